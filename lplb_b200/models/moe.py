@@ -101,6 +101,7 @@ class MoELayer:
             dist.barrier(group=group)
         self.fuse_dispatch = False
         self.send_ctas = 0  # fused dispatch only: this many CTAs send rows and run no tiles (0: sender warps in every CTA)
+        self._n_sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         self._placed_for: torch.Tensor | None = None
         self.place_weights()
 
@@ -129,6 +130,7 @@ class MoELayer:
         self.w13, self.w2 = w13, w2
         self.engine.set_weights(w13, w2)
         self._placed_for = phy2log.clone()
+        self._placed_version = self.planner.placement_version()
 
     # ------------------------------------------------------------------ routing policies
     def route(self, logical_idx: torch.Tensor, avail_counter: torch.Tensor, policy: str = "lplb") -> torch.Tensor:
@@ -150,9 +152,14 @@ class MoELayer:
         """Run the layer on physical expert ids.  ``fuse_dispatch`` (default: the layer's
         setting) sends the rows from inside the first GEMM kernel, so the tensor cores start on
         an expert as soon as its rows have landed instead of after the whole dispatch."""
-        if self._placed_for is None or not torch.equal(self._placed_for, self.planner.phy2log):
-            raise RuntimeError("expert placement changed: call place_weights() first")
-        n_cta = torch.cuda.get_device_properties(self.device).multi_processor_count
+        # The table itself is compared (three launches and a wait for the device, 30 us per call)
+        # only after something wrote to it; the same experts in the same slots need no new weights.
+        version = self.planner.placement_version()
+        if version is None or version != self._placed_version:
+            if self._placed_for is None or not torch.equal(self._placed_for, self.planner.phy2log):
+                raise RuntimeError("expert placement changed: call place_weights() first")
+            self._placed_version = version
+        n_cta = self._n_sms
         fuse = self.fuse_dispatch if fuse_dispatch is None else fuse_dispatch
         if fuse:
             self.engine.set_send_ctas(int(self.send_ctas))

@@ -26,6 +26,7 @@ Differences that a user can observe, all deliberate:
 from __future__ import annotations
 
 import contextlib
+import itertools
 import logging
 import os
 from typing import Any
@@ -43,6 +44,7 @@ log = logging.getLogger("lplb_b200")
 __all__ = ["Planner", "PlannerStatus"]
 
 _NO_RANGE = contextlib.nullcontext()
+_placement_numbers = itertools.count(1)  # one per placement, over all planners of the process
 
 _ERR_NAMES = {
     0: "ok",
@@ -200,7 +202,6 @@ class Planner:
             self._engine.set_warm_start(bool(warm_start), float(warm_guard), float(warm_snap_mu))
 
         self.mapping: ExpertMapping
-        self.phy2log: torch.Tensor
         self.update_redundancy_mapping()
 
         if comm not in ("auto", "p2p", "nccl", "none"):
@@ -217,6 +218,25 @@ class Planner:
                     if comm == "p2p":
                         raise
                     log.warning("peer-memory exchange unavailable (%s); using torch.distributed.all_reduce", exc)
+
+    # ------------------------------------------------------------------ placement
+    @property
+    def phy2log(self) -> torch.Tensor:
+        """``[P]`` int32: the logical expert held by every physical slot."""
+        return self._phy2log
+
+    @phy2log.setter
+    def phy2log(self, value: torch.Tensor) -> None:
+        self._phy2log = value
+        self._placement_number = next(_placement_numbers)
+
+    def placement_version(self) -> tuple[int, int] | None:
+        """Changes whenever ``phy2log`` is replaced or written to, so that whoever depends on the
+        placement can ask on the host, every step, whether it still holds.  ``None``: not known
+        (the table was made in inference mode, where tensors carry no version), compare the table."""
+        if self._phy2log.is_inference():
+            return None
+        return self._placement_number, self._phy2log._version
 
     # ------------------------------------------------------------------ communicator
     def init_peer_exchange(self) -> None:

@@ -97,3 +97,26 @@ def test_default_cta_count_follows_the_batch_size():
     assert planner._default_ctas(384 * 3) == min(sms, 4)
     assert planner._default_ctas(384 * 3 + 1) == min(sms, 5)
     assert planner._default_ctas(10**9) == sms
+
+
+def test_placement_version_follows_every_change_of_the_table():
+    import torch
+
+    from lplb_b200 import Planner, cube
+
+    planner = Planner(cube(), 32 + 16, 32, 8, device="cpu")
+    other = Planner(cube(), 32 + 16, 32, 8, device="cpu")
+    seen = [planner.placement_version(), other.placement_version()]
+    assert planner.placement_version() == seen[0]  # asking changes nothing
+    planner.update_redundancy_mapping(torch.arange(32))
+    seen.append(planner.placement_version())
+    planner.load_state_dict(other.state_dict())
+    seen.append(planner.placement_version())
+    planner.phy2log[0] = 3
+    seen.append(planner.placement_version())
+    planner.phy2log = planner.phy2log.clone()
+    seen.append(planner.placement_version())
+    assert len(set(seen)) == len(seen)
+    with torch.inference_mode():
+        planner.update_redundancy_mapping()
+    assert planner.placement_version() is None
