@@ -35,13 +35,13 @@ struct LayerBuffers {
   // local
   void* act;                           // bf16 [capacity, I]
   int* plan;                           // int32 plan block, see plan_words()
-  int* by_cta;                         // int32 [n_cta, n_ranks * n_local] prefix rows of the pair histogram
+  int* ordinal;                        // int32 [max_tokens * topk] position of every pair among its expert's
+  int* totals;                         // int32 [n_ranks * n_local], zero between launches
   int* pair_slot;                      // int32 [max_tokens * topk] return slot of every pair
   int* send_pair;                      // int32 [max_tokens * topk] pair index at every send position
   int* send_target;                    // int32 [max_tokens * topk] (rank << 24) | row, or -1
   uint32_t* arrived[kApiMaxRanks];     // per rank: uint32 [n_local] rows that have landed, cumulative
   unsigned long long* debug;           // optional uint64 [n_cta * 4] timing of the fused kernel, may be null
-  void* planner_workspace;             // counting kernel workspace (ticket)
   unsigned* tickets;                   // uint32 [4], zero
   int* status;                         // int32 [16]
 };
@@ -64,15 +64,16 @@ size_t gemm_smem_bytes();
 // `box_rows` x 64 elements.  Returns 0 on success.
 int make_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
-// Step 1: all-gather the per-expert pair counts of this launch and derive row offsets.
-cudaError_t launch_plan(const LayerShape& sh, const LayerBuffers& b, int n_cta, uint32_t epoch,
-                        unsigned long long timeout_ns, int fused, cudaStream_t stream);
+// Step 1: rank the pairs of every physical expert, all-gather the per-expert counts of this
+// launch and derive row offsets.
+cudaError_t launch_route(const LayerShape& sh, const LayerBuffers& b, const void* phys_idx, int idx_is64, int n_tokens,
+                         int n_sms, uint32_t epoch, unsigned long long timeout_ns, int fused, cudaStream_t stream);
 // Step 2: copy every (token, k) pair's hidden state into its expert's rows on the target rank.
 cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const void* x, const void* phys_idx,
                             int idx_is64, int n_tokens, int n_cta, uint32_t epoch, cudaStream_t stream);
 // Step 2a (fused path only): decide the send order and every pair's target row and return slot.
 cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const void* phys_idx, int idx_is64,
-                            int n_tokens, int n_cta, cudaStream_t stream);
+                            int n_tokens, cudaStream_t stream);
 // Step 2b+3 fused: the first grouped GEMM, which also streams this rank's rows to their targets
 // while the tensor cores work on the experts whose rows have landed.  send_ctas == 0: four
 // extra warps in every CTA send.  send_ctas > 0: that many of the n_cta CTAs only send and the

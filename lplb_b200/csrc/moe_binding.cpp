@@ -15,7 +15,6 @@
 #include <vector>
 
 #include "moe_api.h"
-#include "planner_api.h"
 
 namespace py = pybind11;
 
@@ -88,7 +87,8 @@ class MoeEngine {
     auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, device_);
     act_ = torch::empty({sh_.capacity, sh_.inter}, i32.dtype(torch::kBFloat16));
     plan_ = torch::zeros({lplb::moe::plan_words(sh_.n_ranks, sh_.n_local)}, i32);
-    workspace_ = torch::zeros({(int64_t)((lplb::planner_workspace_bytes(p_) + 3) / 4)}, i32);
+    totals_ = torch::zeros({p_}, i32);
+    ordinal_ = torch::zeros({(int64_t)sh_.max_tokens * sh_.topk}, i32);
     tickets_ = torch::zeros({4}, i32);
     pair_slot_ = torch::full({(int64_t)sh_.max_tokens * sh_.topk}, -1, i32);
     send_pair_ = torch::zeros({(int64_t)sh_.max_tokens * sh_.topk}, i32);
@@ -181,23 +181,19 @@ class MoeEngine {
     cudaStream_t s = c10::cuda::getCurrentCUDAStream(device_).stream();
     const int is64 = phys_idx.scalar_type() == torch::kInt64;
     ++epoch_;
-    if (!by_cta_.defined() || by_cta_.size(0) != n_cta)
-      by_cta_ = torch::empty({n_cta, p_}, status_.options());
-    buf_.by_cta = by_cta_.data_ptr<int>();
     auto out = torch::empty({n_tokens, sh_.hidden}, x.options());
-    MOE_CUDA(lplb::launch_count(phys_idx.data_ptr(), is64, phys_idx.numel(), p_, n_cta, buf_.by_cta,
-                                workspace_.data_ptr(), status_.data_ptr<int>() + 8, s));
     // The fused path cannot stop between dispatch and the first GEMM: stage 2 then means both.
     const bool fused = fuse_dispatch && upto >= 3;
-    MOE_CUDA(lplb::moe::launch_plan(sh_, buf_, n_cta, epoch_, timeout_ns_, fused ? 1 : 0, s));
+    MOE_CUDA(lplb::moe::launch_route(sh_, buf_, phys_idx.data_ptr(), is64, n_tokens, n_cta, epoch_, timeout_ns_,
+                                     fused ? 1 : 0, s));
     if (upto <= 1) return out;
     if (fused) {
-      MOE_CUDA(lplb::moe::launch_schedule(sh_, buf_, phys_idx.data_ptr(), is64, n_tokens, n_cta, s));
+      MOE_CUDA(lplb::moe::launch_schedule(sh_, buf_, phys_idx.data_ptr(), is64, n_tokens, s));
       MOE_CUDA(lplb::moe::launch_dispatch_gemm(sh_, buf_, tm_x_, tm_w13_, x.data_ptr(), epoch_, timeout_ns_,
                                                gemm_ctas(), send_ctas_, s));
     } else {
-      MOE_CUDA(lplb::moe::launch_dispatch(sh_, buf_, x.data_ptr(), phys_idx.data_ptr(), is64, n_tokens, n_cta,
-                                          epoch_, s));
+      MOE_CUDA(lplb::moe::launch_dispatch(sh_, buf_, x.data_ptr(), phys_idx.data_ptr(), is64, n_tokens,
+                                          4 * n_cta, epoch_, s));
       if (upto <= 2) return out;
       MOE_CUDA(lplb::moe::launch_gemm(sh_, buf_, tm_x_, tm_w13_, 0, epoch_, timeout_ns_, gemm_ctas(), s));
     }
@@ -248,7 +244,7 @@ class MoeEngine {
     plan_.zero_();
     tickets_.zero_();
     status_.zero_();
-    workspace_.zero_();
+    totals_.zero_();
     epoch_ = 0;
     MOE_CUDA(cudaDeviceSynchronize());
   }
@@ -286,12 +282,12 @@ class MoeEngine {
     }
     buf_.act = act_.data_ptr();
     buf_.plan = plan_.data_ptr<int>();
-    buf_.by_cta = nullptr;
+    buf_.ordinal = ordinal_.data_ptr<int>();
+    buf_.totals = totals_.data_ptr<int>();
     buf_.debug = nullptr;
     buf_.pair_slot = pair_slot_.data_ptr<int>();
     buf_.send_pair = send_pair_.data_ptr<int>();
     buf_.send_target = send_target_.data_ptr<int>();
-    buf_.planner_workspace = workspace_.data_ptr();
     buf_.tickets = reinterpret_cast<unsigned*>(tickets_.data_ptr<int>());
     buf_.status = status_.data_ptr<int>();
     ready_ = true;
@@ -304,7 +300,7 @@ class MoeEngine {
   void* block_ = nullptr;
   std::vector<char*> bases_;
   std::vector<void*> opened_;
-  torch::Tensor act_, plan_, workspace_, tickets_, status_, by_cta_, pair_slot_, send_pair_, send_target_, debug_, w13_, w2_;
+  torch::Tensor act_, plan_, totals_, ordinal_, tickets_, status_, pair_slot_, send_pair_, send_target_, debug_, w13_, w2_;
   CUtensorMap tm_x_{}, tm_w13_{}, tm_act_{}, tm_w2_{};
   bool ready_ = false, have_weights_ = false;
   uint32_t epoch_ = 0;

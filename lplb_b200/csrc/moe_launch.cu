@@ -4,7 +4,6 @@
 #include <cudaTypedefs.h>
 
 #include "moe_support.cuh"
-#include "planner_api.h"
 
 namespace lplb {
 namespace moe {
@@ -51,15 +50,39 @@ int make_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
   return rc == CUDA_SUCCESS ? 0 : (int)rc;
 }
 
-cudaError_t launch_plan(const LayerShape& sh, const LayerBuffers& b, int n_cta, uint32_t epoch,
-                        unsigned long long timeout_ns, int fused, cudaStream_t stream) {
-  if (!shape_ok(sh) || n_cta < 1) return cudaErrorInvalidValue;
+namespace {
+struct PlanView {  // see plan_words()
+  int *rows, *row_start, *dst_row_start, *tail, *order_base, *send_base, *arrive_target;
+};
+PlanView plan_view(const LayerShape& sh, const LayerBuffers& b) {
   const int P = sh.n_ranks * sh.n_local;
-  PlanArgs a{};
+  PlanView v;
+  v.rows = b.plan;
+  v.row_start = b.plan + sh.n_local;
+  v.dst_row_start = b.plan + 2 * sh.n_local;
+  v.tail = v.dst_row_start + P + sh.n_ranks * P;
+  v.order_base = v.tail + 8;
+  v.send_base = v.order_base + P;
+  v.arrive_target = v.send_base + P;
+  return v;
+}
+}  // namespace
+
+cudaError_t launch_route(const LayerShape& sh, const LayerBuffers& b, const void* phys_idx, int idx_is64, int n_tokens,
+                         int n_sms, uint32_t epoch, unsigned long long timeout_ns, int fused, cudaStream_t stream) {
+  if (!shape_ok(sh) || n_sms < 1 || n_tokens < 0 || n_tokens > sh.max_tokens) return cudaErrorInvalidValue;
+  const int P = sh.n_ranks * sh.n_local;
+  RouteArgs a{};
+  a.idx = phys_idx;
+  a.ordinal = b.ordinal;
+  a.totals = b.totals;
+  a.ticket = b.tickets + 3;
+  a.count_status = b.status + 8;
   for (int r = 0; r < sh.n_ranks; ++r) a.cnt_words[r] = b.cnt_words[r];
-  a.local_counts = b.by_cta + (size_t)(n_cta - 1) * P;  // last prefix row = totals
   a.plan = b.plan;
   a.status = b.status;
+  a.n_pairs = (long long)n_tokens * sh.topk;
+  a.idx_is64 = idx_is64;
   a.n_ranks = sh.n_ranks;
   a.my_rank = sh.my_rank;
   a.n_local = sh.n_local;
@@ -67,14 +90,20 @@ cudaError_t launch_plan(const LayerShape& sh, const LayerBuffers& b, int n_cta, 
   a.fused = fused;
   a.epoch = epoch;
   a.timeout_ns = timeout_ns;
-  plan_kernel<<<1, kSupportThreads, sizeof(int) * 2 * P, stream>>>(a);
+  // one pair per thread while that fits one CTA per SM, up to four (what a thread keeps in registers) above
+  long long grid = (a.n_pairs + kSupportThreads - 1) / kSupportThreads;
+  if (grid > n_sms) grid = n_sms;
+  const long long least = (a.n_pairs + 4 * kSupportThreads - 1) / (4 * kSupportThreads);
+  if (grid < least) grid = least;
+  if (grid < 1) grid = 1;
+  route_kernel<<<(unsigned)grid, kSupportThreads, sizeof(int) * 4 * P, stream>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const void* x, const void* phys_idx,
                             int idx_is64, int n_tokens, int n_cta, uint32_t epoch, cudaStream_t stream) {
   if (!shape_ok(sh) || n_cta < 1 || n_tokens < 0 || n_tokens > sh.max_tokens) return cudaErrorInvalidValue;
-  const int P = sh.n_ranks * sh.n_local;
+  const PlanView plan = plan_view(sh, b);
   DispatchArgs a{};
   for (int r = 0; r < sh.n_ranks; ++r) {
     a.recv_x[r] = static_cast<__nv_bfloat16*>(b.recv_x[r]);
@@ -83,12 +112,13 @@ cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const v
   }
   a.x = static_cast<const __nv_bfloat16*>(x);
   a.idx = phys_idx;
-  a.dst_row_start = b.plan + 2 * sh.n_local;
-  a.by_cta = b.by_cta;
+  a.ordinal = b.ordinal;
+  a.dst_row_start = plan.dst_row_start;
+  a.send_base = plan.send_base;
   a.pair_slot = b.pair_slot;
   a.status = b.status;
   a.ticket = b.tickets + 0;
-  a.n_pairs = (long long)n_tokens * sh.topk;
+  a.n_tokens = n_tokens;
   a.idx_is64 = idx_is64;
   a.topk = sh.topk;
   a.hidden = sh.hidden;
@@ -97,29 +127,20 @@ cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const v
   a.my_rank = sh.my_rank;
   a.capacity = sh.capacity;
   a.epoch = epoch;
-  const size_t smem = sizeof(int) * (3 * (size_t)P + kDispatchChunk);
-  dispatch_kernel<<<n_cta, kSupportThreads, smem, stream>>>(a);
+  dispatch_kernel<<<n_cta, kSupportThreads, 0, stream>>>(a);
   return cudaGetLastError();
 }
 
-namespace {
-int* plan_tail(const LayerShape& sh, const LayerBuffers& b) {
-  const int P = sh.n_ranks * sh.n_local;
-  return b.plan + 2 * sh.n_local + P + sh.n_ranks * P;
-}
-}  // namespace
-
 cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const void* phys_idx, int idx_is64,
-                            int n_tokens, int n_cta, cudaStream_t stream) {
-  if (!shape_ok(sh) || n_cta < 1 || n_tokens < 0 || n_tokens > sh.max_tokens) return cudaErrorInvalidValue;
-  const int P = sh.n_ranks * sh.n_local;
-  int* tail = plan_tail(sh, b);
+                            int n_tokens, cudaStream_t stream) {
+  if (!shape_ok(sh) || n_tokens < 0 || n_tokens > sh.max_tokens) return cudaErrorInvalidValue;
+  const PlanView plan = plan_view(sh, b);
   ScheduleArgs a{};
   a.idx = phys_idx;
-  a.by_cta = b.by_cta;
-  a.dst_row_start = b.plan + 2 * sh.n_local;
-  a.order_base = tail + 8;
-  a.send_base = tail + 8 + P;
+  a.ordinal = b.ordinal;
+  a.dst_row_start = plan.dst_row_start;
+  a.order_base = plan.order_base;
+  a.send_base = plan.send_base;
   a.pair_slot = b.pair_slot;
   a.send_pair = b.send_pair;
   a.send_target = b.send_target;
@@ -129,7 +150,8 @@ cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const v
   a.n_local = sh.n_local;
   a.n_ranks = sh.n_ranks;
   a.capacity = sh.capacity;
-  schedule_kernel<<<n_cta, kSupportThreads, sizeof(int) * P, stream>>>(a);
+  const long long grid = (a.n_pairs + kSupportThreads - 1) / kSupportThreads;
+  schedule_kernel<<<(unsigned)(grid < 1 ? 1 : grid), kSupportThreads, 0, stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -137,12 +159,11 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
                                  const CUtensorMap& tmap_b, const void* x, uint32_t epoch,
                                  unsigned long long timeout_ns, int n_cta, int send_ctas, cudaStream_t stream) {
   if (!shape_ok(sh) || n_cta < 1 || send_ctas < 0 || send_ctas >= n_cta) return cudaErrorInvalidValue;
-  const int P = sh.n_ranks * sh.n_local;
-  int* tail = plan_tail(sh, b);
+  const PlanView plan = plan_view(sh, b);
   GemmArgs a{};
   a.send_ctas = send_ctas;
-  a.rows = b.plan;
-  a.row_start = b.plan + sh.n_local;
+  a.rows = plan.rows;
+  a.row_start = plan.row_start;
   a.n_experts = sh.n_local;
   a.n_ranks = sh.n_ranks;
   a.my_rank = sh.my_rank;
@@ -160,8 +181,8 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
   a.send_pair = b.send_pair;
   a.send_target = b.send_target;
   a.pair_slot = b.pair_slot;
-  a.n_send = tail + 2;
-  a.arrive_target = tail + 8 + 2 * P;
+  a.n_send = plan.tail + 2;
+  a.arrive_target = plan.arrive_target;
   for (int r = 0; r < sh.n_ranks; ++r) {
     a.recv_x[r] = static_cast<__nv_bfloat16*>(b.recv_x[r]);
     a.recv_meta[r] = b.recv_meta[r];
@@ -197,7 +218,7 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUten
     a.n_per_expert = 2 * sh.inter;
     a.act = static_cast<__nv_bfloat16*>(b.act);
     a.act_ld = sh.inter;
-    a.wait_flags = b.flags[sh.my_rank];  // dispatch done, one word per source rank
+    a.wait_flags = sh.n_ranks > 1 ? b.flags[sh.my_rank] : nullptr;  // dispatch done, one word per source rank
     a.ticket = b.tickets + 1;
     auto kernel = grouped_gemm_kernel<kSwiGLU, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
