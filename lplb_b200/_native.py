@@ -41,6 +41,7 @@ if BOUNDS_CHECK:
 SOURCES = [
     "binding.cpp",
     "planner_launch.cu",
+    "place_kernel.cu",
     "count_noalloc.cu",
     "moe_binding.cpp",
     "moe_launch.cu",

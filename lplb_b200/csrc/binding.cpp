@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include "place_api.h"
 #include "planner_api.h"
 
 namespace py = pybind11;
@@ -111,6 +112,56 @@ class PlannerEngine {
       store_i32(log2slot_, table);
     }
     invalidate_warm_start();  // a new placement is a new LP
+  }
+
+  // Place the experts and rebuild every table on the device (place_kernel.cu), ordered on the
+  // current stream like set_mapping; nothing waits for the device.  `history`: contiguous int32
+  // or int64 [E] on this device, or none for the natural order.  Returns (phy2log, log2phy,
+  // logcnt, log2edge), or none when the shape does not fit one CTA's shared memory.
+  py::object place(const c10::optional<torch::Tensor>& history, int n_nodes) {
+    LPLB_CHECK(r2o_.defined(), "topology must be set first");
+    LPLB_CHECK(n_nodes >= 1, "n_nodes must be positive");
+    lplb::PlaceArgs a{};
+    a.n_logical = e_;
+    a.ep_size = n_group_ * g_;
+    a.n_group = n_group_;
+    a.g = g_;
+    a.dup = d_;
+    a.combined = c_;
+    a.n_nodes = n_nodes;
+    if (lplb::place_shared_bytes(a) > 227 * 1024) return py::none();
+    c10::cuda::CUDAGuard guard(device_);
+    auto stream = c10::cuda::getCurrentCUDAStream(device_);
+    if (history.has_value()) {
+      const torch::Tensor& h = *history;
+      LPLB_CHECK(h.is_cuda() && h.get_device() == device_ && h.is_contiguous() && h.numel() == e_ &&
+                     (h.scalar_type() == torch::kInt64 || h.scalar_type() == torch::kInt32),
+                 "history must be contiguous int32/int64 [E] on cuda:" << device_);
+      a.history = h.data_ptr();
+      a.is64 = h.scalar_type() == torch::kInt64;
+      h.record_stream(stream);  // the caller may drop it before the kernel has read it
+    }
+    const int64_t p = (int64_t)n_group_ * g_ * (ll_ + c_ * d_);
+    auto i32 = status_.options();
+    auto phy2log = torch::empty({p}, i32), log2phy = torch::empty({e_, 2}, i32);
+    auto logcnt = torch::empty({e_}, i32), log2edge = torch::empty({e_}, i32);
+    if (!phy2log_.defined()) phy2log_ = torch::empty({p}, i32);
+    if (!log2phy_.defined()) log2phy_ = torch::empty({e_, 2}, i32);
+    if (!log2edge_.defined()) log2edge_ = torch::empty({e_}, i32);
+    if (!log2slot_.defined()) log2slot_ = torch::empty({e_}, i32);
+    a.r2o = r2o_.data_ptr<int>();
+    a.o2r = o2r_.data_ptr<int>();
+    a.phy2log = phy2log.data_ptr<int>();
+    a.log2phy = log2phy.data_ptr<int>();
+    a.logcnt = logcnt.data_ptr<int>();
+    a.log2edge = log2edge.data_ptr<int>();
+    a.table_phy2log = phy2log_.data_ptr<int>();
+    a.table_log2phy = log2phy_.data_ptr<int>();
+    a.table_log2edge = log2edge_.data_ptr<int>();
+    a.table_log2slot = log2slot_.data_ptr<int>();
+    LPLB_CUDA(lplb::launch_place(a, stream.stream()));
+    invalidate_warm_start();  // a new placement is a new LP
+    return py::make_tuple(phy2log, log2phy, logcnt, log2edge);
   }
 
   // Warm starts: keep a centred iterate per group on the device and start the next solve from
@@ -480,6 +531,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("dup_per_rank"), py::arg("n_local_logical"), py::arg("n_combined"), py::arg("device"))
       .def("set_topology", &PlannerEngine::set_topology)
       .def("set_mapping", &PlannerEngine::set_mapping)
+      .def("place", &PlannerEngine::place, py::arg("history"), py::arg("n_nodes"))
       .def("set_params", &PlannerEngine::set_params)
       .def("set_warm_start", &PlannerEngine::set_warm_start)
       .def("set_solver", &PlannerEngine::set_solver)

@@ -1,0 +1,22 @@
+// Host-side launch interface of the placement kernel.  Plain C++, no torch headers.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace lplb {
+
+struct PlaceArgs {
+  const void* history;  // [n_logical] int32/int64 loads; null = natural order
+  int is64;
+  const int *r2o, *o2r;  // [g, dup]
+  int n_logical, ep_size, n_group, g, dup, combined, n_nodes;
+  // results, and the engine's own copies of them (which keep their addresses)
+  int *phy2log, *log2phy, *logcnt, *log2edge;
+  int *table_phy2log, *table_log2phy, *table_log2edge, *table_log2slot;
+};
+
+size_t place_shared_bytes(const PlaceArgs& a);
+cudaError_t launch_place(const PlaceArgs& a, cudaStream_t stream);
+
+}  // namespace lplb

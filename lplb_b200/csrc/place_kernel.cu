@@ -1,0 +1,227 @@
+// Expert placement from the load history and every table derived from it, in one launch (sm_100a).
+//
+// The same decisions as the host balancer (lplb_b200/eplb.py, lplb_b200/mapping.py), item by item:
+// expert groups to nodes, experts to the ranks of a node, both heaviest first into the lightest
+// pack with room (reference lplb/eplb.py:6-46, :80-148), then the tables (reference
+// lplb/planner.py:115-182).  Loads are float64 on both sides and are added in the same order, so
+// the results are identical.
+//
+// One CTA.  What bounds it is the greedy packing, one dependent step per expert: a warp holds the
+// packs (one per lane up to 32) and finds the lightest with two 32-bit warp reductions over the
+// order-preserving halves of the double and a ballot, with no shared memory on the chain, instead
+// of five shuffle rounds of a double and an index.  The orders come from counting, for every
+// expert, the experts in front of it.  256 experts on 8 ranks: 33 us for the whole call; on the
+// host, some twenty tensor operations per expert, 8.9 ms including a wait for the device.
+#include "place_api.h"
+
+#include <stdint.h>
+
+namespace lplb {
+
+namespace {
+
+constexpr int kPlaceThreads = 1024;
+constexpr unsigned kAll = 0xffffffffu;
+
+struct Shared {
+  double* w;      // [E] loads in node-major order
+  double* gw;     // [n_group] group loads
+  double* load;   // [packs] of one packing, per node
+  int* fill;      // [packs]
+  int* order;     // [E] items of a packing, heaviest first
+  int* nlog2log;  // [E]
+  int* own;       // [E] expert in every rank's own slots
+};
+
+size_t shared_bytes(const PlaceArgs& a) {
+  const size_t e = a.n_logical, packs = a.ep_size > a.n_group ? a.ep_size : a.n_group;
+  return 8 * (e + a.n_group + packs) + 4 * (packs + 3 * e);
+}
+
+__device__ __forceinline__ double load_of(const PlaceArgs& a, int e) {
+  return a.is64 ? (double)((const long long*)a.history)[e] : (double)((const int*)a.history)[e];
+}
+
+// Unsigned order of the result = order of the doubles.
+__device__ __forceinline__ unsigned long long ordered(double x) {
+  const long long b = __double_as_longlong(x);
+  return (unsigned long long)b ^ ((unsigned long long)(b >> 63) | 0x8000000000000000ull);
+}
+
+// order[k] = the item with k items in front of it: heavier ones, and equal ones of lower index.
+// Rows of `n` items each, `rows` of them, by all threads of the CTA.
+__device__ void sort_rows(const double* w, int* order, int rows, int n) {
+  for (int i = threadIdx.x; i < rows * n; i += kPlaceThreads) {
+    const int base = i / n * n, me = i - base;
+    const double mine = w[i];
+    int front = 0;
+    for (int j = 0; j < n; ++j) {
+      const double other = w[base + j];
+      front += other > mine || (other == mine && j < me);
+    }
+    order[base + front] = me;
+  }
+}
+
+// One warp: items order[0], order[1], ... each into the lightest of `packs` packs of `cap` items that
+// has room, the lowest-numbered one among equals.  put(item, pack, position in the pack).
+template <typename Put>
+__device__ void pack_items(const double* w, const int* order, int n, int packs, int cap, double* load, int* fill,
+                           Put put) {
+  const int lane = threadIdx.x & 31;
+  if (packs <= 32) {  // a pack per lane, in registers
+    double mine = 0.0;
+    int held = 0;
+    int item = order[0];
+    double weight = w[item];
+    for (int step = 0; step < n; ++step) {
+      const int next = order[min(step + 1, n - 1)];
+      const double next_weight = w[next];
+      const bool room = lane < packs && held < cap;
+      const unsigned long long key = room ? ordered(mine) : ~0ull;
+      const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+      const unsigned least_hi = __reduce_min_sync(kAll, hi);
+      const unsigned least_lo = __reduce_min_sync(kAll, hi == least_hi ? lo : ~0u);
+      const int pack = __ffs(__ballot_sync(kAll, room && hi == least_hi && lo == least_lo)) - 1;
+      if (lane == pack) {
+        put(item, lane, held);
+        mine += weight;
+        ++held;
+      }
+      item = next;
+      weight = next_weight;
+    }
+    return;
+  }
+  for (int p = lane; p < packs; p += 32) {
+    load[p] = 0.0;
+    fill[p] = 0;
+  }
+  __syncwarp();
+  for (int step = 0; step < n; ++step) {
+    unsigned long long best = ~0ull;
+    int best_pack = 0x7fffffff;
+    for (int p = lane; p < packs; p += 32) {
+      if (fill[p] >= cap) continue;
+      const unsigned long long key = ordered(load[p]);
+      if (best_pack == 0x7fffffff || key < best) {
+        best = key;
+        best_pack = p;
+      }
+    }
+    const bool room = best_pack != 0x7fffffff;
+    const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
+    const unsigned least_hi = __reduce_min_sync(kAll, hi);
+    const unsigned least_lo = __reduce_min_sync(kAll, hi == least_hi ? lo : ~0u);
+    const int pack = (int)__reduce_min_sync(
+        kAll, room && hi == least_hi && lo == least_lo ? (unsigned)best_pack : 0x7fffffffu);
+    if (lane == 0) {
+      const int item = order[step];
+      put(item, pack, fill[pack]);
+      load[pack] += w[item];
+      ++fill[pack];
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(kPlaceThreads) place_kernel(const PlaceArgs a) {
+  extern __shared__ double sm[];
+  const int tid = threadIdx.x, warp = tid >> 5, n_warps = kPlaceThreads / 32;
+  const int E = a.n_logical, ranks = a.ep_size, ll = E / ranks, rep = a.combined * a.dup, pl = ll + rep;
+  const int max_packs = ranks > a.n_group ? ranks : a.n_group;
+  Shared s;
+  s.w = sm;
+  s.gw = s.w + E;
+  s.load = s.gw + a.n_group;
+  s.fill = reinterpret_cast<int*>(s.load + max_packs);
+  s.order = s.fill + max_packs;
+  s.nlog2log = s.order + E;
+  s.own = s.nlog2log + E;
+
+  if (a.history == nullptr) {  // natural order
+    for (int e = tid; e < E; e += kPlaceThreads) s.own[e] = e;
+  } else {
+    // whole groups to nodes; without groups that divide over the nodes, one group on one node
+    const bool hier = a.n_group % a.n_nodes == 0;
+    const int groups = hier ? a.n_group : 1, nodes = hier ? a.n_nodes : 1;
+    const int per_group = E / groups, groups_per_node = groups / nodes, per_node = E / nodes;
+    int* place_of_group = s.own;  // position of the group in node-major order
+    if (groups_per_node == 1) {
+      for (int g = tid; g < groups; g += kPlaceThreads) place_of_group[g] = g;
+    } else {
+      for (int g = warp; g < groups; g += n_warps) {
+        double sum = 0.0;
+        for (int i = tid & 31; i < per_group; i += 32) sum += load_of(a, g * per_group + i);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
+        if ((tid & 31) == 0) s.gw[g] = sum;
+      }
+      __syncthreads();
+      sort_rows(s.gw, s.order, 1, groups);
+      __syncthreads();
+      if (warp == 0)
+        pack_items(s.gw, s.order, groups, nodes, groups_per_node, s.load, s.fill,
+                   [&](int g, int node, int pos) { place_of_group[g] = node * groups_per_node + pos; });
+    }
+    __syncthreads();
+    for (int e = tid; e < E; e += kPlaceThreads) {
+      const int to = place_of_group[e / per_group] * per_group + e % per_group;
+      s.nlog2log[to] = e;
+      s.w[to] = load_of(a, e);
+    }
+    __syncthreads();
+    const int packs = ranks / nodes;
+    if (ll == 1) {
+      for (int e = tid; e < E; e += kPlaceThreads) s.own[e] = s.nlog2log[e];
+    } else {
+      sort_rows(s.w, s.order, nodes, per_node);
+      __syncthreads();
+      // A pack fills heaviest first, so every rank's own slots are in the order of the history.
+      for (int node = warp; node < nodes; node += n_warps) {
+        const int base = node * per_node;
+        pack_items(s.w + base, s.order + base, per_node, packs, ll, s.load + node * packs, s.fill + node * packs,
+                   [&](int item, int pack, int pos) { s.own[base + pack * ll + pos] = s.nlog2log[base + item]; });
+      }
+    }
+  }
+  __syncthreads();
+
+  for (int i = tid; i < ranks * pl; i += kPlaceThreads) {
+    const int rank = i / pl, slot = i - rank * pl;
+    int e;
+    if (slot < ll) {
+      e = s.own[rank * ll + slot];
+      const int first = slot < rep ? slot % a.dup : a.dup;  // bundle of the slot; dup = not replicated
+      int replica = -1;
+      if (slot < rep) {
+        const int grp = rank / a.g;
+        replica = (grp * a.g + a.o2r[(rank - grp * a.g) * a.dup + first]) * pl + ll + slot;
+      }
+      const int edge = slot < rep ? rank * a.dup + first : -1;
+      a.log2phy[2 * e] = a.table_log2phy[2 * e] = i;
+      a.log2phy[2 * e + 1] = a.table_log2phy[2 * e + 1] = replica;
+      a.logcnt[e] = replica >= 0 ? 2 : 1;
+      a.log2edge[e] = a.table_log2edge[e] = edge;
+      a.table_log2slot[e] = rank * (a.dup + 1) + first;
+    } else {
+      const int grp = rank / a.g, at = slot - ll;
+      const int src = grp * a.g + a.r2o[(rank - grp * a.g) * a.dup + at % a.dup];
+      e = s.own[src * ll + at];
+    }
+    a.phy2log[i] = a.table_phy2log[i] = e;
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_place(const PlaceArgs& a, cudaStream_t stream) {
+  const size_t bytes = shared_bytes(a);
+  const cudaError_t err = cudaFuncSetAttribute(place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err != cudaSuccess) return err;
+  place_kernel<<<1, kPlaceThreads, bytes, stream>>>(a);
+  return cudaGetLastError();
+}
+
+size_t place_shared_bytes(const PlaceArgs& a) { return shared_bytes(a); }
+
+}  // namespace lplb

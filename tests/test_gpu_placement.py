@@ -1,0 +1,59 @@
+"""The placement kernel against the host balancer: the same tables, whatever the shape and the history."""
+
+import pytest
+import torch
+
+from lplb_b200 import Planner, cube, ring, topology
+from lplb_b200.mapping import build_mapping
+
+pytestmark = pytest.mark.gpu
+
+# (topology, LP groups, experts per rank, combined, nodes): one group, groups on one node, on fewer
+# nodes, one per node, nodes that the groups do not divide over; one expert per rank; packs below
+# and above a warp's 32 lanes; the largest number of experts
+SHAPES = [
+    (cube(), 1, 32, 1, 1), (cube(), 4, 8, 2, 1), (cube(), 4, 8, 1, 2), (cube(), 4, 9, 1, 4), (cube(), 2, 16, 1, 3),
+    (ring(8), 2, 1, 1, 1), (ring(3), 5, 7, 2, 1), (topology.torus(8, 4), 1, 16, 1, 1), (topology.torus(8, 8), 1, 8, 1, 1),
+    (ring(40), 4, 3, 1, 2), (ring(128), 1, 1, 1, 1), (cube(), 16, 64, 1, 4),
+]
+
+
+def _histories(n, seed):
+    g = torch.Generator().manual_seed(seed)
+    yield (torch.rand(n, generator=g) * 1e7).long()
+    yield torch.randint(0, 3, (n,), generator=g)  # ties everywhere
+    yield torch.zeros(n, dtype=torch.int32)
+    yield torch.randint(-1000, 1000, (n,), generator=g, dtype=torch.int32)
+    yield torch.randint(0, 2**40, (n,), generator=g)
+    yield torch.randint(-100, 100, (n,), generator=g, dtype=torch.int8)
+    yield torch.randint(0, 9, (2 * n,), generator=g)[::2]
+    yield torch.rand(n, generator=g)  # not whole numbers: placed on the host
+
+
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+def test_same_tables_as_the_host(shape):
+    r2o, n_group, ll, c, nodes = SHAPES[shape]
+    ep = n_group * r2o.shape[0]
+    n = ep * ll
+    planner = Planner(r2o, n + ep * r2o.shape[1] * c, n, ep, device="cuda", n_nodes=nodes)
+    twin = Planner(r2o, n + ep * r2o.shape[1] * c, n, ep, device="cuda", n_nodes=nodes)
+    idx = torch.randint(-1, n, (777, 3), device="cuda", generator=torch.Generator("cuda").manual_seed(shape))
+    for i, hist in enumerate([None, *_histories(n, shape)]):
+        if n > 1024 and i not in (1, 2, 4):  # the host takes a second or so for these
+            continue
+        want = build_mapping(r2o, n_group, ll, c, hist, n_nodes=nodes)
+        on_gpu = hist is not None and i % 2 == 0
+        got = planner.update_redundancy_mapping(hist.cuda() if on_gpu else hist)
+        for a, b in zip(got, (want.phy2log, want.log2phy, want.logcnt)):
+            assert a.dtype == torch.int32 and torch.equal(a.cpu(), b), i
+        assert torch.equal(planner.mapping.log2edge.cpu(), want.log2edge), i
+        # the engine's own tables: the same routing as a planner that was handed the host's tables
+        twin.load_state_dict(planner.state_dict())
+        a, b = (p.run(idx, torch.zeros(1, dtype=torch.int32, device="cuda")) for p in (planner, twin))
+        assert torch.equal(planner.last_probs, twin.last_probs)
+        assert torch.equal(planner.count_workload(idx, 4)[0], twin.count_workload(idx, 4)[0])
+        flat = idx.reshape(-1) >= 0
+        assert torch.equal(planner.phy2log[a.reshape(-1)[flat]].long(), idx.reshape(-1)[flat])
+        assert torch.equal(torch.bincount(a.reshape(-1)[flat]), torch.bincount(b.reshape(-1)[flat]))
+    with pytest.raises(ValueError):
+        planner.update_redundancy_mapping(torch.ones(n + 1, dtype=torch.int64, device="cuda"))
