@@ -42,7 +42,7 @@ struct LayerBuffers {
   int* send_target;                    // int32 [max_tokens * topk] (rank << 24) | row, or -1
   uint32_t* arrived[kApiMaxRanks];     // per rank: uint32 [n_local] rows that have landed, cumulative
   unsigned long long* debug;           // optional uint64 [n_cta * 4] timing of the fused kernel, may be null
-  unsigned* tickets;                   // uint32 [4], zero
+  unsigned* tickets;                   // uint32 [5], zero: dispatch, first GEMM, second GEMM, routing, GEMM tiles
   int* status;                         // int32 [16]
 };
 
@@ -60,9 +60,15 @@ inline int plan_words(int n_ranks, int n_local) {
 
 size_t gemm_smem_bytes();
 
-// Encodes a 2-D bf16 row-major tensor map with 128-byte swizzle and a box of
-// `box_rows` x 64 elements.  Returns 0 on success.
-int make_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// Tensor maps of one grouped GEMM (128-byte swizzle, 64 elements of K per box): weights, received
+// rows in boxes of half a tile, received rows in small boxes.
+struct GemmMaps {
+  CUtensorMap w, t, s;
+};
+// tokens: bf16 [rows, cols]; weights: bf16 [weight_rows, cols], with `gate_up` in blocks of 128
+// gate rows and their 128 up rows.  Returns 0 on success.
+int make_gemm_maps(GemmMaps* out, const void* tokens, uint64_t rows, const void* weights, uint64_t weight_rows,
+                   uint64_t cols, bool gate_up);
 
 // Step 1: rank the pairs of every physical expert, all-gather the per-expert counts of this
 // launch and derive row offsets.
@@ -76,14 +82,12 @@ cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const v
                             int n_tokens, cudaStream_t stream);
 // Step 2b+3 fused: the first grouped GEMM, which also streams this rank's rows to their targets
 // while the tensor cores work on the experts whose rows have landed.  send_ctas == 0: four
-// extra warps in every CTA send.  send_ctas > 0: that many of the n_cta CTAs only send and the
-// other n_cta - send_ctas only run tiles.
-cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUtensorMap& tmap_a,
-                                 const CUtensorMap& tmap_b, const void* x, uint32_t epoch,
+// extra warps in every CTA send.  send_ctas > 0: that many of the n_cta CTAs (rounded up to whole
+// pairs) only send and the others only run tiles.
+cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, const void* x, uint32_t epoch,
                                  unsigned long long timeout_ns, int n_cta, int send_ctas, cudaStream_t stream);
 // Step 3/4: grouped GEMMs.  which = 0: recv_x x w13 -> SwiGLU -> act.  which = 1: act x w2 -> peers' comb.
-cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUtensorMap& tmap_a,
-                        const CUtensorMap& tmap_b, int which, uint32_t epoch, unsigned long long timeout_ns,
+cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, int which, uint32_t epoch, unsigned long long timeout_ns,
                         int n_cta, cudaStream_t stream);
 // Step 5: out[t] = sum_k weight[t, k] * comb[pair_slot[t * topk + k]].
 cudaError_t launch_combine(const LayerShape& sh, const LayerBuffers& b, const float* weights, void* out, int n_tokens,

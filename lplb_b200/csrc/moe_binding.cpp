@@ -89,7 +89,7 @@ class MoeEngine {
     plan_ = torch::zeros({lplb::moe::plan_words(sh_.n_ranks, sh_.n_local)}, i32);
     totals_ = torch::zeros({p_}, i32);
     ordinal_ = torch::zeros({(int64_t)sh_.max_tokens * sh_.topk}, i32);
-    tickets_ = torch::zeros({4}, i32);
+    tickets_ = torch::zeros({8}, i32);
     pair_slot_ = torch::full({(int64_t)sh_.max_tokens * sh_.topk}, -1, i32);
     send_pair_ = torch::zeros({(int64_t)sh_.max_tokens * sh_.topk}, i32);
     send_target_ = torch::full({(int64_t)sh_.max_tokens * sh_.topk}, -1, i32);
@@ -149,14 +149,12 @@ class MoeEngine {
     w13_ = w13;
     w2_ = w2;
     c10::cuda::CUDAGuard guard(device_);
-    int rc = lplb::moe::make_tensor_map(&tm_x_, buf_.recv_x[sh_.my_rank], sh_.capacity, sh_.hidden, 128);
-    MOE_CHECK(rc == 0, "tensor map for the receive buffer failed with code " << rc);
-    rc = lplb::moe::make_tensor_map(&tm_w13_, w13.data_ptr(), (uint64_t)sh_.n_local * 2 * sh_.inter, sh_.hidden, 256);
-    MOE_CHECK(rc == 0, "tensor map for w13 failed with code " << rc);
-    rc = lplb::moe::make_tensor_map(&tm_act_, act_.data_ptr(), sh_.capacity, sh_.inter, 128);
-    MOE_CHECK(rc == 0, "tensor map for the activation buffer failed with code " << rc);
-    rc = lplb::moe::make_tensor_map(&tm_w2_, w2.data_ptr(), (uint64_t)sh_.n_local * sh_.hidden, sh_.inter, 256);
-    MOE_CHECK(rc == 0, "tensor map for w2 failed with code " << rc);
+    int rc = lplb::moe::make_gemm_maps(&maps1_, buf_.recv_x[sh_.my_rank], sh_.capacity, w13.data_ptr(),
+                                       (uint64_t)sh_.n_local * 2 * sh_.inter, sh_.hidden, true);
+    MOE_CHECK(rc == 0, "tensor maps for the receive buffer and w13 failed with code " << rc);
+    rc = lplb::moe::make_gemm_maps(&maps2_, act_.data_ptr(), sh_.capacity, w2.data_ptr(),
+                                   (uint64_t)sh_.n_local * sh_.hidden, sh_.inter, false);
+    MOE_CHECK(rc == 0, "tensor maps for the activation buffer and w2 failed with code " << rc);
     have_weights_ = true;
   }
 
@@ -189,16 +187,16 @@ class MoeEngine {
     if (upto <= 1) return out;
     if (fused) {
       MOE_CUDA(lplb::moe::launch_schedule(sh_, buf_, phys_idx.data_ptr(), is64, n_tokens, s));
-      MOE_CUDA(lplb::moe::launch_dispatch_gemm(sh_, buf_, tm_x_, tm_w13_, x.data_ptr(), epoch_, timeout_ns_,
+      MOE_CUDA(lplb::moe::launch_dispatch_gemm(sh_, buf_, maps1_, x.data_ptr(), epoch_, timeout_ns_,
                                                gemm_ctas(), send_ctas_, s));
     } else {
       MOE_CUDA(lplb::moe::launch_dispatch(sh_, buf_, x.data_ptr(), phys_idx.data_ptr(), is64, n_tokens,
                                           4 * n_cta, epoch_, s));
       if (upto <= 2) return out;
-      MOE_CUDA(lplb::moe::launch_gemm(sh_, buf_, tm_x_, tm_w13_, 0, epoch_, timeout_ns_, gemm_ctas(), s));
+      MOE_CUDA(lplb::moe::launch_gemm(sh_, buf_, maps1_, 0, epoch_, timeout_ns_, gemm_ctas(), s));
     }
     if (upto <= 3) return out;
-    MOE_CUDA(lplb::moe::launch_gemm(sh_, buf_, tm_act_, tm_w2_, 1, epoch_, timeout_ns_, gemm_ctas(), s));
+    MOE_CUDA(lplb::moe::launch_gemm(sh_, buf_, maps2_, 1, epoch_, timeout_ns_, gemm_ctas(), s));
     if (upto <= 4) return out;
     MOE_CUDA(lplb::moe::launch_combine(sh_, buf_, weights.data_ptr<float>(), out.data_ptr(), n_tokens, epoch_,
                                        timeout_ns_, 4 * sm_count(), s));
@@ -301,7 +299,7 @@ class MoeEngine {
   std::vector<char*> bases_;
   std::vector<void*> opened_;
   torch::Tensor act_, plan_, totals_, ordinal_, tickets_, status_, pair_slot_, send_pair_, send_target_, debug_, w13_, w2_;
-  CUtensorMap tm_x_{}, tm_w13_{}, tm_act_{}, tm_w2_{};
+  lplb::moe::GemmMaps maps1_{}, maps2_{};
   bool ready_ = false, have_weights_ = false;
   uint32_t epoch_ = 0;
   unsigned long long timeout_ns_ = 2000000000ull;

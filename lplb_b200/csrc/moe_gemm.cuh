@@ -1,6 +1,7 @@
 // Grouped expert GEMM for the benchmark MoE layer on sm_100a: bf16 x bf16 -> fp32 on the
-// 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), operands staged
-// by TMA into 128-byte-swizzled shared memory, persistent warp-specialised CTAs.
+// 5th-generation tensor cores (tcgen05.mma.cta_group::2, accumulators in tensor memory),
+// operands staged by TMA into 128-byte-swizzled shared memory, persistent warp-specialised
+// CTA pairs.
 //
 //   C_e[rows_e, N] = A_e[rows_e, K] * B_e[N, K]^T        for every local expert e
 //
@@ -8,17 +9,31 @@
 // row_start[e]); B is the weight tensor [experts * N, K].  Rows per expert are only known
 // on the device, so the tile list is derived in-kernel from `rows`.
 //
-// Roles inside a CTA (192 threads):
-//   warp 0      TMA producer: A tile 128 x 64 and B tile 256 x 64 per stage, 4 stages
-//   warp 1      allocates 512 TMEM columns, issues tcgen05.mma (one elected lane)
-//   warps 2-5   epilogue: tcgen05.ld their 32-lane quarter, apply the epilogue, store
-// Two 128 x 256 fp32 accumulators (2 x 256 TMEM columns) let the epilogue of tile i overlap
-// the main loop of tile i+1.
+// A pair of CTAs computes a tile of 256 weight rows x up to 256 received rows, weights on the
+// tensor core's M side (128 per CTA), received rows on its N side (half of them staged by each
+// CTA).  Why this way round: the number of rows an expert receives is arbitrary, and N comes in
+// steps of 32 where M does not shrink, so the work for padding is 16 rows per expert on average
+// and a decode step's few rows cost few cycles and few bytes.
 //
-// Epilogues:
-//   kSwiGLU   columns [0,128) of a tile are gate, [128,256) the matching up projections
-//             (the weight rows are stored in that order); writes silu(gate)*up as bf16
-//             into act[row, n_tile*128 + c].
+// Which pair computes which tile is decided as they go: a pair that finishes takes the next tile
+// of the list.  With many rows the kernel is bound by the board's power limit, and there DRAM
+// traffic is what costs most.  The pairs that share a weight tile must therefore read it at the
+// same time, before L2 has lost it.  Tiles of different experts differ in size, so dealing the
+// list out in turn lets the pairs drift apart: 13.9 GB read from DRAM (8192 tokens x top-8, 48
+// experts, 7168 x 2048, first GEMM; 3.8 GB is every operand once).
+//
+// Roles inside a CTA (192 threads):
+//   warp 0      TMA producer: 128 weight rows and half of the tile's received rows per stage
+//   warp 1      allocates 512 TMEM columns; in the pair's first CTA issues tcgen05.mma (one lane)
+//   warps 2-5   epilogue: tcgen05.ld their 32-lane quarter, transpose through shared memory, store
+// Two accumulators (2 x 256 TMEM columns) let the epilogue of tile i overlap the main loop of
+// tile i+1.
+//
+// Epilogues (a TMEM lane is an output feature, a column is a received row; stmatrix.trans turns
+// the 8 x 8 fragments round so that a row's features leave as contiguous 16-byte stores):
+//   kSwiGLU   the weight tensor holds 128 gate rows, then the 128 matching up rows, and so on;
+//             the tensor map deals them out so that every warp's 32 lanes are 16 gate rows and
+//             their 16 up rows.  Writes silu(gate)*up as bf16 into act[row, feature].
 //   kScatter  converts to bf16 and stores each row to the buffer of the GPU the token came
 //             from (peer memory over NVLink), at the return slot meta[row] & 0xFFFFF: this is the
 //             combine step of the MoE layer fused into the last GEMM.
@@ -34,13 +49,24 @@
 namespace lplb {
 namespace moe {
 
-constexpr int kBM = 128, kBN = 256, kBK = 64, kStages = 4, kUmmaK = 16;
+constexpr int kBM = 256, kBN = 256, kBK = 64, kStages = 6, kUmmaK = 16;
+constexpr int kCtaM = kBM / 2;       // weight rows per CTA of a pair
+constexpr int kStepN = 32;           // received rows per tile are rounded up to this
+constexpr int kSmallBox = 16;        // received rows per TMA box where a CTA's half is not 128 rows
+constexpr int kGateRows = 16;        // gate (and up) rows of one epilogue warp
+constexpr int kGateBlock = 128;      // gate rows in front of their up rows in the weight tensor
 constexpr int kGemmThreads = 192;
 constexpr int kTmemCols = 512;
-constexpr uint32_t kStageBytesA = kBM * kBK * 2, kStageBytesB = kBN * kBK * 2;
-// per epilogue warp: 32 rows x 128 bf16 columns, staged so that rows leave as 256-byte segments
-constexpr uint32_t kStageOutBytes = 32 * 128 * 2;
-constexpr size_t kGemmSmem = 1024 + (size_t)kStages * (kStageBytesA + kStageBytesB) + 256 + 4 * kStageOutBytes;
+// Tile numbers on their way to the roles.  The producer announces tile i + 1 when it begins tile
+// i; then all k blocks but the last kStages have been computed, so with two or more k blocks per
+// tile the accumulator of tile i - 4 is complete, the epilogue is through with tile i - 6, and no
+// role still has to read a number older than that of tile i - 5.
+constexpr int kTileSlots = 8;
+static_assert(kStages <= 6, "a slot would be overwritten before the epilogue has read it");
+constexpr uint32_t kStageBytesW = kCtaM * kBK * 2, kStageBytesT = kBN / 2 * kBK * 2;
+constexpr uint32_t kTurnBytes = kStepN * kCtaM * 2;  // 32 received rows x 128 features, two of these
+constexpr uint32_t kBarBytes = 256;
+constexpr size_t kGemmSmem = 1024 + (size_t)kStages * (kStageBytesW + kStageBytesT) + kBarBytes + 2 * kTurnBytes;
 constexpr int kMaxLocalExperts = 128;
 constexpr int kMaxRanks = 8;
 
@@ -52,9 +78,8 @@ struct GemmArgs {
   const int* rows;        // [n_experts] rows received per local expert
   const int* row_start;   // [n_experts] first row of each expert in the A buffer
   int n_experts;
-  int n_tiles_n;          // N / 256
+  int n_tiles_w;          // N / 256
   int k_blocks;           // K / 64
-  int n_per_expert;       // N (rows of B per expert)
   // kSwiGLU
   __nv_bfloat16* act;     // [capacity, act_ld]
   int act_ld;             // N / 2
@@ -70,12 +95,14 @@ struct GemmArgs {
   int n_ranks, my_rank;
   uint32_t epoch;
   unsigned* ticket;       // zero before launch; left at zero
+  unsigned* next_tile;    // tiles taken beyond the first of every pair; zero before launch, left at zero
   int* status;            // first error code
   unsigned long long timeout_ns;
   // fused dispatch (FUSED kernels only): this rank's rows are sent while the tensor cores
   // work; an expert's tiles start once `arrived[e]` reached `arrive_target[e]`.  With
-  // send_ctas == 0 warps 6-9 of every CTA send; with send_ctas > 0 the last `send_ctas`
-  // CTAs of the grid do nothing but send (all their warps) and the others only run tiles.
+  // send_ctas == 0 warps 6-9 of every CTA send; with send_ctas > 0 (even: whole pairs) the last
+  // `send_ctas` CTAs of the grid do nothing but send (all their warps) and the others only run
+  // tiles.
   const __nv_bfloat16* x;        // [tokens, hidden] local hidden states
   const int* send_pair;          // [n_send] (local expert << 20) | pair index, in send order
   const int* send_target;        // [n_send] (rank << 24) | row, or -1
@@ -141,19 +168,28 @@ __device__ __forceinline__ void send_rows(const GemmArgs& a, int gw, int n_gw, i
   }
 }
 
+// Walks the tile list: expert by expert, received rows fastest, so that the pairs at work at any
+// moment share few weight tiles.  An expert's rows, in steps of kStepN, are split evenly over its
+// tiles: tiles of one size keep the pairs that share operands in step.
 struct TileCursor {
   int expert = 0, first_tile = 0;  // first tile id of `expert`
-  int tiles_m = 0;
-  // Advance to the expert that owns tile `t`; returns false when t is past the last tile.
-  __device__ __forceinline__ bool seek(int t, const GemmArgs& a) {
-    for (;;) {
-      if (expert >= a.n_experts) return false;
-      tiles_m = (a.rows[expert] + kBM - 1) / kBM;
-      const int n = tiles_m * a.n_tiles_n;
-      if (t < first_tile + n) return true;
-      first_tile += n;
-      ++expert;
+  int w = 0, row0 = 0, n = 0;      // the tile: weight tile, first row within the expert, rows rounded up to kStepN
+  // Advance to tile `t`; returns false when t is past the last tile.
+  __device__ __forceinline__ bool seek(int t, const int* rows, int n_experts, int n_tiles_w) {
+    for (; expert < n_experts; ++expert) {
+      const int steps = (rows[expert] + kStepN - 1) / kStepN;
+      const int tiles = (steps + kBN / kStepN - 1) / (kBN / kStepN);
+      if (t < first_tile + tiles * n_tiles_w) {
+        const int local = t - first_tile;
+        w = local / tiles;
+        const int i = local - w * tiles, base = steps / tiles, extra = steps - base * tiles;
+        row0 = (i * base + min(i, extra)) * kStepN;
+        n = (base + (i < extra)) * kStepN;
+        return true;
+      }
+      first_tile += tiles * n_tiles_w;
     }
+    return false;
   }
 };
 
@@ -167,28 +203,39 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// tmap_w: weights (kSwiGLU: five dimensions, see gate_up_map; kScatter: boxes of 128 rows);
+// tmap_t: received rows in boxes of 128; tmap_s: the same in boxes of kSmallBox.
 template <int EPI, bool FUSED = false>
-__global__ void __launch_bounds__(FUSED ? kFusedThreads : kGemmThreads, 1)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                    const GemmArgs args) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FUSED ? kFusedThreads : kGemmThreads, 1)
+grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_t,
+                    const __grid_constant__ CUtensorMap tmap_s, const GemmArgs args) {
   using namespace sm100;
   extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment is required by the 128-byte swizzle atoms
+  // 1024-byte alignment is required by the 128-byte swizzle atoms; the offset is the same in both
+  // CTAs of a pair, which the pair's matrix instructions rely on
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* smem_a = smem;
-  uint8_t* smem_b = smem + kStages * kStageBytesA;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_b + kStages * kStageBytesB);
-  uint8_t* smem_out = smem_b + kStages * kStageBytesB + 256;  // 4 x kStageOutBytes, 256-byte aligned
-  // bars: full[kStages], empty[kStages], tmem_full[2], tmem_empty[2]
+  uint8_t* smem_w = smem;
+  uint8_t* smem_t = smem + kStages * kStageBytesW;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_t + kStages * kStageBytesT);
+  uint8_t* smem_turn = smem_t + kStages * kStageBytesT + kBarBytes;  // 2 x kTurnBytes, 256-byte aligned
+  // bars: full[kStages], empty[kStages], tmem_full[2], tmem_empty[2], tile[kTileSlots]; full and
+  // tmem_empty are used in the pair's first CTA only, the others in both
   const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kStages);
   const uint32_t bar_tfull = smem_u32(bars + 2 * kStages), bar_tempty = smem_u32(bars + 2 * kStages + 2);
+  const uint32_t bar_tile = smem_u32(bars + 2 * kStages + 4);
+  static_assert((2 * kStages + 4 + kTileSlots) * 8 <= kBarBytes, "barriers");
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ int s_flags_ok;
+  __shared__ int s_tile[kTileSlots];
+  __shared__ int s_rows[kMaxLocalExperts], s_start[kMaxLocalExperts];
+  __shared__ unsigned long long s_dst[EPI == kScatter ? 2 * kBN : 1];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = (int)cluster_cta_rank();  // which CTA of the pair
   // CTAs [0, n_gemm) run tiles; in the fused kernel the rest (if any) only send rows
   const int n_gemm = FUSED ? (int)gridDim.x - args.send_ctas : (int)gridDim.x;
+  const int n_pairs = n_gemm / 2, pair = (int)blockIdx.x / 2;
   const bool sender_cta = FUSED && (int)blockIdx.x >= n_gemm;
   unsigned long long* dbg = FUSED && args.debug ? args.debug + 4 * blockIdx.x : nullptr;
 
@@ -202,11 +249,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(bar_tfull + 8 * b, 1);
-      mbar_init(bar_tempty + 8 * b, 4);
+      mbar_init(bar_tempty + 8 * b, 8);  // four epilogue warps of either CTA
     }
+    for (int s = 0; s < kTileSlots; ++s) mbar_init(bar_tile + 8 * s, 1);
     fence_barrier_init();
-    tma_prefetch_desc(&tmap_a);
-    tma_prefetch_desc(&tmap_b);
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_t);
+    tma_prefetch_desc(&tmap_s);
     // every source rank must have finished writing this launch's A rows
     if (args.wait_flags != nullptr) {
       const uint64_t t0 = timer_ns();
@@ -226,13 +275,28 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   }
   if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), kTmemCols);
+  for (int e = threadIdx.x; e < args.n_experts; e += blockDim.x) {
+    s_rows[e] = args.rows[e];
+    s_start[e] = args.row_start[e];
+  }
   tc_fence_before_sync();
   __syncthreads();
+  cluster_sync();  // the peer's barriers are initialised and its tensor memory is allocated
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
   volatile int* abort = &abort_flag;
   const uint64_t budget = args.timeout_ns;
   const bool go = s_flags_ok != 0;
+  TileCursor cur;
+  // Number of this pair's i-th tile, for every role but the one that hands them out; past the end
+  // of the list (which ends the role) when the wait was given up.
+  auto tile_number = [&](uint32_t i) -> int {
+    if (i == 0) return pair;
+    const uint32_t slot = i % kTileSlots;
+    if (!mbar_wait_cluster(bar_tile + 8 * slot, ((i / kTileSlots) & 1) ^ (slot == 0), abort, budget)) return 0x7fffffff;
+    return *(volatile int*)&s_tile[slot];
+  };
+  auto find = [&](int t) { return cur.seek(t, s_rows, args.n_experts, args.n_tiles_w); };
 
   if (sender_cta) {
     // ---------------- dedicated sender CTA (never waits on anything) ----------------
@@ -241,10 +305,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   } else if (go && warp == 0) {
     // ---------------- TMA producer ----------------
     if (elect_one()) {
-      TileCursor cur;
-      uint32_t it = 0;  // running k-block counter over all tiles of this CTA
-      int ready_expert = -1;
-      for (int t = blockIdx.x; cur.seek(t, args) && !*abort; t += n_gemm) {
+      const uint32_t lead_full = map_to_rank(bar_full, 0);
+      uint32_t it = 0;  // running k-block counter over all tiles of this pair
+      int ready_expert = -1, t = pair;
+      for (uint32_t i = 0; find(t) && !*abort;) {
+        ++i;
+        if (half == 0) {  // the pair's next tile, fetched while this one is loaded
+          t = n_pairs + (int)atomicAdd(args.next_tile, 1u);
+          const uint32_t slot = i % kTileSlots;
+          for (uint32_t r = 0; r < 2; ++r) {
+            st_cluster(map_to_rank(smem_u32(&s_tile[slot]), r), t);
+            mbar_arrive_remote(map_to_rank(bar_tile + 8 * slot, r));
+          }
+        }
         if (FUSED && cur.expert != ready_expert) {
           // all rows of this expert must have landed (senders on every GPU count them in)
           const uint32_t* ctr = args.arrived[args.my_rank] + cur.expert;
@@ -266,30 +339,40 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           fence_proxy_async_global();
           ready_expert = cur.expert;
         }
-        const int local = t - cur.first_tile;
-        const int m = local % cur.tiles_m, n = local / cur.tiles_m;
-        const int row_a = args.row_start[cur.expert] + m * kBM;
-        const int row_b = cur.expert * args.n_per_expert + n * kBN;
+        const int mine = cur.n / 2;  // received rows that this CTA stages
+        const int row_t = s_start[cur.expert] + cur.row0 + half * mine;
+        const int w_tile = cur.expert * args.n_tiles_w + cur.w;
+        const uint32_t pair_bytes = 2 * (kStageBytesW + (uint32_t)mine * kBK * 2);
         for (int kb = 0; kb < args.k_blocks; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort, budget)) break;
-          mbar_expect_tx(bar_full + 8 * s, kStageBytesA + kStageBytesB);
-          tma_load_2d(smem_u32(smem_a + s * kStageBytesA), &tmap_a, bar_full + 8 * s, kb * kBK, row_a);
-          tma_load_2d(smem_u32(smem_b + s * kStageBytesB), &tmap_b, bar_full + 8 * s, kb * kBK, row_b);
+          const uint32_t full = lead_full + 8 * s;
+          if (half == 0) mbar_expect_tx(bar_full + 8 * s, pair_bytes);
+          const uint32_t dst_w = smem_u32(smem_w + s * kStageBytesW), dst_t = smem_u32(smem_t + s * kStageBytesT);
+          if constexpr (EPI == kSwiGLU)
+            tma_pair_load_5d(dst_w, &tmap_w, full, kb * kBK, half * (kCtaM / (2 * kGateRows)), w_tile);
+          else
+            tma_pair_load_2d(dst_w, &tmap_w, full, kb * kBK, w_tile * kBM + half * kCtaM);
+          if (mine == kBN / 2) {
+            tma_pair_load_2d(dst_t, &tmap_t, full, kb * kBK, row_t);
+          } else {
+            for (int r = 0; r < mine; r += kSmallBox)
+              tma_pair_load_2d(dst_t + r * kBK * 2, &tmap_s, full, kb * kBK, row_t + r);
+          }
         }
+        if (half != 0) t = tile_number(i);
       }
     }
   } else if (go && warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(kBM, kBN);
-      TileCursor cur;
+    // ---------------- MMA issuer, for both CTAs ----------------
+    if (half == 0 && elect_one()) {
       uint32_t it = 0, tile_n = 0;
-      for (int t = blockIdx.x; cur.seek(t, args) && !*abort; t += n_gemm, ++tile_n) {
+      for (; find(tile_number(tile_n)) && !*abort; ++tile_n) {
         const uint32_t acc = tile_n & 1, acc_ph = (tile_n >> 1) & 1;
         if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort, budget)) break;
         tc_fence_after_sync();
+        const uint32_t idesc = umma_idesc_bf16(kBM, cur.n);
         const uint32_t tmem_d = tmem_base + acc * kBN;
         bool ok = true;
         for (int kb = 0; kb < args.k_blocks; ++kb, ++it) {
@@ -300,18 +383,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             break;
           }
           tc_fence_after_sync();
-          const uint64_t da = umma_desc_sw128(smem_u32(smem_a + s * kStageBytesA));
-          const uint64_t db = umma_desc_sw128(smem_u32(smem_b + s * kStageBytesB));
+          const uint64_t dw = umma_desc_sw128(smem_u32(smem_w + s * kStageBytesW));
+          const uint64_t dt = umma_desc_sw128(smem_u32(smem_t + s * kStageBytesT));
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             // advance 16 elements = 32 bytes along K inside the swizzled 128-byte row
-            umma_bf16(tmem_d, da + (uint64_t)(k * kUmmaK * 2 >> 4), db + (uint64_t)(k * kUmmaK * 2 >> 4), idesc,
-                      (kb | k) != 0);
+            umma_pair_bf16(tmem_d, dw + (uint64_t)(k * kUmmaK * 2 >> 4), dt + (uint64_t)(k * kUmmaK * 2 >> 4), idesc,
+                           (kb | k) != 0);
           }
-          umma_commit(bar_empty + 8 * s);  // stage reusable once these MMAs have read it
+          umma_pair_commit(bar_empty + 8 * s);  // stage reusable, in both CTAs, once these MMAs have read it
         }
         if (!ok) break;
-        umma_commit(bar_tfull + 8 * acc);  // accumulator complete
+        umma_pair_commit(bar_tfull + 8 * acc);  // accumulator complete, in both CTAs
       }
     }
   } else if (FUSED && warp >= 6) {
@@ -323,86 +406,88 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   } else if (go && warp >= 2) {
     // ---------------- epilogue ----------------
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 are the ones this warp may read
-    TileCursor cur;
-    uint32_t tile_n = 0;
-    for (int t = blockIdx.x; cur.seek(t, args) && !*abort; t += n_gemm, ++tile_n) {
+    const int et = threadIdx.x - 64;
+    uint32_t turn = 0;
+    for (uint32_t tile_n = 0;; ++tile_n) {
+      // All four warps leave the loop together: they meet at barriers below, and tcgen05.ld is a
+      // whole-warp instruction.  A thread that gave up a wait finds no tile.
+      const bool more = find(tile_number(tile_n));
+      if (!epilogue_all(more && !*abort)) break;
       const uint32_t acc = tile_n & 1, acc_ph = (tile_n >> 1) & 1;
-      const int local = t - cur.first_tile;
-      const int m = local % cur.tiles_m, n = local / cur.tiles_m;
-      const int row_in_expert = m * kBM + quarter * 32 + lane;
-      const bool valid = row_in_expert < args.rows[cur.expert];
-      const size_t row = (size_t)args.row_start[cur.expert] + row_in_expert;
-      // tcgen05.ld is a whole-warp instruction: leave the loop only if every lane agrees
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * acc, acc_ph, abort, budget))) break;
+      const int left = s_rows[cur.expert] - cur.row0;  // rows of the expert from this tile's first on
+      const size_t row0 = (size_t)s_start[cur.expert] + cur.row0;
+      if constexpr (EPI == kScatter) {  // where every row of the tile goes
+        for (int r = et; r < cur.n; r += 128) {
+          unsigned long long to = 0;
+          if (r < left) {
+            const int mt = args.meta[row0 + r];
+            to = reinterpret_cast<unsigned long long>(args.comb[(mt >> 20) & (kMaxRanks - 1)] +
+                                                      (size_t)(mt & 0xFFFFF) * args.out_ld);
+          }
+          s_dst[acc * kBN + r] = to;
+        }
+      }
+      if (!epilogue_all(mbar_wait(bar_tfull + 8 * acc, acc_ph, abort, budget))) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * kBN;
-      if constexpr (EPI == kSwiGLU) {
-        __nv_bfloat16* dst = args.act + row * args.act_ld + (size_t)n * (kBN / 2);
-#pragma unroll 1
-        for (int c0 = 0; c0 < kBN / 2; c0 += 32) {
-          uint32_t g[32], u[32];
-          tmem_ld32(taddr + c0, g);
-          tmem_ld32(taddr + kBN / 2 + c0, u);
-          tmem_ld_wait();
-          if (valid) {
+      for (int c0 = 0; c0 < cur.n; c0 += kStepN, turn ^= 1) {
+        uint8_t* stage = smem_turn + turn * kTurnBytes;
+        const uint32_t mine = smem_u32(stage);
+        // fragments: thread l holds lanes l/4 and l/4 + 8 of a 16-lane half, columns 8j + 2(l%4) and the next
+        uint32_t a[16], b[16];
+        __syncwarp();
+        tmem_ld_16x32(taddr + c0, a);                // lanes 0-15
+        tmem_ld_16x32(taddr + (16u << 16) + c0, b);  // lanes 16-31
+        tmem_ld_wait();
+        if constexpr (EPI == kSwiGLU) {
+          uint32_t o[8];
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint32_t o[4];
+          for (int j = 0; j < 8; ++j) {
+            const float v0 = silu(__uint_as_float(a[2 * j])) * __uint_as_float(b[2 * j]);
+            const float v1 = silu(__uint_as_float(a[2 * j + 1])) * __uint_as_float(b[2 * j + 1]);
+            o[j] = pack_bf16(v0, v1);
+          }
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const float a0 = silu(__uint_as_float(g[j + 2 * q])) * __uint_as_float(u[j + 2 * q]);
-                const float a1 = silu(__uint_as_float(g[j + 2 * q + 1])) * __uint_as_float(u[j + 2 * q + 1]);
-                o[q] = pack_bf16(a0, a1);
-              }
-              st_global_v4(dst + c0 + j, o[0], o[1], o[2], o[3]);
-            }
-          }
-        }
-      } else {
-        // Each lane owns one output row in TMEM, but a row's 512 bytes should leave the SM
-        // as long contiguous stores (they cross NVLink).  Stage 32 rows x 128 columns in
-        // shared memory (16-byte chunks XOR-swizzled by row against bank conflicts), then
-        // let 16 lanes write one row's 256 bytes: two rows per store instruction.
-        unsigned long long dst_addr = 0;
-        if (valid) {
-          const int mt = args.meta[row];
-          dst_addr = reinterpret_cast<unsigned long long>(args.comb[(mt >> 20) & (kMaxRanks - 1)] +
-                                                          (size_t)(mt & 0xFFFFF) * args.out_ld + (size_t)n * kBN);
-        }
-        uint8_t* stage = smem_out + (warp - 2) * kStageOutBytes;
-#pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-#pragma unroll 1
-          for (int c0 = 0; c0 < 128; c0 += 32) {
-            uint32_t v[32];
-            tmem_ld32(taddr + half * 128 + c0, v);
-            tmem_ld_wait();
+          for (int h = 0; h < 2; ++h)  // 8 features each; 128-byte rows, 16-byte chunks swizzled by row
+            stmatrix_trans(mine + lane * 128 + (((2 * quarter + h) ^ (lane & 7)) << 4), o[h], o[2 + h], o[4 + h], o[6 + h]);
+          epilogue_sync();
+          __nv_bfloat16* dst = args.act + (row0 + c0) * args.act_ld + (size_t)cur.w * (kBM / 2) + half * (kCtaM / 2);
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              const int chunk = (c0 + j) >> 3;  // 16-byte chunk index within the 256-byte row
-              uint4 o;
-              o.x = pack_bf16(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-              o.y = pack_bf16(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-              o.z = pack_bf16(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
-              o.w = pack_bf16(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
-              *reinterpret_cast<uint4*>(stage + lane * 256 + ((chunk ^ (lane & 15)) << 4)) = o;
-            }
+          for (int i = 0; i < 2; ++i) {
+            const int r = (et >> 3) + 16 * i, chunk = et & 7;
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
+            if (c0 + r < left) st_global_v4(dst + (size_t)r * args.act_ld + chunk * 8, v.x, v.y, v.z, v.w);
           }
-          __syncwarp();
-#pragma unroll 4
-          for (int i = 0; i < 16; ++i) {
-            const int r = 2 * i + (lane >> 4), chunk = lane & 15;
-            const unsigned long long base = __shfl_sync(0xffffffffu, dst_addr, r);
-            const uint4 o = *reinterpret_cast<const uint4*>(stage + r * 256 + ((chunk ^ (r & 15)) << 4));
-            if (base != 0)
-              st_global_v4(reinterpret_cast<void*>(base + (size_t)half * 256 + (size_t)chunk * 16), o.x, o.y, o.z, o.w);
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t row = mine + lane * 256;
+            stmatrix_trans(row + (((4 * quarter + h) ^ (lane & 7)) << 4),
+                           pack_bf16(__uint_as_float(a[2 * h]), __uint_as_float(a[2 * h + 1])),
+                           pack_bf16(__uint_as_float(a[4 + 2 * h]), __uint_as_float(a[5 + 2 * h])),
+                           pack_bf16(__uint_as_float(a[8 + 2 * h]), __uint_as_float(a[9 + 2 * h])),
+                           pack_bf16(__uint_as_float(a[12 + 2 * h]), __uint_as_float(a[13 + 2 * h])));
+            stmatrix_trans(row + (((4 * quarter + 2 + h) ^ (lane & 7)) << 4),
+                           pack_bf16(__uint_as_float(b[2 * h]), __uint_as_float(b[2 * h + 1])),
+                           pack_bf16(__uint_as_float(b[4 + 2 * h]), __uint_as_float(b[5 + 2 * h])),
+                           pack_bf16(__uint_as_float(b[8 + 2 * h]), __uint_as_float(b[9 + 2 * h])),
+                           pack_bf16(__uint_as_float(b[12 + 2 * h]), __uint_as_float(b[13 + 2 * h])));
           }
-          __syncwarp();
+          epilogue_sync();
+          // 16 lanes write 256 contiguous bytes of a row (they cross NVLink)
+          const size_t col = ((size_t)cur.w * kBM + half * kCtaM) * 2;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = (et >> 4) + 8 * i, chunk = et & 15;
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + r * 256 + ((chunk ^ (r & 7)) << 4));
+            const unsigned long long to = s_dst[acc * kBN + c0 + r];
+            if (to != 0) st_global_v4(reinterpret_cast<void*>(to + col + (size_t)chunk * 16), v.x, v.y, v.z, v.w);
+          }
         }
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+      if (lane == 0) mbar_arrive_remote(map_to_rank(bar_tempty + 8 * acc, 0));
     }
   }
 
@@ -417,12 +502,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if constexpr (EPI == kScatter) __threadfence_system();  // rows stored to peers are visible before the flag
   tc_fence_before_sync();
   __syncthreads();
+  cluster_sync();  // neither CTA leaves while the other may still signal it or read its operands
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
   if (dbg && threadIdx.x == 0) dbg[3] = timer_ns();
   if (threadIdx.x == 0 && args.ticket != nullptr) {
     __threadfence();
     if (atomicAdd(args.ticket, 1u) == gridDim.x - 1) {
       *args.ticket = 0;
+      *args.next_tile = 0;  // every pair has taken its last number
       if constexpr (EPI == kScatter) {
         __threadfence_system();
         for (int r = 0; r < args.n_ranks; ++r)

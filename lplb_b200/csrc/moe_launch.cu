@@ -29,25 +29,48 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 bool shape_ok(const LayerShape& sh) {
   return sh.n_ranks >= 1 && sh.n_ranks <= kMaxRanks && sh.my_rank >= 0 && sh.my_rank < sh.n_ranks &&
-         sh.n_local >= 1 && sh.n_local <= kMaxLocalExperts && sh.hidden % kBN == 0 && sh.hidden % kBK == 0 &&
-         (2 * sh.inter) % kBN == 0 && sh.inter % kBK == 0 && sh.topk >= 1 && sh.topk <= kCombineMaxTopk &&
+         sh.n_local >= 1 && sh.n_local <= kMaxLocalExperts && sh.hidden % kBM == 0 && sh.hidden % kBK == 0 &&
+         (2 * sh.inter) % kBM == 0 && sh.inter % kBK == 0 && sh.topk >= 1 && sh.topk <= kCombineMaxTopk &&
          (long long)sh.max_tokens * sh.topk < (1 << 20) && sh.capacity > 0 && sh.capacity < (1 << 24);
 }
 
 }  // namespace
 
-int make_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+namespace {
+int encode_map(CUtensorMap* out, const void* base, uint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides,
+               const cuuint32_t* box) {
   auto fn = encode_fn();
   if (!fn) return -1;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (cols * 2) % 16 || box_rows == 0 || box_rows > 256) return -2;
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  const CUresult rc = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || strides[0] % 16) return -2;
+  const cuuint32_t elem_strides[5] = {1, 1, 1, 1, 1};
+  const CUresult rc = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box,
                          elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS ? 0 : (int)rc;
+}
+int row_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
+  return encode_map(out, base, 2, dims, strides, box);
+}
+// The gate/up weight tensor as [256-row block][group of 16][gate, up][16 rows][cols]: a box of four
+// groups arrives in shared memory as 16 gate rows, their 16 up rows, the next 16 gate rows, ...
+int gate_up_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols) {
+  const cuuint64_t row = cols * 2;
+  const cuuint64_t dims[5] = {cols, kGateRows, 2, kGateBlock / kGateRows, rows / (2 * kGateBlock)};
+  const cuuint64_t strides[4] = {row, kGateBlock * row, kGateRows * row, 2 * kGateBlock * row};
+  const cuuint32_t box[5] = {(cuuint32_t)kBK, kGateRows, 2, kCtaM / (2 * kGateRows), 1};
+  return encode_map(out, base, 5, dims, strides, box);
+}
+}  // namespace
+
+int make_gemm_maps(GemmMaps* out, const void* tokens, uint64_t rows, const void* weights, uint64_t weight_rows,
+                   uint64_t cols, bool gate_up) {
+  int rc = row_map(&out->t, tokens, rows, cols, kBN / 2);
+  if (rc == 0) rc = row_map(&out->s, tokens, rows, cols, kSmallBox);
+  if (rc == 0) rc = gate_up ? gate_up_map(&out->w, weights, weight_rows, cols) : row_map(&out->w, weights, weight_rows, cols, kCtaM);
+  return rc;
 }
 
 namespace {
@@ -155,13 +178,15 @@ cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const v
   return cudaGetLastError();
 }
 
-cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUtensorMap& tmap_a,
-                                 const CUtensorMap& tmap_b, const void* x, uint32_t epoch,
+cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, const void* x, uint32_t epoch,
                                  unsigned long long timeout_ns, int n_cta, int send_ctas, cudaStream_t stream) {
-  if (!shape_ok(sh) || n_cta < 1 || send_ctas < 0 || send_ctas >= n_cta) return cudaErrorInvalidValue;
+  if (!shape_ok(sh) || n_cta < 2 || send_ctas < 0 || send_ctas >= n_cta) return cudaErrorInvalidValue;
+  n_cta &= ~1;  // tiles are run by pairs, so the CTAs that only send come in pairs too
   const PlanView plan = plan_view(sh, b);
   GemmArgs a{};
-  a.send_ctas = send_ctas;
+  a.send_ctas = (send_ctas + 1) & ~1;
+  if (a.send_ctas > n_cta - 2) a.send_ctas = n_cta - 2;
+  a.next_tile = b.tickets + 4;
   a.rows = plan.rows;
   a.row_start = plan.row_start;
   a.n_experts = sh.n_local;
@@ -170,9 +195,8 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
   a.epoch = epoch;
   a.status = b.status;
   a.timeout_ns = timeout_ns;
-  a.n_tiles_n = 2 * sh.inter / kBN;
+  a.n_tiles_w = 2 * sh.inter / kBM;
   a.k_blocks = sh.hidden / kBK;
-  a.n_per_expert = 2 * sh.inter;
   a.act = static_cast<__nv_bfloat16*>(b.act);
   a.act_ld = sh.inter;
   a.wait_flags = nullptr;
@@ -194,15 +218,16 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
   auto kernel = grouped_gemm_kernel<kSwiGLU, true>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
   if (err != cudaSuccess) return err;
-  kernel<<<n_cta, kFusedThreads, kGemmSmem, stream>>>(tmap_a, tmap_b, a);
+  kernel<<<n_cta, kFusedThreads, kGemmSmem, stream>>>(maps.w, maps.t, maps.s, a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUtensorMap& tmap_a,
-                        const CUtensorMap& tmap_b, int which, uint32_t epoch, unsigned long long timeout_ns,
+cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, int which, uint32_t epoch, unsigned long long timeout_ns,
                         int n_cta, cudaStream_t stream) {
-  if (!shape_ok(sh) || n_cta < 1 || (which != 0 && which != 1)) return cudaErrorInvalidValue;
+  if (!shape_ok(sh) || n_cta < 2 || (which != 0 && which != 1)) return cudaErrorInvalidValue;
+  n_cta &= ~1;
   GemmArgs a{};
+  a.next_tile = b.tickets + 4;
   a.rows = b.plan;
   a.row_start = b.plan + sh.n_local;
   a.n_experts = sh.n_local;
@@ -213,9 +238,8 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUten
   a.timeout_ns = timeout_ns;
   cudaError_t err;
   if (which == 0) {
-    a.n_tiles_n = 2 * sh.inter / kBN;
+    a.n_tiles_w = 2 * sh.inter / kBM;
     a.k_blocks = sh.hidden / kBK;
-    a.n_per_expert = 2 * sh.inter;
     a.act = static_cast<__nv_bfloat16*>(b.act);
     a.act_ld = sh.inter;
     a.wait_flags = sh.n_ranks > 1 ? b.flags[sh.my_rank] : nullptr;  // dispatch done, one word per source rank
@@ -223,11 +247,10 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUten
     auto kernel = grouped_gemm_kernel<kSwiGLU, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     if (err != cudaSuccess) return err;
-    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(tmap_a, tmap_b, a);
+    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, maps.t, maps.s, a);
   } else {
-    a.n_tiles_n = sh.hidden / kBN;
+    a.n_tiles_w = sh.hidden / kBM;
     a.k_blocks = sh.inter / kBK;
-    a.n_per_expert = sh.hidden;
     a.meta = b.recv_meta[sh.my_rank];
     for (int r = 0; r < sh.n_ranks; ++r) {
       a.comb[r] = static_cast<__nv_bfloat16*>(b.comb[r]);
@@ -239,7 +262,7 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const CUten
     auto kernel = grouped_gemm_kernel<kScatter, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     if (err != cudaSuccess) return err;
-    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(tmap_a, tmap_b, a);
+    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, maps.t, maps.s, a);
   }
   return cudaGetLastError();
 }
