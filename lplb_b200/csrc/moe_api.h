@@ -61,9 +61,9 @@ inline int plan_words(int n_ranks, int n_local) {
 size_t gemm_smem_bytes();
 
 // Tensor maps of one grouped GEMM (128-byte swizzle, 64 elements of K per box): weights, received
-// rows in boxes of half a tile, received rows in small boxes.
+// rows in boxes of 128, 64, 32 and 16 rows.
 struct GemmMaps {
-  CUtensorMap w, t, s;
+  CUtensorMap w, rows[4];
 };
 // tokens: bf16 [rows, cols]; weights: bf16 [weight_rows, cols], with `gate_up` in blocks of 128
 // gate rows and their 128 up rows.  Returns 0 on success.

@@ -49,30 +49,39 @@
 namespace lplb {
 namespace moe {
 
-constexpr int kBM = 256, kBN = 256, kBK = 64, kStages = 6, kUmmaK = 16;
+constexpr int kBM = 256, kBN = 256, kBK = 64, kUmmaK = 16;
 constexpr int kCtaM = kBM / 2;       // weight rows per CTA of a pair
 constexpr int kStepN = 32;           // received rows per tile are rounded up to this
-constexpr int kSmallBox = 16;        // received rows per TMA box where a CTA's half is not 128 rows
+constexpr int kRowBoxes = 4;         // received rows come in TMA boxes of 128, 64, 32 and 16 rows
 constexpr int kGateRows = 16;        // gate (and up) rows of one epilogue warp
 constexpr int kGateBlock = 128;      // gate rows in front of their up rows in the weight tensor
 constexpr int kGemmThreads = 192;
 constexpr int kTmemCols = 512;
+constexpr uint32_t kStageBytesW = kCtaM * kBK * 2;
+// The ring of operand stages.  A stage holds the weights and as many received rows as the launch's
+// largest tile stages per CTA, so the ring is as deep as it can be: 6 stages with tiles of 256
+// rows, 11 when no expert received more than 32 (64 tokens, both GEMMs: 643 us, with 6 stages 685).
+constexpr uint32_t kRingBytes = 200 * 1024;
+constexpr int kMaxStages = 11;
 // Tile numbers on their way to the roles.  The producer announces tile i + 1 when it begins tile
-// i; then all k blocks but the last kStages have been computed, so with two or more k blocks per
-// tile the accumulator of tile i - 4 is complete, the epilogue is through with tile i - 6, and no
-// role still has to read a number older than that of tile i - 5.
-constexpr int kTileSlots = 8;
-static_assert(kStages <= 6, "a slot would be overwritten before the epilogue has read it");
-constexpr uint32_t kStageBytesW = kCtaM * kBK * 2, kStageBytesT = kBN / 2 * kBK * 2;
+// i; then all k blocks but the last kMaxStages have been computed, so with two or more k blocks
+// per tile the accumulators of tile i - 7 are complete, the epilogue is through with tile i - 9,
+// and no role still has to read a number older than that of tile i - 8.
+constexpr int kTileSlots = 16;
+static_assert(kMaxStages <= 12, "a slot could be overwritten before the epilogue has read it");
 constexpr uint32_t kTurnBytes = kStepN * kCtaM * 2;  // 32 received rows x 128 features, two of these
-constexpr uint32_t kBarBytes = 256;
-constexpr size_t kGemmSmem = 1024 + (size_t)kStages * (kStageBytesW + kStageBytesT) + kBarBytes + 2 * kTurnBytes;
+constexpr uint32_t kBarBytes = 512;
+constexpr size_t kGemmSmem = 1024 + kRingBytes + kBarBytes + 2 * kTurnBytes;
 constexpr int kMaxLocalExperts = 128;
 constexpr int kMaxRanks = 8;
 
 enum Epilogue : int { kSwiGLU = 0, kScatter = 1 };
 
 enum MoeErr : int { kMoeOk = 0, kMoeGemmTimeout = 11, kMoeFlagTimeout = 12, kMoeOverflow = 13 };
+
+struct RowMaps {
+  CUtensorMap box[kRowBoxes];
+};
 
 struct GemmArgs {
   const int* rows;        // [n_experts] rows received per local expert
@@ -170,16 +179,19 @@ __device__ __forceinline__ void send_rows(const GemmArgs& a, int gw, int n_gw, i
 
 // Walks the tile list: expert by expert, received rows fastest, so that the pairs at work at any
 // moment share few weight tiles.  An expert's rows, in steps of kStepN, are split evenly over its
-// tiles: tiles of one size keep the pairs that share operands in step.
+// tiles: tiles of one size keep the pairs that share operands in step.  (Tiles of 512 rows, two
+// accumulators side by side, load a quarter less but lose more to the shallower ring and the
+// uncovered epilogue: first GEMM at 8192 tokens 3170 us against 2906 us.)
 struct TileCursor {
   int expert = 0, first_tile = 0;  // first tile id of `expert`
   int w = 0, row0 = 0, n = 0;      // the tile: weight tile, first row within the expert, rows rounded up to kStepN
+  static __device__ __forceinline__ int steps_of(int rows) { return (rows + kStepN - 1) / kStepN; }
+  static __device__ __forceinline__ int tiles_of(int steps) { return (steps + kBN / kStepN - 1) / (kBN / kStepN); }
   // Advance to tile `t`; returns false when t is past the last tile.
-  __device__ __forceinline__ bool seek(int t, const int* rows, int n_experts, int n_tiles_w) {
-    for (; expert < n_experts; ++expert) {
-      const int steps = (rows[expert] + kStepN - 1) / kStepN;
-      const int tiles = (steps + kBN / kStepN - 1) / (kBN / kStepN);
-      if (t < first_tile + tiles * n_tiles_w) {
+  __device__ __forceinline__ bool seek(int t, const int* rows, const GemmArgs& a) {
+    for (; expert < a.n_experts; ++expert) {
+      const int steps = steps_of(rows[expert]), tiles = tiles_of(steps);
+      if (t < first_tile + tiles * a.n_tiles_w) {
         const int local = t - first_tile;
         w = local / tiles;
         const int i = local - w * tiles, base = steps / tiles, extra = steps - base * tiles;
@@ -187,7 +199,7 @@ struct TileCursor {
         n = (base + (i < extra)) * kStepN;
         return true;
       }
-      first_tile += tiles * n_tiles_w;
+      first_tile += tiles * a.n_tiles_w;
     }
     return false;
   }
@@ -204,26 +216,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // tmap_w: weights (kSwiGLU: five dimensions, see gate_up_map; kScatter: boxes of 128 rows);
-// tmap_t: received rows in boxes of 128; tmap_s: the same in boxes of kSmallBox.
+// rows: received rows in boxes of 128, 64, 32 and 16.  Issuing a box takes the producer some 55
+// cycles whatever its size: in boxes of 16 rows, eight per K block, it held up the tensor cores.
 template <int EPI, bool FUSED = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FUSED ? kFusedThreads : kGemmThreads, 1)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_t,
-                    const __grid_constant__ CUtensorMap tmap_s, const GemmArgs args) {
+grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ RowMaps rows,
+                    const GemmArgs args) {
   using namespace sm100;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment is required by the 128-byte swizzle atoms; the offset is the same in both
   // CTAs of a pair, which the pair's matrix instructions rely on
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* smem_w = smem;
-  uint8_t* smem_t = smem + kStages * kStageBytesW;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_t + kStages * kStageBytesT);
-  uint8_t* smem_turn = smem_t + kStages * kStageBytesT + kBarBytes;  // 2 x kTurnBytes, 256-byte aligned
-  // bars: full[kStages], empty[kStages], tmem_full[2], tmem_empty[2], tile[kTileSlots]; full and
-  // tmem_empty are used in the pair's first CTA only, the others in both
-  const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kStages);
-  const uint32_t bar_tfull = smem_u32(bars + 2 * kStages), bar_tempty = smem_u32(bars + 2 * kStages + 2);
-  const uint32_t bar_tile = smem_u32(bars + 2 * kStages + 4);
-  static_assert((2 * kStages + 4 + kTileSlots) * 8 <= kBarBytes, "barriers");
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kRingBytes);
+  uint8_t* smem_turn = smem + kRingBytes + kBarBytes;  // 2 x kTurnBytes, 256-byte aligned
+  // bars: full[kMaxStages], empty[kMaxStages], tmem_full[2], tmem_empty[2], tile[kTileSlots]; full
+  // and tmem_empty are used in the pair's first CTA only, the others in both
+  const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kMaxStages);
+  const uint32_t bar_tfull = smem_u32(bars + 2 * kMaxStages), bar_tempty = smem_u32(bars + 2 * kMaxStages + 2);
+  const uint32_t bar_tile = smem_u32(bars + 2 * kMaxStages + 4);
+  static_assert((2 * kMaxStages + 4 + kTileSlots) * 8 <= kBarBytes, "barriers");
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ int s_flags_ok;
@@ -243,7 +254,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (dbg) dbg[0] = timer_ns();
     abort_flag = 0;
     s_flags_ok = 1;
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
@@ -254,8 +265,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     for (int s = 0; s < kTileSlots; ++s) mbar_init(bar_tile + 8 * s, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmap_w);
-    tma_prefetch_desc(&tmap_t);
-    tma_prefetch_desc(&tmap_s);
+    for (int b = 0; b < kRowBoxes; ++b) tma_prefetch_desc(&rows.box[b]);
     // every source rank must have finished writing this launch's A rows
     if (args.wait_flags != nullptr) {
       const uint64_t t0 = timer_ns();
@@ -288,6 +298,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const uint64_t budget = args.timeout_ns;
   const bool go = s_flags_ok != 0;
   TileCursor cur;
+  int largest = 1;  // steps of the launch's largest tile
+  for (int e = lane; e < args.n_experts; e += 32) {
+    const int steps = TileCursor::steps_of(s_rows[e]), tiles = TileCursor::tiles_of(steps);
+    if (tiles > 0) largest = max(largest, (steps + tiles - 1) / tiles);
+  }
+  largest = __reduce_max_sync(0xffffffffu, largest);
+  const uint32_t stage_bytes = kStageBytesW + largest * (kStepN / 2) * kBK * 2;
+  const uint32_t stages = min((uint32_t)kMaxStages, kRingBytes / stage_bytes);
   // Number of this pair's i-th tile, for every role but the one that hands them out; past the end
   // of the list (which ends the role) when the wait was given up.
   auto tile_number = [&](uint32_t i) -> int {
@@ -296,7 +314,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (!mbar_wait_cluster(bar_tile + 8 * slot, ((i / kTileSlots) & 1) ^ (slot == 0), abort, budget)) return 0x7fffffff;
     return *(volatile int*)&s_tile[slot];
   };
-  auto find = [&](int t) { return cur.seek(t, s_rows, args.n_experts, args.n_tiles_w); };
+  auto find = [&](int t) { return cur.seek(t, s_rows, args); };
 
   if (sender_cta) {
     // ---------------- dedicated sender CTA (never waits on anything) ----------------
@@ -306,7 +324,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     // ---------------- TMA producer ----------------
     if (elect_one()) {
       const uint32_t lead_full = map_to_rank(bar_full, 0);
-      uint32_t it = 0;  // running k-block counter over all tiles of this pair
+      uint32_t s = 0, ph = 0;  // stage and its phase, running over all tiles of this pair
       int ready_expert = -1, t = pair;
       for (uint32_t i = 0; find(t) && !*abort;) {
         ++i;
@@ -343,23 +361,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int row_t = s_start[cur.expert] + cur.row0 + half * mine;
         const int w_tile = cur.expert * args.n_tiles_w + cur.w;
         const uint32_t pair_bytes = 2 * (kStageBytesW + (uint32_t)mine * kBK * 2);
-        for (int kb = 0; kb < args.k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
+        for (int kb = 0; kb < args.k_blocks; ++kb) {
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort, budget)) break;
           const uint32_t full = lead_full + 8 * s;
           if (half == 0) mbar_expect_tx(bar_full + 8 * s, pair_bytes);
-          const uint32_t dst_w = smem_u32(smem_w + s * kStageBytesW), dst_t = smem_u32(smem_t + s * kStageBytesT);
+          uint32_t dst = smem_u32(smem) + s * stage_bytes;
           if constexpr (EPI == kSwiGLU)
-            tma_pair_load_5d(dst_w, &tmap_w, full, kb * kBK, half * (kCtaM / (2 * kGateRows)), w_tile);
+            tma_pair_load_5d(dst, &tmap_w, full, kb * kBK, half * (kCtaM / (2 * kGateRows)), w_tile);
           else
-            tma_pair_load_2d(dst_w, &tmap_w, full, kb * kBK, w_tile * kBM + half * kCtaM);
-          if (mine == kBN / 2) {
-            tma_pair_load_2d(dst_t, &tmap_t, full, kb * kBK, row_t);
-          } else {
-            for (int r = 0; r < mine; r += kSmallBox)
-              tma_pair_load_2d(dst_t + r * kBK * 2, &tmap_s, full, kb * kBK, row_t + r);
+            tma_pair_load_2d(dst, &tmap_w, full, kb * kBK, w_tile * kBM + half * kCtaM);
+          dst += kStageBytesW;
+          int row = row_t;
+#pragma unroll
+          for (int b = 0; b < kRowBoxes; ++b) {
+            const int n = kBN / 2 >> b;
+            if (mine & n) {
+              tma_pair_load_2d(dst, &rows.box[b], full, kb * kBK, row);
+              dst += n * kBK * 2;
+              row += n;
+            }
           }
+          if (++s == stages) s = 0, ph ^= 1;
         }
         if (half != 0) t = tile_number(i);
       }
@@ -367,24 +389,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   } else if (go && warp == 1) {
     // ---------------- MMA issuer, for both CTAs ----------------
     if (half == 0 && elect_one()) {
-      uint32_t it = 0, tile_n = 0;
-      for (; find(tile_number(tile_n)) && !*abort; ++tile_n) {
+      uint32_t s = 0, ph = 0;
+      for (uint32_t tile_n = 0; find(tile_number(tile_n)) && !*abort; ++tile_n) {
         const uint32_t acc = tile_n & 1, acc_ph = (tile_n >> 1) & 1;
         if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort, budget)) break;
         tc_fence_after_sync();
         const uint32_t idesc = umma_idesc_bf16(kBM, cur.n);
         const uint32_t tmem_d = tmem_base + acc * kBN;
         bool ok = true;
-        for (int kb = 0; kb < args.k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
+        for (int kb = 0; kb < args.k_blocks; ++kb) {
           if (!mbar_wait(bar_full + 8 * s, ph, abort, budget)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const uint64_t dw = umma_desc_sw128(smem_u32(smem_w + s * kStageBytesW));
-          const uint64_t dt = umma_desc_sw128(smem_u32(smem_t + s * kStageBytesT));
+          const uint32_t base = smem_u32(smem) + s * stage_bytes;
+          const uint64_t dw = umma_desc_sw128(base), dt = umma_desc_sw128(base + kStageBytesW);
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             // advance 16 elements = 32 bytes along K inside the swizzled 128-byte row
@@ -392,6 +412,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                            (kb | k) != 0);
           }
           umma_pair_commit(bar_empty + 8 * s);  // stage reusable, in both CTAs, once these MMAs have read it
+          if (++s == stages) s = 0, ph ^= 1;
         }
         if (!ok) break;
         umma_pair_commit(bar_tfull + 8 * acc);  // accumulator complete, in both CTAs

@@ -67,8 +67,8 @@ int gate_up_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols
 
 int make_gemm_maps(GemmMaps* out, const void* tokens, uint64_t rows, const void* weights, uint64_t weight_rows,
                    uint64_t cols, bool gate_up) {
-  int rc = row_map(&out->t, tokens, rows, cols, kBN / 2);
-  if (rc == 0) rc = row_map(&out->s, tokens, rows, cols, kSmallBox);
+  int rc = 0;
+  for (int b = 0; b < kRowBoxes && rc == 0; ++b) rc = row_map(&out->rows[b], tokens, rows, cols, kBN / 2 >> b);
   if (rc == 0) rc = gate_up ? gate_up_map(&out->w, weights, weight_rows, cols) : row_map(&out->w, weights, weight_rows, cols, kCtaM);
   return rc;
 }
@@ -178,6 +178,14 @@ cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const v
   return cudaGetLastError();
 }
 
+namespace {
+RowMaps row_maps(const GemmMaps& m) {
+  RowMaps r;
+  for (int b = 0; b < kRowBoxes; ++b) r.box[b] = m.rows[b];
+  return r;
+}
+}  // namespace
+
 cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, const void* x, uint32_t epoch,
                                  unsigned long long timeout_ns, int n_cta, int send_ctas, cudaStream_t stream) {
   if (!shape_ok(sh) || n_cta < 2 || send_ctas < 0 || send_ctas >= n_cta) return cudaErrorInvalidValue;
@@ -218,7 +226,7 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
   auto kernel = grouped_gemm_kernel<kSwiGLU, true>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
   if (err != cudaSuccess) return err;
-  kernel<<<n_cta, kFusedThreads, kGemmSmem, stream>>>(maps.w, maps.t, maps.s, a);
+  kernel<<<n_cta, kFusedThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
   return cudaGetLastError();
 }
 
@@ -247,7 +255,7 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmM
     auto kernel = grouped_gemm_kernel<kSwiGLU, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     if (err != cudaSuccess) return err;
-    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, maps.t, maps.s, a);
+    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
   } else {
     a.n_tiles_w = sh.hidden / kBM;
     a.k_blocks = sh.inter / kBK;
@@ -262,7 +270,7 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmM
     auto kernel = grouped_gemm_kernel<kScatter, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     if (err != cudaSuccess) return err;
-    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, maps.t, maps.s, a);
+    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
   }
   return cudaGetLastError();
 }
