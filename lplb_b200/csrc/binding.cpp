@@ -115,9 +115,11 @@ class PlannerEngine {
   }
 
   // Place the experts and rebuild every table on the device (place_kernel.cu), ordered on the
-  // current stream like set_mapping; nothing waits for the device.  `history`: contiguous int32
-  // or int64 [E] on this device, or none for the natural order.  Returns (phy2log, log2phy,
-  // logcnt, log2edge), or none when the shape does not fit one CTA's shared memory.
+  // current stream like set_mapping, and wait for it: whoever holds the returned tables may read
+  // them on any stream (weights are usually moved on a stream of their own).  `history`:
+  // contiguous int32 or int64 [E] on this device, or none for the natural order.  Returns
+  // (phy2log, log2phy, logcnt, log2edge), or none when the shape does not fit one CTA's shared
+  // memory.
   py::object place(const c10::optional<torch::Tensor>& history, int n_nodes) {
     LPLB_CHECK(r2o_.defined(), "topology must be set first");
     LPLB_CHECK(n_nodes >= 1, "n_nodes must be positive");
@@ -139,7 +141,6 @@ class PlannerEngine {
                  "history must be contiguous int32/int64 [E] on cuda:" << device_);
       a.history = h.data_ptr();
       a.is64 = h.scalar_type() == torch::kInt64;
-      h.record_stream(stream);  // the caller may drop it before the kernel has read it
     }
     const int64_t p = (int64_t)n_group_ * g_ * (ll_ + c_ * d_);
     auto i32 = status_.options();
@@ -161,6 +162,10 @@ class PlannerEngine {
     a.table_log2slot = log2slot_.data_ptr<int>();
     LPLB_CUDA(lplb::launch_place(a, stream.stream()));
     invalidate_warm_start();  // a new placement is a new LP
+    {
+      py::gil_scoped_release other_threads_run;
+      LPLB_CUDA(cudaStreamSynchronize(stream.stream()));
+    }
     return py::make_tuple(phy2log, log2phy, logcnt, log2edge);
   }
 

@@ -298,8 +298,9 @@ class Planner:
         """Re-place experts from load history and rebuild every lookup table.
 
         Returns ``(phy2log [P], log2phy [E, 2], logcnt [E])`` int32 on the planner's
-        device (reference ``lplb/planner.py:115-182``).  Moving the expert *weights* to
-        match ``phy2log`` is the caller's job, as in the reference.
+        device (reference ``lplb/planner.py:115-182``), ready to be read on any stream: the call
+        waits for the device.  Moving the expert *weights* to match ``phy2log`` is the caller's
+        job, as in the reference.
         """
         placed = self._place_on_device(workload)
         if placed is not None:
@@ -324,8 +325,8 @@ class Planner:
         return self.mapping.phy2log, self.mapping.log2phy, self.mapping.logcnt
 
     def _place_on_device(self, workload: torch.Tensor | None) -> tuple | None:
-        """The same placement and tables from one kernel, without a wait for the device (256
-        experts: 33 us, 8.9 ms on the host), or ``None`` where the host has to do it.  Histories of
+        """The same placement and tables from one kernel and one wait for it (256 experts: 49 us,
+        8.9 ms on the host), or ``None`` where the host has to do it.  Histories of
         whole numbers only: their sums are exact in any order, and they hold no NaN or infinity,
         for which the host's sort and arg-min have rules of their own."""
         if self._engine is None or self.n_nodes < 1:

@@ -57,3 +57,17 @@ def test_same_tables_as_the_host(shape):
         assert torch.equal(torch.bincount(a.reshape(-1)[flat]), torch.bincount(b.reshape(-1)[flat]))
     with pytest.raises(ValueError):
         planner.update_redundancy_mapping(torch.ones(n + 1, dtype=torch.int64, device="cuda"))
+
+
+def test_the_tables_are_ready_on_every_stream():
+    hist = torch.randperm(32, generator=torch.Generator().manual_seed(3))
+    want = build_mapping(cube(), 1, 4, 1, hist)
+    planner = Planner(cube(), 32 + 16, 32, 8, device="cuda", n_nodes=1)
+    hist = hist.cuda()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)  # the current stream is busy for a while
+    planner.update_redundancy_mapping(hist)
+    with torch.cuda.stream(torch.cuda.Stream()):  # where a program moves its weights
+        got = [t.cpu() for t in vars(planner.mapping).values()]
+    for a, b in zip(got, vars(want).values()):
+        assert torch.equal(a, b)
