@@ -116,7 +116,9 @@ class PlannerEngine {
 
   // Place the experts and rebuild every table on the device (place_kernel.cu), ordered on the
   // current stream like set_mapping, and wait for it: whoever holds the returned tables may read
-  // them on any stream (weights are usually moved on a stream of their own).  `history`:
+  // them on any stream (weights are usually moved on a stream of their own).  Refused during a
+  // graph capture: a replay would change the placement behind the back of whoever holds weights
+  // or tables for the one of the capture.  `history`:
   // contiguous int32 or int64 [E] on this device, or none for the natural order.  Returns
   // (phy2log, log2phy, logcnt, log2edge), or none when the shape does not fit one CTA's shared
   // memory.
@@ -134,6 +136,9 @@ class PlannerEngine {
     if (lplb::place_shared_bytes(a) > 227 * 1024) return py::none();
     c10::cuda::CUDAGuard guard(device_);
     auto stream = c10::cuda::getCurrentCUDAStream(device_);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    LPLB_CUDA(cudaStreamIsCapturing(stream.stream(), &capture));
+    LPLB_CHECK(capture == cudaStreamCaptureStatusNone, "a new placement cannot be captured in a CUDA graph");
     if (history.has_value()) {
       const torch::Tensor& h = *history;
       LPLB_CHECK(h.is_cuda() && h.get_device() == device_ && h.is_contiguous() && h.numel() == e_ &&

@@ -71,3 +71,19 @@ def test_the_tables_are_ready_on_every_stream():
         got = [t.cpu() for t in vars(planner.mapping).values()]
     for a, b in zip(got, vars(want).values()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("history", ["none", "device", "host", "float"])
+def test_a_graph_capture_refuses_a_new_placement(history):
+    planner = Planner(cube(), 32 + 16, 32, 8, device="cuda", n_nodes=1)
+    kept = planner.phy2log
+    before, version = kept.clone(), planner.placement_version()
+    hist = {"none": None, "device": torch.arange(32, device="cuda"), "host": torch.arange(32),
+            "float": torch.rand(32, device="cuda")}[history]
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="captur"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            planner.update_redundancy_mapping(hist)
+    torch.cuda.synchronize()
+    assert planner.phy2log is kept and torch.equal(kept, before) and planner.placement_version() == version
+    planner.update_redundancy_mapping(hist)  # and works again outside
