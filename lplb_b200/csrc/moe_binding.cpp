@@ -203,6 +203,14 @@ class MoeEngine {
     return out;
   }
 
+  // Whether the device's current stream is being captured.
+  bool capturing() const {
+    c10::cuda::CUDAGuard guard(device_);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    MOE_CUDA(cudaStreamIsCapturing(c10::cuda::getCurrentCUDAStream(device_).stream(), &status));
+    return status != cudaStreamCaptureStatusNone;
+  }
+
   void set_timeout_us(double us) { timeout_ns_ = (unsigned long long)(us * 1e3); }
   // Fused dispatch: 0 = four sender warps beside the tile roles in every CTA; n > 0 = n CTAs
   // (of one per SM) only send rows and the rest only run tiles.
@@ -320,6 +328,7 @@ void bind_moe(py::module_& m) {
       .def("set_weights", &MoeEngine::set_weights)
       .def("forward", &MoeEngine::forward, py::arg("x"), py::arg("phys_idx"), py::arg("weights"), py::arg("n_cta"),
            py::arg("upto") = 5, py::arg("fuse_dispatch") = false)
+      .def("capturing", &MoeEngine::capturing)
       .def("set_timeout_us", &MoeEngine::set_timeout_us)
       .def("set_send_ctas", &MoeEngine::set_send_ctas)
       .def("reset", &MoeEngine::reset)

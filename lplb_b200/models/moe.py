@@ -152,6 +152,10 @@ class MoELayer:
         """Run the layer on physical expert ids.  ``fuse_dispatch`` (default: the layer's
         setting) sends the rows from inside the first GEMM kernel, so the tensor cores start on
         an expert as soon as its rows have landed instead of after the whole dispatch."""
+        # A replay would skip the comparison below, run on weights that place_weights() has replaced
+        # since, and repeat a launch number that the ranks must not see twice.
+        if self.engine.capturing():
+            raise RuntimeError("MoELayer cannot be captured in a CUDA graph")
         # The table itself is compared (three launches and a wait for the device, 30 us per call)
         # only after something wrote to it; the same experts in the same slots need no new weights.
         version = self.planner.placement_version()

@@ -229,3 +229,26 @@ def test_receive_buffer_overflow_drops_pairs_and_reports(fused):
     assert layer.check() == 0
     ref = layer.reference_forward(*small).float()
     assert float((out.float() - ref).abs().max() / ref.abs().max()) < 2e-2
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_a_graph_capture_refuses_the_layer(fused):
+    planner, layer = _layer(256, 128, 32, 2, 64)
+    layer.fuse_dispatch = fused
+    x, idx, w = _inputs(64, 256, 32, 2)
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = layer.forward(x, idx, w, avail)  # first launches outside the capture
+    phys = planner.run(idx, avail)
+    torch.cuda.synchronize()
+    epoch = layer.engine.epoch()
+    for call in (lambda: layer.forward(x, idx, w, avail), lambda: layer.forward_physical(x, phys, w)):
+        with pytest.raises(RuntimeError, match="captur"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                call()
+    torch.cuda.synchronize()
+    assert layer.engine.epoch() == epoch
+    again = layer.forward(x, idx, w, avail)
+    torch.cuda.synchronize()
+    assert layer.check() == 0
+    # another split over the replicas gives the same rows: identical weights, the same order of every sum
+    assert torch.equal(again, want)
