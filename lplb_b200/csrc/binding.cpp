@@ -15,6 +15,7 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include <mutex>
 #include <sstream>
 #include <stdexcept>
 #include <string>
@@ -120,8 +121,8 @@ class PlannerEngine {
   // graph capture: a replay would change the placement behind the back of whoever holds weights
   // or tables for the one of the capture.  `history`:
   // contiguous int32 or int64 [E] on this device, or none for the natural order.  Returns
-  // (phy2log, log2phy, logcnt, log2edge), or none when the shape does not fit one CTA's shared
-  // memory.
+  // (phy2log, log2phy, logcnt, log2edge), or none where the host has to place the experts: the
+  // shape does not fit one CTA's shared memory, or the loads are too large for sums in any order.
   py::object place(const c10::optional<torch::Tensor>& history, int n_nodes) {
     LPLB_CHECK(r2o_.defined(), "topology must be set first");
     LPLB_CHECK(n_nodes >= 1, "n_nodes must be positive");
@@ -165,12 +166,20 @@ class PlannerEngine {
     a.table_log2phy = log2phy_.data_ptr<int>();
     a.table_log2edge = log2edge_.data_ptr<int>();
     a.table_log2slot = log2slot_.data_ptr<int>();
-    LPLB_CUDA(lplb::launch_place(a, stream.stream()));
-    invalidate_warm_start();  // a new placement is a new LP
+    int report;
     {
       py::gil_scoped_release other_threads_run;
+      std::lock_guard<std::mutex> one_at_a_time(place_mutex_);  // there is one report word
+      if (!place_report_.defined()) place_report_ = torch::zeros({1}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
+      volatile int* word = place_report_.data_ptr<int>();
+      *word = lplb::kPlaceOk;
+      LPLB_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&a.report), place_report_.data_ptr<int>(), 0));
+      LPLB_CUDA(lplb::launch_place(a, stream.stream()));
+      invalidate_warm_start();  // a new placement is a new LP
       LPLB_CUDA(cudaStreamSynchronize(stream.stream()));
+      report = *word;
     }
+    if (report == lplb::kPlaceInexact) return py::none();
     return py::make_tuple(phy2log, log2phy, logcnt, log2edge);
   }
 
@@ -520,6 +529,8 @@ class PlannerEngine {
   torch::Tensor r2o_, o2r_, phy2log_, log2phy_, log2edge_, log2slot_;
   bool warm_ = false;
   torch::Tensor workspace_, status_, probs_, trace_, anchor_, anchor_valid_;
+  std::mutex place_mutex_;
+  torch::Tensor place_report_;  // pinned [1], written by place_kernel
   int max_cta64_ = -1, max_cta32_ = -1;
   // exchange
   IpcBlock block_;

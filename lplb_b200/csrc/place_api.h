@@ -6,6 +6,11 @@
 
 namespace lplb {
 
+enum PlaceReport : int {
+  kPlaceOk = 0,
+  kPlaceInexact = 1,  // loads of expert groups beyond 2^53: their sums depend on the order of adding; no table was written
+};
+
 struct PlaceArgs {
   const void* history;  // [n_logical] int32/int64 loads; null = natural order
   int is64;
@@ -13,6 +18,7 @@ struct PlaceArgs {
   int n_logical, ep_size, n_group, g, dup, combined, n_nodes;
   // results, and the engine's own copies of them (which keep their addresses)
   int *phy2log, *log2phy, *logcnt, *log2edge;
+  int* report;  // host memory: kPlaceOk before the launch, written only where there is something to report
   int *table_phy2log, *table_log2phy, *table_log2edge, *table_log2slot;
 };
 

@@ -3,14 +3,16 @@
 // The same decisions as the host balancer (lplb_b200/eplb.py, lplb_b200/mapping.py), item by item:
 // expert groups to nodes, experts to the ranks of a node, both heaviest first into the lightest
 // pack with room (reference lplb/eplb.py:6-46, :80-148), then the tables (reference
-// lplb/planner.py:115-182).  Loads are float64 on both sides and are added in the same order, so
-// the results are identical.
+// lplb/planner.py:115-182).  Loads are float64 on both sides.  A rank's load grows item by item, in
+// the same order on both; a group's load is added in another order than on the host, which gives
+// the same sum as long as no partial sum can pass 2^53.  Where one could, the kernel writes no table
+// and reports it, and the host places the experts.  So the results are identical.
 //
 // One CTA.  What bounds it is the greedy packing, one dependent step per expert: a warp holds the
 // packs (one per lane up to 32) and finds the lightest with two 32-bit warp reductions over the
 // order-preserving halves of the double and a ballot, with no shared memory on the chain, instead
 // of five shuffle rounds of a double and an index.  The orders come from counting, for every
-// expert, the experts in front of it.  256 experts on 8 ranks: 29 us, 49 us for the whole call with its
+// expert, the experts in front of it.  256 experts on 8 ranks: 27 us, 48 us for the whole call with its
 // wait for the device; on the host, some twenty tensor operations per expert, 8.9 ms.
 #include "place_api.h"
 
@@ -74,6 +76,8 @@ __device__ void pack_items(const double* w, const int* order, int n, int packs, 
     int held = 0;
     int item = order[0];
     double weight = w[item];
+    // left to the compiler the unrolling moves with lines elsewhere in the kernel: 31 or 35 us, so 29
+#pragma unroll 8
     for (int step = 0; step < n; ++step) {
       const int next = order[min(step + 1, n - 1)];
       const double next_weight = w[next];
@@ -125,6 +129,28 @@ __device__ void pack_items(const double* w, const int* order, int n, int packs, 
   }
 }
 
+// gw[g] = the load of group g, a warp per group.  Returns whether a partial sum, in some order of
+// adding, could pass 2^53 (in a group of the calling warp).
+__device__ bool group_loads(const PlaceArgs& a, double* gw, int groups, int per_group) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  bool large = false;
+  for (int g = warp; g < groups; g += kPlaceThreads / 32) {
+    double sum = 0.0, size = 0.0;
+    for (int i = lane; i < per_group; i += 32) {
+      const double x = load_of(a, g * per_group + i);
+      sum += x;
+      size += fabs(x);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(kAll, sum, o);
+      size += __shfl_xor_sync(kAll, size, o);
+    }
+    if (lane == 0) gw[g] = sum;
+    large |= size >= 9007199254740992.0;  // 2^53
+  }
+  return large;
+}
+
 __global__ void __launch_bounds__(kPlaceThreads) place_kernel(const PlaceArgs a) {
   extern __shared__ double sm[];
   const int tid = threadIdx.x, warp = tid >> 5, n_warps = kPlaceThreads / 32;
@@ -150,13 +176,11 @@ __global__ void __launch_bounds__(kPlaceThreads) place_kernel(const PlaceArgs a)
     if (groups_per_node == 1) {
       for (int g = tid; g < groups; g += kPlaceThreads) place_of_group[g] = g;
     } else {
-      for (int g = warp; g < groups; g += n_warps) {
-        double sum = 0.0;
-        for (int i = tid & 31; i < per_group; i += 32) sum += load_of(a, g * per_group + i);
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
-        if ((tid & 31) == 0) s.gw[g] = sum;
+      const bool inexact = group_loads(a, s.gw, groups, per_group);
+      if (__syncthreads_or(inexact)) {
+        if (tid == 0) *a.report = kPlaceInexact;
+        return;
       }
-      __syncthreads();
       sort_rows(s.gw, s.order, 1, groups);
       __syncthreads();
       if (warp == 0)
@@ -176,12 +200,16 @@ __global__ void __launch_bounds__(kPlaceThreads) place_kernel(const PlaceArgs a)
     } else {
       sort_rows(s.w, s.order, nodes, per_node);
       __syncthreads();
-      // A pack fills heaviest first, so every rank's own slots are in the order of the history.
+      // A pack fills heaviest first, so every rank's own slots are in the order of the history.  The
+      // packing warp stores positions; looking the experts up there would put a load on its chain
+      // (41 instead of 35 us).
       for (int node = warp; node < nodes; node += n_warps) {
         const int base = node * per_node;
         pack_items(s.w + base, s.order + base, per_node, packs, ll, s.load + node * packs, s.fill + node * packs,
-                   [&](int item, int pack, int pos) { s.own[base + pack * ll + pos] = s.nlog2log[base + item]; });
+                   [&](int item, int pack, int pos) { s.own[base + pack * ll + pos] = base + item; });
       }
+      __syncthreads();
+      for (int i = tid; i < E; i += kPlaceThreads) s.own[i] = s.nlog2log[s.own[i]];
     }
   }
   __syncthreads();

@@ -87,3 +87,19 @@ def test_a_graph_capture_refuses_a_new_placement(history):
     torch.cuda.synchronize()
     assert planner.phy2log is kept and torch.equal(kept, before) and planner.placement_version() == version
     planner.update_redundancy_mapping(hist)  # and works again outside
+
+
+def test_groups_whose_loads_pass_2_53_are_placed_as_on_the_host():
+    # The groups hold the same loads in different orders: which of them is the heaviest is decided by
+    # the rounding of the sums alone, so by the order in which the host adds them.
+    planner = Planner(cube(), 4 * 48, 4 * 32, 32, device="cuda", n_nodes=2)
+    g = torch.Generator().manual_seed(0)
+    for bits in (48, 49, 55, 62):  # 32 loads of 48 bits stay below 2^53, of 49 bits may pass it
+        for sign in (1, -1):
+            loads = sign * (torch.randint(2 ** (bits - 1), 2**bits, (32,), generator=g) | 1)
+            hist = torch.cat([loads[torch.randperm(32, generator=g)] for _ in range(4)])
+            want = build_mapping(cube(), 4, 4, 1, hist, n_nodes=2)
+            for h in (hist, hist.cuda()):
+                got = planner.update_redundancy_mapping(h)
+                for a, b in zip(got, (want.phy2log, want.log2phy, want.logcnt)):
+                    assert torch.equal(a.cpu(), b), (bits, sign)
