@@ -84,6 +84,14 @@ class PlannerEngine {
     LPLB_CHECK(o2r.sizes() == r2o.sizes(), "o2r must match r2o");
     r2o_ = to_dev_i32(r2o);
     o2r_ = to_dev_i32(o2r);
+    const auto to = r2o.to(torch::kCPU, torch::kInt64).contiguous(), from = o2r.to(torch::kCPU, torch::kInt64).contiguous();
+    const int64_t *t = to.data_ptr<int64_t>(), *f = from.data_ptr<int64_t>();
+    inverse_topology_ = true;
+    for (int rank = 0; rank < g_; ++rank)
+      for (int d = 0; d < d_; ++d) {
+        const int64_t a = t[rank * d_ + d], b = f[rank * d_ + d];
+        inverse_topology_ &= a >= 0 && a < g_ && b >= 0 && b < g_ && f[a * d_ + d] == rank && t[b * d_ + d] == rank;
+      }
   }
 
   void set_mapping(const torch::Tensor& phy2log, const torch::Tensor& log2phy, const torch::Tensor& log2edge) {
@@ -134,6 +142,10 @@ class PlannerEngine {
     a.dup = d_;
     a.combined = c_;
     a.n_nodes = n_nodes;
+    if (!inverse_topology_) {
+      PyErr_SetString(PyExc_AssertionError, "replica slots disagree with the inverse topology");
+      throw py::error_already_set();
+    }
     if (lplb::place_shared_bytes(a) > 227 * 1024) return py::none();
     c10::cuda::CUDAGuard guard(device_);
     auto stream = c10::cuda::getCurrentCUDAStream(device_);
@@ -180,6 +192,10 @@ class PlannerEngine {
       report = *word;
     }
     if (report == lplb::kPlaceInexact) return py::none();
+    if (report == lplb::kPlaceUncovered) {
+      phy2log_ = log2phy_ = log2edge_ = log2slot_ = torch::Tensor();  // launches are refused until a placement succeeds
+      throw py::value_error("placement does not cover every logical expert exactly once");
+    }
     return py::make_tuple(phy2log, log2phy, logcnt, log2edge);
   }
 
@@ -529,6 +545,7 @@ class PlannerEngine {
   torch::Tensor r2o_, o2r_, phy2log_, log2phy_, log2edge_, log2slot_;
   bool warm_ = false;
   torch::Tensor workspace_, status_, probs_, trace_, anchor_, anchor_valid_;
+  bool inverse_topology_ = false;  // r2o_ and o2r_ are each other's inverse
   std::mutex place_mutex_;
   torch::Tensor place_report_;  // pinned [1], written by place_kernel
   int max_cta64_ = -1, max_cta32_ = -1;

@@ -8,9 +8,11 @@ namespace lplb {
 
 enum PlaceReport : int {
   kPlaceOk = 0,
-  kPlaceInexact = 1,  // loads of expert groups beyond 2^53: their sums depend on the order of adding; no table was written
+  kPlaceInexact = 1,    // loads of expert groups beyond 2^53: their sums depend on the order of adding; no table was written
+  kPlaceUncovered = 2,  // some expert does not sit in exactly one of the ranks' own slots; the tables are not usable
 };
 
+// r2o and o2r: each the inverse of the other, which the caller has checked.
 struct PlaceArgs {
   const void* history;  // [n_logical] int32/int64 loads; null = natural order
   int is64;

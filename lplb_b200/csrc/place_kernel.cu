@@ -12,7 +12,7 @@
 // packs (one per lane up to 32) and finds the lightest with two 32-bit warp reductions over the
 // order-preserving halves of the double and a ballot, with no shared memory on the chain, instead
 // of five shuffle rounds of a double and an index.  The orders come from counting, for every
-// expert, the experts in front of it.  256 experts on 8 ranks: 27 us, 48 us for the whole call with its
+// expert, the experts in front of it.  256 experts on 8 ranks: 32 us, 53 us for the whole call with its
 // wait for the device; on the host, some twenty tensor operations per expert, 8.9 ms.
 #include "place_api.h"
 
@@ -76,7 +76,8 @@ __device__ void pack_items(const double* w, const int* order, int n, int packs, 
     int held = 0;
     int item = order[0];
     double weight = w[item];
-    // left to the compiler the unrolling moves with lines elsewhere in the kernel: 31 or 35 us, so 29
+    // left to the compiler the unrolling moves with lines elsewhere in the kernel (one launch after
+    // the other: 31 or 35 us, with 8 steps 29)
 #pragma unroll 8
     for (int step = 0; step < n; ++step) {
       const int next = order[min(step + 1, n - 1)];
@@ -212,6 +213,9 @@ __global__ void __launch_bounds__(kPlaceThreads) place_kernel(const PlaceArgs a)
       for (int i = tid; i < E; i += kPlaceThreads) s.own[i] = s.nlog2log[s.own[i]];
     }
   }
+  int* slot_of = reinterpret_cast<int*>(s.w);  // the packing is through with the loads
+  for (int i = tid; i < E; i += kPlaceThreads)
+    if ((unsigned)s.own[i] < (unsigned)E) slot_of[s.own[i]] = i;
   __syncthreads();
 
   for (int i = tid; i < ranks * pl; i += kPlaceThreads) {
@@ -219,6 +223,10 @@ __global__ void __launch_bounds__(kPlaceThreads) place_kernel(const PlaceArgs a)
     int e;
     if (slot < ll) {
       e = s.own[rank * ll + slot];
+      if ((unsigned)e >= (unsigned)E || slot_of[e] != rank * ll + slot) {  // every expert in exactly one own slot
+        *a.report = kPlaceUncovered;
+        continue;
+      }
       const int first = slot < rep ? slot % a.dup : a.dup;  // bundle of the slot; dup = not replicated
       int replica = -1;
       if (slot < rep) {

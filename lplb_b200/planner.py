@@ -325,7 +325,7 @@ class Planner:
         return self.mapping.phy2log, self.mapping.log2phy, self.mapping.logcnt
 
     def _place_on_device(self, workload: torch.Tensor | None) -> tuple | None:
-        """The same placement and tables from one kernel and one wait for it (256 experts: 48 us,
+        """The same placement and tables from one kernel and one wait for it (256 experts: 53 us,
         8.9 ms on the host), or ``None`` where the host has to do it.  Histories of whole numbers
         only: their sums are exact in any order up to 2^53 (the kernel finds out whether a sum
         could pass that), and they hold no NaN or infinity, for which the host's sort and arg-min

@@ -103,3 +103,25 @@ def test_groups_whose_loads_pass_2_53_are_placed_as_on_the_host():
                 got = planner.update_redundancy_mapping(h)
                 for a, b in zip(got, (want.phy2log, want.log2phy, want.logcnt)):
                     assert torch.equal(a.cpu(), b), (bits, sign)
+
+
+@pytest.mark.parametrize("entry", [None, (0, 3, 1, 8), (1, 2, 0, 8), (0, 0, 0, -1), (1, 7, 1, -1)])
+def test_tables_that_disagree_with_the_topology_are_refused(entry):
+    planner = Planner(cube(), 32 + 16, 32, 8, device="cuda", n_nodes=1)
+    kept, version = planner.phy2log, planner.placement_version()
+    before = kept.clone()
+    tables = [planner.r2o.clone(), planner.o2r.clone()]
+    if entry is None:  # ranks within range, but not the inverse
+        tables[1] = tables[1].roll(1, 0)
+    else:  # one past the last rank, or in front of the first
+        which, rank, d, value = entry
+        tables[which][rank, d] = value
+    planner._engine.set_topology(*tables)
+    with pytest.raises(AssertionError, match="inverse topology"):
+        planner.update_redundancy_mapping(torch.arange(32))
+    assert planner.phy2log is kept and torch.equal(kept, before) and planner.placement_version() == version
+    planner._engine.set_topology(planner.r2o, planner.o2r)
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    idx = torch.arange(32, device="cuda").unsqueeze(1)
+    assert torch.equal(before[planner.run(idx, avail).long()].long(), idx)  # the engine's tables are untouched
+    planner.update_redundancy_mapping(torch.arange(32))
