@@ -323,6 +323,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   } else if (go && warp == 0) {
     // ---------------- TMA producer ----------------
     if (elect_one()) {
+      // Peers wrote the received rows with ordinary stores, seen through thread 0's acquire of their
+      // flags; the TMA loads below are another proxy.
+      if (args.wait_flags != nullptr) fence_proxy_async_global();
       const uint32_t lead_full = map_to_rank(bar_full, 0);
       uint32_t s = 0, ph = 0;  // stage and its phase, running over all tiles of this pair
       int ready_expert = -1, t = pair;
