@@ -80,12 +80,26 @@ cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const v
 // Step 2a (fused path only): decide the send order and every pair's target row and return slot.
 cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const void* phys_idx, int idx_is64,
                             int n_tokens, cudaStream_t stream);
+// How the fused kernel's CTAs are dealt out: `tile` of them run tiles and `send` only send rows.
+struct FusedGrid {
+  int tile, send;
+};
+// The tile CTAs wait for rows that every sender of the launch sends, so all CTAs have to be resident
+// at once: no more pairs than the device holds (a GPC with an odd number of SMs leaves one without a
+// partner).  send_ctas is rounded up to whole pairs; one pair at least runs tiles.
+inline FusedGrid fused_grid(int n_cta, int send_ctas, int resident_pairs) {
+  const int pairs = n_cta / 2 < resident_pairs ? n_cta / 2 : resident_pairs;
+  int send = (send_ctas + 1) / 2;
+  if (send > pairs - 1) send = pairs - 1;
+  return FusedGrid{2 * (pairs - send), 2 * send};
+}
+// CTA pairs of the fused kernel that fit on the current device at once.
+cudaError_t fused_resident_pairs(int* pairs);
 // Step 2b+3 fused: the first grouped GEMM, which also streams this rank's rows to their targets
-// while the tensor cores work on the experts whose rows have landed.  send_ctas == 0: four
-// extra warps in every CTA send.  send_ctas > 0: that many of the n_cta CTAs (rounded up to whole
-// pairs) only send and the others only run tiles.
+// while the tensor cores work on the experts whose rows have landed.  grid.send == 0: four
+// extra warps in every CTA send.
 cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, const void* x, uint32_t epoch,
-                                 unsigned long long timeout_ns, int n_cta, int send_ctas, cudaStream_t stream);
+                                 unsigned long long timeout_ns, FusedGrid grid, cudaStream_t stream);
 // Step 3/4: grouped GEMMs.  which = 0: recv_x x w13 -> SwiGLU -> act.  which = 1: act x w2 -> peers' comb.
 cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, int which, uint32_t epoch, unsigned long long timeout_ns,
                         int n_cta, cudaStream_t stream);

@@ -178,17 +178,22 @@ class MoeEngine {
     c10::cuda::CUDAGuard guard(device_);
     cudaStream_t s = c10::cuda::getCurrentCUDAStream(device_).stream();
     const int is64 = phys_idx.scalar_type() == torch::kInt64;
-    ++epoch_;
     auto out = torch::empty({n_tokens, sh_.hidden}, x.options());
     // The fused path cannot stop between dispatch and the first GEMM: stage 2 then means both.
     const bool fused = fuse_dispatch && upto >= 3;
+    lplb::moe::FusedGrid grid{};
+    if (fused) {
+      if (resident_pairs_ == 0) MOE_CUDA(lplb::moe::fused_resident_pairs(&resident_pairs_));
+      MOE_CHECK(resident_pairs_ > 0, "the fused kernel's CTA pairs do not fit on this device");
+      grid = lplb::moe::fused_grid(gemm_ctas(), send_ctas_, resident_pairs_);
+    }
+    ++epoch_;
     MOE_CUDA(lplb::moe::launch_route(sh_, buf_, phys_idx.data_ptr(), is64, n_tokens, n_cta, epoch_, timeout_ns_,
                                      fused ? 1 : 0, s));
     if (upto <= 1) return out;
     if (fused) {
       MOE_CUDA(lplb::moe::launch_schedule(sh_, buf_, phys_idx.data_ptr(), is64, n_tokens, s));
-      MOE_CUDA(lplb::moe::launch_dispatch_gemm(sh_, buf_, maps1_, x.data_ptr(), epoch_, timeout_ns_,
-                                               gemm_ctas(), send_ctas_, s));
+      MOE_CUDA(lplb::moe::launch_dispatch_gemm(sh_, buf_, maps1_, x.data_ptr(), epoch_, timeout_ns_, grid, s));
     } else {
       MOE_CUDA(lplb::moe::launch_dispatch(sh_, buf_, x.data_ptr(), phys_idx.data_ptr(), is64, n_tokens,
                                           4 * n_cta, epoch_, s));
@@ -301,7 +306,7 @@ class MoeEngine {
 
   lplb::moe::LayerShape sh_{};
   lplb::moe::LayerBuffers buf_{};
-  int device_, p_ = 0, sms_ = 0;
+  int device_, p_ = 0, sms_ = 0, resident_pairs_ = 0;
   size_t off_recv_x_ = 0, off_meta_ = 0, off_comb_ = 0, off_cnt_ = 0, off_flags_ = 0, off_arrived_ = 0, block_bytes_ = 0;
   void* block_ = nullptr;
   std::vector<char*> bases_;
@@ -317,6 +322,10 @@ class MoeEngine {
 }  // namespace
 
 void bind_moe(py::module_& m) {
+  m.def("moe_fused_grid", [](int n_cta, int send_ctas, int resident_pairs) {
+    const auto grid = lplb::moe::fused_grid(n_cta, send_ctas, resident_pairs);
+    return py::make_tuple(grid.tile, grid.send);
+  });
   py::class_<MoeEngine>(m, "MoeEngine")
       .def(py::init<int, int, int, int, int, int, int, int, int>(), py::arg("hidden"), py::arg("inter"),
            py::arg("n_local"), py::arg("n_ranks"), py::arg("my_rank"), py::arg("topk"), py::arg("max_tokens"),

@@ -186,14 +186,29 @@ RowMaps row_maps(const GemmMaps& m) {
 }
 }  // namespace
 
+cudaError_t fused_resident_pairs(int* pairs) {
+  auto kernel = grouped_gemm_kernel<kSwiGLU, true>;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+  if (err != cudaSuccess) return err;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = 2;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(2);
+  config.blockDim = dim3(kFusedThreads);
+  config.dynamicSmemBytes = kGemmSmem;
+  config.attrs = &cluster;
+  config.numAttrs = 1;
+  return cudaOccupancyMaxActiveClusters(pairs, kernel, &config);
+}
+
 cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, const void* x, uint32_t epoch,
-                                 unsigned long long timeout_ns, int n_cta, int send_ctas, cudaStream_t stream) {
-  if (!shape_ok(sh) || n_cta < 2 || send_ctas < 0 || send_ctas >= n_cta) return cudaErrorInvalidValue;
-  n_cta &= ~1;  // tiles are run by pairs, so the CTAs that only send come in pairs too
+                                 unsigned long long timeout_ns, FusedGrid grid, cudaStream_t stream) {
+  if (!shape_ok(sh) || grid.tile < 2 || grid.tile % 2 || grid.send < 0 || grid.send % 2) return cudaErrorInvalidValue;
   const PlanView plan = plan_view(sh, b);
   GemmArgs a{};
-  a.send_ctas = (send_ctas + 1) & ~1;
-  if (a.send_ctas > n_cta - 2) a.send_ctas = n_cta - 2;
+  a.send_ctas = grid.send;
   a.next_tile = b.tickets + 4;
   a.rows = plan.rows;
   a.row_start = plan.row_start;
@@ -226,7 +241,7 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
   auto kernel = grouped_gemm_kernel<kSwiGLU, true>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
   if (err != cudaSuccess) return err;
-  kernel<<<n_cta, kFusedThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
+  kernel<<<grid.tile + grid.send, kFusedThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
   return cudaGetLastError();
 }
 
