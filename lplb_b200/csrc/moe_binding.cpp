@@ -1,5 +1,5 @@
 // Python binding of the benchmark MoE layer engine: buffers, peer mapping, weights and the
-// forward pass (count -> plan -> dispatch -> GEMM1+SwiGLU -> GEMM2+combine -> reduce).
+// forward pass (route -> dispatch -> GEMM1+SwiGLU -> GEMM2+combine -> reduce).
 // The reference has no MoE layer; this exists for the end-to-end measurement that consumes
 // the planner's redirected indices.
 #include <c10/cuda/CUDAGuard.h>
@@ -160,7 +160,7 @@ class MoeEngine {
 
   // One forward pass.  x: [T, hidden] bf16, phys_idx: [T, topk] int64/int32 physical expert
   // ids (-1 = dropped), weights: [T, topk] float32.  `upto` stops after a stage for tests:
-  // 1 plan, 2 dispatch, 3 first GEMM, 4 second GEMM, 5 (default) everything.
+  // 1 route (counts and plan), 2 dispatch, 3 first GEMM, 4 second GEMM, 5 (default) everything.
   torch::Tensor forward(const torch::Tensor& x, const torch::Tensor& phys_idx, const torch::Tensor& weights,
                         int n_cta, int upto, bool fuse_dispatch) {
     MOE_CHECK(ready_ && have_weights_, "engine is not ready: open peers and set weights first");

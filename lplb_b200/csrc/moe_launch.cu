@@ -56,6 +56,10 @@ int row_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, ui
 }
 // The gate/up weight tensor as [256-row block][group of 16][gate, up][16 rows][cols]: a box of four
 // groups arrives in shared memory as 16 gate rows, their 16 up rows, the next 16 gate rows, ...
+// Its strides do not ascend (128 rows, then 16 rows): the documentation of cuTensorMapEncodeTiled has
+// every stride a multiple of the one before.  The encoder takes the map as it is, and set_weights
+// reports the code where one should refuse it.  With ascending strides either the layout that callers
+// lay their weights out in would change, or a stage would take four boxes instead of one.
 int gate_up_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols) {
   const cuuint64_t row = cols * 2;
   const cuuint64_t dims[5] = {cols, kGateRows, 2, kGateBlock / kGateRows, rows / (2 * kGateBlock)};

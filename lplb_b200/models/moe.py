@@ -4,7 +4,7 @@ SwiGLU experts (``hidden -> 2*inter -> hidden``), top-k routing, expert parallel
 ranks of one NVLink domain.  A forward pass is::
 
     logical ids --Planner.run--> physical ids
-    count pairs per physical expert, all-gather the counts over peer memory   (plan)
+    rank the pairs of every physical expert, all-gather the counts over peer memory, plan   (route)
     push every (token, k) hidden state into its expert's rows on the target GPU (dispatch)
     grouped GEMM 1 on tcgen05 + SwiGLU epilogue
     grouped GEMM 2 on tcgen05, epilogue stores rows straight into the source GPU (combine)
@@ -37,6 +37,7 @@ class MoELayer:
 
     With ``group=None`` a single GPU hosts every physical expert of the (virtual)
     ``ep_size`` ranks; with a process group each rank hosts ``n_physical / ep_size``.
+    A forward pass cannot be captured in a CUDA graph (``RuntimeError``).
     Weights are random-init and derived from a per-logical-expert seed, so a replica holds
     the same values as its original without any weight traffic.
     """
@@ -57,7 +58,8 @@ class MoELayer:
         """``capacity_rows`` sets the receive buffer's size in rows directly (rounded up to a
         multiple of 128) instead of deriving it from ``max_tokens * topk * capacity_factor``.
         Pairs that would land beyond it are dropped by their senders, contribute nothing to
-        the output and are reported (``check()`` returns the overflow code)."""
+        the output and are reported (``check()`` returns the overflow code); which of an expert's
+        pairs they are is not fixed."""
         from .. import _native
 
         if planner.device.type != "cuda":

@@ -233,7 +233,10 @@ class Planner:
 
     def placement_version(self) -> tuple[int, int] | None:
         """Changes whenever ``phy2log`` is replaced or written to, so that whoever depends on the
-        placement can ask on the host, every step, whether it still holds.  ``None``: not known
+        placement can ask on the host, every step, whether it still holds.  (Routing uses the
+        engine's tables, which only ``update_redundancy_mapping`` and ``load_state_dict`` write;
+        both replace ``phy2log``.  A write past autograd's version counter, through ``.data`` or by
+        a collective, changes neither the routing nor this number.)  ``None``: not known
         (the table was made in inference mode, where tensors carry no version), compare the table."""
         if self._phy2log.is_inference():
             return None
