@@ -54,6 +54,7 @@ NVCC_FLAGS = [
     "-O3",
     "-std=c++17",
     "--expt-relaxed-constexpr",
+    "--split-compile=0",  # optimise the many instantiations of one source in parallel
 ] + (["-DLPLB_BOUNDS_CHECK"] if BOUNDS_CHECK else [])
 
 _module = None

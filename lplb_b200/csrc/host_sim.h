@@ -2,7 +2,8 @@
 //
 // When LPLB_HOST_SIM is defined, lp_solver.cuh and lp_block_solver.cuh compile as plain
 // C++: the CUDA function qualifiers vanish and the intrinsics they use (__shfl_sync,
-// __shfl_xor_sync, __all_sync, __syncwarp, __syncthreads, a named barrier) are served by
+// __shfl_xor_sync, __all_sync, __reduce_max_sync, the double-precision matrix instruction,
+// __syncwarp, __syncthreads, a named barrier) are served by
 // host threads that meet at a barrier on every intrinsic.  A warp is 32 threads; a block
 // (run_block) is a set of warps that also share a block-wide and a named barrier, with
 // "shared memory" being an ordinary buffer that the caller passes in.  This works because
@@ -58,6 +59,7 @@ class Barrier {
 struct Warp {
   Barrier barrier{32};
   uint64_t slot[32];
+  double a[32], b[32];
   int pred[32];
 };
 
@@ -95,6 +97,34 @@ inline T exchange(T v, int src_lane) {
   std::memcpy(&out, &raw, sizeof(T));
   return out;
 }
+
+// mma.sync.m8n8k4.f64: lane 4 r + c passes A[r][c], B[c][r] and holds C and D at [r][2 c], [r][2 c + 1].
+inline void mma8(double& d0, double& d1, double a, double b, double c0, double c1) {
+  g_warp->a[g_lane] = a;
+  g_warp->b[g_lane] = b;
+  g_warp->barrier.wait();
+  const int r = g_lane >> 2, n = 2 * (g_lane & 3);
+  for (int k = 0; k < 4; ++k) {
+    c0 = std::fma(g_warp->a[4 * r + k], g_warp->b[4 * n + k], c0);
+    c1 = std::fma(g_warp->a[4 * r + k], g_warp->b[4 * (n + 1) + k], c1);
+  }
+  g_warp->barrier.wait();
+  d0 = c0;
+  d1 = c1;
+}
+struct double2 {
+  double x, y;
+};
+template <typename To, typename From>
+inline To bits(From v) {
+  static_assert(sizeof(To) == sizeof(From), "same size");
+  To out;
+  std::memcpy(&out, &v, sizeof(To));
+  return out;
+}
+inline int hi_word(double x) { return (int)(bits<uint64_t>(x) >> 32); }
+inline int lo_word(double x) { return (int)(uint32_t)bits<uint64_t>(x); }
+inline double from_words(int hi, int lo) { return bits<double>(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo); }
 
 // Run fn(lane) on 32 lock-stepped lanes.
 inline void run_warp(const std::function<void(int)>& fn) {
@@ -160,6 +190,17 @@ inline int __any_sync(unsigned, int pred) {
   lplb_sim::g_warp->barrier.wait();
   return any;
 }
+template <typename T>
+inline T __reduce_max_sync(unsigned, T v) {
+  T best = v;
+  for (int l = 0; l < 32; ++l) {
+    const T other = lplb_sim::exchange(v, l);
+    best = other > best ? other : best;
+  }
+  return best;
+}
+inline int max(int a, int b) { return a > b ? a : b; }
+inline unsigned max(unsigned a, unsigned b) { return a > b ? a : b; }
 inline double rsqrt(double x) { return 1.0 / std::sqrt(x); }
 inline float __fdividef(float a, float b) { return a / b; }
 

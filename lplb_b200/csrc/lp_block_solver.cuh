@@ -1,4 +1,6 @@
-// Thread-block interior-point solver for LP groups of any size (sm_100a).
+// Thread-block interior-point solver for LP groups of any size (sm_100a).  Groups of up to 64 ranks
+// with up to 4 replicas go to the tile solver (lp_tile_solver.cuh) instead, which takes less than half
+// the time.
 //
 // Same LP, same Mehrotra predictor-corrector iteration and same warm-start rule as the warp
 // solver in lp_solver.cuh, organised for groups that do not fit one warp's registers: the

@@ -1,4 +1,6 @@
-// Warp-level interior-point solver for the per-group balancing LP (sm_100a).
+// Warp-level interior-point solver for the per-group balancing LP (sm_100a).  It runs groups of 8
+// ranks where one CTA has more of them than warps, and groups of 16 and 32 ranks on request; all
+// others go to the tile solver (lp_tile_solver.cuh) or the thread-block solver.
 //
 //   min t  s.t.  base_i + sum_k M[i,k] f_k <= t,  0 <= f <= 1
 //
@@ -51,6 +53,9 @@ struct IpmParams {
   // next check after `*stop` (a word in shared memory that another warp sets) becomes
   // non-zero.  Null for every real solve.
   const volatile int* stop = nullptr;
+  // Tile solver, groups of fewer than 8 ranks: the rows up to 8 take part as ranks without load,
+  // as they do in the warp solver.
+  bool pad_rows = false;
 };
 
 struct IpmOutcome {

@@ -43,10 +43,10 @@ struct SolveParams {
   int solver = 0;                // kSolverAuto / kSolverWarp / kSolverBlock
 };
 
-// Two device solvers.  The warp solver keeps a group of up to 32 ranks (up to 4 replicas per
-// rank) in one warp's registers; the thread-block solver takes any group of up to
-// kMaxGroupSize ranks with up to kMaxDup replicas per rank, its matrix in shared memory.
-// kSolverAuto picks the warp solver for groups of up to 8 ranks and the block solver above.
+// What a caller can ask for: one warp per group (up to 32 ranks, up to 4 replicas per rank), or as
+// much of a thread block as the group needs (up to kMaxGroupSize ranks with up to kMaxDup
+// replicas).  kSolverAuto is one warp for groups of up to 8 ranks and the block above.  Which of
+// the three device codes runs a shape is decided in planner_launch.cu.
 enum SolverKind : int { kSolverAuto = 0, kSolverWarp = 1, kSolverBlock = 2 };
 constexpr int kMaxWarpGroupSize = 32;
 constexpr int kMaxWarpDup = 4;

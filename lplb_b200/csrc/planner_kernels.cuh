@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "lp_block_solver.cuh"
 #include "lp_solver.cuh"
+#include "lp_tile_solver.cuh"
 
 namespace lplb {
 
@@ -396,6 +397,53 @@ __device__ __forceinline__ void solve_groups_block(const int* __restrict__ bundl
   }
 }
 
+// Tile solver: NB warps per group, `team_warp` is the calling warp's place among them; the team
+// solves groups first_group, first_group + group_stride, ...  `scratch` is tile_solver_smem_bytes(tp.g, D)
+// of shared memory per team, 16-byte aligned (NB == 1: unused).
+template <int NB, int D>
+__device__ __forceinline__ void solve_groups_tiles(const int* __restrict__ bundle, const Topo& tp, int first_group, int group_stride,
+                                   int team_warp, IpmParams prm, float* __restrict__ probs, Counter avail, int* status,
+                                   double* scratch) {
+  const int lane = threadIdx.x & 31, rank = 8 * team_warp + (lane >> 2);
+  const bool live = rank < tp.g;
+  for (int grp = first_group; grp < tp.n_group; grp += group_stride) {
+    double w[D], fixed = 0.0, f[D];
+    int src[D], dst[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      w[d] = 0.0;
+      src[d] = dst[d] = rank;
+    }
+    if (live) {
+      const int* mine = bundle + ((size_t)grp * tp.g + rank) * (D + 1);
+      fixed = (double)mine[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        w[d] = (double)mine[d];
+        const int s = tp.r2o[rank * D + d], t = tp.o2r[rank * D + d];
+        if (LPLB_CHECKED(s, tp.g, status, kPhSolve) && LPLB_CHECKED(t, tp.g, status, kPhSolve)) {
+          src[d] = s;
+          dst[d] = t;
+        }
+      }
+    }
+    double *anchor = nullptr, *group_anchor = nullptr;
+    int* anchor_valid = nullptr;
+    if (prm.anchor != nullptr) {
+      group_anchor = prm.anchor + (size_t)grp * tp.g * (4 * D + 3);
+      if (live) anchor = group_anchor + (size_t)rank * (4 * D + 3);
+      anchor_valid = prm.anchor_valid + grp;
+    }
+    const IpmOutcome res = ipm_solve_tiles<NB, D>(team_warp, lane, NB == 1 && prm.pad_rows ? 8 : tp.g, w, fixed, src, dst, prm, f,
+                                                  anchor, group_anchor, anchor_valid, scratch);
+    if (live && (lane & 3) == 0) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) probs[((size_t)grp * tp.g + rank) * D + d] = (float)f[d];
+    }
+    if (rank == 0 && lane == 0) report_group(res, grp, avail, status);
+  }
+}
+
 // Counts divided by their maximum, which the Python API returns next to the shares
 // (reference csrc/plugin.cpp:504-506, :577).  Called by one CTA.
 __device__ __forceinline__ void normalise_counts(const int* __restrict__ workload, int e, float* __restrict__ normalised) {
@@ -434,8 +482,6 @@ __global__ void __launch_bounds__(kBlock) solve_kernel(const int* __restrict__ w
     solve_groups<GP, D>(bundle, tp, blockIdx.x * per_cta, gridDim.x * per_cta, prm, probs, avail, status);
 }
 
-// Stand-alone solve kernel, thread-block solver: one CTA per group (the reference launches
-// one block per group too, reference csrc/plugin.cpp:559-565).
 // Shared memory for the bundle sums plus the slack that lets the solver's scratch area start on
 // a 16-byte boundary whatever precedes the sums.
 __host__ __device__ inline size_t bundle_bytes_aligned(int n_ranks, int d) {
@@ -445,6 +491,29 @@ __device__ __forceinline__ double* scratch_after(int* bundle, int n_ranks, int d
   const uintptr_t end = reinterpret_cast<uintptr_t>(bundle + (size_t)n_ranks * (d + 1));
   return reinterpret_cast<double*>((end + 15) & ~(uintptr_t)15);
 }
+
+// Stand-alone solve kernel, tile solver: `teams` groups per CTA (several warps per group: one), and a last
+// CTA that only normalises the counts, beside the solves instead of in front of the first.
+template <int NB, int D>
+__global__ void __launch_bounds__(kBlock) solve_tile_kernel(const int* __restrict__ workload, Topo tp, IpmParams prm,
+                                                            float* __restrict__ probs, float* __restrict__ normalised,
+                                                            Counter avail, int* status, int teams) {
+  if (blockIdx.x == gridDim.x - 1) {
+    normalise_counts(workload, tp.e, normalised);
+    return;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) status[kStLpIters] = status[kStGapPpb] = 0;
+  extern __shared__ __align__(16) int smem[];
+  int* bundle = smem;
+  const int first = (int)blockIdx.x * teams, warp = threadIdx.x >> 5;
+  bundle_sums(workload, tp, bundle, min(tp.n_group, first) * tp.g, min(tp.n_group, first + teams) * tp.g, status);
+  if (warp < teams * NB)
+    solve_groups_tiles<NB, D>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, NB == 1 ? 0 : warp, prm, probs, avail, status,
+                              scratch_after(bundle, tp.n_group * tp.g, tp.d));
+}
+
+// Stand-alone solve kernel, thread-block solver: one CTA per group (the reference launches
+// one block per group too, reference csrc/plugin.cpp:559-565).
 template <int DP>
 __global__ void __launch_bounds__(kBlock) solve_block_kernel(const int* __restrict__ workload, Topo tp, IpmParams prm,
                                                              float* __restrict__ probs,
@@ -719,8 +788,8 @@ __global__ void __launch_bounds__(kBlock) exchange_kernel(const int* __restrict_
 // to run; quotas are exact regardless.  Shared memory: the five E-sized redirect tables
 // (workers) or the statistics vector (solver), the (D + 1) bundle sums per rank, and for
 // GP == 0 the scratch area of the thread-block solver.  GP = 8, 16, 32 selects the warp solver
-// for groups of up to GP ranks, GP = 0 the thread-block solver for any group size; D is the
-// instantiated replica count (>= tp.d when GP == 0).
+// for groups of up to GP ranks, GP = 0 the thread-block solver for any group size, GP = -NB the tile
+// solver with NB warps per group; D is the instantiated replica count (>= tp.d when GP == 0).
 constexpr int kTraceWords = 16;
 
 // Optional phase stamps (globaltimer, ns): 0 solver CTA started, 1 first worker arrived, 2 all
@@ -782,15 +851,15 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
       atomicAdd(&status[kStCalls], 1);
     }
   } else if (warp == 0) {
-    if constexpr (GP != 0) {
+    if constexpr (GP > 0 || GP == -1) {
       // Rehearsal while the workers count: the warp that will solve runs the solver on made-up
       // loads until the counts are in.  Whatever ran since the last step has evicted the
       // solver's code from the caches, the instruction caches included, and one warp running
       // two thousand straight-line instructions per iteration waits for every line of it; here
       // it takes the first of those waits while it has nothing else to do.  Nothing it
       // computes is kept.
-      const int li = lane, g = tp.g;
-      if (lane < GP) {
+      const int li = GP == -1 ? lane >> 2 : lane, g = tp.g;
+      if (GP == -1 || lane < GP) {
       double w[D], f[D];
       int src[D], dst[D];
 #pragma unroll
@@ -802,8 +871,9 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
       }
       IpmParams rehearsal{3, 0.0};
       rehearsal.stop = &s_stop;
-      ipm_solve_segment<GP, D>(li, w, li < g ? 3.0 + 0.2 * li : 0.0, src, dst, rehearsal, f, nullptr, nullptr,
-                               first_lanes(GP));
+      const double fixed = li < g ? 3.0 + 0.2 * li : 0.0;
+      if constexpr (GP == -1) ipm_solve_tiles<1, D>(0, lane, 8, w, fixed, src, dst, rehearsal, f, nullptr, nullptr, nullptr, nullptr);
+      else ipm_solve_segment<GP, D>(li, w, fixed, src, dst, rehearsal, f, nullptr, nullptr, first_lanes(GP));
       }
     }
   }
@@ -847,6 +917,11 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
   team_sync<NT>();
   if constexpr (GP == 0) {
     solve_groups_block<D>(bundle, tp, 0, 1, prm, probs, avail, status, scratch_after(bundle, tp.n_group * tp.g, tp.d));
+  } else if constexpr (GP < 0) {
+    constexpr int kTeams = GP == -1 ? kWarps : 1;  // one group per warp, or one group at a time
+    if (GP == -1 || warp < -GP)
+      solve_groups_tiles<-GP, D>(bundle, tp, GP == -1 ? warp : 0, kTeams, GP == -1 ? 0 : warp, prm, probs, avail, status,
+                                 scratch_after(bundle, tp.n_group * tp.g, tp.d));
   } else {
     solve_groups<GP, D, true>(bundle, tp, 0, (NT / 32) * (32 / GP), prm, probs, avail, status);
   }

@@ -35,11 +35,28 @@ bool shape_ok(const TopoDesc& t, bool need_solver = true, int solver = kSolverAu
   return tables && (!need_solver || resolve_solver(t.g, t.d, solver) > 0);
 }
 
-// Calls fn.template operator()<GP, D>() for the instantiation that covers (g, d): GP = 8, 16,
-// 32 for the warp solver, GP = 0 for the thread-block solver (D is then the padded count).
+// Calls fn.template operator()<GP, D>() for the instantiation that covers the topology: GP = -1, -2, -4,
+// -8 for the tile solver with that many warps per group, 8, 16, 32 for the warp solver, 0 for the
+// thread-block solver (D is then the padded count).  The tile solver takes every group that it
+// covers (8 ranks 22.6 -> 11.3 us a call, 16 ranks 40.6 -> 16.9, 32 ranks 64 -> 27, 64 ranks 147 -> 63 against the
+// other two), except that the warp solver packs four groups of 8 ranks into a warp: `packed` asks for
+// that where one CTA has more groups than warps.  The warp solver's larger groups run on request only.
 template <typename Fn>
-cudaError_t dispatch_shape(int g, int d, int solver, Fn&& fn) {
+cudaError_t dispatch_shape(int g, int d, int solver, bool packed, Fn&& fn) {
   const int kind = resolve_solver(g, d, solver);
+  if (kind != kSolverWarp && kind != kSolverBlock) return cudaErrorInvalidValue;
+  const bool tiles = d <= kTileMaxDup && (kind == kSolverWarp ? g <= 8 && !packed : g <= kTileMaxGroup);
+  if (tiles) {
+    const int nb = tile_rows(g);
+#define LPLB_CASE(NB_, D_) \
+  if (nb == NB_ && d == D_) return fn.template operator()<-NB_, D_>();
+    LPLB_CASE(1, 1) LPLB_CASE(1, 2) LPLB_CASE(1, 3) LPLB_CASE(1, 4)
+    LPLB_CASE(2, 1) LPLB_CASE(2, 2) LPLB_CASE(2, 3) LPLB_CASE(2, 4)
+    LPLB_CASE(4, 1) LPLB_CASE(4, 2) LPLB_CASE(4, 3) LPLB_CASE(4, 4)
+    LPLB_CASE(8, 1) LPLB_CASE(8, 2) LPLB_CASE(8, 3) LPLB_CASE(8, 4)
+#undef LPLB_CASE
+    return cudaErrorInvalidValue;
+  }
   if (kind == kSolverBlock) {
     const int dp = padded_dup(d);
 #define LPLB_CASE(D_) \
@@ -48,7 +65,6 @@ cudaError_t dispatch_shape(int g, int d, int solver, Fn&& fn) {
 #undef LPLB_CASE
     return cudaErrorInvalidValue;
   }
-  if (kind != kSolverWarp) return cudaErrorInvalidValue;
   const int gp = padded_group(g);
 #define LPLB_CASE(GP_, D_) \
   if (gp == GP_ && d == D_) return fn.template operator()<GP_, D_>();
@@ -61,8 +77,15 @@ cudaError_t dispatch_shape(int g, int d, int solver, Fn&& fn) {
 
 size_t fused_smem(int e) { return sizeof(int) * 5 * (size_t)e; }
 size_t bundle_smem(const Topo& tp) { return sizeof(int) * (size_t)tp.n_group * tp.g * (tp.d + 1); }
-// bundle sums followed by the thread-block solver's scratch area
-size_t block_smem(int n_ranks, int g, int d) { return bundle_bytes_aligned(n_ranks, d) + block_solver_smem_bytes(g, padded_dup(d)); }
+// bundle sums followed by the solver's scratch area, if it has one
+template <int GP>
+size_t solver_smem(const Topo& tp) {
+  if constexpr (GP > 0 || GP == -1) return bundle_smem(tp);
+  else return bundle_bytes_aligned(tp.n_group * tp.g, tp.d) +
+              (GP == 0 ? block_solver_smem_bytes(tp.g, padded_dup(tp.d)) : tile_solver_smem_bytes(tp.g, tp.d));
+}
+// The fused kernel's one solver CTA has a warp for each of this many groups of 8 ranks.
+bool pack_groups(const Topo& tp) { return tp.n_group > kWarps; }
 
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
@@ -71,8 +94,10 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-IpmParams make_params(const SolveParams& prm) {
-  return IpmParams{prm.max_iters, prm.tol, prm.anchor, prm.anchor_valid, prm.guard, prm.snap_mu};
+IpmParams make_params(const SolveParams& prm, int g, int d) {
+  IpmParams p{prm.max_iters, prm.tol, prm.anchor, prm.anchor_valid, prm.guard, prm.snap_mu};
+  p.pad_rows = resolve_solver(g, d, prm.solver) == kSolverWarp;
+  return p;
 }
 
 }  // namespace
@@ -115,24 +140,36 @@ struct SolveLaunch {
   cudaStream_t stream;
   template <int GP, int D>
   cudaError_t operator()() const {
-    if constexpr (GP == 0) {
-      const size_t smem = block_smem(tp.n_group * tp.g, tp.g, tp.d);
-      cudaError_t err = allow_smem(solve_block_kernel<D>, smem);
-      if (err != cudaSuccess) return err;
-      solve_block_kernel<D><<<tp.n_group, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status);
+    const size_t smem = solver_smem<GP>(tp);
+    cudaError_t err;
+    if constexpr (GP == 8) {
+      return cudaErrorInvalidValue;  // groups of 8 ranks are packed in the fused kernel only
+    } else if constexpr (GP == 0 || GP < -1) {
+      auto kernel = [] {
+        if constexpr (GP == 0) return solve_block_kernel<D>;
+        else return solve_tile_kernel<-GP, D>;
+      }();
+      if ((err = allow_smem(kernel, smem)) != cudaSuccess) return err;
+      if constexpr (GP == 0) kernel<<<tp.n_group, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status);
+      else kernel<<<tp.n_group + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, 1);
     } else {
       // As few solving warps per CTA as still fit the groups on one wave of CTAs.
+      constexpr int kPerWarp = GP == -1 ? 1 : 32 / GP;
       int dev = 0, sms = 1;
-      cudaError_t err = cudaGetDevice(&dev);
+      err = cudaGetDevice(&dev);
       if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       if (err != cudaSuccess) return err;
       int warps = 1;
-      while (warps < kWarps && (tp.n_group + warps * (32 / GP) - 1) / (warps * (32 / GP)) > sms) warps *= 2;
-      const int per_cta = warps * (32 / GP);
+      while (warps < kWarps && (tp.n_group + warps * kPerWarp - 1) / (warps * kPerWarp) > sms) warps *= 2;
+      const int per_cta = warps * kPerWarp;
       const int grid = (tp.n_group + per_cta - 1) / per_cta;
-      const size_t smem = bundle_smem(tp);
-      if ((err = allow_smem(solve_kernel<GP, D>, smem)) != cudaSuccess) return err;
-      solve_kernel<GP, D><<<grid, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
+      if constexpr (GP == -1) {
+        if ((err = allow_smem(solve_tile_kernel<1, D>, smem)) != cudaSuccess) return err;
+        solve_tile_kernel<1, D><<<grid + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
+      } else {
+        if ((err = allow_smem(solve_kernel<GP, D>, smem)) != cudaSuccess) return err;
+        solve_kernel<GP, D><<<grid, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
+      }
     }
     return cudaGetLastError();
   }
@@ -141,9 +178,9 @@ struct SolveLaunch {
 cudaError_t launch_solve(const int* workload, const TopoDesc& topo, SolveParams prm, float* probs, float* normalised,
                          void* avail, int avail_is64, int* status, cudaStream_t stream) {
   if (!shape_ok(topo, true, prm.solver)) return cudaErrorInvalidValue;
-  SolveLaunch l{workload, make_topo(topo), make_params(prm), probs, normalised, Counter{avail, avail_is64}, status,
+  SolveLaunch l{workload, make_topo(topo), make_params(prm, topo.g, topo.d), probs, normalised, Counter{avail, avail_is64}, status,
                 stream};
-  return dispatch_shape(topo.g, topo.d, prm.solver, l);
+  return dispatch_shape(topo.g, topo.d, prm.solver, false, l);
 }
 
 cudaError_t launch_redirect(const void* idx, int idx_is64, long long n, const float* probs, const int* by_cta,
@@ -196,7 +233,7 @@ struct FusedLaunch {
   template <int GP, int D>
   cudaError_t operator()() {
     auto kernel = fused_run_kernel<GP, D, IdxT>;
-    const size_t smem = fused_smem(tp.e) + (GP == 0 ? block_smem(tp.n_group * tp.g, tp.g, tp.d) : bundle_smem(tp));
+    const size_t smem = fused_smem(tp.e) + solver_smem<GP>(tp);
     cudaError_t err = allow_smem(kernel, smem);
     if (err != cudaSuccess) return err;
     void* args[] = {&idx, &n, &tp, &ex, &prm, &ws, &probs, &avail, &status, &out, &grid_timeout_ns, &trace};
@@ -214,23 +251,24 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
   if (!shape_ok(topo, true, prm.solver) || n_cta < 2 || exd.n_ranks > kMaxRanks) return cudaErrorInvalidValue;
   Exchange ex{exd.recv, exd.n_ranks, exd.my_rank, exd.node_size, exd.timeout_ns};
   if (idx_is64) {
-    FusedLaunch<int64_t> l{static_cast<const int64_t*>(idx), n, make_topo(topo), ex, make_params(prm),
+    FusedLaunch<int64_t> l{static_cast<const int64_t*>(idx), n, make_topo(topo), ex, make_params(prm, topo.g, topo.d),
                            static_cast<Workspace*>(workspace), probs, Counter{avail, avail_is64}, status,
                            static_cast<int64_t*>(out), n_cta, grid_timeout_ns, trace, cooperative, stream};
-    return dispatch_shape(topo.g, topo.d, prm.solver, l);
+    return dispatch_shape(topo.g, topo.d, prm.solver, pack_groups(l.tp), l);
   }
-  FusedLaunch<int32_t> l{static_cast<const int32_t*>(idx), n, make_topo(topo), ex, make_params(prm),
+  FusedLaunch<int32_t> l{static_cast<const int32_t*>(idx), n, make_topo(topo), ex, make_params(prm, topo.g, topo.d),
                          static_cast<Workspace*>(workspace), probs, Counter{avail, avail_is64}, status,
                          static_cast<int32_t*>(out), n_cta, grid_timeout_ns, trace, cooperative, stream};
-  return dispatch_shape(topo.g, topo.d, prm.solver, l);
+  return dispatch_shape(topo.g, topo.d, prm.solver, pack_groups(l.tp), l);
 }
 
 struct OccupancyQuery {
-  size_t smem;
+  Topo tp;
   int is64;
   int* result;
   template <int GP, int D>
   cudaError_t operator()() const {
+    const size_t smem = fused_smem(tp.e) + solver_smem<GP>(tp);
     int per_sm = 0, dev = 0, sms = 0;
     cudaError_t err;
     if (is64) {
@@ -252,10 +290,8 @@ int max_fused_ctas(const TopoDesc& topo, int solver, int idx_is64) {
   int result = 0;
   if (!shape_ok(topo, true, solver)) return 0;
   const Topo tp = make_topo(topo);
-  const bool block = resolve_solver(topo.g, topo.d, solver) == kSolverBlock;
-  OccupancyQuery q{fused_smem(tp.e) + (block ? block_smem(tp.n_group * tp.g, tp.g, tp.d) : bundle_smem(tp)), idx_is64,
-                   &result};
-  if (dispatch_shape(topo.g, topo.d, solver, q) != cudaSuccess) return 0;
+  OccupancyQuery q{tp, idx_is64, &result};
+  if (dispatch_shape(topo.g, topo.d, solver, pack_groups(tp), q) != cudaSuccess) return 0;
   return result;
 }
 

@@ -3,6 +3,7 @@
 #define LPLB_HOST_SIM 1
 #include "lp_block_solver.cuh"
 #include "lp_solver.cuh"
+#include "lp_tile_solver.cuh"
 
 namespace {
 
@@ -85,7 +86,64 @@ void solve_batch_block(int g, int d, const int* r2o, const int* o2r, int nb, con
   }
 }
 
+// The tile solver, NB emulated warps per instance.
+template <int NB, int D>
+void solve_batch_tiles(int g, int rows, const int* r2o, const int* o2r, int nb, const double* w, const double* fixed,
+                       int max_iters, double tol, double* f_out, int* iters, int* converged, double* anchor,
+                       int* anchor_valid, double guard, double snap_mu) {
+  std::vector<double> scratch(lplb::tile_layout(NB, D).total + 2);
+  for (int b = 0; b < nb; ++b) {
+    lplb_sim::run_block(32 * NB, [&](int tid) {
+      const int warp = tid >> 5, lane = tid & 31, rank = 8 * warp + (lane >> 2);
+      const bool live = rank < g;
+      double wl[D], f[D], fx = 0.0;
+      int src[D], dst[D];
+      for (int k = 0; k < D; ++k) {
+        wl[k] = 0.0;
+        src[k] = dst[k] = rank;
+      }
+      if (live) {
+        fx = fixed[(size_t)b * g + rank];
+        for (int k = 0; k < D; ++k) {
+          wl[k] = w[((size_t)b * g + rank) * D + k];
+          src[k] = r2o[rank * D + k];
+          dst[k] = o2r[rank * D + k];
+        }
+      }
+      lplb::IpmParams prm{max_iters, tol, anchor, anchor_valid, guard, snap_mu};
+      double* group = anchor ? anchor + (size_t)b * g * (4 * D + 3) : nullptr;
+      const lplb::IpmOutcome res = lplb::ipm_solve_tiles<NB, D>(
+          warp, lane, rows, wl, fx, src, dst, prm, f, live && anchor ? group + (size_t)rank * (4 * D + 3) : nullptr, group,
+          anchor ? anchor_valid + b : nullptr, scratch.data());
+      if (live && (lane & 3) == 0) {
+        for (int k = 0; k < D; ++k) f_out[((size_t)b * g + rank) * D + k] = f[k];
+        if (rank == 0) {
+          iters[b] = res.iters;
+          converged[b] = res.converged ? 1 : 0;
+        }
+      }
+    });
+  }
+}
+
 }  // namespace
+
+// Tile solver: groups of up to 64 ranks and 4 replicas.  `rows`: ranks that take part, g or (one warp) 8.
+extern "C" int lplb_sim_solve_tiles(int g, int d, int rows, const int* r2o, const int* o2r, int nb, const double* w,
+                                    const double* fixed, int max_iters, double tol, double* f_out, int* iters,
+                                    int* converged, double* anchor, int* anchor_valid, double guard, double snap_mu) {
+  if (g < 1 || g > lplb::kTileMaxGroup || d < 1 || d > lplb::kTileMaxDup) return 1;
+#define LPLB_CASE(NB_, D_)                                                                                          \
+  if (lplb::tile_rows(g) == NB_ && d == D_) {                                                                       \
+    solve_batch_tiles<NB_, D_>(g, rows, r2o, o2r, nb, w, fixed, max_iters, tol, f_out, iters, converged, anchor,    \
+                               anchor_valid, guard, snap_mu);                                                       \
+    return 0;                                                                                                       \
+  }
+  LPLB_CASE(1, 1) LPLB_CASE(1, 2) LPLB_CASE(1, 3) LPLB_CASE(1, 4) LPLB_CASE(2, 1) LPLB_CASE(2, 2) LPLB_CASE(2, 3)
+  LPLB_CASE(2, 4) LPLB_CASE(4, 1) LPLB_CASE(4, 2) LPLB_CASE(4, 4) LPLB_CASE(8, 1) LPLB_CASE(8, 2) LPLB_CASE(8, 3)
+#undef LPLB_CASE
+  return 1;
+}
 
 // Thread-block solver for any group size up to kBlkMaxGroup and up to 8 replicas per rank.
 // anchor [nb][g][4*DP+3] with DP = d for d <= 4, else 8; null for cold solves only.

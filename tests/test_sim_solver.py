@@ -257,3 +257,82 @@ int main() {
                          env=dict(__import__("os").environ, ASAN_OPTIONS="detect_leaks=0"))
     assert run.returncode == 0, run.stdout[-1000:] + run.stderr[-3000:]
     assert "SANITIZED_OK 0" in run.stdout
+
+
+# ---------------------------------------------------------------- tile solver
+def _solve_tiles(lib, r2o, w, fixed, rows=None, max_iters=24, tol=1e-4, anchor=None, valid=None, guard=0.1):
+    g, d = r2o.shape
+    nb = w.shape[0]
+    r = np.ascontiguousarray(r2o.numpy().astype(np.int32))
+    o = np.ascontiguousarray(topology.invert_r2o(r2o).numpy().astype(np.int32))
+    wa = np.ascontiguousarray(w.numpy().astype(np.float64))
+    fa = np.ascontiguousarray(fixed.numpy().astype(np.float64))
+    f = np.zeros((nb, g, d))
+    iters = np.zeros(nb, np.int32)
+    conv = np.zeros(nb, np.int32)
+    ptr = lambda a: None if a is None else ctypes.c_void_p(a.ctypes.data)  # noqa: E731
+    rc = lib.lplb_sim_solve_tiles(g, d, rows or g, ptr(r), ptr(o), nb, ptr(wa), ptr(fa), max_iters, ctypes.c_double(tol),
+                                  ptr(f), ptr(iters), ptr(conv), ptr(anchor), ptr(valid), ctypes.c_double(guard),
+                                  ctypes.c_double(1e-3))
+    assert rc == 0
+    return torch.from_numpy(f), iters, conv
+
+
+@pytest.mark.parametrize("g,offsets", [
+    (2, (1,)), (5, (1,)), (8, (1, 4)), (8, (1, 2, 3, 4)), (9, (1, 2)), (16, (3, 8)), (16, (1, 2, 3, 4)), (17, (1,)),
+    (32, (1, 16)), (33, (1, 2)), (64, (1, 8)),
+])
+def test_tile_solver_device_code_matches_the_torch_restatement(sim, g, offsets):
+    """Group sizes at the edges of the tile counts (1, 2, 4 and 8 warps), with rows that are only padding, and
+    offsets of half the group, whose two terms fall into one column of the normal matrix.  The
+    iterates differ by the rounding of the step lengths (2^-26, times at most seven iterations and
+    the conditioning of the last ones); 1e-5 is what the other solvers are held to."""
+    r2o = topology.circulant(g, offsets)
+    d = r2o.shape[1]
+    gen = torch.Generator().manual_seed(7)
+    cnt = ((torch.randn(1, g, d + 6, generator=gen, dtype=torch.float64) * 0.3 + 1).clamp_min(0) * 4096).floor()
+    w, fixed = cnt[:, :, :d].contiguous(), cnt[:, :, d:].sum(-1)
+    f, iters, conv = _solve_tiles(sim, r2o, w, fixed)
+    ref = lp.solve_ipm(w, fixed, r2o, tol=1e-4)
+    assert conv.all() and bool(((f >= 0) & (f <= 1)).all())
+    assert iters.tolist() == ref.iters.tolist()
+    assert float((f - ref.f).abs().max()) < 1e-5
+    if g < 8 and d == 1:  # with the padding rows taking part, as in the warp solver
+        f8, it8, _ = _solve_tiles(sim, r2o, w, fixed, rows=8)
+        ref8, ref_it, _ = _solve(sim, r2o, w, fixed)
+        assert it8.tolist() == ref_it.tolist() and float((f8 - ref8).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("name", ["cube", "ring5", "hypercube"])
+def test_tile_solver_warm_start_follows_the_torch_restatement(sim, name):
+    r2o = topology.by_name(name)
+    g, d = r2o.shape
+    gen = torch.Generator().manual_seed(13)
+    mean = (torch.rand(g, 8, generator=gen, dtype=torch.float64) + 0.5) * 4096
+    anchor_c, valid_c, anchor_t = np.zeros((1, g, 4 * d + 3)), np.zeros(1, np.int32), None
+    seen = []
+    for step in range(4):
+        if step == 3:
+            mean = mean.flip(0) * torch.linspace(0.3, 2.0, 8, dtype=torch.float64)
+        cnt = (mean * (1 + 0.02 * torch.randn(g, 8, generator=gen, dtype=torch.float64))).floor().unsqueeze(0)
+        w, fixed = cnt[:, :, :d].contiguous(), cnt[:, :, d:].sum(-1)
+        ref = lp.solve_ipm(w, fixed, r2o, tol=1e-4, warm_start=True, anchor=anchor_t, guard=0.1)
+        anchor_t = ref.anchor
+        f, iters, conv = _solve_tiles(sim, r2o, w, fixed, anchor=anchor_c, valid=valid_c)
+        assert conv[0] == 1 and int(iters[0]) == int(ref.iters[0])
+        assert float((f - ref.f).abs().max()) < 1e-5
+        seen.append((bool(ref.warm[0]), int(iters[0])))
+    assert [s[0] for s in seen] == [False, True, True, name == "ring5"]  # the small shift of five loads stays in the guard
+    assert seen[1][1] < seen[0][1]
+
+
+def test_tile_solver_handles_empty_groups_and_the_iteration_cap(sim):
+    for r2o in (topology.cube(), topology.hypercube()):
+        g, d = r2o.shape
+        zero = torch.zeros(1, g, d, dtype=torch.float64)
+        f, iters, conv = _solve_tiles(sim, r2o, zero, zero[:, :, 0])
+        assert conv[0] == 1 and iters[0] == 0 and torch.equal(f, torch.ones(1, g, d, dtype=torch.float64))
+        w = torch.rand(1, g, d, dtype=torch.float64, generator=torch.Generator().manual_seed(1)) * 1000
+        fixed = torch.rand(1, g, dtype=torch.float64, generator=torch.Generator().manual_seed(2)) * 1000
+        f, iters, conv = _solve_tiles(sim, r2o, w, fixed, max_iters=1, tol=1e-9)
+        assert conv[0] == 0 and iters[0] == 1 and bool(((f >= 0) & (f <= 1)).all())
