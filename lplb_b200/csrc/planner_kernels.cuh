@@ -495,7 +495,7 @@ __device__ __forceinline__ double* scratch_after(int* bundle, int n_ranks, int d
 // Stand-alone solve kernel, tile solver: `teams` groups per CTA (several warps per group: one), and a last
 // CTA that only normalises the counts, beside the solves instead of in front of the first.
 template <int NB, int D>
-__global__ void __launch_bounds__(kBlock) solve_tile_kernel(const int* __restrict__ workload, Topo tp, IpmParams prm,
+__global__ void __launch_bounds__(kBlock) tile_solve_kernel(const int* __restrict__ workload, Topo tp, IpmParams prm,
                                                             float* __restrict__ probs, float* __restrict__ normalised,
                                                             Counter avail, int* status, int teams) {
   if (blockIdx.x == gridDim.x - 1) {

@@ -147,7 +147,7 @@ struct SolveLaunch {
     } else if constexpr (GP == 0 || GP < -1) {
       auto kernel = [] {
         if constexpr (GP == 0) return solve_block_kernel<D>;
-        else return solve_tile_kernel<-GP, D>;
+        else return tile_solve_kernel<-GP, D>;
       }();
       if ((err = allow_smem(kernel, smem)) != cudaSuccess) return err;
       if constexpr (GP == 0) kernel<<<tp.n_group, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status);
@@ -164,8 +164,8 @@ struct SolveLaunch {
       const int per_cta = warps * kPerWarp;
       const int grid = (tp.n_group + per_cta - 1) / per_cta;
       if constexpr (GP == -1) {
-        if ((err = allow_smem(solve_tile_kernel<1, D>, smem)) != cudaSuccess) return err;
-        solve_tile_kernel<1, D><<<grid + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
+        if ((err = allow_smem(tile_solve_kernel<1, D>, smem)) != cudaSuccess) return err;
+        tile_solve_kernel<1, D><<<grid + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
       } else {
         if ((err = allow_smem(solve_kernel<GP, D>, smem)) != cudaSuccess) return err;
         solve_kernel<GP, D><<<grid, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
