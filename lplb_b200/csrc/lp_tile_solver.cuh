@@ -16,8 +16,9 @@
 //     tile a sweep takes two pivots at a time (one reciprocal, of the 2 x 2 determinant); between
 //     tiles it takes a whole 8 x 8 tile, and the warp that owns the next pivot tile inverts it
 //     while the others still update theirs.
-//   * Warp I holds tile row I and is the ranks 8 I .. 8 I + 7, four lanes each with the same
-//     values.  With one warp nothing goes through shared memory and there is no barrier.
+//   * Warp I holds tile row I and is the ranks 8 I .. 8 I + 7, four lanes each; a lane is one of the
+//     rank's edges, so that no instruction is spent once per edge (8 ranks 11.3 -> 10.3 us, with
+//     the sweep below).  With one warp there is no barrier.
 //   * Sums over ranks are two matrix instructions by a matrix of ones for two sums at a time
 //     (65 cycles; three rounds of shuffles take 96 for one).
 //   * Maxima are taken on integers that order like the doubles they stand for.
@@ -25,9 +26,9 @@
 //     corrector's step is linear in it.
 //
 // Solve kernel, two replicas per rank, unrelated instances, us a call back to back (the warp solver
-// for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 11.3, 64 groups of 8 ranks
-// 26.2 -> 13.1, 16 ranks 40.6 -> 16.9, 32 ranks 64.4 -> 27.4, 64 ranks 147 -> 63.  An iteration: 8 ranks 3.5 -> 1.5,
-// 64 ranks 22.5 -> 9.4 us.
+// for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 10.3, 64 groups of 8 ranks
+// 26.2 -> 11.8, 16 ranks 40.6 -> 17.0, 32 ranks 64.4 -> 25.4, 64 ranks 147 -> 52.  An iteration: 8 ranks 3.5 -> 1.2,
+// 64 ranks 22.5 -> 7.4 us.
 #pragma once
 
 #include "lp_solver.cuh"
@@ -121,69 +122,98 @@ __device__ __forceinline__ double warp_max_positive(double x) {
 // -U P, columns of the pivots pass -1 at their own place as operand B and all others U, and
 // the accumulator is zero in both.  (k = 2, 3 of the instruction stay empty.)  A pivot block
 // that rounding drove singular counts as infinite: its unknowns become zero in the solves.
-__device__ __forceinline__ void sweep_tile(double& n0, double& n1, int lane) {
+//
+// A sweep is one dependent chain: block, determinant, reciprocal, matrix instruction.  The tile goes
+// through shared memory, where every lane reads just the elements that it needs, zeros and ones
+// included, because the ten shuffles and the selections between their results take longer:
+// 641 cycles for the four sweeps, with shuffles 715 to 930, with the next pivot block computed ahead of
+// the matrix instruction 710 to 1000 (more instructions on the same warp).
+// `scratch`: kSweepScratch doubles per warp, prepared by sweep_scratch_init.
+constexpr int kSweepZero = 128, kSweepOne = 144, kSweepScratch = 146;
+__device__ __forceinline__ void sweep_scratch_init(double* scratch, int lane) {
+  if (lane < kSweepScratch - kSweepZero) scratch[kSweepZero + lane] = lane == kSweepOne - kSweepZero ? -1.0 : 0.0;
+  __syncwarp();
+}
+__device__ __forceinline__ void sweep_tile(double& n0, double& n1, int lane, double* scratch) {
   const int r = lane >> 2, c = lane & 3;
-  const bool odd = c & 1, used = c < 2;
+  const bool odd = c & 1, used = c < 2, own = (r & 1) == (c & 1);
+  // offsets in `scratch` of this lane's element of U in its own column, of the other one, of the opposite
+  // diagonal element of the pivot block, and of what replaces the first two in the pivots' rows
+  const int mine_at = used ? 2 * (lane & 28) + odd : kSweepZero, other_at = used ? 2 * (lane & 28) + !odd : kSweepZero;
+  const int opposite_at = odd ? 0 : 9;
+  const int mine_pivot = kSweepOne + !(used && own), other_pivot = kSweepOne + !(used && !own);
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
-    const double u0 = lane_get(n0, (lane & 28) | h), u1 = lane_get(n1, (lane & 28) | h);
-    const double a = lane_get(n0, 9 * h), b = lane_get(n1, 9 * h), d = lane_get(n1, 9 * h + 4);
-    const double det = fma(a, d, -(b * b));
-    const double inv = rcp3(det);
+    const int copy = (h & 1) * 64;
+    double* tile = scratch + copy;
+    *reinterpret_cast<double2*>(tile + 2 * lane) = double2{n0, n1};
+    __syncwarp();
+    const bool pivot = (r >> 1) == h;
+    const double2 ab = *reinterpret_cast<const double2*>(tile + 18 * h);  // the block is a b / b d
+    const double d = tile[18 * h + 9], opposite = tile[18 * h + opposite_at];
+    const double mine = scratch[pivot ? mine_pivot : mine_at + 2 * h + (used ? copy : 0)];
+    const double other = scratch[pivot ? other_pivot : other_at + 2 * h + (used ? copy : 0)];
+    const double det = fma(ab.x, d, -(ab.y * ab.y)), inv = rcp3(det);
     const bool ok = (unsigned)(hi_word(det) - 0x01000000) < 0x7E000000u;  // a positive, finite number
-    const bool pivot = (r >> 1) == h, own = (r & 1) == (c & 1);
-    const double mine = odd ? u1 : u0, other = odd ? u0 : u1, p = odd ? a : d;
-    double num = fma(other, b, -(mine * p));
-    if (pivot) num = own ? p : -b;
-    double bop = pivot ? (own ? -1.0 : 0.0) : mine;
-    num = used ? num : 0.0;
-    bop = used ? bop : 0.0;
+    const double num = fma(other, ab.y, -(mine * opposite));
+    const double scale = from_words(ok ? hi_word(inv) : 0, lo_word(inv));  // finite, and times zero if not ok
     const bool fresh = pivot || c == h;
-    mma8(n0, n1, num * (ok ? inv : 0.0), bop, fresh ? 0.0 : n0, fresh ? 0.0 : n1);
+    mma8(n0, n1, (ok ? num : 0.0) * scale, mine, fresh ? 0.0 : n0, fresh ? 0.0 : n1);
   }
 }
 
 // ---- exchange between ranks -----------------------------------------------------------------
-// With one warp a value of another rank is a shuffle away; otherwise it is published in a
-// shared-memory vector, one vector per use so that one barrier per use suffices.
-enum TileVec : int {  // after the D-fold vectors
-  kVecY, kVecComp, kVecDual, kVecLoad, kVecG, kVecG1, kVecX, kVecX1, kVecBorder, kVecCp, kVecCpd, kVecG0, kVecX0, kVecMisc, kVecCount
-};
-constexpr int kTileFold = 5;  // D-fold vectors: w f, theta w^2, and the products of the three right-hand sides
+// Every rank has up to four lanes; lane c is its edge c % L, L = 1, 2 or 4 (of three edges the fourth is
+// a dummy that carries no load).  With one warp a value of another rank is a shuffle away;
+// otherwise it is published in a shared-memory vector, one vector per use so that one barrier
+// per use suffices.
+enum TileVec : int { kVecY, kVecG, kVecG1, kVecX, kVecX1, kVecBorder, kVecG0, kVecX0, kVecCount };  // per rank
+enum TileEdgeVec : int { kEdgeF, kEdgeCw, kEdgeRhs, kEdgeOne, kEdgeCor, kEdgeCount };               // per edge
+enum TileSum : int { kSumStart, kSumCold, kSumMu, kSumDual, kSumX, kSumX1, kSumAffine, kSumX0, kSumCount };
+enum TileMax : int { kMaxLoad, kMaxDown, kMaxCount };
+constexpr int kTileKeys = 4;
 
 struct TileLayout {
-  int rows_mat, u, pi, vec, keys, total;  // in doubles
+  int sweep, rows_mat, u, pi, vec, edge, sums, maxes, keys, total;  // in doubles; every part starts on 16 bytes
 };
 __host__ __device__ constexpr TileLayout tile_layout(int nb, int d) {
   TileLayout l{};
-  if (nb == 1) return l;
-  const int n = 8 * nb;
+  const int n = 8 * nb, many = nb > 1;
   int o = 0;
-  l.rows_mat = o, o += nb * nb * 64;  // normal matrix, tile by tile (16-byte aligned)
-  l.u = o, o += 2 * nb * 64;          // pivot columns, two alternating copies
-  l.pi = o, o += 2 * 64;              // minus the inverse of the pivot tile, likewise
-  l.vec = o, o += (kTileFold * d + kVecCount) * n;
-  l.keys = o, o += 2 * nb;         // unsigned: four keys per warp
+  l.sweep = o, o += nb * kSweepScratch;
+  l.rows_mat = o, o += many * nb * nb * 64;  // normal matrix, tile by tile
+  l.u = o, o += many * 2 * nb * 64;          // pivot columns, two alternating copies
+  l.pi = o, o += many * 2 * 64;              // minus the inverse of the pivot tile, likewise
+  l.vec = o, o += many * kVecCount * n;
+  l.edge = o, o += many * kEdgeCount * d * n;
+  l.sums = o, o += many * kSumCount * nb * 2;
+  l.maxes = o, o += many * kMaxCount * nb;
+  l.keys = o, o += many * kTileKeys * nb / 2;  // unsigned
   l.total = o;
   return l;
 }
-__host__ __device__ inline size_t tile_solver_smem_bytes(int g, int d) {
-  return sizeof(double) * (size_t)tile_layout(tile_rows(g), d).total;
+// Shared memory of `teams` groups solved side by side by one CTA.
+__host__ __device__ inline size_t tile_solver_smem_bytes(int g, int d, int teams = 1) {
+  return sizeof(double) * (size_t)tile_layout(tile_rows(g), d).total * teams;
 }
 
 template <int NB, int D>
 struct TileTeam {
-  int warp, lane, r, c, rank;
+  static constexpr int kRanks = 8 * NB, kLanes = D == 3 ? 4 : D;  // distinct lanes per rank
+  static constexpr TileLayout kLay = tile_layout(NB, D);
+  int warp, lane, r, c, edge, rank;
   double* sm;
-  static constexpr int kRanks = 8 * NB;
   __device__ __forceinline__ TileTeam(int warp_, int lane_, double* sm_)
-      : warp(warp_), lane(lane_), r(lane_ >> 2), c(lane_ & 3), rank(8 * warp_ + (lane_ >> 2)), sm(sm_) {}
-  __device__ __forceinline__ double* vec(int v) const { return sm + tile_layout(NB, D).vec + (kTileFold * D + v) * kRanks; }
-  __device__ __forceinline__ double* fold(int v, int d) const { return sm + tile_layout(NB, D).vec + (v * D + d) * kRanks; }
-  __device__ __forceinline__ unsigned* keys() const { return reinterpret_cast<unsigned*>(sm + tile_layout(NB, D).keys); }
-  __device__ __forceinline__ double2* mat() const { return reinterpret_cast<double2*>(sm + tile_layout(NB, D).rows_mat) + warp * NB * 32; }
-  __device__ __forceinline__ double2* pivot_col(int parity) const { return reinterpret_cast<double2*>(sm + tile_layout(NB, D).u) + parity * NB * 32; }
-  __device__ __forceinline__ double2* pivot_inv(int parity) const { return reinterpret_cast<double2*>(sm + tile_layout(NB, D).pi) + parity * 32; }
+      : warp(warp_), lane(lane_), r(lane_ >> 2), c(lane_ & 3), edge(lane_ & (kLanes - 1)), rank(8 * warp_ + (lane_ >> 2)), sm(sm_) {}
+  __device__ __forceinline__ double* sweep() const { return sm + kLay.sweep + warp * kSweepScratch; }
+  __device__ __forceinline__ double* vec(int v) const { return sm + kLay.vec + v * kRanks; }
+  __device__ __forceinline__ double* edges(int v) const { return sm + kLay.edge + (v * D + (edge < D ? edge : 0)) * kRanks; }
+  __device__ __forceinline__ double2* sums(int v) const { return reinterpret_cast<double2*>(sm + kLay.sums) + v * NB; }
+  __device__ __forceinline__ double* maxes(int v) const { return sm + kLay.maxes + v * NB; }
+  __device__ __forceinline__ unsigned* keys(int v) const { return reinterpret_cast<unsigned*>(sm + kLay.keys) + v * NB; }
+  __device__ __forceinline__ double2* mat() const { return reinterpret_cast<double2*>(sm + kLay.rows_mat) + warp * NB * 32; }
+  __device__ __forceinline__ double2* pivot_col(int parity) const { return reinterpret_cast<double2*>(sm + kLay.u) + parity * NB * 32; }
+  __device__ __forceinline__ double2* pivot_inv(int parity) const { return reinterpret_cast<double2*>(sm + kLay.pi) + parity * 32; }
 
   __device__ __forceinline__ void sync() const {
     if constexpr (NB > 1) {
@@ -194,55 +224,96 @@ struct TileTeam {
 #endif
     }
   }
-  __device__ __forceinline__ void put(double* where, double v) const {
+  __device__ __forceinline__ void put(int v, double x) const {
     if constexpr (NB > 1) {
-      if (c == 0) where[rank] = v;
+      if (c == 0) vec(v)[rank] = x;
     }
   }
-  __device__ __forceinline__ double get(const double* where, double mine, int of) const {
-    if constexpr (NB > 1) return where[of];
+  __device__ __forceinline__ double get(int v, double mine, int of) const {
+    if constexpr (NB > 1) return vec(v)[of];
     else return lane_get(mine, 4 * of);
   }
-  // Sums over the ranks of two values; (va, vb) hold them where they have been published.
-  __device__ __forceinline__ void sum2(const double* va, double a, const double* vb, double b, double& sa, double& sb) const {
-    double d0, d1;
-    if constexpr (NB == 1) {
-      // lanes of one rank hold the same values: every other one passes b
-      mma8(d0, d1, c == (r & 1) ? 1.0 : 0.0, (c & 1) ? b : a, 0.0, 0.0);  // even rows: all ranks' a, odd rows: their b
-      mma8(sa, sb, 1.0, d0 + d1, 0.0, 0.0);
-    } else {
-      const double* v = (r & 1) ? vb : va;
-      const int first = (r >> 1) * 4 + c;
-      double acc = v[first];
-#pragma unroll
-      for (int k = 16; k < kRanks; k += 16) acc += v[first + k];
-      mma8(d0, d1, 1.0, acc, 0.0, 0.0);
-      mma8(sa, sb, 1.0, (r & 1) ? d1 : d0, 0.0, 0.0);
-    }
-  }
-  __device__ __forceinline__ double max_positive(const double* where, double x) const {
+  // the same edge of another rank
+  __device__ __forceinline__ void put_edge(int v, double x) const {
     if constexpr (NB > 1) {
-      x = where[lane % kRanks];
-      if constexpr (kRanks > 32) {
-        const double other = where[lane + 32];
-        // positive doubles order like their bit patterns, negative ones lie below
-        const bool more = hi_word(other) > hi_word(x) ||
-                          (hi_word(other) == hi_word(x) && (unsigned)lo_word(other) > (unsigned)lo_word(x));
-        x = more ? other : x;
-      }
+      if (c < D) edges(v)[rank] = x;
     }
-    return warp_max_positive(x);
   }
-  // Largest key over the ranks, in two halves around a barrier.
+  __device__ __forceinline__ double get_edge(int v, double mine, int of) const {
+    if constexpr (NB > 1) return edges(v)[of];
+    else return lane_get(mine, 4 * of + c);
+  }
+  // Sum over the rank's edges, on all its lanes.
+  __device__ __forceinline__ double edge_sum(double x) const {
+    if constexpr (D == 1) return x;
+    double sum, same;
+    mma8(sum, same, x, c < D ? 1.0 : 0.0, 0.0, 0.0);
+    return sum;
+  }
+  // Sums over all lanes of all ranks (copies of an edge count once) of two values, in two halves around a barrier.
+  __device__ __forceinline__ void sum_put(int slot, double& a, double& b) const {
+    double d0, d1, s;
+    if constexpr (kLanes <= 2) {
+      // lanes with copies pass b instead: even rows of the product are the ranks' a, odd rows their b
+      const int half = kLanes == 1 ? c : c >> 1;
+      mma8(d0, d1, half == (r & 1) ? 1.0 : 0.0, (half & 1) ? b : a, 0.0, 0.0);
+      s = d0 + d1;
+    } else {
+      double e0, e1;
+      mma8(d0, d1, 1.0, a, 0.0, 0.0);
+      mma8(e0, e1, 1.0, b, 0.0, 0.0);
+      s = (r & 1) ? e0 + e1 : d0 + d1;
+    }
+    mma8(a, b, 1.0, s, 0.0, 0.0);
+    if constexpr (NB > 1) {
+      if (lane == 0) sums(slot)[warp] = double2{a, b};
+    }
+  }
+  __device__ __forceinline__ void sum_put(int slot, double& a) const {
+    double none = 0.0;
+    sum_put(slot, a, none);
+  }
+  __device__ __forceinline__ void sum_get(int slot, double& a) const {
+    double none = 0.0;
+    sum_get(slot, a, none);
+  }
+  __device__ __forceinline__ void sum_get(int slot, double& a, double& b) const {
+    if constexpr (NB > 1) {
+      double2 v[NB];
+#pragma unroll
+      for (int k = 0; k < NB; ++k) v[k] = sums(slot)[k];
+#pragma unroll
+      for (int o = NB / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; ++k) {
+          v[k].x += v[k + o].x;
+          v[k].y += v[k + o].y;
+        }
+      a = v[0].x;
+      b = v[0].y;
+    }
+  }
+  // Largest value, exactly; it must be positive.
+  __device__ __forceinline__ double max_put(int slot, double x) const {
+    x = warp_max_positive(x);
+    if constexpr (NB > 1) {
+      if (lane == 0) maxes(slot)[warp] = x;
+    }
+    return x;
+  }
+  __device__ __forceinline__ double max_get(int slot, double x) const {
+    if constexpr (NB > 1) x = warp_max_positive(maxes(slot)[lane % NB]);
+    return x;
+  }
   __device__ __forceinline__ unsigned key_put(int slot, unsigned key) const {
     key = __reduce_max_sync(0xffffffffu, key);
     if constexpr (NB > 1) {
-      if (lane == 0) keys()[slot * NB + warp] = key;
+      if (lane == 0) keys(slot)[warp] = key;
     }
     return key;
   }
   __device__ __forceinline__ unsigned key_get(int slot, unsigned key) const {
-    if constexpr (NB > 1) key = __reduce_max_sync(0xffffffffu, keys()[slot * NB + lane % NB]);
+    if constexpr (NB > 1) key = __reduce_max_sync(0xffffffffu, keys(slot)[lane % NB]);
     return key;
   }
   __device__ __forceinline__ bool all(int slot, bool ok) const {  // several warps: key_put(slot, !ok) and a barrier before
@@ -259,11 +330,11 @@ struct TileTeam {
 template <int NB, int D>
 __device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (&n0)[NB], double (&n1)[NB]) {
   if constexpr (NB == 1) {
-    sweep_tile(n0[0], n1[0], tm.lane);
+    sweep_tile(n0[0], n1[0], tm.lane, tm.sweep());
   } else {
     if (tm.warp == 0) {
       double p0 = n0[0], p1 = n1[0];
-      sweep_tile(p0, p1, tm.lane);
+      sweep_tile(p0, p1, tm.lane, tm.sweep());
       tm.pivot_inv(0)[tm.lane] = double2{p0, p1};
     }
 #pragma unroll 1
@@ -287,11 +358,11 @@ __device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (
         n1[j - 1] = d1;
       };
       update(1);
-      if (tm.warp == p + 1) {  // the next pivot tile is ready: invert it beside the other updates
+      if (tm.warp == p + 1) {
+        // The next pivot tile is ready: invert it while the others update theirs.  (The other tiles of
+        // this row are due to be replaced by P U_J^T, so they need no update: 62 -> 52 us at 64 ranks.)
         double p0 = n0[0], p1 = n1[0];
-        sweep_tile(p0, p1, tm.lane);
-#pragma unroll
-        for (int j = 2; j < NB; ++j) update(j);
+        sweep_tile(p0, p1, tm.lane, tm.sweep());
         tm.pivot_inv((p + 1) & 1)[tm.lane] = double2{p0, p1};
       } else {
 #pragma unroll
@@ -304,39 +375,34 @@ __device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (
 }
 
 // One group of at most 8 NB ranks, solved by NB warps (all of them call; `warp` counts from 0 within the
-// group).  Lane 4 r + c of warp I is rank 8 I + r and passes that rank's data, as in ipm_solve_segment;
-// ranks from `rows` on do not take part (w = 0, fixed = 0, src = dst = the rank itself, no anchor).
-// `sm`: tile_solver_smem_bytes of shared memory, 16-byte aligned (one warp: unused).  `anchor`:
-// the rank's slot of the warm-start state or null; `group_anchor` the slot of the group's first rank.
-// The outcome is the same on every lane.
+// group).  Lane 4 r + c of warp I is edge c of rank 8 I + r (see above) and passes that bundle's load, the
+// rank's non-replicated load, and the ranks whose bundle it holds (`src`) and that hold its own (`dst`); dummies
+// and ranks from `rows` on, which do not take part, pass no load and themselves.  All four lanes of a
+// rank pass `mine`, the rank's whole own load.  `sm`: tile_solver_smem_bytes of shared memory, 16-byte
+// aligned.  `anchor`: the rank's slot of the warm-start state or null; `group_anchor` the slot of the
+// group's first rank.  The outcome is the same on every lane, the share is the lane's own.
 template <int NB, int D>
-__device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int lane, const int rows,
-                                                      const double (&w_in)[D], const double fixed,
-                                                      const int (&src_in)[D], const int (&dst_in)[D],
-                                                      const IpmParams prm, double (&f_out)[D], double* anchor,
+__device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int lane, const int rows, const double w_in,
+                                                      const double fixed, const double own_load, const int src,
+                                                      const int dst, const IpmParams prm, double& f_out, double* anchor,
                                                       const double* group_anchor, int* anchor_valid, double* sm) {
   constexpr double kEta = 0.995;
   const TileTeam<NB, D> tm(warp, lane, sm);
   const int c = tm.c, rank = tm.rank;
-  const bool live = rank < rows;
-  int src[D], dst[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    src[d] = src_in[d];
-    dst[d] = dst_in[d];
-  }
+  const bool live = rank < rows, real = tm.edge < D;
+  const bool first = tm.edge == 0;  // the lane that adds the rank's own part to sums over lanes
+  sweep_scratch_init(tm.sweep(), lane);
   // The saved iterate is read first, valid or not (the slot is always allocated): its loads are
   // in flight while the scaling is computed.
-  double fa[D], va[D], za[D], qa[D], sa = 1.0, ya = 0.0, ta = 0.0;
   const bool slot = anchor != nullptr && live;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    fa[d] = slot ? anchor[d] : 0.5;
-    va[d] = slot ? anchor[D + d] : 0.5;
-    za[d] = slot ? anchor[2 * D + d] : 1.0;
-    qa[d] = slot ? anchor[3 * D + d] : 1.0;
-  }
+  double fa = 0.5, va = 0.5, za = 1.0, qa = 1.0, sa = 1.0, ya = 0.0, ta = 0.0;
   if (slot) {
+    if (real) {
+      fa = anchor[tm.edge];
+      va = anchor[D + tm.edge];
+      za = anchor[2 * D + tm.edge];
+      qa = anchor[3 * D + tm.edge];
+    }
     sa = anchor[4 * D];
     ya = anchor[4 * D + 1];
   }
@@ -346,78 +412,64 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
   const double kcomp = (double)(rows + 2 * rows * D), inv_kcomp = rcp3(kcomp), inv_rows = rcp3((double)rows);
 
   // ---- where this lane's off-diagonal terms of the matrix go -----------------------------------
-  // One warp: factors 0 or -1 for the lane's two columns.  Several: places in the tile row, written
-  // once per iteration; terms that share a column are merged (the first collects the later ones).
+  // One warp: factors 0 or -1 of all the rank's terms for the lane's two columns.  Several: the places of the
+  // lane's two terms in the tile row, written once per iteration.  Terms of a rank that share a
+  // column are merged, in one order, so that whoever writes such a place writes the same.
   double cd[NB == 1 ? D : 1][2], cs[NB == 1 ? D : 1][2];
-  double* place[NB > 1 ? 2 * D : 1];
-  unsigned merge = 0;  // bit a * 2 D + b: term b > a goes to term a's place
-  double* diag_place = nullptr;
-  if constexpr (NB == 1) {
-#pragma unroll
-    for (int d = 0; d < D; ++d)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        cd[d][e] = dst[d] == 2 * c + e ? -1.0 : 0.0;
-        cs[d][e] = src[d] == 2 * c + e ? -1.0 : 0.0;
-      }
-  } else {
-    static_assert(kTileMaxDup <= 4, "the pairs of terms share one word: (2 D)^2 bits with a < b");
-    double2* mat = tm.mat();
-    for (int j = 0; j < NB; ++j) mat[j * 32 + lane] = double2{0.0, 0.0};
-    auto at = [&](int col) { return reinterpret_cast<double*>(mat) + ((col >> 3) * 32 + 4 * tm.r + ((col & 7) >> 1)) * 2 + (col & 1); };
-    int col[2 * D];
+  double *place_dst = nullptr, *place_src = nullptr, *place_diag = nullptr;
+  unsigned same_dst = 0, same_src = 0;  // bit 2 d: the dst term of edge d shares the column, bit 2 d + 1: its src term
+  {
+    int all_dst[D], all_src[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      col[2 * d] = dst[d];
-      col[2 * d + 1] = src[d];
+      all_dst[d] = __shfl_sync(0xffffffffu, dst, (lane & 28) | d);
+      all_src[d] = __shfl_sync(0xffffffffu, src, (lane & 28) | d);
     }
-    int bit = 0;
+    if constexpr (NB == 1) {
 #pragma unroll
-    for (int a = 0; a < 2 * D; ++a) {
-      bool first = col[a] != rank && live && c == 0;
+      for (int d = 0; d < D; ++d)
 #pragma unroll
-      for (int b = 0; b < a; ++b)
-        if (col[b] == col[a]) first = false;
+        for (int e = 0; e < 2; ++e) {
+          cd[d][e] = all_dst[d] == 2 * c + e ? -1.0 : 0.0;
+          cs[d][e] = all_src[d] == 2 * c + e ? -1.0 : 0.0;
+        }
+    } else {
+      double2* mat = tm.mat();
+      for (int j = 0; j < NB; ++j) mat[j * 32 + lane] = double2{0.0, 0.0};
+      auto at = [&](int col) { return reinterpret_cast<double*>(mat) + ((col >> 3) * 32 + 4 * tm.r + ((col & 7) >> 1)) * 2 + (col & 1); };
 #pragma unroll
-      for (int b = a + 1; b < 2 * D; ++b, ++bit)
-        if (col[b] == col[a]) merge |= 1u << bit;
-      place[a] = first ? at(col[a]) : nullptr;
+      for (int d = 0; d < D; ++d) {
+        same_dst |= (all_dst[d] == dst ? 1u : 0u) << (2 * d) | (all_src[d] == dst ? 2u : 0u) << (2 * d);
+        same_src |= (all_dst[d] == src ? 1u : 0u) << (2 * d) | (all_src[d] == src ? 2u : 0u) << (2 * d);
+      }
+      if (live && c < D) {  // a self edge has no terms
+        if (dst != rank) place_dst = at(dst);
+        if (src != rank) place_src = at(src);
+      }
+      if (c == 0) place_diag = at(rank);
+      __syncwarp();
     }
-    if (c == 0) diag_place = at(rank);
-    __syncwarp();
   }
 
   // ---- scale so that the mean rank load is 1 ---------------------------------------
-  double mine = fixed;
-#pragma unroll
-  for (int d = 0; d < D; ++d) mine += w_in[d];
-  if (!live) mine = 0.0;
-#pragma unroll
-  for (int d = 0; d < D; ++d) tm.put(tm.fold(0, d), w_in[d]);
-  tm.put(tm.vec(kVecMisc), mine);
+  double total = first && live ? own_load : 0.0;
+  tm.put_edge(kEdgeF, w_in);
+  tm.sum_put(kSumStart, total);
   tm.sync();
-  double total, unused;
-  tm.sum2(tm.vec(kVecMisc), mine, tm.vec(kVecMisc), mine, total, unused);
+  tm.sum_get(kSumStart, total);
   const bool empty = !(total > 0.0);
   const double inv_scale = empty ? 0.0 : (double)rows * rcp3(total);
-  double w[D], base = fixed;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    base += tm.get(tm.fold(0, d), w_in[d], src[d]);
-    // a self edge moves no load: its column of M is zero, its load is already part of `base`
-    w[d] = dst[d] == rank ? 0.0 : w_in[d] * inv_scale;
-  }
-  base *= inv_scale;
+  const double base = (fixed + tm.edge_sum(tm.get_edge(kEdgeF, w_in, src))) * inv_scale;
+  // a self edge moves no load: its column of M is zero, its load is already part of `base`
+  const double w = dst == rank ? 0.0 : w_in * inv_scale, ww = w * w;
 
   // ---- warm start from the anchor, if it still fits the data -----------------------------
   bool cold;
   {
-    double mfa = 0.0;
-#pragma unroll
-    for (int d = 0; d < D; ++d) tm.put(tm.fold(1, d), w[d] * fa[d]);
+    const double x = w * fa;
+    tm.put_edge(kEdgeCw, x);
     tm.sync();
-#pragma unroll
-    for (int d = 0; d < D; ++d) mfa += w[d] * fa[d] - tm.get(tm.fold(1, d), w[d] * fa[d], src[d]);
+    const double mfa = tm.edge_sum(x - tm.get_edge(kEdgeCw, x, src));
     const bool near = !slot || fabs(ta - base - mfa - sa) <= prm.guard;
     if constexpr (NB > 1) {
       tm.key_put(0, near ? 0u : 1u);
@@ -428,46 +480,27 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
   // With one warp the rows past a smaller group's last rank take part; they save no iterate and start
   // cold beside a warm group.  A rank that does not take part keeps s = 1, y = 0 all along.
   const bool start_cold = cold || !slot;
-  double f[D], v[D], z[D], q[D], t = ta, s = 1.0, y = live ? inv_rows : 0.0;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    f[d] = start_cold ? 0.5 : fa[d];
-    v[d] = start_cold ? 0.5 : va[d];
-    z[d] = start_cold ? 1.0 : za[d];
-    q[d] = start_cold ? 1.0 : qa[d];
-  }
-  if (!start_cold) {
-    s = sa;
-    y = ya;
-  }
+  double f = start_cold ? 0.5 : fa, v = start_cold ? 0.5 : va, z = start_cold ? 1.0 : za, q = start_cold ? 1.0 : qa;
+  double t = ta, s = start_cold ? 1.0 : sa, y = start_cold ? (live ? inv_rows : 0.0) : ya;
   if (NB == 1 ? __any_sync(0xffffffffu, live && start_cold) : cold) {  // feasible start
-    double load = base;
-#pragma unroll
-    for (int d = 0; d < D; ++d) tm.put(tm.fold(2, d), 0.5 * w[d]);
+    const double x = 0.5 * w;
+    tm.put_edge(kEdgeRhs, x);
     tm.sync();
-#pragma unroll
-    for (int d = 0; d < D; ++d) load += 0.5 * w[d] - tm.get(tm.fold(2, d), 0.5 * w[d], src[d]);
-    tm.put(tm.vec(kVecLoad), live ? load : -1.0);
+    const double load = base + tm.edge_sum(x - tm.get_edge(kEdgeRhs, x, src));
+    double lmax = tm.max_put(kMaxLoad, live ? load : -1.0);
     tm.sync();
-    const double lmax = tm.max_positive(tm.vec(kVecLoad), live ? load : -1.0);
-    const double down = live ? (lmax + 1.0) - load : -1.0;
-    tm.put(tm.vec(kVecDual), down);
+    lmax = tm.max_get(kMaxLoad, lmax);
+    double down = tm.max_put(kMaxDown, live ? (lmax + 1.0) - load : -1.0);
     tm.sync();
-    const double lmin = (lmax + 1.0) - tm.max_positive(tm.vec(kVecDual), down);
+    const double lmin = (lmax + 1.0) - tm.max_get(kMaxDown, down);
     const double ct = lmax + 0.5 * (lmax - lmin) + 0.05;
     if (live && start_cold) s = ct - load;
     if (cold) t = ct;
-    const double sy = live ? (ct - load) * inv_rows : 0.0;
-    tm.put(tm.vec(kVecComp), sy);
+    double sum = live && first ? (ct - load) * inv_rows : 0.0;
+    tm.sum_put(kSumCold, sum);
     tm.sync();
-    double sum, same;
-    tm.sum2(tm.vec(kVecComp), sy, tm.vec(kVecComp), sy, sum, same);
-    const double mu0 = sum * inv_rows;
-    if (start_cold) {
-#pragma unroll
-      for (int d = 0; d < D; ++d) z[d] = q[d] = 2.0 * mu0;
-    }
-    tm.sync();  // the vectors are used again below
+    tm.sum_get(kSumCold, sum);
+    if (start_cold) z = q = 2.0 * (sum * inv_rows);
   }
   bool saved = false, done = empty;
   int iters = 0;
@@ -476,61 +509,81 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
 #pragma unroll 1
   for (int it = 0;; ++it) {
     if (prm.stop != nullptr && __any_sync(0xffffffffu, *prm.stop != 0)) break;
-    // ---- weights, residuals, gap, stopping test ----------------------------------------------
-    double wf[D], cw[D], theta[D], inv_f[D], inv_v[D];
-    const double inv_y = rcp3(live ? y : 1.0);
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      wf[d] = w[d] * f[d];
-      const double fv = f[d] * v[d], inv_fv = rcp3(fv);
-      theta[d] = fv * rcp3(fma(z[d], v[d], q[d] * f[d]));  // 1 / (z / f + q / v)
-      cw[d] = theta[d] * (w[d] * w[d]);
-      inv_f[d] = v[d] * inv_fv;
-      inv_v[d] = f[d] * inv_fv;
-      tm.put(tm.fold(0, d), wf[d]);
-      tm.put(tm.fold(1, d), cw[d]);
-    }
-    tm.put(tm.vec(kVecY), y);
+    // ---- weights and residuals --------------------------------------------------------------
+    const double fv = f * v, inv_fv = rcp3(fv), inv_y = rcp3(live ? y : 1.0);
+    const double theta = fv * rcp3(fma(z, v, q * f));  // 1 / (z / f + q / v)
+    const double cw = theta * ww, wf = w * f, wt = w * theta;
+    const double inv_f = v * inv_fv, inv_v = f * inv_fv;
+    tm.put_edge(kEdgeF, wf);
+    tm.put_edge(kEdgeCw, cw);
+    tm.put(kVecY, y);
     tm.sync();
-    double load = base, diag = s * inv_y, held[D], wy[D], r_u[D];
-    double comp = s * y, dual = y * base;
-    bool feasible = true;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      load += wf[d] - tm.get(tm.fold(0, d), wf[d], src[d]);
-      held[d] = tm.get(tm.fold(1, d), cw[d], src[d]);
-      wy[d] = w[d] * (y - tm.get(tm.vec(kVecY), y, dst[d]));
-      diag += cw[d] + held[d];
-      r_u[d] = 1.0 - f[d] - v[d];
-      comp = fma(z[d], f[d], fma(q[d], v[d], comp));
-      dual += negative_part(z[d] - q[d] - wy[d]) - q[d];
-      feasible = feasible && fabs(r_u[d]) <= prm.tol;
-    }
-    if (!live) comp = dual = 0.0;
-    tm.put(tm.vec(kVecComp), comp);
-    tm.put(tm.vec(kVecDual), dual);
-    tm.put(tm.vec(kVecLoad), live ? load : -1.0);
+    const double held = tm.get_edge(kEdgeCw, cw, src);
+    const double load = base + tm.edge_sum(wf - tm.get_edge(kEdgeF, wf, src));
+    const double wy = w * (y - tm.get(kVecY, y, dst));
+    const double r_u = 1.0 - f - v;
     // right-hand sides: the predictor's, and the part of the corrector's that goes with sigma mu
-    double qv[D], rd[D], wt[D], x_rhs[D], x_one[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      qv[d] = q[d] * inv_v[d];
-      rd[d] = fma(qv[d], r_u[d], -wy[d]);
-      wt[d] = w[d] * theta[d];
-      x_rhs[d] = wt[d] * rd[d];
-      x_one[d] = wt[d] * (inv_f[d] - inv_v[d]);
-      tm.put(tm.fold(2, d), x_rhs[d]);
-      tm.put(tm.fold(3, d), x_one[d]);
+    const double qv = q * inv_v, rd = fma(qv, r_u, -wy), x_rhs = wt * rd, x_one = wt * (inv_f - inv_v);
+    tm.put_edge(kEdgeRhs, x_rhs);
+    tm.put_edge(kEdgeOne, x_one);
+    // gap, complementarity and feasibility
+    double mu = real ? fma(z, f, q * v) : 0.0, dual_sum = real ? negative_part(z - q - wy) - q : 0.0, sum_y = 0.0;
+    if (first) {
+      mu = fma(s, y, mu);
+      dual_sum = fma(y, base, dual_sum);
+      sum_y = y;
     }
-    if constexpr (NB > 1) tm.key_put(0, live && !feasible ? 1u : 0u);
+    if (!live) mu = dual_sum = 0.0;
+    const bool feasible = !live || !real || fabs(r_u) <= prm.tol;
+    tm.sum_put(kSumMu, mu, sum_y);
+    tm.sum_put(kSumDual, dual_sum);
+    double primal = tm.max_put(kMaxLoad, live ? load : -1.0);
+    if constexpr (NB > 1) tm.key_put(0, feasible ? 0u : 1u);
+    // ---- normal matrix ----------------------------------------------------------------------
+    double n0[NB], n1[NB];
+    {
+      double val[2 * D], diag = s * inv_y;  // the rank's terms: theta w^2 of its own and of the held bundles
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        val[2 * d] = D == 1 ? cw : lane_get(cw, (lane & 28) | d);
+        val[2 * d + 1] = D == 1 ? held : lane_get(held, (lane & 28) | d);
+        diag += val[2 * d] + val[2 * d + 1];
+      }
+      if (!live) diag = 1.0;
+      if constexpr (NB == 1) {
+        double e0 = rank == 2 * c ? diag : 0.0, e1 = rank == 2 * c + 1 ? diag : 0.0, h0 = 0.0, h1 = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          e0 = fma(cd[d][0], val[2 * d], e0);
+          e1 = fma(cd[d][1], val[2 * d], e1);
+          h0 = fma(cs[d][0], val[2 * d + 1], h0);
+          h1 = fma(cs[d][1], val[2 * d + 1], h1);
+        }
+        n0[0] = e0 + h0;
+        n1[0] = e1 + h1;
+      } else {
+        double at_dst = 0.0, at_src = 0.0;
+#pragma unroll
+        for (int k = 0; k < 2 * D; ++k) {
+          at_dst -= (same_dst >> k) & 1u ? val[k] : 0.0;
+          at_src -= (same_src >> k) & 1u ? val[k] : 0.0;
+        }
+        if (place_dst != nullptr) *place_dst = at_dst;
+        if (place_src != nullptr) *place_src = at_src;
+        if (place_diag != nullptr) *place_diag = diag;
+      }
+    }
     tm.sync();
-    double mu, sum_y, dual_sum, same;
-    tm.sum2(tm.vec(kVecComp), comp, tm.vec(kVecY), y, mu, sum_y);
-    tm.sum2(tm.vec(kVecDual), dual, tm.vec(kVecDual), dual, dual_sum, same);
+    const double g_edges = tm.edge_sum(x_rhs - tm.get_edge(kEdgeRhs, x_rhs, src));
+    const double o_edges = tm.edge_sum(x_one - tm.get_edge(kEdgeOne, x_one, src));
+    const double g = live ? load - t + g_edges : 0.0, g_one = live ? inv_y + o_edges : 0.0;
+    // ---- stopping test ------------------------------------------------------------------------
+    tm.sum_get(kSumMu, mu, sum_y);
+    tm.sum_get(kSumDual, dual_sum);
+    primal = tm.max_get(kMaxLoad, primal);
     mu *= inv_kcomp;
     const double r_t = 1.0 - sum_y;
-    const double primal = tm.max_positive(tm.vec(kVecLoad), live ? load : -1.0);
-    const bool all_feasible = tm.all(0, !live || feasible);
+    const bool all_feasible = tm.all(0, feasible);
     if (!done) {
       gap = primal - dual_sum;  // absolute here, made relative once at the end
       gap_scale = fabs(primal);
@@ -539,57 +592,25 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     }
     // A cold solve leaves its first iterate at or below snap_mu behind as the next anchor.
     if (cold && !saved && !empty && mu <= prm.snap_mu) {
-      if (slot && c == 0) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          anchor[d] = f[d];
-          anchor[D + d] = v[d];
-          anchor[2 * D + d] = z[d];
-          anchor[3 * D + d] = q[d];
+      if (slot && c < D) {
+        anchor[c] = f;
+        anchor[D + c] = v;
+        anchor[2 * D + c] = z;
+        anchor[3 * D + c] = q;
+        if (c == 0) {
+          anchor[4 * D] = s;
+          anchor[4 * D + 1] = y;
+          anchor[4 * D + 2] = t;
+          if (rank == 0) *anchor_valid = 1;
         }
-        anchor[4 * D] = s;
-        anchor[4 * D + 1] = y;
-        anchor[4 * D + 2] = t;
-        if (rank == 0) *anchor_valid = 1;
       }
       saved = true;
     }
     if (done || it >= prm.max_iters) break;
     ++iters;
 
-    // ---- normal matrix and its inverse ---------------------------------------------------------
-    double n0[NB], n1[NB];
-    if (!live) diag = 1.0;
-    if constexpr (NB == 1) {
-      double e0 = rank == 2 * c ? diag : 0.0, e1 = rank == 2 * c + 1 ? diag : 0.0;
-      double h0 = 0.0, h1 = 0.0;
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        e0 = fma(cd[d][0], cw[d], e0);
-        e1 = fma(cd[d][1], cw[d], e1);
-        h0 = fma(cs[d][0], held[d], h0);
-        h1 = fma(cs[d][1], held[d], h1);
-      }
-      n0[0] = e0 + h0;
-      n1[0] = e1 + h1;
-    } else {
-      double val[2 * D];
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        val[2 * d] = cw[d];
-        val[2 * d + 1] = held[d];
-      }
-      int bit = 0;
-#pragma unroll
-      for (int a = 0; a < 2 * D; ++a) {
-        double acc = val[a];
-#pragma unroll
-        for (int b = a + 1; b < 2 * D; ++b, ++bit)
-          if ((merge >> bit) & 1u) acc += val[b];
-        if (place[a] != nullptr) *place[a] = -acc;
-      }
-      if (diag_place != nullptr) *diag_place = diag;
-      __syncwarp();
+    // ---- inverse, and its products with (g, g_one) and with ones: the border column of sum(dy) = r_t --------
+    if constexpr (NB > 1) {
       const double2* mat = tm.mat();
 #pragma unroll
       for (int j = 0; j < NB; ++j) {
@@ -598,24 +619,15 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
         n1[j] = e.y;
       }
     }
-    double g = load - t, g_one = inv_y;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      g += x_rhs[d] - tm.get(tm.fold(2, d), x_rhs[d], src[d]);
-      g_one += x_one[d] - tm.get(tm.fold(3, d), x_one[d], src[d]);
-    }
-    if (!live) g = g_one = 0.0;
-    tm.put(tm.vec(kVecG), g);
-    tm.put(tm.vec(kVecG1), g_one);
+    tm.put(kVecG, g);
+    tm.put(kVecG1, g_one);
     sweep_matrix<NB, D>(tm, n0, n1);  // with several warps its barriers also publish the right-hand sides
-
-    // inverse times (g, g_one), and times a vector of ones: the border column that carries sum(dy) = r_t
-    double x, x1, border;
+    double x, x1, border, same;
     {
-      double rs = 0.0, same_b;
+      double rs = 0.0;
 #pragma unroll
       for (int j = 0; j < NB; ++j) rs += n0[j] + n1[j];
-      mma8(border, same_b, rs, -1.0, 0.0, 0.0);
+      mma8(border, same, rs, -1.0, 0.0, 0.0);
       if constexpr (NB == 1) {
         // even columns of the product carry g, odd ones g_one: lane 4 r + c fetches the element of ranks
         // 2 c and 2 c + 1 from a lane that holds the one that column r is made of
@@ -627,7 +639,7 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
       } else {
         const double2* gv = reinterpret_cast<const double2*>(tm.vec(kVecG));
         const double2* ov = reinterpret_cast<const double2*>(tm.vec(kVecG1));
-        double p0 = 0.0, p1 = 0.0, o0 = 0.0, o1 = 0.0, unused_x;
+        double p0 = 0.0, p1 = 0.0, o0 = 0.0, o1 = 0.0;
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
           const double2 a = gv[4 * j + c], b = ov[4 * j + c];
@@ -636,77 +648,55 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
           o0 = fma(n0[j], b.x, o0);
           o1 = fma(n1[j], b.y, o1);
         }
-        mma8(x, unused_x, p0 + p1, -1.0, 0.0, 0.0);
-        mma8(x1, unused_x, o0 + o1, -1.0, 0.0, 0.0);
+        mma8(x, same, p0 + p1, -1.0, 0.0, 0.0);
+        mma8(x1, same, o0 + o1, -1.0, 0.0, 0.0);
       }
     }
     if (!live) border = 0.0;
-    tm.put(tm.vec(kVecX), x);
-    tm.put(tm.vec(kVecX1), x1);
-    tm.put(tm.vec(kVecBorder), border);
+    tm.put(kVecX, x);
+    tm.put(kVecX1, x1);
+    tm.put(kVecBorder, border);
+    double sum_x = first ? x : 0.0, sum_b = first ? border : 0.0, sum_x1 = first ? x1 : 0.0;
+    tm.sum_put(kSumX, sum_x, sum_b);
+    tm.sum_put(kSumX1, sum_x1);
     tm.sync();
-    double sum_x, sum_b, sum_x1;
-    tm.sum2(tm.vec(kVecX), x, tm.vec(kVecBorder), border, sum_x, sum_b);
-    tm.sum2(tm.vec(kVecX1), x1, tm.vec(kVecX1), x1, sum_x1, same);
-    const double inv_sum_b = rcp3(sum_b);
-    const double inv_mu = rcp3(kcomp * mu);
+    tm.sum_get(kSumX, sum_x, sum_b);
+    tm.sum_get(kSumX1, sum_x1);
+    const double inv_sum_b = rcp3(sum_b), inv_mu = rcp3(kcomp * mu);
     // ---- predictor ---------------------------------------------------------------------------
     // df = theta (rd - w (dy - dy_dst)) with dy = x - dt border, as e + dt e_b
-    double e[D], e_b[D], e_1[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      e[d] = fma(-wt[d], x - tm.get(tm.vec(kVecX), x, dst[d]), theta[d] * rd[d]);
-      e_b[d] = wt[d] * (border - tm.get(tm.vec(kVecBorder), border, dst[d]));
-      e_1[d] = fma(-wt[d], x1 - tm.get(tm.vec(kVecX1), x1, dst[d]), theta[d] * (inv_f[d] - inv_v[d]));
-    }
+    const double e = fma(-wt, x - tm.get(kVecX, x, dst), theta * rd);
+    const double e_b = wt * (border - tm.get(kVecBorder, border, dst));
+    const double e_1 = fma(-wt, x1 - tm.get(kVecX1, x1, dst), theta * (inv_f - inv_v));
+    const double si = s * inv_y, zi = z * inv_f;
     double dt = (sum_x - r_t) * inv_sum_b;
-    double dy = fma(-dt, border, x);
-    const double si = s * inv_y;
-    double ds = fma(-si, dy, -s);
-    double df[D], dv[D], dz[D], dq[D], zi[D], p_f[D], p_v[D], x_cor[D], rc[D];
+    double dy = fma(-dt, border, x), ds = fma(-si, dy, -s);
+    double df = fma(dt, e_b, e), dv = r_u - df, dz = fma(-zi, df, -z), dq = fma(-qv, dv, -q);
     // the predictor takes every complementarity product to zero, so dz / z = -1 - df / f, and so on
-    const double ty = -dy * inv_y;
-    unsigned key_p = step_key(1.0 - ty), key_d = step_key(ty);
-    double c_p = y * ds, c_pd = ds * dy;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      zi[d] = z[d] * inv_f[d];
-      df[d] = fma(dt, e_b[d], e[d]);
-      dv[d] = r_u[d] - df[d];
-      dz[d] = fma(-zi[d], df[d], -z[d]);
-      dq[d] = fma(-qv[d], dv[d], -q[d]);
-      const double tf = -df[d] * inv_f[d], tv = -dv[d] * inv_v[d];
-      key_p = max(key_p, max(step_key(tf), step_key(tv)));
-      key_d = max(key_d, max(step_key(1.0 - tf), step_key(1.0 - tv)));
-      c_p = fma(z[d], df[d], fma(q[d], dv[d], c_p));
-      c_pd = fma(df[d], dz[d], fma(dv[d], dq[d], c_pd));
-      p_f[d] = dz[d] * -tf;  // dz df / f
-      p_v[d] = dq[d] * -tv;
-      rc[d] = rd[d] - p_f[d] + p_v[d];
-      x_cor[d] = wt[d] * rc[d];
-      tm.put(tm.fold(4, d), x_cor[d]);
+    const double tf = -df * inv_f, tv = -dv * inv_v, ty = -dy * inv_y;
+    unsigned key_p = max(step_key(1.0 - ty), max(step_key(tf), step_key(tv)));
+    unsigned key_d = max(step_key(ty), max(step_key(1.0 - tf), step_key(1.0 - tv)));
+    double c_p = real ? fma(z, df, q * dv) : 0.0, c_pd = real ? fma(df, dz, dv * dq) : 0.0;
+    if (first) {
+      c_p = fma(y, ds, c_p);
+      c_pd = fma(ds, dy, c_pd);
     }
-    if (!live) {
-      c_p = c_pd = 0.0;
-      key_p = key_d = 0;
-    }
-    const double p_s = ds * -ty;  // ds dy / y
-    key_p = tm.key_put(0, key_p);
-    key_d = tm.key_put(1, key_d);
-    tm.put(tm.vec(kVecCp), c_p);
-    tm.put(tm.vec(kVecCpd), c_pd);
+    const double p_f = dz * -tf, p_v = dq * -tv, p_s = ds * -ty;  // dz df / f, dq dv / v, ds dy / y
+    const double rc = rd - p_f + p_v, x_cor = wt * rc;
+    tm.put_edge(kEdgeCor, x_cor);
+    if (!live) c_p = c_pd = 0.0;
+    key_p = tm.key_put(0, live && real ? key_p : 0u);
+    key_d = tm.key_put(1, live && real ? key_d : 0u);
+    tm.sum_put(kSumAffine, c_p, c_pd);
     tm.sync();
     // ---- corrector ---------------------------------------------------------------------------
-    double g0 = load - t - p_s;
-#pragma unroll
-    for (int d = 0; d < D; ++d) g0 += x_cor[d] - tm.get(tm.fold(4, d), x_cor[d], src[d]);
-    if (!live) g0 = 0.0;
-    tm.put(tm.vec(kVecG0), g0);
-    double sum_cp, sum_cpd;
-    tm.sum2(tm.vec(kVecCp), c_p, tm.vec(kVecCpd), c_pd, sum_cp, sum_cpd);
+    const double c_edges = tm.edge_sum(x_cor - tm.get_edge(kEdgeCor, x_cor, src));
+    const double g0 = live ? load - t - p_s + c_edges : 0.0;
+    tm.put(kVecG0, g0);
+    tm.sum_get(kSumAffine, c_p, c_pd);
     const double ap0 = step_from_key(tm.key_get(0, key_p), 1.0), ad0 = step_from_key(tm.key_get(1, key_d), 1.0);
     // complementarity after the affine step; sum x dz = -kcomp mu - sum z dx
-    const double comp_aff = fma(ap0 * ad0, sum_cpd, fma(ap0 - ad0, sum_cp, kcomp * mu * (1.0 - ad0)));
+    const double comp_aff = fma(ap0 * ad0, c_pd, fma(ap0 - ad0, c_p, kcomp * mu * (1.0 - ad0)));
     const double ratio = clamp01(comp_aff * inv_mu);
     const double sig_mu = ratio * ratio * ratio * mu;
     double x0;
@@ -725,65 +715,49 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
         p1 = fma(n1[j], a.y, p1);
       }
       mma8(x0, same, p0 + p1, -1.0, 0.0, 0.0);
-      tm.put(tm.vec(kVecX0), x0);
-      tm.sync();
+      tm.put(kVecX0, x0);
     }
-    double sum_x0;
-    tm.sum2(tm.vec(kVecX0), x0, tm.vec(kVecX0), x0, sum_x0, same);
+    double sum_x0 = first ? x0 : 0.0;
+    tm.sum_put(kSumX0, sum_x0);
+    tm.sync();
+    tm.sum_get(kSumX0, sum_x0);
+    const double e0 = fma(-wt, x0 - tm.get(kVecX0, x0, dst), theta * rc);
     dt = (fma(sig_mu, sum_x1, sum_x0) - r_t) * inv_sum_b;
     dy = fma(-dt, border, fma(sig_mu, x1, x0));
     ds = fma(-si, dy, fma(sig_mu, inv_y, -s - p_s));
-    key_p = step_key(-ds * rcp_seed(s));
-    key_d = step_key(-dy * inv_y);
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      const double e0 = fma(-wt[d], x0 - tm.get(tm.vec(kVecX0), x0, dst[d]), theta[d] * rc[d]);
-      df[d] = fma(dt, e_b[d], fma(sig_mu, e_1[d], e0));
-      dv[d] = r_u[d] - df[d];
-      dz[d] = fma(-zi[d], df[d], fma(sig_mu, inv_f[d], -z[d] - p_f[d]));
-      dq[d] = fma(-qv[d], dv[d], fma(sig_mu, inv_v[d], -q[d] - p_v[d]));
-      key_p = max(key_p, max(step_key(-df[d] * inv_f[d]), step_key(-dv[d] * inv_v[d])));
-      key_d = max(key_d, max(step_key(-dz[d] * rcp_seed(z[d])), step_key(-dq[d] * rcp_seed(q[d]))));
-    }
-    if (!live) key_p = key_d = 0;
-    key_p = tm.key_put(2, key_p);
-    key_d = tm.key_put(3, key_d);
+    df = fma(dt, e_b, fma(sig_mu, e_1, e0));
+    dv = r_u - df;
+    dz = fma(-zi, df, fma(sig_mu, inv_f, -z - p_f));
+    dq = fma(-qv, dv, fma(sig_mu, inv_v, -q - p_v));
+    key_p = max(step_key(-ds * rcp_seed(s)), max(step_key(-df * inv_f), step_key(-dv * inv_v)));
+    key_d = max(step_key(-dy * inv_y), max(step_key(-dz * rcp_seed(z)), step_key(-dq * rcp_seed(q))));
+    key_p = tm.key_put(2, live && real ? key_p : 0u);
+    key_d = tm.key_put(3, live && real ? key_d : 0u);
     tm.sync();
     const double ap = step_from_key(tm.key_get(2, key_p), kEta), ad = step_from_key(tm.key_get(3, key_d), kEta);
     t = fma(ap, dt, t);
     if (live) {
       s = fma(ap, ds, s);
       y = fma(ad, dy, y);
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        f[d] = fma(ap, df[d], f[d]);
-        v[d] = fma(ap, dv[d], v[d]);
-        z[d] = fma(ad, dz[d], z[d]);
-        q[d] = fma(ad, dq[d], q[d]);
-      }
+    }
+    if (live && real) {
+      f = fma(ap, df, f);
+      v = fma(ap, dv, v);
+      z = fma(ad, dz, z);
+      q = fma(ad, dq, q);
     }
   }
 
-  bool ok = true;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    ok = ok && (f[d] == f[d]) && fabs(f[d]) < 1e300;
-    f_out[d] = fmin(fmax(f[d], 0.0), 1.0);
-  }
+  const bool ok = !live || !real || (f == f && fabs(f) < 1e300);
+  f_out = fmin(fmax(f, 0.0), 1.0);
   if constexpr (NB > 1) {
     tm.sync();  // every warp is through with key 0
-    tm.key_put(0, live && !ok ? 1u : 0u);
+    tm.key_put(0, ok ? 0u : 1u);
     tm.sync();
   }
-  const bool finite = tm.all(0, !live || ok);
-  if (!finite) {
-#pragma unroll
-    for (int d = 0; d < D; ++d) f_out[d] = 0.5;
-  }
-  if (empty) {  // nothing to balance: keep everything on the origin
-#pragma unroll
-    for (int d = 0; d < D; ++d) f_out[d] = 1.0;
-  }
+  const bool finite = tm.all(0, ok);
+  if (!finite) f_out = 0.5;
+  if (empty) f_out = 1.0;  // nothing to balance: keep everything on the origin
   IpmOutcome out;
   out.iters = iters;
   out.converged = done && finite;

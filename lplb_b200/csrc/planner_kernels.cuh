@@ -43,18 +43,23 @@ struct Exchange {
 struct Workspace {
   uint32_t epoch;      // launches completed
   uint32_t arrive[2];  // by launch parity: CTAs of that launch that published their counts
-  uint32_t lp_done;    // epoch whose shares are ready
   uint32_t count_ticket;  // used by the stand-alone counting kernel
   uint32_t exit_cnt;   // tracing only: CTAs of the running launch that finished
-  uint32_t pad[2];
-  // followed by: int total[2][E]; int global_cnt[E];
+  uint32_t pad[3];
+  // followed by: int total[2][E]; int global_cnt[E]; (on 16 bytes) uint64 result[E][2]
 };
 static_assert(sizeof(Workspace) == 32, "the tables that follow the header start at byte 32");
-__host__ __device__ inline size_t workspace_bytes(int e) { return sizeof(Workspace) + sizeof(int) * 3 * (size_t)e; }
+__host__ __device__ inline size_t ws_result_offset(int e) { return (sizeof(Workspace) + sizeof(int) * 3 * (size_t)e + 15) & ~(size_t)15; }
+__host__ __device__ inline size_t workspace_bytes(int e) { return ws_result_offset(e) + 16 * (size_t)e; }
 __device__ __forceinline__ int* ws_total(Workspace* ws, int parity, int e) {
   return reinterpret_cast<int*>(ws + 1) + (size_t)parity * e;
 }
 __device__ __forceinline__ int* ws_global(Workspace* ws, int e) { return reinterpret_cast<int*>(ws + 1) + 2 * (size_t)e; }
+// What the solver CTA hands to the workers, per expert: two words (epoch << 32) | value with the quota of
+// tokens that stay on the original and the rank-local total.
+__device__ __forceinline__ unsigned long long* ws_result(Workspace* ws, int e) {
+  return reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(ws) + ws_result_offset(e));
+}
 
 // ---------------------------------------------------------------------------------------
 // Histogram of one CTA's token slice into shared memory.  Indices outside [-1, E) are
@@ -109,9 +114,9 @@ __device__ __forceinline__ bool even_pick(unsigned k, unsigned quota, unsigned t
 }
 
 // Quota of expert e's local tokens that stay on the original.
-__device__ __forceinline__ int quota_of(int total, int edge, const float* __restrict__ probs) {
+__device__ __forceinline__ int quota_of(int total, int edge, const float* probs) {
   if (edge < 0) return total;
-  float p = __ldcg(&probs[edge]);  // may have been written by another CTA of this launch
+  float p = probs[edge];
   p = p != p ? 0.5f : fminf(fmaxf(p, 0.f), 1.f);
   int q = __float2int_rn(p * (float)total);
   return q < 0 ? 0 : (q > total ? total : q);
@@ -301,7 +306,7 @@ __device__ __forceinline__ void report_group(const IpmOutcome& res, int grp, Cou
 // costs 1.5-2 us per call.
 template <int GP, int D, bool SKIP_IDLE = false>
 __device__ __forceinline__ void solve_groups(const int* __restrict__ bundle, const Topo& tp, int first_group, int group_stride,
-                             IpmParams prm, float* __restrict__ probs, Counter avail, int* status) {
+                             IpmParams prm, float* __restrict__ probs, float* share, Counter avail, int* status) {
   constexpr int kSeg = 32 / GP;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int seg = lane / GP, li = lane % GP;
@@ -342,7 +347,11 @@ __device__ __forceinline__ void solve_groups(const int* __restrict__ bundle, con
     else res = ipm_solve_segment<GP, D>(li, w, fixed, src, dst, prm, f, anchor, anchor_valid, lanes);
     if (live) {
 #pragma unroll
-      for (int d = 0; d < D; ++d) probs[((size_t)grp * tp.g + li) * D + d] = (float)f[d];
+      for (int d = 0; d < D; ++d) {
+        const size_t at = ((size_t)grp * tp.g + li) * D + d;
+        probs[at] = (float)f[d];
+        if (share != nullptr) share[at] = (float)f[d];
+      }
       if (li == 0) report_group(res, grp, avail, status);
     }
   }
@@ -353,7 +362,7 @@ __device__ __forceinline__ void solve_groups(const int* __restrict__ bundle, con
 // block_solver_smem_bytes(tp.g, DP) of shared memory, 8-byte aligned.
 template <int DP>
 __device__ __forceinline__ void solve_groups_block(const int* __restrict__ bundle, const Topo& tp, int first_group, int group_stride,
-                                   IpmParams prm, float* __restrict__ probs, Counter avail, int* status,
+                                   IpmParams prm, float* __restrict__ probs, float* share, Counter avail, int* status,
                                    double* scratch) {
   const int tid = threadIdx.x, dd = tp.d;
   for (int grp = first_group; grp < tp.n_group; grp += group_stride) {
@@ -389,8 +398,12 @@ __device__ __forceinline__ void solve_groups_block(const int* __restrict__ bundl
     const IpmOutcome res = ipm_solve_block<DP>(tid, tp.g, w, fixed, src, dst, prm, f, anchor, anchor_valid, scratch);
     if (live) {
 #pragma unroll
-      for (int d = 0; d < DP; ++d)
-        if (d < dd) probs[((size_t)grp * tp.g + tid) * dd + d] = (float)f[d];
+      for (int d = 0; d < DP; ++d) {
+        if (d >= dd) continue;
+        const size_t at = ((size_t)grp * tp.g + tid) * dd + d;
+        probs[at] = (float)f[d];
+        if (share != nullptr) share[at] = (float)f[d];
+      }
       if (tid == 0) report_group(res, grp, avail, status);
     }
     __syncthreads();  // the scratch area is reused by the next group
@@ -398,34 +411,32 @@ __device__ __forceinline__ void solve_groups_block(const int* __restrict__ bundl
 }
 
 // Tile solver: NB warps per group, `team_warp` is the calling warp's place among them; the team
-// solves groups first_group, first_group + group_stride, ...  `scratch` is tile_solver_smem_bytes(tp.g, D)
-// of shared memory per team, 16-byte aligned (NB == 1: unused).
+// solves groups first_group, first_group + group_stride, ...  `scratch` is the team's
+// tile_solver_smem_bytes(tp.g, D) of shared memory, 16-byte aligned.  `share`: a copy of the shares in
+// shared memory, or null.
 template <int NB, int D>
 __device__ __forceinline__ void solve_groups_tiles(const int* __restrict__ bundle, const Topo& tp, int first_group, int group_stride,
-                                   int team_warp, IpmParams prm, float* __restrict__ probs, Counter avail, int* status,
-                                   double* scratch) {
+                                   int team_warp, IpmParams prm, float* __restrict__ probs, float* share, Counter avail,
+                                   int* status, double* scratch) {
   const int lane = threadIdx.x & 31, rank = 8 * team_warp + (lane >> 2);
-  const bool live = rank < tp.g;
-  for (int grp = first_group; grp < tp.n_group; grp += group_stride) {
-    double w[D], fixed = 0.0, f[D];
-    int src[D], dst[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      w[d] = 0.0;
-      src[d] = dst[d] = rank;
+  const int d = lane & (TileTeam<NB, D>::kLanes - 1);
+  const bool live = rank < tp.g, real = live && d < D;
+  int src = rank, dst = rank;
+  if (real) {
+    const int s = tp.r2o[rank * D + d], t = tp.o2r[rank * D + d];
+    if (LPLB_CHECKED(s, tp.g, status, kPhSolve) && LPLB_CHECKED(t, tp.g, status, kPhSolve)) {
+      src = s;
+      dst = t;
     }
+  }
+  for (int grp = first_group; grp < tp.n_group; grp += group_stride) {
+    double w = 0.0, fixed = 0.0, own = 0.0, f;
     if (live) {
       const int* mine = bundle + ((size_t)grp * tp.g + rank) * (D + 1);
-      fixed = (double)mine[D];
+      fixed = own = (double)mine[D];
 #pragma unroll
-      for (int d = 0; d < D; ++d) {
-        w[d] = (double)mine[d];
-        const int s = tp.r2o[rank * D + d], t = tp.o2r[rank * D + d];
-        if (LPLB_CHECKED(s, tp.g, status, kPhSolve) && LPLB_CHECKED(t, tp.g, status, kPhSolve)) {
-          src[d] = s;
-          dst[d] = t;
-        }
-      }
+      for (int k = 0; k < D; ++k) own += (double)mine[k];
+      if (real) w = (double)mine[d];
     }
     double *anchor = nullptr, *group_anchor = nullptr;
     int* anchor_valid = nullptr;
@@ -434,11 +445,12 @@ __device__ __forceinline__ void solve_groups_tiles(const int* __restrict__ bundl
       if (live) anchor = group_anchor + (size_t)rank * (4 * D + 3);
       anchor_valid = prm.anchor_valid + grp;
     }
-    const IpmOutcome res = ipm_solve_tiles<NB, D>(team_warp, lane, NB == 1 && prm.pad_rows ? 8 : tp.g, w, fixed, src, dst, prm, f,
-                                                  anchor, group_anchor, anchor_valid, scratch);
-    if (live && (lane & 3) == 0) {
-#pragma unroll
-      for (int d = 0; d < D; ++d) probs[((size_t)grp * tp.g + rank) * D + d] = (float)f[d];
+    const IpmOutcome res = ipm_solve_tiles<NB, D>(team_warp, lane, NB == 1 && prm.pad_rows ? 8 : tp.g, w, fixed, own, src, dst, prm,
+                                                  f, anchor, group_anchor, anchor_valid, scratch);
+    if (live && (lane & 3) < D) {
+      const size_t at = ((size_t)grp * tp.g + rank) * D + d;
+      probs[at] = (float)f;
+      if (share != nullptr) share[at] = (float)f;
     }
     if (rank == 0 && lane == 0) report_group(res, grp, avail, status);
   }
@@ -479,7 +491,7 @@ __global__ void __launch_bounds__(kBlock) solve_kernel(const int* __restrict__ w
   bundle_sums(workload, tp, bundle, min(tp.n_group, (int)blockIdx.x * per_cta) * tp.g,
               min(tp.n_group, ((int)blockIdx.x + 1) * per_cta) * tp.g, status);
   if ((int)(threadIdx.x >> 5) < solver_warps)
-    solve_groups<GP, D>(bundle, tp, blockIdx.x * per_cta, gridDim.x * per_cta, prm, probs, avail, status);
+    solve_groups<GP, D>(bundle, tp, blockIdx.x * per_cta, gridDim.x * per_cta, prm, probs, nullptr, avail, status);
 }
 
 // Shared memory for the bundle sums plus the slack that lets the solver's scratch area start on
@@ -508,8 +520,8 @@ __global__ void __launch_bounds__(kBlock) tile_solve_kernel(const int* __restric
   const int first = (int)blockIdx.x * teams, warp = threadIdx.x >> 5;
   bundle_sums(workload, tp, bundle, min(tp.n_group, first) * tp.g, min(tp.n_group, first + teams) * tp.g, status);
   if (warp < teams * NB)
-    solve_groups_tiles<NB, D>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, NB == 1 ? 0 : warp, prm, probs, avail, status,
-                              scratch_after(bundle, tp.n_group * tp.g, tp.d));
+    solve_groups_tiles<NB, D>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, NB == 1 ? 0 : warp, prm, probs, nullptr, avail,
+                              status, scratch_after(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total);
 }
 
 // Stand-alone solve kernel, thread-block solver: one CTA per group (the reference launches
@@ -528,7 +540,7 @@ __global__ void __launch_bounds__(kBlock) solve_block_kernel(const int* __restri
   double* scratch = scratch_after(bundle, tp.n_group * tp.g, tp.d);
   const int grp = blockIdx.x;
   bundle_sums(workload, tp, bundle, grp * tp.g, (grp + 1) * tp.g, status);
-  solve_groups_block<DP>(bundle, tp, grp, gridDim.x, prm, probs, avail, status, scratch);
+  solve_groups_block<DP>(bundle, tp, grp, gridDim.x, prm, probs, nullptr, avail, status, scratch);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -572,6 +584,24 @@ __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned lon
 }
 __device__ __forceinline__ void st_volatile_u64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.volatile.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void ld_volatile_u64x2(const unsigned long long* p, unsigned long long (&v)[2]) {
+  asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "l"(p) : "memory");
+}
+// Wait until both words carry the launch number; false when `budget_ns` ran out first.
+__device__ __forceinline__ bool wait_result(const unsigned long long* p, uint32_t epoch, uint64_t budget_ns,
+                                            unsigned long long (&v)[2]) {
+  uint64_t t0 = 0;
+  for (uint32_t spins = 0;; ++spins) {
+    ld_volatile_u64x2(p, v);
+    if ((uint32_t)(v[0] >> 32) == epoch && (uint32_t)(v[1] >> 32) == epoch) return true;
+    if ((spins & 63u) == 63u) {
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > budget_ns) return false;
+    }
+    __nanosleep(20);
+  }
 }
 // Two adjacent words in one 16-byte store.  Each 8-byte half carries its own epoch, so it does
 // not matter whether the two halves become visible together.
@@ -772,9 +802,11 @@ __global__ void __launch_bounds__(kBlock) exchange_kernel(const int* __restrict_
 //   CTAs 1..n  ("workers"): histogram their slice of the indices; reserve an ordinal range per
 //                expert with one returning atomicAdd on the rank-local totals; arrive.
 //   CTA 0      ("solver"):  meanwhile pulls the solver's inputs into its caches; waits for the
-//                arrivals; exchanges the totals with the peers; solves the LPs; publishes the
-//                shares; raises lp_done.
-//   workers:     wait for lp_done; turn shares into integer quotas; rewrite their slice.
+//                arrivals; exchanges the totals with the peers; solves the LPs; turns the shares into
+//                integer quotas and hands them out, each in a word that carries the launch number.
+//   workers:     poll those words, one expert per thread; rewrite their slice.
+//
+// Handing the quotas out took a fence, a flag and two more round trips to L2 before (0.6 us of the step).
 //
 // The solver CTA touches no indices.  Its code path shares no registers with the workers' (the
 // workers keep indices and table pointers live across their wait; inlined into one path with
@@ -830,9 +862,23 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
   const int parity = epoch & 1;
   int* total_g = ws_total(ws, parity, e);
   int* vec = smem;  // rank-local, then group-wide totals
-  int* bundle = smem + e;
+  int* local = smem + e;
+  float* share = reinterpret_cast<float*>(smem + 2 * (size_t)e);  // [n_group * g * d], at most e
+  int* bundle = smem + 3 * (size_t)e;
   constexpr int NT = kBlock;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first = threadIdx.x;  // its table entries are in flight while the workers count
+  const int first_slot = first < e ? tp.log2slot[first] : 0;
+  const int first_edge = first < e ? tp.log2edge[first] : -1;
+  int* glob = ws_global(ws, e);
+  const int n_bundle = tp.n_group * tp.g * (tp.d + 1);
+  for (int i = threadIdx.x; i < n_bundle; i += NT) bundle[i] = 0;
+  // one expert's group-wide count -> its rank's bundle load, and a copy for the host
+  auto add_count = [&](int i, int c) {
+    glob[i] = c;
+    const int slot = i == first ? first_slot : tp.log2slot[i];
+    if (c && LPLB_CHECKED(slot, n_bundle, status, kPhSolve)) atomicAdd(&bundle[slot], c);
+  };
   if (warp == 1) {
     if (lane == 0) {
       if (!bounded_wait_ge<false>(&ws->arrive[parity], (uint32_t)n_workers, grid_timeout_ns)) {
@@ -851,40 +897,39 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
       atomicAdd(&status[kStCalls], 1);
     }
   } else if (warp == 0) {
-    if constexpr (GP > 0 || GP == -1) {
+    if constexpr (GP > 0) {
       // Rehearsal while the workers count: the warp that will solve runs the solver on made-up
       // loads until the counts are in.  Whatever ran since the last step has evicted the
       // solver's code from the caches, the instruction caches included, and one warp running
       // two thousand straight-line instructions per iteration waits for every line of it; here
       // it takes the first of those waits while it has nothing else to do.  Nothing it
-      // computes is kept.
-      const int li = GP == -1 ? lane >> 2 : lane, g = tp.g;
-      if (GP == -1 || lane < GP) {
-      double w[D], f[D];
-      int src[D], dst[D];
+      // computes is kept.  (The tile solver's code is less than half as long: a rehearsal costs it 0.2 to 1.4 us
+      // a step more than it gives, one through the very code that solves 1 us or more.)
+      const int li = lane, g = tp.g;
+      if (lane < GP) {
+        double w[D], f[D];
+        int src[D], dst[D];
 #pragma unroll
-      for (int d = 0; d < D; ++d) {
-        const bool real = li < g && (d + 1) % g != 0;
-        w[d] = real ? 1.0 + 0.37 * li + 0.11 * d : 0.0;
-        src[d] = real ? (li + d + 1) % g : li;
-        dst[d] = real ? (li + g - (d + 1) % g) % g : li;
-      }
-      IpmParams rehearsal{3, 0.0};
-      rehearsal.stop = &s_stop;
-      const double fixed = li < g ? 3.0 + 0.2 * li : 0.0;
-      if constexpr (GP == -1) ipm_solve_tiles<1, D>(0, lane, 8, w, fixed, src, dst, rehearsal, f, nullptr, nullptr, nullptr, nullptr);
-      else ipm_solve_segment<GP, D>(li, w, fixed, src, dst, rehearsal, f, nullptr, nullptr, first_lanes(GP));
+        for (int d = 0; d < D; ++d) {
+          const bool real = li < g && (d + 1) % g != 0;
+          w[d] = real ? 1.0 + 0.37 * li + 0.11 * d : 0.0;
+          src[d] = real ? (li + d + 1) % g : li;
+          dst[d] = real ? (li + g - (d + 1) % g) % g : li;
+        }
+        IpmParams rehearsal{3, 0.0};
+        rehearsal.stop = &s_stop;
+        ipm_solve_segment<GP, D>(li, w, li < g ? 3.0 + 0.2 * li : 0.0, src, dst, rehearsal, f, nullptr, nullptr,
+                                 first_lanes(GP));
       }
     }
   }
   team_sync<NT>();
   // the workers' counts are in total_g: their atomics precede their arrivals
   int* other = ws_total(ws, parity ^ 1, e);
-  const int first = threadIdx.x;
-  const int first_slot = first < e ? tp.log2slot[first] : 0;  // in flight while the exchange runs
   for (int i = threadIdx.x; i < e; i += NT) {
-    vec[i] = __ldcg(&total_g[i]);
+    vec[i] = local[i] = __ldcg(&total_g[i]);
     other[i] = 0;  // ready for the next launch
+    if (ex.n_ranks <= 1) add_count(i, vec[i]);
   }
   team_sync<NT>();
   if (ex.n_ranks > 1) {
@@ -901,33 +946,29 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
         raise_status(status, kErrPeerTimeout, kPhExchange, (int)miss);
       }
     }
+    for (int i = threadIdx.x; i < e; i += NT) add_count(i, vec[i]);
+    team_sync<NT>();
   }
   if (tracing) trace[3] = global_timer_ns();
-  // group-wide counts -> per-rank bundle loads, and a copy for the host
-  int* glob = ws_global(ws, e);
-  const int n_bundle = tp.n_group * tp.g * (tp.d + 1);
-  for (int i = threadIdx.x; i < n_bundle; i += NT) bundle[i] = 0;
-  team_sync<NT>();
-  for (int i = threadIdx.x; i < e; i += NT) {
-    const int c = vec[i];
-    glob[i] = c;
-    const int slot = i == first ? first_slot : tp.log2slot[i];
-    if (c && LPLB_CHECKED(slot, n_bundle, status, kPhSolve)) atomicAdd(&bundle[slot], c);
-  }
-  team_sync<NT>();
+  double* scratch = scratch_after(bundle, tp.n_group * tp.g, tp.d);
   if constexpr (GP == 0) {
-    solve_groups_block<D>(bundle, tp, 0, 1, prm, probs, avail, status, scratch_after(bundle, tp.n_group * tp.g, tp.d));
+    solve_groups_block<D>(bundle, tp, 0, 1, prm, probs, share, avail, status, scratch);
+  } else if constexpr (GP == -1) {  // one group per warp
+    solve_groups_tiles<1, D>(bundle, tp, warp, kWarps, 0, prm, probs, share, avail, status, scratch + warp * tile_layout(1, D).total);
   } else if constexpr (GP < 0) {
-    constexpr int kTeams = GP == -1 ? kWarps : 1;  // one group per warp, or one group at a time
-    if (GP == -1 || warp < -GP)
-      solve_groups_tiles<-GP, D>(bundle, tp, GP == -1 ? warp : 0, kTeams, GP == -1 ? 0 : warp, prm, probs, avail, status,
-                                 scratch_after(bundle, tp.n_group * tp.g, tp.d));
+    if (warp < -GP) solve_groups_tiles<-GP, D>(bundle, tp, 0, 1, warp, prm, probs, share, avail, status, scratch);
   } else {
-    solve_groups<GP, D, true>(bundle, tp, 0, (NT / 32) * (32 / GP), prm, probs, avail, status);
+    solve_groups<GP, D, true>(bundle, tp, 0, (NT / 32) * (32 / GP), prm, probs, share, avail, status);
   }
-  __threadfence();
   team_sync<NT>();
-  if (threadIdx.x == 0) st_release_gpu(&ws->lp_done, epoch);
+  // Quotas and totals go out as words that carry the launch number, so a worker that sees one has it:
+  // no fence, no flag, no second round trip.
+  unsigned long long* result = ws_result(ws, e);
+  const unsigned long long tag = (unsigned long long)epoch << 32;
+  for (int i = threadIdx.x; i < e; i += NT) {
+    const int tot = local[i], quota = quota_of(tot, i == first ? first_edge : tp.log2edge[i], share);
+    st_volatile_u64x2(result + 2 * (size_t)i, tag | (uint32_t)quota, tag | (uint32_t)tot);
+  }
   if (tracing) trace[4] = global_timer_ns();
 }
 
@@ -941,7 +982,6 @@ __device__ __forceinline__ void worker_cta(const IdxT* __restrict__ idx, long lo
   const RedirectTables tb = redirect_tables(smem, e);
   int* hist = tb.total;  // this CTA's counts, later the rank-local totals
   __shared__ uint32_t s_epoch;
-  __shared__ int s_ok;
   // Everything that does not depend on the launch number is issued before the first barrier:
   // the launch number itself, this thread's indices, the static lookup tables.
   if (threadIdx.x == 0) s_epoch = ld_acquire_gpu(&ws->epoch) + 1;
@@ -950,7 +990,6 @@ __device__ __forceinline__ void worker_cta(const IdxT* __restrict__ idx, long lo
   load_keep(idx, begin, end, keep);
   for (int i = threadIdx.x; i < e; i += kBlock) {
     hist[i] = 0;
-    tb.quota[i] = tp.log2edge[i];  // the edge ids, until the shares are known
     tb.phys[i] = reinterpret_cast<const int2*>(tp.log2phy)[i];
   }
   __syncthreads();
@@ -962,26 +1001,29 @@ __device__ __forceinline__ void worker_cta(const IdxT* __restrict__ idx, long lo
     const int c = hist[i];
     tb.cur[i] = c ? atomicAdd(&total_g[i], c) : 0;
   }
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&ws->arrive[epoch & 1], 1u);
+  if (threadIdx.x == 0) {  // every thread's atomics have returned: this CTA's counts are in the totals
+    red_release_gpu(&ws->arrive[epoch & 1], 1u);
     if (tracing) trace[1] = global_timer_ns();
-    s_ok = bounded_wait_ge<false>(&ws->lp_done, epoch, grid_timeout_ns);
-    if (!s_ok) {
-      atomicAdd(&status[kStTimeouts], 1);
-      raise_status(status, kErrLpTimeout, kPhRedirect, q);
+  }
+  const unsigned long long* result = ws_result(ws, e);
+  bool late = false;
+  for (int i = threadIdx.x; i < e; i += kBlock) {
+    unsigned long long word[2];
+    late = late || !wait_result(result + 2 * (size_t)i, epoch, grid_timeout_ns, word);
+    if (!late) {
+      tb.quota[i] = (int)(uint32_t)word[0];
+      tb.total[i] = (int)(uint32_t)word[1];
+    } else {  // no shares: half of a replicated expert's tokens stay
+      const int tot = __ldcg(&total_g[i]);
+      tb.total[i] = tot;
+      tb.quota[i] = tp.log2edge[i] < 0 ? tot : tot / 2;
     }
   }
-  __syncthreads();
-  const bool have_probs = s_ok;
-  for (int i = threadIdx.x; i < e; i += kBlock) {
-    const int tot = __ldcg(&total_g[i]);
-    tb.total[i] = tot;
-    const int edge = tb.quota[i];
-    tb.quota[i] = have_probs ? quota_of(tot, edge, probs) : (edge < 0 ? tot : tot / 2);
+  if (__syncthreads_or(late) && threadIdx.x == 0) {
+    atomicAdd(&status[kStTimeouts], 1);
+    raise_status(status, kErrLpTimeout, kPhRedirect, q);
   }
-  __syncthreads();
   redirect_keep(idx, begin, end, e, tb.cur, tb.total, tb.quota, tb.phys, out, keep);
   if (trace != nullptr) {  // tracing only: find the worker that leaves last
     __syncthreads();

@@ -38,7 +38,7 @@ bool shape_ok(const TopoDesc& t, bool need_solver = true, int solver = kSolverAu
 // Calls fn.template operator()<GP, D>() for the instantiation that covers the topology: GP = -1, -2, -4,
 // -8 for the tile solver with that many warps per group, 8, 16, 32 for the warp solver, 0 for the
 // thread-block solver (D is then the padded count).  The tile solver takes every group that it
-// covers (8 ranks 22.6 -> 11.3 us a call, 16 ranks 40.6 -> 16.9, 32 ranks 64 -> 27, 64 ranks 147 -> 63 against the
+// covers (8 ranks 22.6 -> 10.3 us a call, 16 ranks 40.6 -> 17.0, 32 ranks 64 -> 25, 64 ranks 147 -> 52 against the
 // other two), except that the warp solver packs four groups of 8 ranks into a warp: `packed` asks for
 // that where one CTA has more groups than warps.  The warp solver's larger groups run on request only.
 template <typename Fn>
@@ -79,10 +79,10 @@ size_t fused_smem(int e) { return sizeof(int) * 5 * (size_t)e; }
 size_t bundle_smem(const Topo& tp) { return sizeof(int) * (size_t)tp.n_group * tp.g * (tp.d + 1); }
 // bundle sums followed by the solver's scratch area, if it has one
 template <int GP>
-size_t solver_smem(const Topo& tp) {
-  if constexpr (GP > 0 || GP == -1) return bundle_smem(tp);
+size_t solver_smem(const Topo& tp, int teams = kWarps) {
+  if constexpr (GP > 0) return bundle_smem(tp);
   else return bundle_bytes_aligned(tp.n_group * tp.g, tp.d) +
-              (GP == 0 ? block_solver_smem_bytes(tp.g, padded_dup(tp.d)) : tile_solver_smem_bytes(tp.g, tp.d));
+              (GP == 0 ? block_solver_smem_bytes(tp.g, padded_dup(tp.d)) : tile_solver_smem_bytes(tp.g, tp.d, GP == -1 ? teams : 1));
 }
 // The fused kernel's one solver CTA has a warp for each of this many groups of 8 ranks.
 bool pack_groups(const Topo& tp) { return tp.n_group > kWarps; }
@@ -164,6 +164,7 @@ struct SolveLaunch {
       const int per_cta = warps * kPerWarp;
       const int grid = (tp.n_group + per_cta - 1) / per_cta;
       if constexpr (GP == -1) {
+        const size_t smem = solver_smem<GP>(tp, warps);
         if ((err = allow_smem(tile_solve_kernel<1, D>, smem)) != cudaSuccess) return err;
         tile_solve_kernel<1, D><<<grid + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
       } else {

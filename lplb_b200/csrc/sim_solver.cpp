@@ -95,28 +95,20 @@ void solve_batch_tiles(int g, int rows, const int* r2o, const int* o2r, int nb, 
   for (int b = 0; b < nb; ++b) {
     lplb_sim::run_block(32 * NB, [&](int tid) {
       const int warp = tid >> 5, lane = tid & 31, rank = 8 * warp + (lane >> 2);
-      const bool live = rank < g;
-      double wl[D], f[D], fx = 0.0;
-      int src[D], dst[D];
-      for (int k = 0; k < D; ++k) {
-        wl[k] = 0.0;
-        src[k] = dst[k] = rank;
-      }
-      if (live) {
-        fx = fixed[(size_t)b * g + rank];
-        for (int k = 0; k < D; ++k) {
-          wl[k] = w[((size_t)b * g + rank) * D + k];
-          src[k] = r2o[rank * D + k];
-          dst[k] = o2r[rank * D + k];
-        }
-      }
+      const int d = lane & (lplb::TileTeam<NB, D>::kLanes - 1);
+      const bool live = rank < g, real = live && d < D;
+      const double* mine = w + ((size_t)b * g + rank) * D;
+      double own = 0.0, f = 0.0;
+      if (live) own = fixed[(size_t)b * g + rank];
+      for (int k = 0; live && k < D; ++k) own += mine[k];
       lplb::IpmParams prm{max_iters, tol, anchor, anchor_valid, guard, snap_mu};
       double* group = anchor ? anchor + (size_t)b * g * (4 * D + 3) : nullptr;
       const lplb::IpmOutcome res = lplb::ipm_solve_tiles<NB, D>(
-          warp, lane, rows, wl, fx, src, dst, prm, f, live && anchor ? group + (size_t)rank * (4 * D + 3) : nullptr, group,
+          warp, lane, rows, real ? mine[d] : 0.0, live ? fixed[(size_t)b * g + rank] : 0.0, own, real ? r2o[rank * D + d] : rank,
+          real ? o2r[rank * D + d] : rank, prm, f, live && anchor ? group + (size_t)rank * (4 * D + 3) : nullptr, group,
           anchor ? anchor_valid + b : nullptr, scratch.data());
+      if (live && (lane & 3) < D) f_out[((size_t)b * g + rank) * D + d] = f;
       if (live && (lane & 3) == 0) {
-        for (int k = 0; k < D; ++k) f_out[((size_t)b * g + rank) * D + k] = f[k];
         if (rank == 0) {
           iters[b] = res.iters;
           converged[b] = res.converged ? 1 : 0;
