@@ -44,6 +44,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include "common.cuh"
 #include "tcgen05.cuh"
 
 namespace lplb {
@@ -250,6 +251,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const bool sender_cta = FUSED && (int)blockIdx.x >= n_gemm;
   unsigned long long* dbg = FUSED && args.debug ? args.debug + 4 * blockIdx.x : nullptr;
 
+  allow_successor();
   if (threadIdx.x == 0) {
     if (dbg) dbg[0] = timer_ns();
     abort_flag = 0;
@@ -266,6 +268,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     fence_barrier_init();
     tma_prefetch_desc(&tmap_w);
     for (int b = 0; b < kRowBoxes; ++b) tma_prefetch_desc(&rows.box[b]);
+  }
+  if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), kTmemCols);
+  wait_predecessors();
+  if (threadIdx.x == 0) {
     // every source rank must have finished writing this launch's A rows
     if (args.wait_flags != nullptr) {
       const uint64_t t0 = timer_ns();
@@ -284,7 +290,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       }
     }
   }
-  if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), kTmemCols);
   for (int e = threadIdx.x; e < args.n_experts; e += blockDim.x) {
     s_rows[e] = args.rows[e];
     s_start[e] = args.row_start[e];

@@ -123,8 +123,7 @@ cudaError_t launch_route(const LayerShape& sh, const LayerBuffers& b, const void
   const long long least = (a.n_pairs + 4 * kSupportThreads - 1) / (4 * kSupportThreads);
   if (grid < least) grid = least;
   if (grid < 1) grid = 1;
-  route_kernel<<<(unsigned)grid, kSupportThreads, sizeof(int) * 4 * P, stream>>>(a);
-  return cudaGetLastError();
+  return launch_after(route_kernel, (unsigned)grid, kSupportThreads, sizeof(int) * 4 * P, stream, a);
 }
 
 cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const void* x, const void* phys_idx,
@@ -154,8 +153,7 @@ cudaError_t launch_dispatch(const LayerShape& sh, const LayerBuffers& b, const v
   a.my_rank = sh.my_rank;
   a.capacity = sh.capacity;
   a.epoch = epoch;
-  dispatch_kernel<<<n_cta, kSupportThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+  return launch_after(dispatch_kernel, n_cta, kSupportThreads, 0, stream, a);
 }
 
 cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const void* phys_idx, int idx_is64,
@@ -178,8 +176,7 @@ cudaError_t launch_schedule(const LayerShape& sh, const LayerBuffers& b, const v
   a.n_ranks = sh.n_ranks;
   a.capacity = sh.capacity;
   const long long grid = (a.n_pairs + kSupportThreads - 1) / kSupportThreads;
-  schedule_kernel<<<(unsigned)(grid < 1 ? 1 : grid), kSupportThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+  return launch_after(schedule_kernel, (unsigned)(grid < 1 ? 1 : grid), kSupportThreads, 0, stream, a);
 }
 
 namespace {
@@ -245,8 +242,7 @@ cudaError_t launch_dispatch_gemm(const LayerShape& sh, const LayerBuffers& b, co
   auto kernel = grouped_gemm_kernel<kSwiGLU, true>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
   if (err != cudaSuccess) return err;
-  kernel<<<grid.tile + grid.send, kFusedThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
-  return cudaGetLastError();
+  return launch_after(kernel, grid.tile + grid.send, kFusedThreads, kGemmSmem, stream, maps.w, row_maps(maps), a);
 }
 
 cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmMaps& maps, int which, uint32_t epoch, unsigned long long timeout_ns,
@@ -274,7 +270,7 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmM
     auto kernel = grouped_gemm_kernel<kSwiGLU, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     if (err != cudaSuccess) return err;
-    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
+    return launch_after(kernel, n_cta, kGemmThreads, kGemmSmem, stream, maps.w, row_maps(maps), a);
   } else {
     a.n_tiles_w = sh.hidden / kBM;
     a.k_blocks = sh.inter / kBK;
@@ -289,9 +285,8 @@ cudaError_t launch_gemm(const LayerShape& sh, const LayerBuffers& b, const GemmM
     auto kernel = grouped_gemm_kernel<kScatter, false>;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     if (err != cudaSuccess) return err;
-    kernel<<<n_cta, kGemmThreads, kGemmSmem, stream>>>(maps.w, row_maps(maps), a);
+    return launch_after(kernel, n_cta, kGemmThreads, kGemmSmem, stream, maps.w, row_maps(maps), a);
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_combine(const LayerShape& sh, const LayerBuffers& b, const float* weights, void* out, int n_tokens,
@@ -310,8 +305,7 @@ cudaError_t launch_combine(const LayerShape& sh, const LayerBuffers& b, const fl
   a.n_ranks = sh.n_ranks;
   a.epoch = epoch;
   a.timeout_ns = timeout_ns;
-  combine_kernel<<<n_cta, kSupportThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+  return launch_after(combine_kernel, n_cta, kSupportThreads, 0, stream, a);
 }
 
 }  // namespace moe

@@ -80,6 +80,8 @@ __device__ __forceinline__ int warp_exclusive_prefix(int n, int lane, Get get, P
 // 512 pairs on 48 experts.
 __global__ void __launch_bounds__(kSupportThreads) route_kernel(const RouteArgs a) {
   extern __shared__ int sm[];
+  allow_successor();
+  wait_predecessors();
   const int P = a.n_ranks * a.n_local, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int* hist = sm;  // [P] this CTA's counts, then its first ordinal per expert
   __shared__ int s_last, s_missing;
@@ -244,6 +246,8 @@ struct ScheduleArgs {
 // Fused dispatch: for the k-th pair this rank sends to physical expert e: target row
 // dst_row_start[e] + k, return slot send_base[e] + k, send position order_base[e] + k.
 __global__ void __launch_bounds__(kSupportThreads) schedule_kernel(const ScheduleArgs a) {
+  allow_successor();
+  wait_predecessors();
   const int P = a.n_ranks * a.n_local;
   const long long stride = (long long)gridDim.x * kSupportThreads;
   for (long long i = (long long)blockIdx.x * kSupportThreads + threadIdx.x; i < a.n_pairs; i += stride) {
@@ -300,6 +304,8 @@ constexpr int kDispatchVec = 4;  // 16-byte vectors per lane and work item: an i
 // consecutive slots: the stores that cross NVLink walk through memory sequentially instead of
 // hitting a random page per row.
 __global__ void __launch_bounds__(kSupportThreads) dispatch_kernel(const DispatchArgs a) {
+  allow_successor();
+  wait_predecessors();
   const int P = a.n_ranks * a.n_local;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int vec_per_row = a.hidden / 8;  // 16-byte vectors per row
@@ -373,6 +379,7 @@ struct CombineArgs {
 // out[t] = sum_k weights[t, k] * comb[pair_slot[t * topk + k]], fp32 accumulation, after every rank has
 // signalled that its expert outputs for this launch are in place.
 __global__ void __launch_bounds__(kSupportThreads) combine_kernel(const CombineArgs a) {
+  wait_predecessors();
   __shared__ int ok;
   if (threadIdx.x == 0) {
     ok = 1;
