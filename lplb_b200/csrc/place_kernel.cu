@@ -8,12 +8,11 @@
 // the same sum as long as no partial sum can pass 2^53.  Where one could, the kernel writes no table
 // and reports it, and the host places the experts.  So the results are identical.
 //
-// One CTA.  What bounds it is the greedy packing, one dependent step per expert: a warp holds the
-// packs (one per lane up to 32) and finds the lightest with two 32-bit warp reductions over the
-// order-preserving halves of the double and a ballot, with no shared memory on the chain, instead
-// of five shuffle rounds of a double and an index.  The orders come from counting, for every
-// expert, the experts in front of it.  256 experts on 8 ranks: 32 us, 53 us for the whole call with its
-// wait for the device; on the host, some twenty tensor operations per expert, 8.9 ms.
+// One CTA.  What bounds it is the greedy packing, a chain of dependent rounds: a warp holds the
+// packs (one per lane up to 32), ranks them by load, and hands out an item to each at once as
+// far as the order of the items allows it.  The orders come from counting, for every
+// expert, the experts in front of it.  256 experts on 8 ranks: 21 us (one
+// item after the other 27 to 32), 43 us for the whole call with its wait for the device; on the host, some twenty tensor operations per expert, 8.9 ms.
 #include "place_api.h"
 
 #include <stdint.h>
@@ -51,17 +50,24 @@ __device__ __forceinline__ unsigned long long ordered(double x) {
 }
 
 // order[k] = the item with k items in front of it: heavier ones, and equal ones of lower index.
-// Rows of `n` items each, `rows` of them, by all threads of the CTA.
+// Rows of `n` items each, `rows` of them, by all threads of the CTA; several neighbouring threads
+// share an item where there are threads to spare (256 items: one 64-step pass instead of 256 steps).
 __device__ void sort_rows(const double* w, int* order, int rows, int n) {
-  for (int i = threadIdx.x; i < rows * n; i += kPlaceThreads) {
-    const int base = i / n * n, me = i - base;
-    const double mine = w[i];
+  int parts = 1;
+  while (parts < 32 && parts * 2 * rows * n <= kPlaceThreads) parts *= 2;
+  const int part = threadIdx.x & (parts - 1);
+  for (int base_slot = 0; base_slot < rows * n * parts; base_slot += kPlaceThreads) {
+    const int i = (base_slot + (int)threadIdx.x) / parts;
+    const bool item = i < rows * n;
+    const int base = item ? i / n * n : 0, me = item ? i - base : 0;
+    const double mine = w[base + me];
     int front = 0;
-    for (int j = 0; j < n; ++j) {
+    for (int j = part; j < n; j += parts) {
       const double other = w[base + j];
       front += other > mine || (other == mine && j < me);
     }
-    order[base + front] = me;
+    for (int o = parts / 2; o > 0; o >>= 1) front += __shfl_xor_sync(kAll, front, o);
+    if (item && part == 0) order[base + front] = me;
   }
 }
 
@@ -71,30 +77,58 @@ template <typename Put>
 __device__ void pack_items(const double* w, const int* order, int n, int packs, int cap, double* load, int* fill,
                            Put put) {
   const int lane = threadIdx.x & 31;
-  if (packs <= 32) {  // a pack per lane, in registers
+  if (packs == 1) {
+    for (int k = lane; k < n; k += 32) put(order[k], 0, k);
+    return;
+  }
+  if (packs <= 32) {
+    // A pack per lane, in registers.  A round hands out one item to each of the lightest packs at once: the
+    // j-th next item goes to the j-th lightest pack, as one after the other it would, as long as that
+    // pack is lighter than every pack is after its item of this round.  So many items of the round
+    // count, at least the first.  (Loads drawn like gate logits: 34 rounds for 256 items on 8 packs; a
+    // Zipf history 99.)
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(load);
     double mine = 0.0;
     int held = 0;
-    int item = order[0];
-    double weight = w[item];
-    // left to the compiler the unrolling moves with lines elsewhere in the kernel (one launch after
-    // the other: 31 or 35 us, with 8 steps 29)
-#pragma unroll 8
-    for (int step = 0; step < n; ++step) {
-      const int next = order[min(step + 1, n - 1)];
-      const double next_weight = w[next];
+    for (int step = 0; step < n;) {
       const bool room = lane < packs && held < cap;
       const unsigned long long key = room ? ordered(mine) : ~0ull;
-      const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-      const unsigned least_hi = __reduce_min_sync(kAll, hi);
-      const unsigned least_lo = __reduce_min_sync(kAll, hi == least_hi ? lo : ~0u);
-      const int pack = __ffs(__ballot_sync(kAll, room && hi == least_hi && lo == least_lo)) - 1;
-      if (lane == pack) {
+      if (lane < packs) {
+        keys[lane] = key;
+        fill[lane] = cap - held;
+      }
+      __syncwarp();
+      int rank = 0;  // packs with room in front of this one
+#pragma unroll 4
+      for (int q = 0; q < packs; ++q) {
+        const unsigned long long other = keys[q];
+        rank += other < key || (other == key && q < lane);
+      }
+      const int takers = min(__popc(__ballot_sync(kAll, room)), n - step);
+      const bool takes = room && rank < takers;
+      const int item = order[step + (takes ? rank : 0)];
+      const double weight = w[item], grown = mine + weight;
+      if (__ballot_sync(kAll, takes && rank == 0 && weight == 0.0) && w[order[n - 1]] == 0.0) {
+        // nothing but empty items left: they fill up the packs, the lightest first
+        int at = step;
+        for (int q = 0; q < packs; ++q) {
+          const unsigned long long other = keys[q];
+          if (other < key || (other == key && q < lane)) at += fill[q];
+        }
+        if (room)
+          for (int k = held; k < cap && at < n; ++k, ++at) put(order[at], lane, k);
+        return;
+      }
+      const unsigned long long after = takes ? ordered(grown) : ~0ull;
+      const unsigned hi = (unsigned)(after >> 32), least_hi = __reduce_min_sync(kAll, hi);
+      const unsigned least_lo = __reduce_min_sync(kAll, hi == least_hi ? (unsigned)after : ~0u);
+      const bool counts = takes && (rank == 0 || key < ((unsigned long long)least_hi << 32 | least_lo));
+      step += __popc(__ballot_sync(kAll, counts));
+      if (counts) {
         put(item, lane, held);
-        mine += weight;
+        mine = grown;
         ++held;
       }
-      item = next;
-      weight = next_weight;
     }
     return;
   }

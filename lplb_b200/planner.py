@@ -121,11 +121,11 @@ class Planner:
         :param exchange_node_size: run the in-kernel statistics exchange in two levels, inside
             nodes of this many consecutive ranks and then between nodes (the schedule for a
             topology that spans nodes, e.g. ``torus(2, 4)`` with 4); 0 = one all-to-all level.
-        :param solver: device LP solver: ``"warp"`` keeps a group of up to 32 ranks (4 replicas
-            per rank) in one warp's registers, ``"block"`` solves a group of up to 128 ranks
-            (8 replicas per rank) with one thread block and the matrix in shared memory,
-            ``"auto"`` uses the warp solver up to 8 ranks and the block solver above.  Larger
-            groups run the same method as tensor ops on the planner's device.
+        :param solver: device LP solver: ``"warp"`` solves a group of up to 32 ranks (4 replicas
+            per rank) with one warp, ``"block"`` a group of up to 128 ranks (8 replicas per rank)
+            with as many warps of a thread block as it needs, ``"auto"`` uses one warp up to
+            8 ranks and the block above.  Larger groups run the same method as tensor ops on
+            the planner's device.
         """
         if device is None:
             device = "cuda" if torch.cuda.is_available() else "cpu"
@@ -328,7 +328,7 @@ class Planner:
         return self.mapping.phy2log, self.mapping.log2phy, self.mapping.logcnt
 
     def _place_on_device(self, workload: torch.Tensor | None) -> tuple | None:
-        """The same placement and tables from one kernel and one wait for it (256 experts: 53 us,
+        """The same placement and tables from one kernel and one wait for it (256 experts: 43 us,
         8.9 ms on the host), or ``None`` where the host has to do it.  Histories of whole numbers
         only: their sums are exact in any order up to 2^53 (the kernel finds out whether a sum
         could pass that), and they hold no NaN or infinity, for which the host's sort and arg-min

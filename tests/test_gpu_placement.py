@@ -125,3 +125,23 @@ def test_tables_that_disagree_with_the_topology_are_refused(entry):
     idx = torch.arange(32, device="cuda").unsqueeze(1)
     assert torch.equal(before[planner.run(idx, avail).long()].long(), idx)  # the engine's tables are untouched
     planner.update_redundancy_mapping(torch.arange(32))
+
+
+@pytest.mark.parametrize("ranks,ll", [(2, 40), (8, 5), (8, 32), (16, 7), (32, 16), (33, 3)])
+def test_packing_in_rounds_places_like_one_item_after_the_other(ranks, ll):
+    """Histories where few items of a round count (a pack far below the others takes several in a
+    row), where all do, and where empty experts fill up what is left."""
+    n = ranks * ll
+    r2o = ring(ranks)
+    planner = Planner(r2o, n + ranks, n, ranks, device="cuda", n_nodes=1)
+    k = torch.arange(1, n + 1)
+    zipf = (1e6 / k**1.2).long()
+    some = (torch.arange(n) % 3 == 0).long() * (k % 7 + 1)  # two thirds empty
+    giant = torch.ones(n, dtype=torch.long)
+    giant[n // 2] = 10**9
+    halves = (2.0 ** (40 - (k % 40))).long()
+    for hist in (zipf, zipf.flip(0), some, giant, giant - 1, halves, k):
+        want = build_mapping(r2o, 1, ll, 1, hist, n_nodes=1)
+        got = planner.update_redundancy_mapping(hist.cuda())
+        for a, b in zip(got, (want.phy2log, want.log2phy, want.logcnt)):
+            assert torch.equal(a.cpu(), b)
