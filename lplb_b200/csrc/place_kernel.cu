@@ -11,8 +11,9 @@
 // One CTA.  What bounds it is the greedy packing, a chain of dependent rounds: a warp holds the
 // packs (one per lane up to 32), ranks them by load, and hands out an item to each at once as
 // far as the order of the items allows it.  The orders come from counting, for every
-// expert, the experts in front of it.  256 experts on 8 ranks: 21 us (one
-// item after the other 27 to 32), 43 us for the whole call with its wait for the device; on the host, some twenty tensor operations per expert, 8.9 ms.
+// expert, the experts in front of it.  256 experts on 8 ranks: 21 us (one item after the
+// other 27 to 32), 43 us for the whole call with its wait for the device; on the host, some twenty
+// tensor operations per expert, 8.9 ms.
 #include "place_api.h"
 
 #include <stdint.h>
