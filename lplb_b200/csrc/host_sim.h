@@ -125,8 +125,6 @@ inline To bits(From v) {
 inline int hi_word(double x) { return (int)(bits<uint64_t>(x) >> 32); }
 inline int lo_word(double x) { return (int)(uint32_t)bits<uint64_t>(x); }
 inline double from_words(int hi, int lo) { return bits<double>(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo); }
-inline float bits_float(unsigned v) { return bits<float>(v); }
-inline unsigned float_bits(float v) { return bits<unsigned>(v); }
 
 // Run fn(lane) on 32 lock-stepped lanes.
 inline void run_warp(const std::function<void(int)>& fn) {

@@ -76,8 +76,6 @@ __device__ __forceinline__ double rcp3(double x) {
 }
 
 #ifdef LPLB_HOST_SIM
-using lplb_sim::bits_float;
-using lplb_sim::float_bits;
 using lplb_sim::from_words;
 using lplb_sim::hi_word;
 using lplb_sim::lo_word;
@@ -85,34 +83,20 @@ using lplb_sim::lo_word;
 __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
 __device__ __forceinline__ int lo_word(double x) { return __double2loint(x); }
 __device__ __forceinline__ double from_words(int hi, int lo) { return __hiloint2double(hi, lo); }
-__device__ __forceinline__ unsigned float_bits(float x) { return __float_as_uint(x); }
-__device__ __forceinline__ float bits_float(unsigned x) { return __uint_as_float(x); }
 #endif
 
-// The variable of this lane that bounds the step most, by how much of itself it would lose (`loss` =
-// -dx / x).  Compared as unsigned integers that order like the doubles in [1/2, 2^63), with 26 bits behind
-// the binary point; a loss below 1/2 bounds no step.  Three integer instructions a variable, where a maximum
-// of doubles takes 24 cycles.
-struct StepBound {
-  unsigned key = 0;
-  double x = 1.0, dx = -1.0;
-  __device__ __forceinline__ void add(double loss, double x_, double dx_) {
-    const unsigned hi = (unsigned)max(hi_word(loss), 0x3FE00000) - 0x3FE00000u;
-    const unsigned k = (hi << 6) | ((unsigned)lo_word(loss) >> 26);
-    if (k > key) {
-      key = k;
-      x = x_;
-      dx = dx_;
-    }
-  }
-  // The step that takes it to its bound, a quotient of floats as in the other solvers (another rounding
-  // here moves the last iterates, and so the shares, by up to 1e-5), as an integer whose maximum over
-  // lanes is the shortest step.
-  __device__ __forceinline__ unsigned shortest() const { return ~float_bits(key != 0 ? __fdividef((float)x, -(float)dx) : 3.0e38f); }
-};
-// min(limit * step, 1)
-__device__ __forceinline__ double step_from(unsigned shortest, double limit) {
-  const double a = limit * (double)bits_float(~shortest);
+// A step of length 1 / x, or `limit` / x, keeps one variable at its bound; only the largest x counts,
+// and only if it is above `limit`.  x in [1/2, 2^63) as an unsigned integer that orders like it, with 26
+// bits behind the binary point, the rest cut off (the float ratios of the other solvers carry 23);
+// anything below 1/2, negative numbers too, becomes 0.  Three integer instructions.
+__device__ __forceinline__ unsigned step_key(double x) {
+  const unsigned hi = (unsigned)max(hi_word(x), 0x3FE00000) - 0x3FE00000u;
+  return (hi << 6) | ((unsigned)lo_word(x) >> 26);
+}
+// min(limit / (the number behind `key`), 1)
+__device__ __forceinline__ double step_from_key(unsigned key, double limit) {
+  const double x = from_words((int)((key >> 6) + 0x3FE00000u), (int)(key << 26));
+  const double r = rcp_seed(x), a = limit * fma(r, fma(-x, r, 1.0), r);
   return hi_word(a) >= 0x3FF00000 ? 1.0 : a;
 }
 // min(max(x, 0), 1)
@@ -690,13 +674,8 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     double df = fma(dt, e_b, e), dv = r_u - df, dz = fma(-zi, df, -z), dq = fma(-qv, dv, -q);
     // the predictor takes every complementarity product to zero, so dz / z = -1 - df / f, and so on
     const double tf = -df * inv_f, tv = -dv * inv_v, ty = -dy * inv_y;
-    StepBound primal_bound, dual_bound;
-    primal_bound.add(1.0 - ty, s, ds);
-    primal_bound.add(tf, f, df);
-    primal_bound.add(tv, v, dv);
-    dual_bound.add(ty, y, dy);
-    dual_bound.add(1.0 - tf, z, dz);
-    dual_bound.add(1.0 - tv, q, dq);
+    unsigned key_p = max(step_key(1.0 - ty), max(step_key(tf), step_key(tv)));
+    unsigned key_d = max(step_key(ty), max(step_key(1.0 - tf), step_key(1.0 - tv)));
     double c_p = real ? fma(z, df, q * dv) : 0.0, c_pd = real ? fma(df, dz, dv * dq) : 0.0;
     if (first) {
       c_p = fma(y, ds, c_p);
@@ -706,8 +685,8 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     const double rc = rd - p_f + p_v, x_cor = wt * rc;
     tm.put_edge(kEdgeCor, x_cor);
     if (!live) c_p = c_pd = 0.0;
-    unsigned key_p = tm.key_put(0, live && real ? primal_bound.shortest() : 0u);
-    unsigned key_d = tm.key_put(1, live && real ? dual_bound.shortest() : 0u);
+    key_p = tm.key_put(0, live && real ? key_p : 0u);
+    key_d = tm.key_put(1, live && real ? key_d : 0u);
     tm.sum_put(kSumAffine, c_p, c_pd);
     tm.sync();
     // ---- corrector ---------------------------------------------------------------------------
@@ -715,7 +694,7 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     const double g0 = live ? load - t - p_s + c_edges : 0.0;
     tm.put(kVecG0, g0);
     tm.sum_get(kSumAffine, c_p, c_pd);
-    const double ap0 = step_from(tm.key_get(0, key_p), 1.0), ad0 = step_from(tm.key_get(1, key_d), 1.0);
+    const double ap0 = step_from_key(tm.key_get(0, key_p), 1.0), ad0 = step_from_key(tm.key_get(1, key_d), 1.0);
     // complementarity after the affine step; sum x dz = -kcomp mu - sum z dx
     const double comp_aff = fma(ap0 * ad0, c_pd, fma(ap0 - ad0, c_p, kcomp * mu * (1.0 - ad0)));
     const double ratio = clamp01(comp_aff * inv_mu);
@@ -750,17 +729,12 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     dv = r_u - df;
     dz = fma(-zi, df, fma(sig_mu, inv_f, -z - p_f));
     dq = fma(-qv, dv, fma(sig_mu, inv_v, -q - p_v));
-    primal_bound = dual_bound = StepBound();
-    primal_bound.add(-ds * rcp_seed(s), s, ds);
-    primal_bound.add(-df * inv_f, f, df);
-    primal_bound.add(-dv * inv_v, v, dv);
-    dual_bound.add(-dy * inv_y, y, dy);
-    dual_bound.add(-dz * rcp_seed(z), z, dz);
-    dual_bound.add(-dq * rcp_seed(q), q, dq);
-    key_p = tm.key_put(2, live && real ? primal_bound.shortest() : 0u);
-    key_d = tm.key_put(3, live && real ? dual_bound.shortest() : 0u);
+    key_p = max(step_key(-ds * rcp_seed(s)), max(step_key(-df * inv_f), step_key(-dv * inv_v)));
+    key_d = max(step_key(-dy * inv_y), max(step_key(-dz * rcp_seed(z)), step_key(-dq * rcp_seed(q))));
+    key_p = tm.key_put(2, live && real ? key_p : 0u);
+    key_d = tm.key_put(3, live && real ? key_d : 0u);
     tm.sync();
-    const double ap = step_from(tm.key_get(2, key_p), kEta), ad = step_from(tm.key_get(3, key_d), kEta);
+    const double ap = step_from_key(tm.key_get(2, key_p), kEta), ad = step_from_key(tm.key_get(3, key_d), kEta);
     t = fma(ap, dt, t);
     if (live) {
       s = fma(ap, ds, s);

@@ -284,9 +284,9 @@ def _solve_tiles(lib, r2o, w, fixed, rows=None, max_iters=24, tol=1e-4, anchor=N
 ])
 def test_tile_solver_device_code_matches_the_torch_restatement(sim, g, offsets):
     """Group sizes at the edges of the tile counts (1, 2, 4 and 8 warps), with rows that are only padding, and
-    offsets of half the group, whose two terms fall into one column of the normal matrix.  The step lengths are
-    floats here and doubles in the oracle (6e-8 each, at most seven iterations, and the conditioning of
-    the last ones); 1e-5 is what the other solvers are held to."""
+    offsets of half the group, whose two terms fall into one column of the normal matrix.  The
+    iterates differ by the rounding of the step lengths (2^-26, times at most seven iterations and
+    the conditioning of the last ones); 1e-5 is what the other solvers are held to."""
     r2o = topology.circulant(g, offsets)
     d = r2o.shape[1]
     gen = torch.Generator().manual_seed(7)
@@ -304,35 +304,26 @@ def test_tile_solver_device_code_matches_the_torch_restatement(sim, g, offsets):
 
 
 @pytest.mark.parametrize("name", ["cube", "ring5", "hypercube"])
-def test_tile_solver_warm_start_follows_the_warp_solver(sim, name):
-    """Same decisions, iterations and shares over a stream and a shift, each with an anchor of its own.
-    Both round their step lengths to the same floats, so only the order of float64 sums is between
-    them; 1e-6 leaves that room for the conditioning of the last iterates."""
+def test_tile_solver_warm_start_follows_the_torch_restatement(sim, name):
     r2o = topology.by_name(name)
     g, d = r2o.shape
     gen = torch.Generator().manual_seed(13)
     mean = (torch.rand(g, 8, generator=gen, dtype=torch.float64) + 0.5) * 4096
-    anchor, valid = np.zeros((1, g, 4 * d + 3)), np.zeros(1, np.int32)
-    anchor_w, valid_w = anchor.copy(), valid.copy()
-    r = np.ascontiguousarray(r2o.numpy().astype(np.int32))
-    o = np.ascontiguousarray(topology.invert_r2o(r2o).numpy().astype(np.int32))
-    ptr = lambda a: ctypes.c_void_p(a.ctypes.data)  # noqa: E731
-    used = []
+    anchor_c, valid_c, anchor_t = np.zeros((1, g, 4 * d + 3)), np.zeros(1, np.int32), None
+    seen = []
     for step in range(4):
         if step == 3:
             mean = mean.flip(0) * torch.linspace(0.3, 2.0, 8, dtype=torch.float64)
         cnt = (mean * (1 + 0.02 * torch.randn(g, 8, generator=gen, dtype=torch.float64))).floor().unsqueeze(0)
         w, fixed = cnt[:, :, :d].contiguous(), cnt[:, :, d:].sum(-1)
-        f, iters, conv = _solve_tiles(sim, r2o, w, fixed, rows=max(g, 8), anchor=anchor, valid=valid)
-        wa, fa = np.ascontiguousarray(w.numpy()), np.ascontiguousarray(fixed.numpy())
-        fw, itw, convw = np.zeros((1, g, d)), np.zeros(1, np.int32), np.zeros(1, np.int32)
-        assert sim.lplb_sim_solve_warm(g, d, ptr(r), ptr(o), 1, ptr(wa), ptr(fa), 24, ctypes.c_double(1e-4), ptr(fw), ptr(itw),
-                                       ptr(convw), ptr(anchor_w), ptr(valid_w), ctypes.c_double(0.1), ctypes.c_double(1e-3)) == 0
-        assert conv[0] == convw[0] == 1 and iters[0] == itw[0]
-        assert float((f - torch.from_numpy(fw)).abs().max()) < 1e-6
-        used.append(int(iters[0]))
-    assert used[1] <= used[0] and used[2] <= used[0]
-    assert np.abs(anchor - anchor_w).max() < 1e-5
+        ref = lp.solve_ipm(w, fixed, r2o, tol=1e-4, warm_start=True, anchor=anchor_t, guard=0.1)
+        anchor_t = ref.anchor
+        f, iters, conv = _solve_tiles(sim, r2o, w, fixed, anchor=anchor_c, valid=valid_c)
+        assert conv[0] == 1 and int(iters[0]) == int(ref.iters[0])
+        assert float((f - ref.f).abs().max()) < 1e-5
+        seen.append((bool(ref.warm[0]), int(iters[0])))
+    assert [s[0] for s in seen] == [False, True, True, name == "ring5"]  # the small shift of five loads stays in the guard
+    assert seen[1][1] < seen[0][1]
 
 
 def test_tile_solver_handles_empty_groups_and_the_iteration_cap(sim):
