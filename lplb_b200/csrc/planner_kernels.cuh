@@ -510,6 +510,8 @@ template <int NB, int D>
 __global__ void __launch_bounds__(kBlock) tile_solve_kernel(const int* __restrict__ workload, Topo tp, IpmParams prm,
                                                             float* __restrict__ probs, float* __restrict__ normalised,
                                                             Counter avail, int* status, int teams) {
+  allow_successor();
+  wait_predecessors();
   if (blockIdx.x == gridDim.x - 1) {
     normalise_counts(workload, tp.e, normalised);
     return;

@@ -151,7 +151,7 @@ struct SolveLaunch {
       }();
       if ((err = allow_smem(kernel, smem)) != cudaSuccess) return err;
       if constexpr (GP == 0) kernel<<<tp.n_group, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status);
-      else kernel<<<tp.n_group + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, 1);
+      else return launch_after(kernel, tp.n_group + 1, kBlock, smem, stream, workload, tp, prm, probs, normalised, avail, status, 1);
     } else {
       // As few solving warps per CTA as still fit the groups on one wave of CTAs.
       constexpr int kPerWarp = GP == -1 ? 1 : 32 / GP;
@@ -166,7 +166,9 @@ struct SolveLaunch {
       if constexpr (GP == -1) {
         const size_t smem = solver_smem<GP>(tp, warps);
         if ((err = allow_smem(tile_solve_kernel<1, D>, smem)) != cudaSuccess) return err;
-        tile_solve_kernel<1, D><<<grid + 1, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
+        // an early launch: 14.3 -> 11.6 us for 64 groups of 8 ranks, one call after the other, 64 ranks 59 -> 52
+        return launch_after(tile_solve_kernel<1, D>, grid + 1, kBlock, smem, stream, workload, tp, prm, probs, normalised, avail,
+                            status, warps);
       } else {
         if ((err = allow_smem(solve_kernel<GP, D>, smem)) != cudaSuccess) return err;
         solve_kernel<GP, D><<<grid, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
