@@ -200,6 +200,7 @@ inline T __reduce_max_sync(unsigned, T v) {
   return best;
 }
 inline int max(int a, int b) { return a > b ? a : b; }
+inline int min(int a, int b) { return a < b ? a : b; }
 inline unsigned max(unsigned a, unsigned b) { return a > b ? a : b; }
 inline double rsqrt(double x) { return 1.0 / std::sqrt(x); }
 inline float __fdividef(float a, float b) { return a / b; }

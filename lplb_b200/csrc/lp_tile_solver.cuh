@@ -87,10 +87,11 @@ __device__ __forceinline__ double from_words(int hi, int lo) { return __hiloint2
 
 // A step of length 1 / x, or `limit` / x, keeps one variable at its bound; only the largest x counts,
 // and only if it is above `limit`.  x in [1/2, 2^63) as an unsigned integer that orders like it, with 26
-// bits behind the binary point, the rest cut off (the float ratios of the other solvers carry 23);
-// anything below 1/2, negative numbers too, becomes 0.  Three integer instructions.
+// bits behind the binary point, the rest cut off (the float ratios of the other solvers carry 23).
+// Anything below 1/2, negative numbers too, becomes at most 63, which stands for a step of 1; anything from
+// 2^63 on, infinity too, one of the 64 largest keys, which stand for next to none.
 __device__ __forceinline__ unsigned step_key(double x) {
-  const unsigned hi = (unsigned)max(hi_word(x), 0x3FE00000) - 0x3FE00000u;
+  const unsigned hi = (unsigned)min(max(hi_word(x), 0x3FE00000), 0x43DFFFFF) - 0x3FE00000u;
   return (hi << 6) | ((unsigned)lo_word(x) >> 26);
 }
 // min(limit / (the number behind `key`), 1)

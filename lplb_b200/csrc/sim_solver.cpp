@@ -176,3 +176,11 @@ extern "C" int lplb_sim_solve(int g, int d, const int* r2o, const int* o2r, int 
   return lplb_sim_solve_warm(g, d, r2o, o2r, nb, w, fixed, max_iters, tol, f_out, iters, converged, nullptr, nullptr,
                              0.05, 1e-3);
 }
+
+// The step lengths' keys: `keys` and `steps` [n] of the values x and of one `limit`.
+extern "C" void lplb_sim_step_keys(int n, const double* x, double limit, unsigned* keys, double* steps) {
+  for (int i = 0; i < n; ++i) {
+    keys[i] = lplb::step_key(x[i]);
+    steps[i] = lplb::step_from_key(keys[i], limit);
+  }
+}

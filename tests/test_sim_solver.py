@@ -336,3 +336,28 @@ def test_tile_solver_handles_empty_groups_and_the_iteration_cap(sim):
         fixed = torch.rand(1, g, dtype=torch.float64, generator=torch.Generator().manual_seed(2)) * 1000
         f, iters, conv = _solve_tiles(sim, r2o, w, fixed, max_iters=1, tol=1e-9)
         assert conv[0] == 0 and iters[0] == 1 and bool(((f >= 0) & (f <= 1)).all())
+
+
+def _step_keys(lib, x, limit):
+    x = np.ascontiguousarray(x, dtype=np.float64)
+    keys, steps = np.zeros(len(x), np.uint32), np.zeros(len(x))
+    lib.lplb_sim_step_keys(len(x), ctypes.c_void_p(x.ctypes.data), ctypes.c_double(limit), ctypes.c_void_p(keys.ctypes.data),
+                           ctypes.c_void_p(steps.ctypes.data))
+    return keys, steps
+
+
+def test_step_keys_order_like_their_values_over_the_whole_range(sim):
+    """From 2^63 on a key is one of the largest 64, whose step is next to nothing, instead of starting
+    over at the small ones; a truncated value is at most 2^-26 of itself too small."""
+    rng = np.random.default_rng(0)
+    x = np.sort(np.concatenate([[0.5, 0.995, 1.0, 2.0**62, np.nextafter(2.0**63, 0)], 2.0 ** rng.uniform(-1, 63, 2000)]))
+    small = [-np.inf, -1e300, -1.0, -0.0, 0.0, 5e-324, 1e-9, 0.25, 0.4999999]
+    huge = [2.0**63, 9.3e18, 2.0**64, 1e25, 1e300, np.inf]
+    for limit in (1.0, 0.995):
+        keys, steps = _step_keys(sim, x, limit)
+        assert bool((np.diff(keys.astype(np.int64)) >= 0).all())
+        assert float(np.abs(steps * np.maximum(x, limit) / limit - 1).max()) < 2.0**-25
+        keys, steps = _step_keys(sim, small, limit)
+        assert bool((keys < 64).all()) and bool((steps == 1.0).all())
+        keys, steps = _step_keys(sim, huge, limit)
+        assert bool((keys >= 2**32 - 64).all()) and bool((steps <= 2.0**-62).all())
