@@ -558,6 +558,15 @@ class PlannerEngine {
   bool cooperative_ = true;
 };
 
+torch::Tensor debug_reciprocals(const torch::Tensor& x) {
+  LPLB_CHECK(x.is_cuda() && x.dtype() == torch::kFloat64 && x.is_contiguous() && x.numel() > 0, "x must be a float64 CUDA tensor");
+  c10::cuda::CUDAGuard guard(x.device());
+  auto out = torch::empty({2, x.numel()}, x.options());
+  LPLB_CUDA(lplb::launch_debug_reciprocals(x.data_ptr<double>(), (int)x.numel(), out.data_ptr<double>(),
+                                           at::cuda::getCurrentCUDAStream()));
+  return out;
+}
+
 }  // namespace
 
 void bind_moe(py::module_& m);  // moe_binding.cpp
@@ -601,6 +610,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("n_logical", &PlannerEngine::n_logical)
       .def("has_native_solver", &PlannerEngine::has_native_solver)
       .def("max_fused_ctas", &PlannerEngine::max_fused_ctas);
+  m.def("debug_reciprocals", &debug_reciprocals);
   bind_moe(m);
   m.attr("MAX_GROUP_SIZE") = lplb::kMaxGroupSize;
   m.attr("MAX_DUP") = lplb::kMaxDup;

@@ -124,6 +124,12 @@ inline To bits(From v) {
 }
 inline int hi_word(double x) { return (int)(bits<uint64_t>(x) >> 32); }
 inline int lo_word(double x) { return (int)(uint32_t)bits<uint64_t>(x); }
+// rcp.approx.ftz.f64 as the PTX manual describes it: 20 bits of mantissa in, 20 bits out.
+inline double rcp_approx(double x) {
+  const double in = bits<double>(bits<uint64_t>(x) & 0xFFFFFFFF00000000ull);
+  const double out = 1.0 / (std::fpclassify(in) == FP_SUBNORMAL ? std::copysign(0.0, in) : in);
+  return bits<double>(bits<uint64_t>(std::fpclassify(out) == FP_SUBNORMAL ? std::copysign(0.0, out) : out) & 0xFFFFFFFF00000000ull);
+}
 inline double from_words(int hi, int lo) { return bits<double>(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo); }
 
 // Run fn(lane) on 32 lock-stepped lanes.

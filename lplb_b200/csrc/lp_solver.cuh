@@ -98,7 +98,7 @@ __device__ __forceinline__ float ratio_to_bound(double val, double dval) {
   return dval < 0.0 ? __fdividef((float)val, -(float)dval) : 3.0e38f;
 }
 
-// 1/x for a positive, finite double: the hardware's ~2^-23 approximation refined by two
+// 1/x for a positive, finite double: the hardware's approximation (20 bits) refined by two
 // Newton steps (error squared each time), five dependent instructions instead of the
 // forty-odd of an IEEE division.  Relative error is a few ulp, far below the solver's needs.
 __device__ __forceinline__ double fast_rcp(double x) {

@@ -58,21 +58,28 @@ __device__ __forceinline__ void mma8(double& d0, double& d1, double a, double b,
 #endif
 }
 
-// The hardware's approximation of 1/x, relative error about 2^-23.
+// The hardware's approximation of 1/x.  By the PTX manual it reads the upper 32 bits of x, of them 20 of the
+// mantissa, and returns as many, so its relative error is near 2^-20; subnormals count as zeros.
 __device__ __forceinline__ double rcp_seed(double x) {
 #ifdef LPLB_HOST_SIM
-  return 1.0 / x;
+  return lplb_sim::rcp_approx(x);
 #else
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   return r;
 #endif
 }
-// 1/x to a few ulp: one third-order step on the approximation, r (1 + e + e^2) with e = 1 - x r.
+// 1/x to a few ulp: one step of Householder's method of third order, r (1 + e + e^2) with e = 1 - x r.
 // Three dependent operations where two Newton steps take four.
 __device__ __forceinline__ double rcp3(double x) {
   const double r = rcp_seed(x), e = fma(-x, r, 1.0);
   return fma(r, fma(e, e, e), r);
+}
+// 1/x to about 2^-38, one Newton step: enough for the 26 bits of a step length, where the approximation
+// alone is not.
+__device__ __forceinline__ double rcp2(double x) {
+  const double r = rcp_seed(x);
+  return fma(r, fma(-x, r, 1.0), r);
 }
 
 #ifdef LPLB_HOST_SIM
@@ -97,9 +104,11 @@ __device__ __forceinline__ unsigned step_key(double x) {
 // min(limit / (the number behind `key`), 1)
 __device__ __forceinline__ double step_from_key(unsigned key, double limit) {
   const double x = from_words((int)((key >> 6) + 0x3FE00000u), (int)(key << 26));
-  const double r = rcp_seed(x), a = limit * fma(r, fma(-x, r, 1.0), r);
+  const double a = limit * rcp2(x);
   return hi_word(a) >= 0x3FF00000 ? 1.0 : a;
 }
+// What a step length of one does to a variable x > 0, in units of x: the ratio that becomes a key.
+__device__ __forceinline__ double step_ratio(double x, double dx) { return -dx * rcp2(x); }
 // min(max(x, 0), 1)
 __device__ __forceinline__ double clamp01(double x) {
   const int hi = hi_word(x);
@@ -730,8 +739,8 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     dv = r_u - df;
     dz = fma(-zi, df, fma(sig_mu, inv_f, -z - p_f));
     dq = fma(-qv, dv, fma(sig_mu, inv_v, -q - p_v));
-    key_p = max(step_key(-ds * rcp_seed(s)), max(step_key(-df * inv_f), step_key(-dv * inv_v)));
-    key_d = max(step_key(-dy * inv_y), max(step_key(-dz * rcp_seed(z)), step_key(-dq * rcp_seed(q))));
+    key_p = max(step_key(step_ratio(s, ds)), max(step_key(-df * inv_f), step_key(-dv * inv_v)));
+    key_d = max(step_key(-dy * inv_y), max(step_key(step_ratio(z, dz)), step_key(step_ratio(q, dq))));
     key_p = tm.key_put(2, live && real ? key_p : 0u);
     key_d = tm.key_put(3, live && real ? key_d : 0u);
     tm.sync();

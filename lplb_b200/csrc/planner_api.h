@@ -91,4 +91,7 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
 // shape has no device solver or its tables do not fit shared memory).
 int max_fused_ctas(const TopoDesc& topo, int solver, int idx_is64);
 
+// For the tests: out [2][n] = 1 / x as the tile solver takes it, and the ratio behind a step of -1 from x.
+cudaError_t launch_debug_reciprocals(const double* x, int n, double* out, cudaStream_t stream);
+
 }  // namespace lplb

@@ -298,4 +298,19 @@ int max_fused_ctas(const TopoDesc& topo, int solver, int idx_is64) {
   return result;
 }
 
+namespace {
+__global__ void debug_reciprocals_kernel(const double* __restrict__ x, int n, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = rcp3(x[i]);
+  out[n + i] = step_ratio(x[i], -1.0);
+}
+}  // namespace
+
+cudaError_t launch_debug_reciprocals(const double* x, int n, double* out, cudaStream_t stream) {
+  if (n < 1) return cudaErrorInvalidValue;
+  debug_reciprocals_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, stream>>>(x, n, out);
+  return cudaGetLastError();
+}
+
 }  // namespace lplb

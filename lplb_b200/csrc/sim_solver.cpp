@@ -184,3 +184,11 @@ extern "C" void lplb_sim_step_keys(int n, const double* x, double limit, unsigne
     steps[i] = lplb::step_from_key(keys[i], limit);
   }
 }
+
+// The reciprocals behind them: [n] each of 1/x to a few ulp, and of -dx / x for the step lengths.
+extern "C" void lplb_sim_reciprocals(int n, const double* x, const double* dx, double* inverse, double* ratio) {
+  for (int i = 0; i < n; ++i) {
+    inverse[i] = lplb::rcp3(x[i]);
+    ratio[i] = lplb::step_ratio(x[i], dx[i]);
+  }
+}

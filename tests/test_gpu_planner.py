@@ -487,6 +487,17 @@ def test_block_and_warp_solver_agree():
         assert float((warp.last_probs - block.last_probs).abs().max()) < 2e-4
 
 
+def test_reciprocals_of_the_tile_solver_hold_their_bounds():
+    # see the CPU test of the same name: a seed of 20 bits, one step of third or second order
+    from lplb_b200 import _native
+
+    gen = torch.Generator("cuda").manual_seed(5)
+    x = 2.0 ** (800 * torch.rand(1 << 20, device="cuda", dtype=torch.float64, generator=gen) - 400)
+    inverse, ratio = _native.load().debug_reciprocals(x)
+    assert float((inverse * x - 1).abs().max()) < 4 * 2.0**-53
+    assert float((ratio * x - 1).abs().max()) < 2.0**-36
+
+
 def test_several_wide_groups_are_solved_side_by_side():
     # hypercube with ep_size 64: four LP groups of 16 ranks.  `run` leaves the single launch so
     # that every group gets a CTA of its own; result and status are as for any other call.

@@ -361,3 +361,17 @@ def test_step_keys_order_like_their_values_over_the_whole_range(sim):
         assert bool((keys < 64).all()) and bool((steps == 1.0).all())
         keys, steps = _step_keys(sim, huge, limit)
         assert bool((keys >= 2**32 - 64).all()) and bool((steps <= 2.0**-62).all())
+
+
+def test_reciprocals_hold_their_bounds_from_a_seed_of_twenty_bits(sim):
+    """The seed's error is at most 2^-18.4 (input and output cut to 20 bits, and one unit of its own): squared
+    below 2^-36 for the ratios behind a step length, which keep 26 bits, and cubed below the roundings of
+    1/x, four of 2^-53."""
+    rng = np.random.default_rng(1)
+    x = 2.0 ** rng.uniform(-400, 400, 20000)
+    dx = x * rng.uniform(-3, 3, 20000)
+    ptr = lambda a: ctypes.c_void_p(a.ctypes.data)  # noqa: E731
+    inverse, ratio = np.zeros_like(x), np.zeros_like(x)
+    sim.lplb_sim_reciprocals(len(x), ptr(x), ptr(dx), ptr(inverse), ptr(ratio))
+    assert float(np.abs(inverse * x - 1).max()) < 4 * 2.0**-53
+    assert float(np.abs(ratio * x / -dx - 1).max()) < 2.0**-36
