@@ -1,5 +1,5 @@
 // Warp-level interior-point solver for the per-group balancing LP (sm_100a).  It runs groups of 8
-// ranks where one CTA has more of them than warps, and groups of 16 and 32 ranks on request; all
+// ranks where one CTA has more than two of them per warp, and groups of 16 and 32 ranks on request; all
 // others go to the tile solver (lp_tile_solver.cuh) or the thread-block solver.
 //
 //   min t  s.t.  base_i + sum_k M[i,k] f_k <= t,  0 <= f <= 1

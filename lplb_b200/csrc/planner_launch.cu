@@ -40,7 +40,7 @@ bool shape_ok(const TopoDesc& t, bool need_solver = true, int solver = kSolverAu
 // thread-block solver (D is then the padded count).  The tile solver takes every group that it
 // covers (8 ranks 22.6 -> 10.3 us a call, 16 ranks 40.6 -> 17.0, 32 ranks 64 -> 25, 64 ranks 147 -> 52 against the
 // other two), except that the warp solver packs four groups of 8 ranks into a warp: `packed` asks for
-// that where one CTA has more groups than warps.  The warp solver's larger groups run on request only.
+// that where one CTA has many of them.  The warp solver's larger groups run on request only.
 template <typename Fn>
 cudaError_t dispatch_shape(int g, int d, int solver, bool packed, Fn&& fn) {
   const int kind = resolve_solver(g, d, solver);
@@ -84,8 +84,13 @@ size_t solver_smem(const Topo& tp, int teams = kWarps) {
   else return bundle_bytes_aligned(tp.n_group * tp.g, tp.d) +
               (GP == 0 ? block_solver_smem_bytes(tp.g, padded_dup(tp.d)) : tile_solver_smem_bytes(tp.g, tp.d, GP == -1 ? teams : 1));
 }
-// The fused kernel's one solver CTA has a warp for each of this many groups of 8 ranks.
-bool pack_groups(const Topo& tp) { return tp.n_group > kWarps; }
+// The fused kernel's one solver CTA gives each of its warps up to two groups of 8 ranks, one after the other;
+// beyond, the warp solver packs four groups to a warp.  Step with L2 flushed, warm-started, packed against a group
+// per warp, us: two replicas 4 groups 24.7 / 16.4, 8 groups 28.8 / 18.4, 9 groups 34.8 / 22.7, 16 groups 36.9 / 26.7, 24
+// groups 36.9 / 36.9, 32 groups 41.0 / 45.0, 64 groups 68.5 / 78.0; one replica 16 groups 28.7 / 26.6, 17 groups 30.8 /
+// 30.8, 32 groups 36.9 / 43.0; four replicas 47 / 27, 51 / 31 and 58 / 43 there.  Up to two rounds a step also
+// solves with the same code as the stand-alone kernel, bit for bit; beyond, shares agree to rounding (1e-6 of their norm).
+bool pack_groups(const Topo& tp) { return tp.n_group > 2 * kWarps; }
 
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {

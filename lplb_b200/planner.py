@@ -125,7 +125,9 @@ class Planner:
             per rank) with one warp, ``"block"`` a group of up to 128 ranks (8 replicas per rank)
             with as many warps of a thread block as it needs, ``"auto"`` uses one warp up to
             8 ranks and the block above.  Larger groups run the same method as tensor ops on
-            the planner's device.
+            the planner's device.  ``run`` solves with the code of ``solve_probs`` and gives the same
+            shares for the same counts, except that with more than 16 groups of up to 8 ranks it
+            packs several into a warp, whose shares differ by rounding (1e-6 of their norm).
         """
         if device is None:
             device = "cuda" if torch.cuda.is_available() else "cpu"
