@@ -41,6 +41,13 @@ if BOUNDS_CHECK:
 SOURCES = [
     "binding.cpp",
     "planner_launch.cu",
+    "planner_tiles1.cu",
+    "planner_tiles2.cu",
+    "planner_tiles4.cu",
+    "planner_tiles8.cu",
+    "planner_warp.cu",
+    "planner_warp32.cu",
+    "planner_block.cu",
     "place_kernel.cu",
     "count_noalloc.cu",
     "moe_binding.cpp",
@@ -54,7 +61,6 @@ NVCC_FLAGS = [
     "-O3",
     "-std=c++17",
     "--expt-relaxed-constexpr",
-    "--split-compile=0",  # optimise the many instantiations of one source in parallel
 ] + (["-DLPLB_BOUNDS_CHECK"] if BOUNDS_CHECK else [])
 
 _module = None

@@ -769,36 +769,6 @@ __device__ __forceinline__ unsigned exchange_counts(const Exchange& ex, Exchange
 }
 
 // ---------------------------------------------------------------------------------------
-// Stand-alone all-reduce of int32[E] counts over the peers (one CTA), for callers that
-// feed their own statistics to the solver.  Shares the epoch with the fused kernel, so it
-// keeps that kernel's invariant: the totals of the other parity are zero when it ends.
-__global__ void __launch_bounds__(kBlock) exchange_kernel(const int* __restrict__ in, int e, Exchange ex,
-                                                          Workspace* ws, int* __restrict__ out, int* status) {
-  extern __shared__ __align__(16) int smem[];
-  __shared__ ExchangeShared xs;
-  int* vec = smem;
-  const uint32_t epoch = ld_acquire_gpu(&ws->epoch) + 1;
-  int* other = ws_total(ws, (epoch & 1) ^ 1, e);
-  exchange_prepare(ex, &xs);
-  for (int i = threadIdx.x; i < e; i += kBlock) {
-    vec[i] = in[i];
-    other[i] = 0;
-  }
-  __syncthreads();
-  const unsigned miss = exchange_counts<kBlock>(ex, &xs, epoch, e, vec, status, nullptr);
-  if (miss && threadIdx.x == 0) {
-    atomicAdd(&status[kStTimeouts], 1);
-    raise_status(status, kErrPeerTimeout, kPhExchange, (int)miss);
-  }
-  for (int i = threadIdx.x; i < e; i += kBlock) out[i] = vec[i];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ws->arrive[(epoch & 1) ^ 1] = 0;  // every launch leaves the next one's arrival counter at zero
-    st_release_gpu(&ws->epoch, epoch);
-  }
-}
-
-// ---------------------------------------------------------------------------------------
 // Single-launch planner step.  Launched cooperatively so that all CTAs are co-resident.
 //
 //   CTAs 1..n  ("workers"): histogram their slice of the indices; reserve an ordinal range per

@@ -1,6 +1,5 @@
 // Launchers for the planner kernels: shape dispatch to the ahead-of-time instantiations.
-#include "planner_api.h"
-#include "planner_kernels.cuh"
+#include "planner_shapes.cuh"
 
 namespace lplb {
 
@@ -25,7 +24,6 @@ Topo make_topo(const TopoDesc& t) {
 }
 
 int padded_group(int g) { return g <= 8 ? 8 : (g <= 16 ? 16 : 32); }
-int padded_dup(int d) { return d <= 4 ? d : 8; }
 
 // The counting and redirect kernels work for any topology; the solvers (and with them the
 // fused kernel) cover groups of up to kMaxGroupSize ranks and kMaxDup replicas.
@@ -75,15 +73,6 @@ cudaError_t dispatch_shape(int g, int d, int solver, bool packed, Fn&& fn) {
   return cudaErrorInvalidValue;
 }
 
-size_t fused_smem(int e) { return sizeof(int) * 5 * (size_t)e; }
-size_t bundle_smem(const Topo& tp) { return sizeof(int) * (size_t)tp.n_group * tp.g * (tp.d + 1); }
-// bundle sums followed by the solver's scratch area, if it has one
-template <int GP>
-size_t solver_smem(const Topo& tp, int teams = kWarps) {
-  if constexpr (GP > 0) return bundle_smem(tp);
-  else return bundle_bytes_aligned(tp.n_group * tp.g, tp.d) +
-              (GP == 0 ? block_solver_smem_bytes(tp.g, padded_dup(tp.d)) : tile_solver_smem_bytes(tp.g, tp.d, GP == -1 ? teams : 1));
-}
 // The fused kernel's one solver CTA gives each of its warps up to two groups of 8 ranks, one after the other;
 // beyond, the warp solver packs four groups to a warp.  Step with L2 flushed, warm-started, packed against a group
 // per warp, us: two replicas 4 groups 24.7 / 16.4, 8 groups 28.8 / 18.4, 9 groups 34.8 / 22.7, 16 groups 36.9 / 26.7, 24
@@ -91,13 +80,6 @@ size_t solver_smem(const Topo& tp, int teams = kWarps) {
 // 30.8, 32 groups 36.9 / 43.0; four replicas 47 / 27, 51 / 31 and 58 / 43 there.  Up to two rounds a step also
 // solves with the same code as the stand-alone kernel, bit for bit; beyond, shares agree to rounding (1e-6 of their norm).
 bool pack_groups(const Topo& tp) { return tp.n_group > 2 * kWarps; }
-
-template <typename K>
-cudaError_t allow_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  if (bytes > 227 * 1024) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 
 IpmParams make_params(const SolveParams& prm, int g, int d) {
   IpmParams p{prm.max_iters, prm.tol, prm.anchor, prm.anchor_valid, prm.guard, prm.snap_mu};
@@ -134,55 +116,6 @@ cudaError_t launch_count(const void* idx, int idx_is64, long long n, int n_logic
   return cudaGetLastError();
 }
 
-struct SolveLaunch {
-  const int* workload;
-  Topo tp;
-  IpmParams prm;
-  float* probs;
-  float* normalised;
-  Counter avail;
-  int* status;
-  cudaStream_t stream;
-  template <int GP, int D>
-  cudaError_t operator()() const {
-    const size_t smem = solver_smem<GP>(tp);
-    cudaError_t err;
-    if constexpr (GP == 8) {
-      return cudaErrorInvalidValue;  // groups of 8 ranks are packed in the fused kernel only
-    } else if constexpr (GP == 0 || GP < -1) {
-      auto kernel = [] {
-        if constexpr (GP == 0) return solve_block_kernel<D>;
-        else return tile_solve_kernel<-GP, D>;
-      }();
-      if ((err = allow_smem(kernel, smem)) != cudaSuccess) return err;
-      if constexpr (GP == 0) kernel<<<tp.n_group, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status);
-      else return launch_after(kernel, tp.n_group + 1, kBlock, smem, stream, workload, tp, prm, probs, normalised, avail, status, 1);
-    } else {
-      // As few solving warps per CTA as still fit the groups on one wave of CTAs.
-      constexpr int kPerWarp = GP == -1 ? 1 : 32 / GP;
-      int dev = 0, sms = 1;
-      err = cudaGetDevice(&dev);
-      if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      if (err != cudaSuccess) return err;
-      int warps = 1;
-      while (warps < kWarps && (tp.n_group + warps * kPerWarp - 1) / (warps * kPerWarp) > sms) warps *= 2;
-      const int per_cta = warps * kPerWarp;
-      const int grid = (tp.n_group + per_cta - 1) / per_cta;
-      if constexpr (GP == -1) {
-        const size_t smem = solver_smem<GP>(tp, warps);
-        if ((err = allow_smem(tile_solve_kernel<1, D>, smem)) != cudaSuccess) return err;
-        // an early launch: 14.3 -> 11.6 us for 64 groups of 8 ranks, one call after the other, 64 ranks 59 -> 52
-        return launch_after(tile_solve_kernel<1, D>, grid + 1, kBlock, smem, stream, workload, tp, prm, probs, normalised, avail,
-                            status, warps);
-      } else {
-        if ((err = allow_smem(solve_kernel<GP, D>, smem)) != cudaSuccess) return err;
-        solve_kernel<GP, D><<<grid, kBlock, smem, stream>>>(workload, tp, prm, probs, normalised, avail, status, warps);
-      }
-    }
-    return cudaGetLastError();
-  }
-};
-
 cudaError_t launch_solve(const int* workload, const TopoDesc& topo, SolveParams prm, float* probs, float* normalised,
                          void* avail, int avail_is64, int* status, cudaStream_t stream) {
   if (!shape_ok(topo, true, prm.solver)) return cudaErrorInvalidValue;
@@ -209,6 +142,37 @@ cudaError_t launch_redirect(const void* idx, int idx_is64, long long n, const fl
   return cudaGetLastError();
 }
 
+namespace {
+// Stand-alone all-reduce of int32[E] counts over the peers (one CTA), for callers that
+// feed their own statistics to the solver.  Shares the epoch with the fused kernel, so it
+// keeps that kernel's invariant: the totals of the other parity are zero when it ends.
+__global__ void __launch_bounds__(kBlock) exchange_kernel(const int* __restrict__ in, int e, Exchange ex,
+                                                          Workspace* ws, int* __restrict__ out, int* status) {
+  extern __shared__ __align__(16) int smem[];
+  __shared__ ExchangeShared xs;
+  int* vec = smem;
+  const uint32_t epoch = ld_acquire_gpu(&ws->epoch) + 1;
+  int* other = ws_total(ws, (epoch & 1) ^ 1, e);
+  exchange_prepare(ex, &xs);
+  for (int i = threadIdx.x; i < e; i += kBlock) {
+    vec[i] = in[i];
+    other[i] = 0;
+  }
+  __syncthreads();
+  const unsigned miss = exchange_counts<kBlock>(ex, &xs, epoch, e, vec, status, nullptr);
+  if (miss && threadIdx.x == 0) {
+    atomicAdd(&status[kStTimeouts], 1);
+    raise_status(status, kErrPeerTimeout, kPhExchange, (int)miss);
+  }
+  for (int i = threadIdx.x; i < e; i += kBlock) out[i] = vec[i];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ws->arrive[(epoch & 1) ^ 1] = 0;  // every launch leaves the next one's arrival counter at zero
+    st_release_gpu(&ws->epoch, epoch);
+  }
+}
+}  // namespace
+
 cudaError_t launch_exchange(const int* in, int n_logical, const ExchangeDesc& exd, void* workspace, int* out,
                             int* status, cudaStream_t stream) {
   if (n_logical < 1 || n_logical > kMaxLogicalExperts || exd.n_ranks < 2 || exd.n_ranks > kMaxRanks)
@@ -220,37 +184,6 @@ cudaError_t launch_exchange(const int* in, int n_logical, const ExchangeDesc& ex
   exchange_kernel<<<1, kBlock, smem, stream>>>(in, n_logical, ex, static_cast<Workspace*>(workspace), out, status);
   return cudaGetLastError();
 }
-
-template <typename IdxT>
-struct FusedLaunch {
-  const IdxT* idx;
-  long long n;
-  Topo tp;
-  Exchange ex;
-  IpmParams prm;
-  Workspace* ws;
-  float* probs;
-  Counter avail;
-  int* status;
-  IdxT* out;
-  int n_cta;
-  unsigned long long grid_timeout_ns;
-  unsigned long long* trace;
-  int cooperative;
-  cudaStream_t stream;
-  template <int GP, int D>
-  cudaError_t operator()() {
-    auto kernel = fused_run_kernel<GP, D, IdxT>;
-    const size_t smem = fused_smem(tp.e) + solver_smem<GP>(tp);
-    cudaError_t err = allow_smem(kernel, smem);
-    if (err != cudaSuccess) return err;
-    void* args[] = {&idx, &n, &tp, &ex, &prm, &ws, &probs, &avail, &status, &out, &grid_timeout_ns, &trace};
-    if (cooperative)
-      return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(n_cta), dim3(kBlock), args, smem,
-                                         stream);
-    return cudaLaunchKernel(reinterpret_cast<void*>(kernel), dim3(n_cta), dim3(kBlock), args, smem, stream);
-  }
-};
 
 cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoDesc& topo, const ExchangeDesc& exd,
                          SolveParams prm, void* workspace, float* probs, void* avail, int avail_is64, int* status,
@@ -269,30 +202,6 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
                          static_cast<int32_t*>(out), n_cta, grid_timeout_ns, trace, cooperative, stream};
   return dispatch_shape(topo.g, topo.d, prm.solver, pack_groups(l.tp), l);
 }
-
-struct OccupancyQuery {
-  Topo tp;
-  int is64;
-  int* result;
-  template <int GP, int D>
-  cudaError_t operator()() const {
-    const size_t smem = fused_smem(tp.e) + solver_smem<GP>(tp);
-    int per_sm = 0, dev = 0, sms = 0;
-    cudaError_t err;
-    if (is64) {
-      if ((err = allow_smem(fused_run_kernel<GP, D, int64_t>, smem)) != cudaSuccess) return err;
-      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_run_kernel<GP, D, int64_t>, kBlock, smem);
-    } else {
-      if ((err = allow_smem(fused_run_kernel<GP, D, int32_t>, smem)) != cudaSuccess) return err;
-      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_run_kernel<GP, D, int32_t>, kBlock, smem);
-    }
-    if (err != cudaSuccess) return err;
-    if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
-    if ((err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return err;
-    *result = per_sm * sms;
-    return cudaSuccess;
-  }
-};
 
 int max_fused_ctas(const TopoDesc& topo, int solver, int idx_is64) {
   int result = 0;
