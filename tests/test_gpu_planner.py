@@ -414,6 +414,47 @@ def test_warm_start_cuts_iterations_and_keeps_the_optimum():
     assert planner.check_status()["lp_iters"] >= iters[0][0] - 1
 
 
+def test_warm_starts_converge_where_only_one_bundle_per_rank_is_loaded():
+    # 64 groups of a skewed gate: parts of a group are connected through loaded bundles only, and the normal
+    # matrix of the most loaded part is singular up to s / y
+    n_group, r2o = 64, topology.cube()
+    planner = _planner(r2o, 64 * 32, 512, 2, warm_start=True)
+    gen = torch.Generator().manual_seed(6)
+    base = torch.rand(n_group, 8, generator=gen, dtype=torch.float64) * 500 + 200
+    anchor = None
+    for step in range(6):
+        counts = torch.zeros(n_group, 8, 4, dtype=torch.float64)
+        counts[:, :, 0] = torch.poisson(base, generator=gen)
+        counts[:, :, 2] = torch.randint(0, 3, (n_group, 8), generator=gen)
+        w, fixed = counts[:, :, :2].contiguous(), counts[:, :, 2:].sum(-1)
+        ref = lp.solve_ipm(w, fixed, r2o, tol=1e-4, warm_start=True, anchor=anchor, guard=planner.warm_guard)
+        anchor = ref.anchor
+        avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+        probs, _ = planner.solve_probs(counts.reshape(-1).int().cuda(), avail)
+        st = planner.check_status(clear=True)
+        assert int(avail) == n_group and st.ok and st["lp_iters"] <= int(ref.iters.max()) + 1
+        realised = lp.rank_loads(probs.cpu().double(), w, fixed, r2o).max(-1).values
+        best = lp.solve_ipm(w, fixed, r2o, tol=1e-7, max_iters=40)
+        assert float(((realised - best.t) / best.t).max()) < 1e-3
+
+
+@pytest.mark.parametrize("name", ["cube", "hypercube", "torus8x4", "torus8x8"])
+def test_small_tolerances_are_reached(name):
+    r2o = topology.by_name(name)
+    g = r2o.shape[0]
+    planner = _planner(r2o, 8 * g, g, 2, tol=1e-7)
+    gen = torch.Generator().manual_seed(12)
+    for _ in range(6):
+        counts = ((torch.randn(1, g, 8, generator=gen, dtype=torch.float64) * 0.3 + 1).clamp_min(0) * 4096).floor()
+        w, fixed = counts[:, :, :2].contiguous(), counts[:, :, 2:].sum(-1)
+        avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+        probs, _ = planner.solve_probs(counts.reshape(-1).int().cuda(), avail)
+        assert int(avail) == 1 and planner.check_status(clear=True).ok
+        best = lp.solve_ipm(w, fixed, r2o, tol=1e-9, max_iters=60)
+        realised = float(lp.rank_loads(probs.cpu().double(), w, fixed, r2o).max())
+        assert realised <= float(best.t[0]) * (1 + 5e-7)  # the gap, and shares of 24 bits
+
+
 # ---------------------------------------------------------------- exchange on one GPU
 def test_exchange_loopback_sums_prefilled_peer():
     planner = _planner(topology.cube(), 64, 8, 2)

@@ -326,6 +326,38 @@ def test_tile_solver_warm_start_follows_the_torch_restatement(sim, name):
     assert seen[1][1] < seen[0][1]
 
 
+def test_tile_solver_warm_start_with_nearly_singular_systems(sim):
+    """Two batches of a skewed gate: one loaded expert per rank, second bundles empty, so that the four most
+    loaded ranks are a part of their own whose normal matrix is singular up to s / y.  The second
+    solve starts from the iterate of the first and takes as long as the restatement does."""
+    r2o = topology.cube()
+    heavy = torch.tensor([[675, 452, 385, 314, 313, 307, 275, 211], [640, 471, 374, 332, 306, 280, 279, 221]], dtype=torch.float64)
+    rest = torch.tensor([[0, 0, 0, 0, 0, 0, 0, 2], [0, 0, 0, 0, 0, 0, 1, 1]], dtype=torch.float64)
+    anchor_c, valid_c, anchor_t = np.zeros((1, 8, 11)), np.zeros(1, np.int32), None
+    for step in range(2):
+        w, fixed = torch.stack([heavy[step], torch.zeros(8, dtype=torch.float64)], -1).unsqueeze(0), rest[step].unsqueeze(0)
+        ref = lp.solve_ipm(w, fixed, r2o, tol=1e-4, warm_start=True, anchor=anchor_t, guard=0.1)
+        anchor_t = ref.anchor
+        f, iters, conv = _solve_tiles(sim, r2o, w, fixed, rows=8, anchor=anchor_c, valid=valid_c)
+        assert conv[0] == 1 and int(iters[0]) == int(ref.iters[0])
+        assert float((f - ref.f).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("g,offsets", [(8, (1, 4)), (16, (3, 8)), (64, (1, 8))])
+def test_tile_solver_reaches_small_tolerances(sim, g, offsets):
+    """A gap of 1e-7, three orders below the default: the systems of the last iterations are the worse conditioned."""
+    r2o = topology.circulant(g, offsets)
+    gen = torch.Generator().manual_seed(3)
+    cnt = ((torch.randn(1, g, 8, generator=gen, dtype=torch.float64) * 0.3 + 1).clamp_min(0) * 4096).floor()
+    w, fixed = cnt[:, :, :2].contiguous(), cnt[:, :, 2:].sum(-1)
+    f, iters, conv = _solve_tiles(sim, r2o, w, fixed, tol=1e-7)
+    ref = lp.solve_ipm(w, fixed, r2o, tol=1e-7)
+    assert bool(ref.converged.all()) and conv[0] == 1 and int(iters[0]) <= int(ref.iters[0]) + 1
+    best = lp.solve_ipm(w, fixed, r2o, tol=1e-9, max_iters=60)
+    realised = float(lp.rank_loads(f, w, fixed, r2o).max())
+    assert realised <= float(best.t[0]) * (1 + 2e-7)
+
+
 def test_tile_solver_handles_empty_groups_and_the_iteration_cap(sim):
     for r2o in (topology.cube(), topology.hypercube()):
         g, d = r2o.shape
