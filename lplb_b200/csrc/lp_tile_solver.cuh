@@ -545,7 +545,6 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
 
 #pragma unroll 1
   for (int it = 0;; ++it) {
-    if (prm.stop != nullptr && __any_sync(0xffffffffu, *prm.stop != 0)) break;
     // ---- weights and residuals --------------------------------------------------------------
     const double fv = f * v, inv_fv = rcp3(fv), inv_y = rcp3(live ? y : 1.0);
     const double theta = fv * rcp3(fma(z, v, q * f));  // 1 / (z / f + q / v)

@@ -252,8 +252,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   unsigned long long* dbg = FUSED && args.debug ? args.debug + 4 * blockIdx.x : nullptr;
 
   allow_successor();
+  const unsigned long long started = dbg ? timer_ns() : 0;
   if (threadIdx.x == 0) {
-    if (dbg) dbg[0] = timer_ns();
     abort_flag = 0;
     s_flags_ok = 1;
     for (int s = 0; s < kMaxStages; ++s) {
@@ -272,6 +272,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), kTmemCols);
   wait_predecessors();
   if (threadIdx.x == 0) {
+    if (dbg) dbg[0] = started;
     // every source rank must have finished writing this launch's A rows
     if (args.wait_flags != nullptr) {
       const uint64_t t0 = timer_ns();

@@ -946,9 +946,8 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
 
 template <typename IdxT>
 __device__ __forceinline__ void worker_cta(const IdxT* __restrict__ idx, long long n, const Topo& tp, Workspace* ws,
-                                           const float* __restrict__ probs, int* status, IdxT* __restrict__ out,
-                                           int q, int n_workers, unsigned long long grid_timeout_ns,
-                                           unsigned long long* __restrict__ trace, int* smem) {
+                                           int* status, IdxT* __restrict__ out, int q, int n_workers,
+                                           unsigned long long grid_timeout_ns, unsigned long long* __restrict__ trace, int* smem) {
   const int e = tp.e;
   const bool tracing = trace != nullptr && threadIdx.x == 0 && q == 0;
   const RedirectTables tb = redirect_tables(smem, e);
@@ -1020,7 +1019,7 @@ __global__ void __launch_bounds__(kBlock) fused_run_kernel(const IdxT* __restric
   extern __shared__ __align__(16) int smem[];
   const int n_workers = (int)gridDim.x - 1;
   if (blockIdx.x == 0) solver_cta<GP, D>(tp, ex, prm, ws, probs, avail, status, n_workers, grid_timeout_ns, trace, smem);
-  else worker_cta<IdxT>(idx, n, tp, ws, probs, status, out, (int)blockIdx.x - 1, n_workers, grid_timeout_ns, trace, smem);
+  else worker_cta<IdxT>(idx, n, tp, ws, status, out, (int)blockIdx.x - 1, n_workers, grid_timeout_ns, trace, smem);
 }
 
 }  // namespace lplb
