@@ -1,4 +1,4 @@
-// CPU build of the warp-level and thread-block LP solvers (see host_sim.h): C entry points
+// CPU build of the LP solvers (see host_sim.h): C entry points
 // for ctypes.  Compiled with -DLPLB_HOST_SIM by the CPU tests; not part of the GPU extension.
 #define LPLB_HOST_SIM 1
 #include "lp_block_solver.cuh"
@@ -91,7 +91,7 @@ template <int NB, int D>
 void solve_batch_tiles(int g, int rows, const int* r2o, const int* o2r, int nb, const double* w, const double* fixed,
                        int max_iters, double tol, double* f_out, int* iters, int* converged, double* anchor,
                        int* anchor_valid, double guard, double snap_mu) {
-  std::vector<double> scratch(lplb::tile_layout(NB, D).total + 2);
+  std::vector<double> scratch(lplb::tile_layout(NB, D).total);  // exactly, so that a sanitizer sees an overrun
   for (int b = 0; b < nb; ++b) {
     lplb_sim::run_block(32 * NB, [&](int tid) {
       const int warp = tid >> 5, lane = tid & 31, rank = 8 * warp + (lane >> 2);
@@ -132,7 +132,8 @@ extern "C" int lplb_sim_solve_tiles(int g, int d, int rows, const int* r2o, cons
     return 0;                                                                                                       \
   }
   LPLB_CASE(1, 1) LPLB_CASE(1, 2) LPLB_CASE(1, 3) LPLB_CASE(1, 4) LPLB_CASE(2, 1) LPLB_CASE(2, 2) LPLB_CASE(2, 3)
-  LPLB_CASE(2, 4) LPLB_CASE(4, 1) LPLB_CASE(4, 2) LPLB_CASE(4, 4) LPLB_CASE(8, 1) LPLB_CASE(8, 2) LPLB_CASE(8, 3)
+  LPLB_CASE(2, 4) LPLB_CASE(4, 1) LPLB_CASE(4, 2) LPLB_CASE(4, 3) LPLB_CASE(4, 4) LPLB_CASE(8, 1) LPLB_CASE(8, 2)
+  LPLB_CASE(8, 3) LPLB_CASE(8, 4)
 #undef LPLB_CASE
   return 1;
 }

@@ -221,6 +221,8 @@ extern "C" int lplb_sim_solve_block(int, int, const int*, const int*, int, const
                                     double*, int*, int*, double*, int*, double, double);
 extern "C" int lplb_sim_solve(int, int, const int*, const int*, int, const double*, const double*, int, double, double*,
                               int*, int*);
+extern "C" int lplb_sim_solve_tiles(int, int, int, const int*, const int*, int, const double*, const double*, int, double,
+                                    double*, int*, int*, double*, int*, double, double);
 int main() {
   int bad = 0;
   for (int g : {5, 8, 19, 40}) {
@@ -234,6 +236,27 @@ int main() {
     for (int rep = 0; rep < 2; ++rep) {
       bad += lplb_sim_solve_block(g, 1, r2o.data(), o2r.data(), 1, w.data(), fixed.data(), 24, 1e-4, f.data(), &iters,
                                   &conv, anchor.data(), &valid, 0.1, 1e-3);
+      bad += conv != 1;
+    }
+    // the tile solver, with one replica and with three (four lanes a rank, one of them a dummy)
+    valid = 0;
+    for (int rep = 0; rep < 2; ++rep) {
+      bad += lplb_sim_solve_tiles(g, 1, g, r2o.data(), o2r.data(), 1, w.data(), fixed.data(), 24, 1e-4, f.data(), &iters,
+                                  &conv, anchor.data(), &valid, 0.1, 1e-3);
+      bad += conv != 1;
+    }
+    std::vector<int> r2o3(3 * g), o2r3(3 * g);
+    std::vector<double> w3(3 * g), f3(3 * g), anchor3((size_t)g * 15, 0.0);
+    for (int i = 0; i < g; ++i)
+      for (int d = 0; d < 3; ++d) {
+        r2o3[3 * i + d] = (i + d + 1) % g;
+        o2r3[3 * ((i + d + 1) % g) + d] = i;
+        w3[3 * i + d] = w[i] / (d + 1);
+      }
+    int valid3 = 0;
+    for (int rep = 0; rep < 2; ++rep) {
+      bad += lplb_sim_solve_tiles(g, 3, g, r2o3.data(), o2r3.data(), 1, w3.data(), fixed.data(), 24, 1e-4, f3.data(), &iters,
+                                  &conv, anchor3.data(), &valid3, 0.1, 1e-3);
       bad += conv != 1;
     }
     if (g <= 32) {
@@ -281,6 +304,7 @@ def _solve_tiles(lib, r2o, w, fixed, rows=None, max_iters=24, tol=1e-4, anchor=N
 @pytest.mark.parametrize("g,offsets", [
     (2, (1,)), (5, (1,)), (8, (1, 4)), (8, (1, 2, 3, 4)), (9, (1, 2)), (16, (3, 8)), (16, (1, 2, 3, 4)), (17, (1,)),
     (32, (1, 16)), (33, (1, 2)), (64, (1, 8)),
+    (8, (1, 2, 4)), (12, (1, 5, 7)), (24, (1, 2, 3)), (40, (1, 2, 3)), (64, (1, 2, 3, 4)),
 ])
 def test_tile_solver_device_code_matches_the_torch_restatement(sim, g, offsets):
     """Group sizes at the edges of the tile counts (1, 2, 4 and 8 warps), with rows that are only padding, and
@@ -324,6 +348,23 @@ def test_tile_solver_warm_start_follows_the_torch_restatement(sim, name):
         seen.append((bool(ref.warm[0]), int(iters[0])))
     assert [s[0] for s in seen] == [False, True, True, name == "ring5"]  # the small shift of five loads stays in the guard
     assert seen[1][1] < seen[0][1]
+
+
+@pytest.mark.parametrize("g,offsets", [(8, (1, 2, 4)), (12, (1, 5, 7)), (24, (1, 2, 3)), (40, (1, 2, 3))])
+def test_tile_solver_warm_starts_with_three_replicas(sim, g, offsets):
+    """Four lanes share three edges and the saved iterate has no fourth."""
+    r2o = topology.circulant(g, offsets)
+    gen = torch.Generator().manual_seed(17)
+    mean = (torch.rand(g, 8, generator=gen, dtype=torch.float64) + 0.5) * 4096
+    anchor_c, valid_c, anchor_t = np.zeros((1, g, 15)), np.zeros(1, np.int32), None
+    for step in range(2):
+        cnt = (mean * (1 + 0.02 * torch.randn(g, 8, generator=gen, dtype=torch.float64))).floor().unsqueeze(0)
+        w, fixed = cnt[:, :, :3].contiguous(), cnt[:, :, 3:].sum(-1)
+        ref = lp.solve_ipm(w, fixed, r2o, tol=1e-4, warm_start=True, anchor=anchor_t, guard=0.1)
+        anchor_t = ref.anchor
+        f, iters, conv = _solve_tiles(sim, r2o, w, fixed, anchor=anchor_c, valid=valid_c)
+        assert conv[0] == 1 and int(iters[0]) == int(ref.iters[0]) and bool(ref.warm[0]) == (step == 1)
+        assert float((f - ref.f).abs().max()) < 1e-5
 
 
 def test_tile_solver_warm_start_with_nearly_singular_systems(sim):
