@@ -242,6 +242,8 @@ class PlannerEngine {
     const int k = lplb::resolve_solver(g_, d_, prm_.solver);
     return k == lplb::kSolverWarp ? "warp" : k == lplb::kSolverBlock ? "block" : "none";
   }
+  // Which of the three device codes that stands for: see planner_launch.cu.
+  std::string solver_code(bool fused) const { return lplb::solver_code(topo(), prm_.solver, fused); }
   // Forget the saved iterates (next solve of every group starts cold).  Stream-ordered.
   void invalidate_warm_start() {
     if (anchor_valid_.defined()) anchor_valid_.zero_();
@@ -583,6 +585,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("set_warm_start", &PlannerEngine::set_warm_start)
       .def("set_solver", &PlannerEngine::set_solver)
       .def("solver", &PlannerEngine::solver)
+      .def("solver_code", &PlannerEngine::solver_code, py::arg("fused"))
       .def("warm_start_valid", &PlannerEngine::warm_start_valid)
       .def("invalidate_warm_start", &PlannerEngine::invalidate_warm_start)
       .def("count_idx", &PlannerEngine::count_idx)

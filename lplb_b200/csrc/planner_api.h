@@ -56,6 +56,9 @@ constexpr int kMaxLogicalExperts = 8192;
 
 // The solver that `requested` resolves to for this shape, or -1 when no device solver fits.
 int resolve_solver(int g, int d, int requested);
+// The device code that runs the topology, in the fused step or in the stand-alone solve: "tile", "warp" or "block", or
+// "none".
+const char* solver_code(const TopoDesc& topo, int requested, bool fused);
 // Replica slots per rank in the warm-start state for this shape and solver.
 int anchor_dup(int g, int d, int requested);
 

@@ -98,6 +98,23 @@ int resolve_solver(int g, int d, int requested) {
   return block_ok ? kSolverBlock : -1;
 }
 
+namespace {
+struct CodeQuery {
+  const char** name;
+  template <int GP, int D>
+  cudaError_t operator()() const {
+    *name = GP < 0 ? "tile" : (GP > 0 ? "warp" : "block");
+    return cudaSuccess;
+  }
+};
+}  // namespace
+
+const char* solver_code(const TopoDesc& topo, int requested, bool fused) {
+  const char* name = "none";
+  if (shape_ok(topo, true, requested)) dispatch_shape(topo.g, topo.d, requested, fused && pack_groups(make_topo(topo)), CodeQuery{&name});
+  return name;
+}
+
 int anchor_dup(int g, int d, int requested) { return resolve_solver(g, d, requested) == kSolverBlock ? padded_dup(d) : d; }
 
 size_t planner_workspace_bytes(int n_logical) { return workspace_bytes(n_logical); }

@@ -22,13 +22,15 @@ def main():
     dev = torch.device("cuda", 0)
     gen = torch.Generator(device=dev).manual_seed(0)
     avail = torch.zeros(1, dtype=torch.int32, device=dev)
-    # clean runs: fused and staged steps on both solvers, odd expert counts, ragged slices, loopback exchange
+    # clean runs: fused and staged steps on the three device solvers, odd expert counts, ragged slices, loopback exchange
     for r2o, ll, n_tokens, n_sms in (
         (topology.cube(), 4, 1000, 7), (topology.ring(5), 3, 257, 3), (topology.hypercube(), 2, 4096, 148),
         (topology.torus(3, 3), 3, 5000, 16), (topology.torus(8, 4), 2, 300, 5),
+        (topology.circulant(12, (1, 5, 7)), 3, 999, 9), (topology.circulant(66, (1, 9)), 2, 3000, 33),
     ):
         g, d = r2o.shape
         planner = Planner(r2o, g * (ll + d), g * ll, g, device=dev)
+        assert planner._engine.solver_code(True) == ("tile" if g <= 64 else "block")
         idx = torch.randint(-1, g * ll, (n_tokens, 2), device=dev, generator=gen)
         for _ in range(2):
             out = planner.run(idx, avail, n_sms)
@@ -38,6 +40,13 @@ def main():
         st = planner.check_status()
         assert st.ok and "bounds_skipped" not in st, st
         assert int(out.max()) < g * (ll + d)
+    # many groups of 8 ranks: two rounds of the tile solver, and the warp solver's packing
+    for n_group, code in ((10, "tile"), (18, "warp")):
+        planner = Planner(topology.cube(), n_group * 8 * 5, n_group * 8 * 3, n_group * 8, device=dev)
+        assert planner._engine.solver_code(True) == code
+        planner.run(torch.randint(-1, n_group * 24, (20000, 2), device=dev, generator=gen), avail)
+        st = planner.check_status()
+        assert st.ok and "bounds_skipped" not in st, st
     planner = Planner(topology.cube(), 80, 64, 8, device=dev)
     eng = planner._engine
     eng.open_exchange_loopback(2, 0)

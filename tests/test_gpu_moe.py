@@ -25,6 +25,28 @@ def _inputs(tokens, hidden, n_logical, topk, seed=0):
     return x, idx, w
 
 
+@pytest.mark.parametrize("fuse", [False, True])
+@pytest.mark.parametrize("hidden,inter,tokens,topk", [(512, 256, 64, 2), (1024, 512, 1000, 4)])
+def test_passes_follow_one_another_without_a_gap(hidden, inter, tokens, topk, fuse):
+    """The layer's kernels start while their predecessors run out, also those of the pass before, whose buffers they
+    use: passes on alternating inputs without a wait give what they give one at a time."""
+    planner, layer = _layer(hidden, inter, 32, topk, 1024)
+    layer.fuse_dispatch = fuse
+    layer.engine.set_timeout_us(1e6)
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    batches = [_inputs(tokens - 7 * i, hidden, 32, topk, seed=i) for i in range(3)]
+    want = []
+    for x, idx, w in batches:
+        want.append(layer.forward(x, idx, w, avail))
+        torch.cuda.synchronize()
+    got = [layer.forward(x, idx, w, avail) for _ in range(8) for x, idx, w in batches]
+    assert layer.check() == 0
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 3])
+    ref = layer.reference_forward(*batches[0]).float()
+    assert float((want[0].float() - ref).norm() / ref.norm()) < 1e-2
+
+
 def test_interleave_layout():
     gate = torch.arange(256).float().unsqueeze(1).expand(256, 4)
     up = gate + 1000

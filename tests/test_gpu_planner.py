@@ -256,6 +256,8 @@ def test_many_groups_of_8_ranks_in_one_step(n_group):
             if step % 2:
                 solved = planner.solve_probs(counts, avail)[0].clone()
             out = planner.run(idx, avail)
+            assert planner._engine.solver_code(True) == ("tile" if n_group <= 16 else "warp")
+            assert planner._engine.solver_code(False) == "tile"
             shares = planner.last_probs.clone()
             if not step % 2:
                 solved, _ = planner.solve_probs(counts, avail)
@@ -479,7 +481,7 @@ def test_exchange_loopback_sums_prefilled_peer():
 
 
 def test_groups_beyond_a_warp_run_the_fused_single_launch_without_a_host_sync():
-    # torus(8, 8): one LP group of 64 ranks, solved by the thread-block solver inside the fused
+    # torus(8, 8): one LP group of 64 ranks, solved by eight warps inside the fused
     # kernel; the whole step is one launch and the host never waits for the device
     planner = _planner(topology.torus(8, 8), 512, 64, 2)
     assert planner._native_solver is True and planner._engine.solver() == "block"
@@ -519,11 +521,12 @@ def test_groups_beyond_a_warp_run_the_fused_single_launch_without_a_host_sync():
     ("circulant128x4", topology.circulant(128, (1, 2, 64, 127)), 8),
 ])
 def test_block_solver_reaches_the_optimum_for_any_group_shape(name, r2o, ll):
-    """The thread-block solver on group sizes that are not multiples of 8 or 32, on every
-    instantiated replica count and on the padded one (5 replicas run as 8), warm and cold."""
+    """What solver="block" stands for, warm and cold: the tile solver up to 64 ranks and four replicas, the
+    thread-block solver beyond (100 and 128 ranks, 5 replicas run as 8)."""
     g, d = r2o.shape
     planner = _planner(r2o, g * ll, g, d, solver="block", warm_start=True)
     assert planner._engine.solver() == "block"
+    assert planner._engine.solver_code(False) == ("tile" if g <= 64 and d <= 4 else "block")
     gen = torch.Generator().manual_seed(11)
     base = (torch.rand(g * ll, generator=gen) + 0.5) * 4000
     iters = []
@@ -550,6 +553,9 @@ def test_block_and_warp_solver_agree():
         warp = _planner(r2o, e, g * n_group, d, solver="warp")
         block = _planner(r2o, e, g * n_group, d, solver="block")
         assert (warp._engine.solver(), block._engine.solver()) == ("warp", "block")
+        # up to 8 ranks both names stand for the tile solver, which more groups compare with the packed one
+        # (test_many_groups_of_8_ranks_in_one_step)
+        assert (warp._engine.solver_code(True), block._engine.solver_code(True)) == ("tile" if g == 8 else "warp", "tile")
         counts = (torch.rand(e, generator=gen) * 5000).int().cuda()
         a1 = torch.zeros(1, dtype=torch.int32, device="cuda")
         a2 = torch.zeros(1, dtype=torch.int32, device="cuda")
@@ -568,6 +574,74 @@ def test_block_and_warp_solver_agree():
         o3 = block.run(idx, a2)
         _check_redirect(block, idx, o3, block.last_probs.clone())
         assert float((warp.last_probs - block.last_probs).abs().max()) < 2e-4
+
+
+@pytest.mark.parametrize("code,g,d", [("tile", g, d) for g in (7, 13, 27, 50) for d in (1, 2, 3, 4)]
+                         + [("block", 65, 1), ("block", 72, 2), ("block", 66, 3), ("block", 100, 4), ("block", 20, 6)])
+def test_every_instantiation_against_the_oracle(code, g, d):
+    """One group size inside every tile count (1, 2, 4, 8 warps) times every replica count, and the
+    thread-block solver's, in the stand-alone kernel and in the step, 32 and 64 bit ids, cold and warm."""
+    r2o = topology.circulant(g, (1, 3, 4, 6, 7, 9)[:d]) if g > 7 else topology.circulant(g, (1, 2, 3, 4)[:d])
+    ll = 2 * d
+    e = g * ll
+    planner = _planner(r2o, e, g, d, warm_start=True)
+    assert planner._engine.solver_code(False) == planner._engine.solver_code(True) == code
+    gen = torch.Generator("cuda").manual_seed(g * 10 + d)
+    p = torch.rand(e, device="cuda", generator=gen) + 0.3
+    for step in range(4):
+        idx = torch.multinomial(p, 1 << 18, replacement=True, generator=gen)
+        idx = idx.int() if step % 2 else idx
+        counts = torch.bincount(idx.long(), minlength=e).int()
+        avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+        if step < 2:
+            out = planner.run(idx, avail)
+            shares = planner.last_probs.clone()
+            _check_redirect(planner, idx, out, shares)
+        else:
+            shares, _ = planner.solve_probs(counts, avail)
+        assert int(avail) == 1 and planner.check_status(clear=True).ok
+        w, fixed = lp.bundle_loads(counts.cpu().double(), planner.phy2log.cpu(), 1, g, d, ll, 1)
+        best = lp.solve_ipm(w, fixed, r2o, tol=1e-7, max_iters=40)
+        realised = float(lp.rank_loads(shares.cpu().double(), w, fixed, r2o).max())
+        assert -1e-6 < (realised - float(best.t[0])) / float(best.t[0]) < 1e-3
+
+
+@pytest.mark.parametrize("name,n_group", [("cube", 64), ("cube", 1), ("torus8x8", 1)])
+def test_solves_follow_one_another_without_a_gap(name, n_group):
+    """The stand-alone kernel starts while its predecessor runs out: launches that follow one another on the same
+    buffers, eager and in a graph, give what they give one at a time."""
+    r2o = topology.by_name(name)
+    e = 4 * r2o.shape[0] * n_group
+    planner = _planner(r2o, e, r2o.shape[0] * n_group, 2)
+    gen = torch.Generator("cuda").manual_seed(3)
+    loads = [torch.randint(0, 5000, (e,), device="cuda", generator=gen, dtype=torch.int32) for _ in range(4)]
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = []
+    for c in loads:
+        want.append([t.clone() for t in planner.solve_probs(c, avail)])
+        torch.cuda.synchronize()
+    counts = torch.empty_like(loads[0])
+    got = []
+    for i in range(40):
+        counts.copy_(loads[i % 4])
+        got.append([t.clone() for t in planner.solve_probs(counts, avail)])
+    first = planner.solve_probs(loads[0], avail)  # and with nothing in between
+    second = planner.solve_probs(loads[1], avail)
+    for i, pair in enumerate(got + [first, second]):
+        ref_pair = want[i % 4] if i < 40 else want[i - 40]
+        assert torch.equal(pair[0], ref_pair[0]) and torch.equal(pair[1], ref_pair[1])
+    avail.zero_()
+    graph = torch.cuda.CUDAGraph()
+    other = torch.empty_like(counts)
+    with torch.cuda.graph(graph):
+        a = planner.solve_probs(counts, avail)
+        b = planner.solve_probs(other, avail)
+    for i in range(4):
+        counts.copy_(loads[i])
+        other.copy_(loads[i - 1])
+        graph.replay()
+        assert torch.equal(a[0], want[i][0]) and torch.equal(b[0], want[i - 1][0]) and torch.equal(b[1], want[i - 1][1])
+    assert int(avail) == 8 * n_group
 
 
 def test_reciprocals_of_the_tile_solver_hold_their_bounds():
