@@ -32,7 +32,7 @@ def main():
     ap.add_argument("--calls", type=int, default=30)
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--modes", default="cold,warm", help="cold: warm_start off; warm: warm_start on")
-    ap.add_argument("--solvers", default="auto", help="comma list of auto, warp, block")
+    ap.add_argument("--solvers", default="auto", help="comma list of auto, warp, block (up to 8 ranks all three are the tile solver)")
     ap.add_argument("--json", default="")
     args = ap.parse_args()
     from lplb_b200.utils.timing import ClockSampler, physical_gpu_index

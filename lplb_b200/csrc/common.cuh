@@ -126,8 +126,9 @@ __device__ __forceinline__ bool bounded_wait_ge(const uint32_t* flag, uint32_t t
 // thread calls it), which is when the predecessor, and with it everything before, has
 // completed.  allow_successor() lets the next such kernel start; its blocks take only what is left of an SM.
 // The five kernels of a MoE forward pass so lose the gaps between them, some 2 us each, and the set-up of
-// the GEMMs' barriers and tensor memory: 64 tokens, hidden 7168, 705 -> 673 us; a small layer 134 -> 98 us (both with
-// the planner's step in front).
+// the GEMMs' barriers and tensor memory.  A pass with the planner's step in front, all kernels early against none, in turn in
+// one process: 64 tokens x 1024 72.4 -> 65.3 us, 128 x 2048 120 -> 109, 64 x 7168 679 -> 668, 1000 x 7168 1032 -> 1018;
+// 4096 and 8192 x 7168 differ by less than 0.5 % either way, which is their noise.
 __device__ __forceinline__ void wait_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

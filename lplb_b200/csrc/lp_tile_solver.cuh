@@ -17,17 +17,18 @@
 //     tiles it takes a whole 8 x 8 tile, and the warp that owns the next pivot tile inverts it
 //     while the others still update theirs.
 //   * Warp I holds tile row I and is the ranks 8 I .. 8 I + 7, four lanes each; a lane is one of the
-//     rank's edges, so that no instruction is spent once per edge (8 ranks 11.3 -> 10.3 us, with
-//     the sweep below).  With one warp there is no barrier.
+//     rank's edges, so that no instruction is spent once per edge (8 ranks 11.3 -> 10.3 us with
+//     the sweep below, before the refinement).  With one warp there is no barrier.
 //   * Sums over ranks are two matrix instructions by a matrix of ones for two sums at a time
 //     (65 cycles; three rounds of shuffles take 96 for one).
 //   * Maxima are taken on integers that order like the doubles they stand for.
 //   * Whatever does not depend on the centring parameter is done before it is known: the
 //     corrector's step is linear in it.
+//   * A product with an inverse is not as good as a substitution, so the step is refined once (kDamping).
 //
 // Solve kernel, two replicas per rank, unrelated instances, us a call back to back (the warp solver
-// for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 10.3, 64 groups of 8 ranks
-// 26.2 -> 11.8, 16 ranks 40.6 -> 17.0, 32 ranks 64.4 -> 25.4, 64 ranks 147 -> 52.  An iteration: 8 ranks 3.5 -> 1.2,
+// for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 11.2, 64 groups of 8 ranks
+// 26.2 -> 12.4, 16 ranks 40.6 -> 18.0, 32 ranks 64.4 -> 26.1, 64 ranks 147 -> 52.  An iteration: 8 ranks 3.5 -> 1.4,
 // 64 ranks 22.5 -> 7.4 us.
 #pragma once
 

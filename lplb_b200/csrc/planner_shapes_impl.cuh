@@ -33,7 +33,8 @@ cudaError_t SolveLaunch::operator()() const {
     if constexpr (GP == -1) {
       const size_t smem = solver_smem<GP>(tp, warps);
       if ((err = allow_smem(tile_solve_kernel<1, D>, smem)) != cudaSuccess) return err;
-      // an early launch: 14.3 -> 11.6 us for 64 groups of 8 ranks, one call after the other, 64 ranks 59 -> 52
+      // an early launch, one call after the other: one group 12.5 -> 11.2 us, 64 groups 14.4 -> 12.4; several warps per
+      // group 16 ranks 19.8 -> 18.0, 32 ranks 28.1 -> 26.1, 64 ranks 53.5 -> 52.1
       return launch_after(tile_solve_kernel<1, D>, grid + 1, kBlock, smem, stream, workload, tp, prm, probs, normalised, avail,
                           status, warps);
     } else {
