@@ -15,10 +15,12 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include <map>
 #include <mutex>
 #include <sstream>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "place_api.h"
@@ -231,6 +233,7 @@ class PlannerEngine {
     LPLB_CHECK(lplb::resolve_solver(g_, d_, k) > 0, "the " << kind << " solver does not cover " << g_ << " ranks x " << d_ << " replicas");
     prm_.solver = k;
     max_cta64_ = max_cta32_ = -1;
+    cluster_limit_.clear();
     if (warm_) set_warm_start(true, prm_.guard, prm_.snap_mu);
     invalidate_warm_start();
   }
@@ -319,8 +322,10 @@ class PlannerEngine {
   // `idx` may also be a pinned host tensor: the kernel then reads it over PCIe itself and,
   // if `out` is a pinned host tensor too, writes the result straight back, which replaces two
   // copy-engine transfers and their launch latencies.  `out` must match `idx` in shape/dtype.
+  // `cluster`: 0 runs the grid-wide kernel of n_cta CTAs, 2 to 16 a cluster of so many, -1 whichever suits the
+  // batch (n_cta then serves where that is the grid-wide kernel).
   torch::Tensor run_fused(const torch::Tensor& idx, torch::Tensor avail, int n_cta, bool use_exchange,
-                          c10::optional<torch::Tensor> out_opt) {
+                          c10::optional<torch::Tensor> out_opt, int cluster) {
     require_mapping();
     const bool host_idx = !idx.is_cuda();
     if (host_idx) {
@@ -336,6 +341,13 @@ class PlannerEngine {
     LPLB_CHECK(has_native_solver(), "the fused kernel needs a group of at most " << lplb::kMaxGroupSize
                                         << " ranks with at most " << lplb::kMaxDup << " replicas each");
     LPLB_CHECK(!use_exchange || n_ranks_ <= 32, "the in-kernel exchange covers at most 32 ranks");
+    const auto topology = topo();
+    if (cluster < 0) {
+      cluster = lplb::cluster_ctas(idx.numel());
+      long long& most = cluster_limit_[{is64, cluster}];  // asked once
+      if (most < 0) most = lplb::cluster_limit(topology, prm_.solver, is64, cluster);
+      if (idx.numel() > most) cluster = 0;
+    }
     int& limit = is64 ? max_cta64_ : max_cta32_;
     if (limit < 0) limit = lplb::max_fused_ctas(topo(), prm_.solver, is64);
     LPLB_CHECK(limit >= 2, "fused kernel cannot be resident on this device");
@@ -358,7 +370,15 @@ class PlannerEngine {
       LPLB_CHECK(exchange_open_, "exchange buffers are not open; call open_exchange first");
       ex = exchange_desc();
     }
-    LPLB_CUDA(lplb::launch_fused(idx.data_ptr(), is64, idx.numel(), topo(), ex, prm_, workspace_.data_ptr(),
+    if (cluster > 0) {
+      LPLB_CUDA(lplb::launch_cluster(idx.data_ptr(), is64, idx.numel(), topology, ex, prm_, workspace_.data_ptr(),
+                                     probs_.data_ptr<float>(), avail.data_ptr(), avail.scalar_type() == torch::kInt64,
+                                     status_.data_ptr<int>(), out.data_ptr(), cluster, grid_timeout_ns_,
+                                     trace_.defined() ? reinterpret_cast<unsigned long long*>(trace_.data_ptr()) : nullptr,
+                                     stream()));
+      return out;
+    }
+    LPLB_CUDA(lplb::launch_fused(idx.data_ptr(), is64, idx.numel(), topology, ex, prm_, workspace_.data_ptr(),
                                  probs_.data_ptr<float>(), avail.data_ptr(), avail.scalar_type() == torch::kInt64,
                                  status_.data_ptr<int>(), out.data_ptr(), n_cta, grid_timeout_ns_,
                                  trace_.defined() ? reinterpret_cast<unsigned long long*>(trace_.data_ptr()) : nullptr,
@@ -551,6 +571,11 @@ class PlannerEngine {
   std::mutex place_mutex_;
   torch::Tensor place_report_;  // pinned [1], written by place_kernel
   int max_cta64_ = -1, max_cta32_ = -1;
+  struct Unknown {
+    long long value = -1;
+    operator long long&() { return value; }
+  };
+  std::map<std::pair<int, int>, Unknown> cluster_limit_;  // by width of the indices and CTAs
   // exchange
   IpcBlock block_;
   std::vector<void*> peers_;
@@ -592,7 +617,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("solve", &PlannerEngine::solve)
       .def("map_idx", &PlannerEngine::map_idx)
       .def("run_fused", &PlannerEngine::run_fused, py::arg("idx"), py::arg("avail"), py::arg("n_cta"),
-           py::arg("use_exchange"), py::arg("out") = py::none())
+           py::arg("use_exchange"), py::arg("out") = py::none(), py::arg("cluster") = 0)
       .def("all_reduce_counts", &PlannerEngine::all_reduce_counts)
       .def("alloc_exchange", &PlannerEngine::alloc_exchange)
       .def("open_exchange", &PlannerEngine::open_exchange)

@@ -412,40 +412,57 @@ __device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (
   }
 }
 
+// A lane's part of the saved iterate of its group, read whether it is valid or not (the slot is always
+// allocated), so that whoever waits for the counts has the loads behind it by then.
+struct TileStart {
+  double f = 0.5, v = 0.5, z = 1.0, q = 1.0, s = 1.0, y = 0.0, t = 0.0;
+  bool saved = false;
+};
+// `anchor`: the rank's slot, or null for a rank that does not take part; `group_anchor`: that of the group's first rank.
+template <int D>
+__device__ __forceinline__ TileStart load_tile_start(int edge, const double* anchor, const double* group_anchor,
+                                                     const int* anchor_valid) {
+  TileStart a;
+  if (anchor != nullptr) {
+    if (edge < D) {
+      a.f = anchor[edge];
+      a.v = anchor[D + edge];
+      a.z = anchor[2 * D + edge];
+      a.q = anchor[3 * D + edge];
+    }
+    a.s = anchor[4 * D];
+    a.y = anchor[4 * D + 1];
+  }
+  if (group_anchor != nullptr) {
+    a.t = group_anchor[4 * D + 2];
+    a.saved = *anchor_valid != 0;
+  }
+  return a;
+}
+
 // One group of at most 8 NB ranks, solved by NB warps (all of them call; `warp` counts from 0 within the
 // group).  Lane 4 r + c of warp I is edge c of rank 8 I + r (see above) and passes that bundle's load, the
 // rank's non-replicated load, and the ranks whose bundle it holds (`src`) and that hold its own (`dst`); dummies
 // and ranks from `rows` on, which do not take part, pass no load and themselves.  All four lanes of a
 // rank pass `mine`, the rank's whole own load.  `sm`: tile_solver_smem_bytes of shared memory, 16-byte
-// aligned.  `anchor`: the rank's slot of the warm-start state or null; `group_anchor` the slot of the
-// group's first rank.  The outcome is the same on every lane, the share is the lane's own.
+// aligned.  `anchor`: the rank's slot of the warm-start state or null; `group_anchor` the slot of the group's first rank;
+// `early`: what load_tile_start found there, or null.  The outcome is the same on every lane, the share is the lane's own.
 template <int NB, int D>
 __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int lane, const int rows, const double w_in,
                                                       const double fixed, const double own_load, const int src,
-                                                      const int dst, const IpmParams prm, double& f_out, double* anchor,
-                                                      const double* group_anchor, int* anchor_valid, double* sm) {
+                                                      const int dst, const IpmParams prm, double& f_out, const TileStart* early,
+                                                      double* anchor, const double* group_anchor, int* anchor_valid, double* sm) {
   constexpr double kEta = 0.995;
   const TileTeam<NB, D> tm(warp, lane, sm);
   const int c = tm.c, rank = tm.rank;
   const bool live = rank < rows, real = tm.edge < D;
   const bool first = tm.edge == 0;  // the lane that adds the rank's own part to sums over lanes
   sweep_scratch_init(tm.sweep(), lane);
-  // The saved iterate is read first, valid or not (the slot is always allocated): its loads are
-  // in flight while the scaling is computed.
+  // The saved iterate's loads are in flight while the scaling is computed, unless the caller has made them already.
+  const TileStart start = early != nullptr ? *early : load_tile_start<D>(tm.edge, live ? anchor : nullptr, group_anchor, anchor_valid);
   const bool slot = anchor != nullptr && live;
-  double fa = 0.5, va = 0.5, za = 1.0, qa = 1.0, sa = 1.0, ya = 0.0, ta = 0.0;
-  if (slot) {
-    if (real) {
-      fa = anchor[tm.edge];
-      va = anchor[D + tm.edge];
-      za = anchor[2 * D + tm.edge];
-      qa = anchor[3 * D + tm.edge];
-    }
-    sa = anchor[4 * D];
-    ya = anchor[4 * D + 1];
-  }
-  if (group_anchor != nullptr) ta = group_anchor[4 * D + 2];
-  const bool saved_before = group_anchor != nullptr && *anchor_valid != 0;
+  const double fa = start.f, va = start.v, za = start.z, qa = start.q, sa = start.s, ya = start.y, ta = start.t;
+  const bool saved_before = start.saved;
 
   const double kcomp = (double)(rows + 2 * rows * D), inv_kcomp = rcp3(kcomp), inv_rows = rcp3((double)rows);
 

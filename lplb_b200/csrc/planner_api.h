@@ -90,6 +90,16 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
                          void* out, int n_cta, unsigned long long grid_timeout_ns, unsigned long long* trace,
                          int cooperative, cudaStream_t stream);
 
+// The same step in one thread-block cluster of n_cta CTAs (2 to 16; CTA 0 exchanges and solves): up to 1024 experts, groups of
+// up to 32 ranks, and at most cluster_limit() indices (cudaErrorInvalidValue otherwise).
+cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const TopoDesc& topo, const ExchangeDesc& ex,
+                           SolveParams prm, void* workspace, float* probs, void* avail, int avail_is64, int* status,
+                           void* out, int n_cta, unsigned long long timeout_ns, unsigned long long* trace, cudaStream_t stream);
+// The cluster that suits a batch of n indices, and how many a cluster takes: up to there it is faster than the grid-wide
+// kernel.  0 where shape or device cannot run one.
+int cluster_ctas(long long n);
+long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_cta);
+
 // Co-resident CTA limit of the fused kernel for this topology on the current device (0 when the
 // shape has no device solver or its tables do not fit shared memory).
 int max_fused_ctas(const TopoDesc& topo, int solver, int idx_is64);

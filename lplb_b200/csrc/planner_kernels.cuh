@@ -410,33 +410,56 @@ __device__ __forceinline__ void solve_groups_block(const int* __restrict__ bundl
   }
 }
 
+// What a lane of the tile solver needs besides the bundle sums: its edge, and its part of the saved iterate of `grp`.
+struct TileLane {
+  int src, dst;
+  TileStart start;
+};
+template <int NB, int D>
+__device__ __forceinline__ TileLane load_tile_lane(const Topo& tp, int team_warp, int* status) {
+  const int lane = threadIdx.x & 31, rank = 8 * team_warp + (lane >> 2);
+  const int d = lane & (TileTeam<NB, D>::kLanes - 1);
+  TileLane l;
+  l.src = l.dst = rank;
+  if (rank < tp.g && d < D) {
+    const int s = tp.r2o[rank * D + d], t = tp.o2r[rank * D + d];
+    if (LPLB_CHECKED(s, tp.g, status, kPhSolve) && LPLB_CHECKED(t, tp.g, status, kPhSolve)) {
+      l.src = s;
+      l.dst = t;
+    }
+  }
+  return l;
+}
+template <int NB, int D>
+__device__ __forceinline__ void load_tile_start_of(const Topo& tp, int grp, int team_warp, const IpmParams& prm, TileLane* l) {
+  if (prm.anchor == nullptr || grp >= tp.n_group) return;
+  const int lane = threadIdx.x & 31, rank = 8 * team_warp + (lane >> 2);
+  const double* group_anchor = prm.anchor + (size_t)grp * tp.g * (4 * D + 3);
+  l->start = load_tile_start<D>(lane & (TileTeam<NB, D>::kLanes - 1), rank < tp.g ? group_anchor + (size_t)rank * (4 * D + 3) : nullptr,
+                                group_anchor, prm.anchor_valid + grp);
+}
+
 // Tile solver: NB warps per group, `team_warp` is the calling warp's place among them; the team
 // solves groups first_group, first_group + group_stride, ...  `scratch` is the team's
-// tile_solver_smem_bytes(tp.g, D) of shared memory, 16-byte aligned.  `share`: a copy of the shares in
-// shared memory, or null.
-template <int NB, int D>
+// tile_solver_smem_bytes(tp.g, D) of shared memory, 16-byte aligned.  EARLY: `mine` holds the saved iterate of the first
+// group.  `probs` and `status` may be null for a solve that leaves nothing behind.  `share`: a copy of the shares in shared
+// memory, or null; shared() is called when the warp's last is there.
+template <int NB, int D, bool EARLY, typename Shared>
 __device__ __forceinline__ void solve_groups_tiles(const int* __restrict__ bundle, const Topo& tp, int first_group, int group_stride,
-                                   int team_warp, IpmParams prm, float* __restrict__ probs, float* share, Counter avail,
-                                   int* status, double* scratch) {
+                                   int team_warp, IpmParams prm, TileLane mine, float* __restrict__ probs, float* share,
+                                   Counter avail, int* status, double* scratch, Shared shared) {
   const int lane = threadIdx.x & 31, rank = 8 * team_warp + (lane >> 2);
   const int d = lane & (TileTeam<NB, D>::kLanes - 1);
   const bool live = rank < tp.g, real = live && d < D;
-  int src = rank, dst = rank;
-  if (real) {
-    const int s = tp.r2o[rank * D + d], t = tp.o2r[rank * D + d];
-    if (LPLB_CHECKED(s, tp.g, status, kPhSolve) && LPLB_CHECKED(t, tp.g, status, kPhSolve)) {
-      src = s;
-      dst = t;
-    }
-  }
   for (int grp = first_group; grp < tp.n_group; grp += group_stride) {
+    if (EARLY && grp != first_group) load_tile_start_of<NB, D>(tp, grp, team_warp, prm, &mine);
     double w = 0.0, fixed = 0.0, own = 0.0, f;
     if (live) {
-      const int* mine = bundle + ((size_t)grp * tp.g + rank) * (D + 1);
-      fixed = own = (double)mine[D];
+      const int* sums = bundle + ((size_t)grp * tp.g + rank) * (D + 1);
+      fixed = own = (double)sums[D];
 #pragma unroll
-      for (int k = 0; k < D; ++k) own += (double)mine[k];
-      if (real) w = (double)mine[d];
+      for (int k = 0; k < D; ++k) own += (double)sums[k];
+      if (real) w = (double)sums[d];
     }
     double *anchor = nullptr, *group_anchor = nullptr;
     int* anchor_valid = nullptr;
@@ -444,15 +467,21 @@ __device__ __forceinline__ void solve_groups_tiles(const int* __restrict__ bundl
       group_anchor = prm.anchor + (size_t)grp * tp.g * (4 * D + 3);
       if (live) anchor = group_anchor + (size_t)rank * (4 * D + 3);
       anchor_valid = prm.anchor_valid + grp;
+    } else {
+      mine.start.saved = false;  // taken back after the load (see exchange_step)
     }
-    const IpmOutcome res = ipm_solve_tiles<NB, D>(team_warp, lane, NB == 1 && prm.pad_rows ? 8 : tp.g, w, fixed, own, src, dst, prm,
-                                                  f, anchor, group_anchor, anchor_valid, scratch);
-    if (live && (lane & 3) < D) {
-      const size_t at = ((size_t)grp * tp.g + rank) * D + d;
-      probs[at] = (float)f;
-      if (share != nullptr) share[at] = (float)f;
+    const IpmOutcome res = ipm_solve_tiles<NB, D>(team_warp, lane, NB == 1 && prm.pad_rows ? 8 : tp.g, w, fixed, own, mine.src,
+                                                  mine.dst, prm, f, EARLY ? &mine.start : nullptr, anchor, group_anchor,
+                                                  anchor_valid, scratch);
+    const bool writes = live && (lane & 3) < D;
+    const size_t at = ((size_t)grp * tp.g + rank) * D + d;
+    if (writes && share != nullptr) share[at] = (float)f;
+    if (grp + group_stride >= tp.n_group) {
+      __syncwarp();
+      shared();
     }
-    if (rank == 0 && lane == 0) report_group(res, grp, avail, status);
+    if (writes && probs != nullptr) probs[at] = (float)f;
+    if (rank == 0 && lane == 0 && status != nullptr) report_group(res, grp, avail, status);
   }
 }
 
@@ -519,11 +548,13 @@ __global__ void __launch_bounds__(kBlock) tile_solve_kernel(const int* __restric
   if (blockIdx.x == 0 && threadIdx.x == 0) status[kStLpIters] = status[kStGapPpb] = 0;
   extern __shared__ __align__(16) int smem[];
   int* bundle = smem;
-  const int first = (int)blockIdx.x * teams, warp = threadIdx.x >> 5;
+  const int first = (int)blockIdx.x * teams, warp = threadIdx.x >> 5, team_warp = NB == 1 ? 0 : warp;
   bundle_sums(workload, tp, bundle, min(tp.n_group, first) * tp.g, min(tp.n_group, first + teams) * tp.g, status);
-  if (warp < teams * NB)
-    solve_groups_tiles<NB, D>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, NB == 1 ? 0 : warp, prm, probs, nullptr, avail,
-                              status, scratch_after(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total);
+  if (warp < teams * NB) {
+    const TileLane mine = load_tile_lane<NB, D>(tp, team_warp, status);
+    solve_groups_tiles<NB, D, false>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, team_warp, prm, mine, probs, nullptr, avail, status,
+                              scratch_after(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total, [] {});
+  }
 }
 
 // Stand-alone solve kernel, thread-block solver: one CTA per group (the reference launches
@@ -769,6 +800,97 @@ __device__ __forceinline__ unsigned exchange_counts(const Exchange& ex, Exchange
 }
 
 // ---------------------------------------------------------------------------------------
+// Parts of the planner step's solver CTA, in the kernel below and in planner_cluster.cuh.
+
+// The solver's inputs go to L2 and to this SM's L1 while the workers count (they were evicted if
+// anything ran since the last step).
+template <int D>
+__device__ __forceinline__ void prefetch_solver_inputs(const Topo& tp, const IpmParams& prm) {
+  const int ranks = tp.n_group * tp.g;
+  for (int b = threadIdx.x * 128; b < tp.e * 4; b += kBlock * 128)
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(tp.log2slot) + b));
+  for (int b = threadIdx.x * 128; b < tp.g * tp.d * 4; b += kBlock * 128) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(tp.r2o) + b));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(tp.o2r) + b));
+  }
+  if (prm.anchor != nullptr) {  // warm-start state: (4 D + 3) doubles per rank
+    for (int b = threadIdx.x * 128; b < ranks * (4 * D + 3) * 8; b += kBlock * 128)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(prm.anchor) + b));
+    if (threadIdx.x == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(prm.anchor_valid));
+  }
+}
+
+// The solver CTA's exchange of `vec` with the peers.
+__device__ __forceinline__ void exchange_step(const Exchange& ex, ExchangeShared* xs, uint32_t epoch, const Topo& tp, int* vec,
+                                              IpmParams& prm, int* status, unsigned long long* trace) {
+  const unsigned miss = exchange_counts<kBlock>(ex, xs, epoch, tp.e, vec, status, trace != nullptr ? trace + 8 : nullptr);
+  if (miss) {
+    // Shares made from substituted statistics must not become the next warm start, and the
+    // saved iterate may no longer match the peers': this solve and the next one start cold.
+    if (prm.anchor_valid != nullptr)
+      for (int g = threadIdx.x; g < tp.n_group; g += kBlock) prm.anchor_valid[g] = 0;
+    prm.anchor = nullptr;
+    prm.anchor_valid = nullptr;
+    if (threadIdx.x == 0) {
+      atomicAdd(&status[kStTimeouts], 1);
+      raise_status(status, kErrPeerTimeout, kPhExchange, (int)miss);
+    }
+  }
+}
+
+// The tile solver inside the solver CTA: a group per warp (GP = -1), or -GP warps on one after the other.
+//
+// Whatever ran since the last step has evicted the solver's code from the SM's instruction caches, and a warp that runs it
+// once from start to end waits for every line of it.  So while the workers count, the CTA's last warp goes through the same
+// code, one iteration on made-up loads, and the solving warps find it in the cache: 8 ranks, one iteration 4.2 -> 2.9 us,
+// two 5.7 -> 4.4.  (It has to be the same code, not a copy of it, and another warp: the solving ones would still be rehearsing
+// when the counts are in.)  Groups of several warps have none left for it that share a barrier of their own: given one, the
+// solve itself got slower (32 ranks 10.6 -> 11.6 us).
+template <int GP>
+struct TileStep {
+  static constexpr int kRehearsing = kWarps - 1;
+  static __device__ __forceinline__ int solving(const Topo& tp) { return GP == -1 ? min(tp.n_group, kWarps) : -GP; }
+  // not beside more than four groups, whose warps would share a scheduler with it and each other
+  static __device__ __forceinline__ bool rehearses(const Topo& tp) { return GP == -1 && tp.n_group <= kWarps / 2; }
+};
+template <int GP, int D>
+__device__ __forceinline__ TileLane load_step_lane(const Topo& tp, const IpmParams& prm, bool rehearses, int* status) {
+  const int warp = threadIdx.x >> 5;
+  TileLane mine{};
+  if (warp < TileStep<GP>::solving(tp) || rehearses) {
+    mine = load_tile_lane<-GP, D>(tp, GP == -1 ? 0 : warp, status);
+    if (!rehearses) load_tile_start_of<-GP, D>(tp, GP == -1 ? warp : 0, GP == -1 ? 0 : warp, prm, &mine);
+  }
+  return mine;
+}
+// The solve, or with `rehearses` one on `made_up` that leaves nothing behind.  Called by the warps that do either.
+template <int GP, int D, typename Shared>
+__device__ __forceinline__ void solve_step_tiles(int* bundle, const int* made_up, bool rehearses, const Topo& tp, IpmParams prm,
+                                                 const TileLane& mine, float* __restrict__ probs, float* share, Counter avail,
+                                                 int* status, Shared shared) {
+  const int warp = threadIdx.x >> 5;
+  double* scratch = scratch_after(bundle, tp.n_group * tp.g, tp.d);
+  if constexpr (GP == -1) {
+    Topo t = tp;
+    if (rehearses) {
+      t.n_group = kWarps;  // the warp's own group and no other
+      prm.anchor = nullptr;
+      prm.max_iters = 1;
+    }
+    solve_groups_tiles<1, D, true>(rehearses ? made_up - TileStep<GP>::kRehearsing * tp.g * (D + 1) : bundle, t, warp, kWarps, 0, prm, mine,
+                                   rehearses ? nullptr : probs, rehearses ? nullptr : share, avail, rehearses ? nullptr : status,
+                                   scratch + warp * tile_layout(1, D).total, shared);
+  } else {
+    solve_groups_tiles<-GP, D, true>(bundle, tp, 0, 1, warp, prm, mine, probs, share, avail, status, scratch, shared);
+  }
+}
+__device__ __forceinline__ void make_up_loads(int* loads, int n) {
+  for (int i = threadIdx.x; i < n; i += kBlock) loads[i] = 100 + 7 * i % 40;
+}
+// Barrier of the first n threads of the CTA.
+__device__ __forceinline__ void sync_threads(int n) { asm volatile("bar.sync 2, %0;" ::"r"(n) : "memory"); }
+
+// ---------------------------------------------------------------------------------------
 // Single-launch planner step.  Launched cooperatively so that all CTAs are co-resident.
 //
 //   CTAs 1..n  ("workers"): histogram their slice of the indices; reserve an ordinal range per
@@ -810,22 +932,7 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
   __shared__ uint32_t s_epoch;
   __shared__ ExchangeShared xs;
   if (threadIdx.x == 0) s_epoch = ld_acquire_gpu(&ws->epoch) + 1;
-  // The solver's inputs go to L2 and to this SM's L1 while the workers count (they were
-  // evicted if anything ran since the last step).
-  {
-    const int ranks = tp.n_group * tp.g;
-    for (int b = threadIdx.x * 128; b < e * 4; b += kBlock * 128)
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(tp.log2slot) + b));
-    for (int b = threadIdx.x * 128; b < tp.g * tp.d * 4; b += kBlock * 128) {
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(tp.r2o) + b));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(tp.o2r) + b));
-    }
-    if (prm.anchor != nullptr) {  // warm-start state: (4 D + 3) doubles per rank
-      for (int b = threadIdx.x * 128; b < ranks * (4 * D + 3) * 8; b += kBlock * 128)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(prm.anchor) + b));
-      if (threadIdx.x == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(prm.anchor_valid));
-    }
-  }
+  prefetch_solver_inputs<D>(tp, prm);
   exchange_prepare(ex, &xs);
   __shared__ int s_stop;
   if (threadIdx.x == 0) s_stop = 0;
@@ -839,12 +946,26 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
   int* bundle = smem + 3 * (size_t)e;
   constexpr int NT = kBlock;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the tile solver's last warp rehearses, and nothing else
+  constexpr bool kTiles = GP < 0, kMayRehearse = GP == -1;
+  const bool rehearsal = kMayRehearse && ex.n_ranks <= 1 && TileStep<GP>::rehearses(tp);
+  const bool rehearses = rehearsal && warp == TileStep<GP>::kRehearsing;
+  const int n_threads = rehearsal ? NT - 32 : NT;  // the others
+  __shared__ int made_up[kMayRehearse ? 8 * (D + 1) : 1];
   const int first = threadIdx.x;  // its table entries are in flight while the workers count
   const int first_slot = first < e ? tp.log2slot[first] : 0;
   const int first_edge = first < e ? tp.log2edge[first] : -1;
   int* glob = ws_global(ws, e);
   const int n_bundle = tp.n_group * tp.g * (tp.d + 1);
   for (int i = threadIdx.x; i < n_bundle; i += NT) bundle[i] = 0;
+  TileLane mine{};
+  if constexpr (kTiles) {
+    mine = load_step_lane<GP, D>(tp, prm, rehearses, status);
+    if (kMayRehearse) {
+      make_up_loads(made_up, 8 * (D + 1));
+      __syncthreads();
+    }
+  }
   // one expert's group-wide count -> its rank's bundle load, and a copy for the host
   auto add_count = [&](int i, int c) {
     glob[i] = c;
@@ -875,8 +996,7 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
       // solver's code from the caches, the instruction caches included, and one warp running
       // two thousand straight-line instructions per iteration waits for every line of it; here
       // it takes the first of those waits while it has nothing else to do.  Nothing it
-      // computes is kept.  (The tile solver's code is less than half as long: a rehearsal costs it 0.2 to 1.4 us
-      // a step more than it gives, one through the very code that solves 1 us or more.)
+      // computes is kept.  (The tile solver rehearses in another way, see TileStep.)
       const int li = lane, g = tp.g;
       if (lane < GP) {
         double w[D], f[D];
@@ -895,49 +1015,38 @@ __device__ __forceinline__ void solver_cta(Topo tp, const Exchange& ex, IpmParam
       }
     }
   }
-  team_sync<NT>();
-  // the workers' counts are in total_g: their atomics precede their arrivals
-  int* other = ws_total(ws, parity ^ 1, e);
-  for (int i = threadIdx.x; i < e; i += NT) {
-    vec[i] = local[i] = __ldcg(&total_g[i]);
-    other[i] = 0;  // ready for the next launch
-    if (ex.n_ranks <= 1) add_count(i, vec[i]);
-  }
-  team_sync<NT>();
-  if (ex.n_ranks > 1) {
-    const unsigned miss = exchange_counts<NT>(ex, &xs, epoch, e, vec, status, trace != nullptr ? trace + 8 : nullptr);
-    if (miss) {
-      // Shares made from substituted statistics must not become the next warm start, and the
-      // saved iterate may no longer match the peers': this solve and the next one start cold.
-      if (prm.anchor_valid != nullptr)
-        for (int g = threadIdx.x; g < tp.n_group; g += NT) prm.anchor_valid[g] = 0;
-      prm.anchor = nullptr;
-      prm.anchor_valid = nullptr;
-      if (threadIdx.x == 0) {
-        atomicAdd(&status[kStTimeouts], 1);
-        raise_status(status, kErrPeerTimeout, kPhExchange, (int)miss);
-      }
+  if (!rehearses) {
+    sync_threads(n_threads);
+    // the workers' counts are in total_g: their atomics precede their arrivals
+    int* other = ws_total(ws, parity ^ 1, e);
+    for (int i = threadIdx.x; i < e; i += n_threads) {
+      vec[i] = local[i] = __ldcg(&total_g[i]);
+      other[i] = 0;  // ready for the next launch
+      if (ex.n_ranks <= 1) add_count(i, vec[i]);
     }
-    for (int i = threadIdx.x; i < e; i += NT) add_count(i, vec[i]);
-    team_sync<NT>();
+    sync_threads(n_threads);
+    if (ex.n_ranks > 1) {
+      exchange_step(ex, &xs, epoch, tp, vec, prm, status, trace);
+      for (int i = threadIdx.x; i < e; i += NT) add_count(i, vec[i]);
+      team_sync<NT>();
+    }
+    if (tracing) trace[3] = global_timer_ns();
   }
-  if (tracing) trace[3] = global_timer_ns();
-  double* scratch = scratch_after(bundle, tp.n_group * tp.g, tp.d);
-  if constexpr (GP == 0) {
-    solve_groups_block<D>(bundle, tp, 0, 1, prm, probs, share, avail, status, scratch);
-  } else if constexpr (GP == -1) {  // one group per warp
-    solve_groups_tiles<1, D>(bundle, tp, warp, kWarps, 0, prm, probs, share, avail, status, scratch + warp * tile_layout(1, D).total);
-  } else if constexpr (GP < 0) {
-    if (warp < -GP) solve_groups_tiles<-GP, D>(bundle, tp, 0, 1, warp, prm, probs, share, avail, status, scratch);
+  if constexpr (kTiles) {
+    if (rehearses || warp < TileStep<GP>::solving(tp))
+      solve_step_tiles<GP, D>(bundle, made_up, rehearses, tp, prm, mine, probs, share, avail, status, [] {});
+  } else if constexpr (GP == 0) {
+    solve_groups_block<D>(bundle, tp, 0, 1, prm, probs, share, avail, status, scratch_after(bundle, tp.n_group * tp.g, tp.d));
   } else {
     solve_groups<GP, D, true>(bundle, tp, 0, (NT / 32) * (32 / GP), prm, probs, share, avail, status);
   }
-  team_sync<NT>();
+  if (rehearses) return;
+  sync_threads(n_threads);
   // Quotas and totals go out as words that carry the launch number, so a worker that sees one has it:
   // no fence, no flag, no second round trip.
   unsigned long long* result = ws_result(ws, e);
   const unsigned long long tag = (unsigned long long)epoch << 32;
-  for (int i = threadIdx.x; i < e; i += NT) {
+  for (int i = threadIdx.x; i < e; i += n_threads) {
     const int tot = local[i], quota = quota_of(tot, i == first ? first_edge : tp.log2edge[i], share);
     st_volatile_u64x2(result + 2 * (size_t)i, tag | (uint32_t)quota, tag | (uint32_t)tot);
   }

@@ -220,6 +220,48 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
   return dispatch_shape(topo.g, topo.d, prm.solver, pack_groups(l.tp), l);
 }
 
+namespace {
+template <typename IdxT>
+cudaError_t cluster_step(const void* idx, long long n, const Topo& tp, const Exchange& ex, const SolveParams& prm, void* workspace,
+                         float* probs, Counter avail, int* status, void* out, int n_cta, unsigned long long timeout_ns,
+                         unsigned long long* trace, cudaStream_t stream, int* fits) {
+  const ClusterLaunch<IdxT> l{static_cast<const IdxT*>(idx), n, tp, ex, make_params(prm, tp.g, tp.d),
+                              static_cast<Workspace*>(workspace), probs, avail, status, static_cast<IdxT*>(out), n_cta,
+                              timeout_ns, trace, stream, fits};
+  return dispatch_shape(tp.g, tp.d, prm.solver, pack_groups(tp), l);
+}
+}  // namespace
+
+cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const TopoDesc& topo, const ExchangeDesc& exd,
+                           SolveParams prm, void* workspace, float* probs, void* avail, int avail_is64, int* status,
+                           void* out, int n_cta, unsigned long long timeout_ns, unsigned long long* trace, cudaStream_t stream) {
+  if (!shape_ok(topo, true, prm.solver) || n_cta < 2 || n_cta > kClusterMaxCtas || exd.n_ranks > kMaxRanks) return cudaErrorInvalidValue;
+  const Topo tp = make_topo(topo);
+  if (tp.e > kClusterMaxExperts) return cudaErrorInvalidValue;
+  const Exchange ex{exd.recv, exd.n_ranks, exd.my_rank, exd.node_size, exd.timeout_ns};
+  return (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(idx, n, tp, ex, prm, workspace, probs, Counter{avail, avail_is64},
+                                                                     status, out, n_cta, timeout_ns, trace, stream, nullptr);
+}
+
+int cluster_ctas(long long n) {
+  int n_cta = 2;
+  while (n_cta < kClusterMaxCtas && n > (long long)(n_cta - 1) * kClusterShare) n_cta *= 2;
+  return n_cta;
+}
+
+long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_cta) {
+  const Topo tp = make_topo(topo);
+  if (!shape_ok(topo, true, solver) || tp.e > kClusterMaxExperts) return 0;
+  SolveParams prm{1, 1.0};
+  prm.solver = solver;
+  const long long n = (long long)(n_cta - 1) * cluster_max_slice(tile_rows(tp.g) == 1 ? -1 : -2);
+  int fits = 0;
+  const cudaError_t err = (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(
+      nullptr, n, tp, Exchange{}, prm, nullptr, nullptr, Counter{}, nullptr, nullptr, n_cta, 0, nullptr, nullptr, &fits);
+  if (err != cudaSuccess) cudaGetLastError();  // this shape does not run in a cluster
+  return err == cudaSuccess && fits > 0 ? n : 0;
+}
+
 int max_fused_ctas(const TopoDesc& topo, int solver, int idx_is64) {
   int result = 0;
   if (!shape_ok(topo, true, solver)) return 0;

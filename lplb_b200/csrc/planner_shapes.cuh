@@ -6,7 +6,7 @@
 #pragma once
 
 #include "planner_api.h"
-#include "planner_kernels.cuh"
+#include "planner_cluster.cuh"
 
 namespace lplb {
 
@@ -19,6 +19,13 @@ size_t solver_smem(const Topo& tp, int teams = kWarps) {
   if constexpr (GP > 0) return bundle_smem(tp);
   else return bundle_bytes_aligned(tp.n_group * tp.g, tp.d) +
               (GP == 0 ? block_solver_smem_bytes(tp.g, padded_dup(tp.d)) : tile_solver_smem_bytes(tp.g, tp.d, GP == -1 ? teams : 1));
+}
+
+template <int GP>
+size_t cluster_smem(const Topo& tp, long long n, int n_cta) {
+  const size_t solver = sizeof(int) * cluster_solver_words(tp, n_cta - 1) + solver_smem<GP>(tp);
+  const size_t worker = cluster_worker_smem(tp, n, n_cta - 1, cluster_threads(GP));
+  return solver > worker ? solver : worker;
 }
 
 template <typename K>
@@ -60,6 +67,28 @@ struct FusedLaunch {
   cudaStream_t stream;
   template <int GP, int D>
   cudaError_t operator()();
+};
+
+// The step in one cluster (planner_cluster.cuh).  `fits` non-null: only asks whether the device can run it.
+template <typename IdxT>
+struct ClusterLaunch {
+  const IdxT* idx;
+  long long n;
+  Topo tp;
+  Exchange ex;
+  IpmParams prm;
+  Workspace* ws;
+  float* probs;
+  Counter avail;
+  int* status;
+  IdxT* out;
+  int n_cta;
+  unsigned long long timeout_ns;
+  unsigned long long* trace;
+  cudaStream_t stream;
+  int* fits;
+  template <int GP, int D>
+  cudaError_t operator()() const;
 };
 
 struct OccupancyQuery {

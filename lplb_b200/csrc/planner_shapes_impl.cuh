@@ -1,6 +1,8 @@
 // Definitions of the launches that planner_shapes.cuh declares; included by the files that instantiate them.
 #pragma once
 
+#include <atomic>
+
 #include "planner_shapes.cuh"
 
 namespace lplb {
@@ -59,6 +61,49 @@ cudaError_t FusedLaunch<IdxT>::operator()() {
   return cudaLaunchKernel(reinterpret_cast<void*>(kernel), dim3(n_cta), dim3(kBlock), args, smem, stream);
 }
 
+template <typename IdxT>
+template <int GP, int D>
+cudaError_t ClusterLaunch<IdxT>::operator()() const {
+  if constexpr (GP >= 0 || GP < -4) {
+    return cudaErrorInvalidValue;
+  } else {
+    if (n > (long long)(n_cta - 1) * cluster_max_slice(GP)) return cudaErrorInvalidValue;
+    auto kernel = cluster_run_kernel<GP, D, IdxT>;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)n_cta;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_after
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(n_cta);
+    config.blockDim = dim3(cluster_threads(GP));
+    config.dynamicSmemBytes = cluster_smem<GP>(tp, n, n_cta);
+    config.stream = stream;
+    config.attrs = attr;
+    config.numAttrs = fits != nullptr ? 1 : 2;
+    // What a launch may ask for at most is set once per device: both calls together cost the host a microsecond.
+    static std::atomic<uint64_t> ready{0};
+    int dev = 0, most = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (dev > 63 || !(ready.load(std::memory_order_acquire) & bit)) {
+      cudaFuncAttributes has{};
+      if ((err = cudaFuncGetAttributes(&has, kernel)) != cudaSuccess) return err;
+      if ((err = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return err;
+      err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)has.sharedSizeBytes);
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (err != cudaSuccess) return err;
+      ready.fetch_or(bit, std::memory_order_release);
+    }
+    if (fits != nullptr) return cudaOccupancyMaxActiveClusters(fits, kernel, &config);
+    const ClusterHead<IdxT> head{idx, out, reinterpret_cast<const int2*>(tp.log2phy), n,
+                                 cluster_slice(n, n_cta - 1, cluster_threads(GP)), tp.e, cluster_replicated(tp)};
+    return cudaLaunchKernelEx(&config, kernel, head, timeout_ns, trace, status, ws, tp, ex, prm, probs, avail);
+  }
+}
+
 template <int GP, int D>
 cudaError_t OccupancyQuery::operator()() const {
   const size_t smem = fused_smem(tp.e) + solver_smem<GP>(tp);
@@ -85,4 +130,6 @@ cudaError_t OccupancyQuery::operator()() const {
   template cudaError_t lplb::SolveLaunch::operator()<GP, D>() const;    \
   template cudaError_t lplb::FusedLaunch<int32_t>::operator()<GP, D>(); \
   template cudaError_t lplb::FusedLaunch<int64_t>::operator()<GP, D>(); \
+  template cudaError_t lplb::ClusterLaunch<int32_t>::operator()<GP, D>() const; \
+  template cudaError_t lplb::ClusterLaunch<int64_t>::operator()<GP, D>() const; \
   template cudaError_t lplb::OccupancyQuery::operator()<GP, D>() const;

@@ -103,10 +103,11 @@ void solve_batch_tiles(int g, int rows, const int* r2o, const int* o2r, int nb, 
       for (int k = 0; live && k < D; ++k) own += mine[k];
       lplb::IpmParams prm{max_iters, tol, anchor, anchor_valid, guard, snap_mu};
       double* group = anchor ? anchor + (size_t)b * g * (4 * D + 3) : nullptr;
+      double* slot = live && anchor ? group + (size_t)rank * (4 * D + 3) : nullptr;
+      int* flag = anchor ? anchor_valid + b : nullptr;
       const lplb::IpmOutcome res = lplb::ipm_solve_tiles<NB, D>(
           warp, lane, rows, real ? mine[d] : 0.0, live ? fixed[(size_t)b * g + rank] : 0.0, own, real ? r2o[rank * D + d] : rank,
-          real ? o2r[rank * D + d] : rank, prm, f, live && anchor ? group + (size_t)rank * (4 * D + 3) : nullptr, group,
-          anchor ? anchor_valid + b : nullptr, scratch.data());
+          real ? o2r[rank * D + d] : rank, prm, f, nullptr, slot, group, flag, scratch.data());
       if (live && (lane & 3) < D) f_out[((size_t)b * g + rank) * D + d] = f;
       if (live && (lane & 3) == 0) {
         if (rank == 0) {

@@ -489,7 +489,9 @@ class Planner:
                 self._staged_probs = None
                 if pick_ctas:
                     n_sms = self._default_ctas(idx.numel())
-                return self._engine.run_fused(idx.contiguous(), avail_counter, int(n_sms), self.comm == "p2p", out)
+                return self._engine.run_fused(
+                    idx.contiguous(), avail_counter, int(n_sms), self.comm == "p2p", out, -1 if pick_ctas else 0
+                )
             if not idx.is_cuda and self._engine is not None:
                 idx = idx.to(self.device, non_blocking=True)
             local, by_sm = self.count_workload(idx, n_sms)

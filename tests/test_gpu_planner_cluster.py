@@ -1,0 +1,168 @@
+"""The planner step in one thread-block cluster against the grid-wide kernel: the same shares, and the same number of
+tokens on every physical expert, at the edges of slices, rounds, rows of counts and lists."""
+
+import re
+from pathlib import Path
+
+import pytest
+import torch
+
+from lplb_b200 import Planner, topology
+
+gpu = pytest.mark.gpu
+CSRC = Path(__file__).resolve().parents[1] / "lplb_b200" / "csrc"
+
+
+def test_the_cluster_kernel_waits_for_its_predecessor_first():
+    text = re.sub(r"//[^\n]*", "", (CSRC / "planner_cluster.cuh").read_text())
+    body = text[re.search(r"cluster_run_kernel\(", text).start() :]
+    statements = [s.strip() for s in body[body.index("{") + 1 :].split(";")]
+    statements = [s for s in statements if "__shared__" not in s]
+    assert statements[:2] == ["allow_successor()", "wait_predecessors()"]
+    assert text.count("wait_predecessors") == 1  # both roles run behind it
+
+
+def _planner(r2o, groups, ll, combined=1, **kw):
+    g, d = r2o.shape
+    ep = g * groups
+    return Planner(r2o, ep * ll + ep * d * combined, ep * ll, ep, device="cuda", n_nodes=1, **kw)
+
+
+def _indices(planner, n, dtype, seed, masked=0.1):
+    gen = torch.Generator("cuda").manual_seed(seed)
+    e = planner.n_logical_routed_experts
+    skew = torch.rand(e, device="cuda", generator=gen) ** 3 + 1e-3
+    idx = torch.multinomial(skew, max(n, 1), replacement=True, generator=gen)[:n]
+    idx[torch.rand(n, device="cuda", generator=gen) < masked] = -1
+    planner.update_redundancy_mapping(torch.bincount(idx + 1, minlength=e + 1)[1:])
+    return idx.to(dtype)
+
+
+def _counts(planner, ids):
+    return torch.bincount(ids.reshape(-1).long() + 1, minlength=planner.n_routed_experts + 1)
+
+
+def _check(planner, idx, cluster, in_place=False):
+    """Two steps in a cluster (a cold and, with warm starts, a warm one) against two of the grid-wide kernel."""
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for step in range(2):
+        results = []
+        for c in (0, cluster):
+            if step == 0:
+                planner.invalidate_warm_start()
+            else:  # the same anchor on both sides
+                planner.invalidate_warm_start()
+                eng.run_fused(idx, avail, 16, False)
+            buf = idx.clone()
+            out = eng.run_fused(buf, avail, 16, False, buf if in_place else None, c)
+            results.append((out, eng.last_probs().clone()))
+        (want, shares), (got, got_shares) = results
+        assert torch.equal(got_shares, shares)
+        assert torch.equal(_counts(planner, got), _counts(planner, want))
+        live = idx >= 0
+        assert torch.equal(planner.phy2log[got[live].long()].long(), idx[live].long())
+        assert bool((got[~live] == -1).all())
+    assert planner.check_status().ok
+
+
+# 512 threads and slices in rounds of them with groups of 8 ranks, 256 with larger ones
+@gpu
+@pytest.mark.parametrize("n", [0, 1, 3, 31, 511, 512, 513, 1024, 1537, 4095, 7681, 30721, 153600])
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+def test_batches_at_the_edges_of_slices_and_rounds(n, dtype):
+    planner = _planner(topology.cube(), 1, 32)
+    idx = _indices(planner, n, dtype, seed=n)
+    for cluster in (2, 4, 8, 16):
+        if n <= (cluster - 1) * 10240:
+            _check(planner, idx, cluster, in_place=cluster == 4)
+
+
+@gpu
+@pytest.mark.parametrize("r2o,groups,ll,combined", [
+    (topology.ring(3), 1, 9, 1),                       # 27 experts: a row that is no whole number of messages
+    (topology.ring(5), 2, 7, 3),                       # fewer ranks than rows of the tile
+    (topology.cube(), 4, 8, 2),                        # one group to each of half of the warps
+    (topology.cube(), 5, 4, 1),                        # more than half of the warps solve: nobody is left to send
+    (topology.cube(), 16, 8, 1),                       # two rounds, 1024 experts
+    (topology.circulant(8, (1, 2, 5)), 1, 6, 2),       # every expert replicated
+    (topology.circulant(7, (1, 2, 3, 6)), 3, 48, 1),   # 1008 experts
+    (topology.hypercube(), 1, 16, 1), (topology.circulant(12, (1, 2, 5, 7)), 2, 5, 1),
+    (topology.torus(8, 4), 1, 32, 1), (topology.circulant(20, (1, 7, 9)), 1, 3, 1),
+])
+@pytest.mark.parametrize("warm", [True, False])
+def test_every_shape_of_groups(r2o, groups, ll, combined, warm):
+    planner = _planner(r2o, groups, ll, combined, warm_start=warm)
+    for n, cluster in ((700, 2), (1025 * 8, 16)):
+        _check(planner, _indices(planner, n, torch.int64, seed=ll), cluster)
+
+
+@gpu
+def test_shapes_and_batches_that_do_not_fit_take_the_grid_wide_kernel():
+    for r2o, groups, ll, n in ((topology.cube(), 1, 32, 153601), (topology.cube(), 17, 8, 4096), (topology.ring(8), 1, 200, 4096),
+                               (topology.torus(8, 4), 1, 8, 15361), (topology.torus(8, 8), 1, 8, 2000), (topology.ring(80), 1, 4, 2000)):
+        planner = _planner(r2o, groups, ll)
+        idx = _indices(planner, n, torch.int64, seed=1)
+        avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+        with pytest.raises(RuntimeError):
+            planner._engine.run_fused(idx, avail, 16, False, None, 16)
+        out = planner.run(idx, avail)
+        assert int(avail) == groups
+        staged = planner._engine.map_idx(idx, planner.last_probs.contiguous(), planner.count_workload(idx, 8)[1], 8)
+        assert torch.equal(_counts(planner, out), _counts(planner, staged))
+
+
+@gpu
+def test_bad_indices_are_counted_and_masked():
+    planner = _planner(topology.cube(), 1, 8)
+    idx = _indices(planner, 2000, torch.int64, seed=4, masked=0.0)
+    idx[::10] = 64
+    idx[1::10] = -7
+    idx[2::10] = (1 << 32) + 5  # in range if its upper half were lost
+    out = planner._engine.run_fused(idx, torch.zeros(1, dtype=torch.int32, device="cuda"), 16, False, None, 8)
+    bad = (idx < 0) | (idx >= 64)
+    assert bool((out[bad] == -1).all()) and bool((out[~bad] >= 0).all())
+    st = planner.check_status(clear=True)
+    assert st["bad_indices"] == int(bad.sum()) and st["error"] == "bad_index"
+
+
+@gpu
+def test_clusters_and_grids_alternate_on_one_engine_without_a_gap():
+    planner = _planner(topology.cube(), 1, 16)
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    batches = [_indices(planner, n, torch.int64, seed=n) for n in (100, 20000, 3000)]
+    outs = []
+    before = eng.completed_launches()
+    for i in range(30):  # each step's indices come from a kernel right in front of it
+        idx = batches[i % 3].clone()
+        outs.append((idx, eng.run_fused(idx, avail, 16, False, None, (0, 4, 16)[i * 7 % 3]), eng.last_probs().clone()))
+    assert eng.completed_launches() == before + 30 and int(avail) == 30 and planner.check_status().ok
+    for idx, out, shares in outs:
+        want = eng.map_idx(idx, shares, planner.count_workload(idx, 8)[1], 8)
+        assert torch.equal(_counts(planner, out), _counts(planner, want))
+
+
+@gpu
+def test_the_exchange_runs_in_a_cluster_too():
+    planner = _planner(topology.cube(), 1, 8, peer_timeout_us=300.0)
+    eng = planner._engine
+    eng.open_exchange_loopback(2, 0)
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    peer = torch.arange(64, dtype=torch.int32) * 3
+    for step in range(3):
+        idx = _indices(planner, 4096, torch.int64, seed=step)
+        eng.debug_fill_slot(1, peer, eng.completed_launches() + 1)
+        out = eng.run_fused(idx, avail, 16, True, None, (2, 8, 16)[step])
+        assert planner.check_status().ok
+        counts = torch.bincount(idx + 1, minlength=65)[1:].int()
+        glob = eng.workspace()[8 + 2 * 64 : 8 + 3 * 64]
+        assert torch.equal(glob.cpu(), counts.cpu() + peer)
+        want = eng.map_idx(idx, eng.last_probs(), planner.count_workload(idx, 8)[1], 8)
+        assert torch.equal(_counts(planner, out), _counts(planner, want))
+    # a peer that never publishes: reported, solved from this rank's counts, nothing kept for a warm start
+    idx = _indices(planner, 4096, torch.int64, seed=9)
+    eng.run_fused(idx, avail, 16, True, None, 8)
+    st = planner.check_status(clear=True)
+    assert st["error"] == "peer_timeout" and st["detail"] == 0b10 and st["timeouts"] == 1
+    assert int(eng.warm_start_valid().sum()) == 0
