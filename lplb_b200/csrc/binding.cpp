@@ -15,6 +15,8 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include <atomic>
+#include <chrono>
 #include <map>
 #include <mutex>
 #include <sstream>
@@ -186,12 +188,23 @@ class PlannerEngine {
       std::lock_guard<std::mutex> one_at_a_time(place_mutex_);  // there is one report word
       if (!place_report_.defined()) place_report_ = torch::zeros({1}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
       volatile int* word = place_report_.data_ptr<int>();
-      *word = lplb::kPlaceOk;
+      *word = lplb::kPlacePending;
       LPLB_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&a.report), place_report_.data_ptr<int>(), 0));
+      if (anchor_valid_.defined()) {
+        a.anchor_valid = anchor_valid_.data_ptr<int>();
+        a.n_anchor = (int)anchor_valid_.numel();
+      }
       LPLB_CUDA(lplb::launch_place(a, stream.stream()));
-      invalidate_warm_start();  // a new placement is a new LP
-      LPLB_CUDA(cudaStreamSynchronize(stream.stream()));
-      report = *word;
+      // The kernel's word is there before the stream is known to be idle; where other work is in front of it, or
+      // the kernel has failed, the stream is waited for.
+      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+      while ((report = *word) == lplb::kPlacePending && std::chrono::steady_clock::now() < until) {}
+      if (report == lplb::kPlacePending) {
+        LPLB_CUDA(cudaStreamSynchronize(stream.stream()));
+        report = *word;
+      }
+      std::atomic_thread_fence(std::memory_order_acquire);
+      LPLB_CHECK(report != lplb::kPlacePending, "the placement kernel has not reported");
     }
     if (report == lplb::kPlaceInexact) return py::none();
     if (report == lplb::kPlaceUncovered) {

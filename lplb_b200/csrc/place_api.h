@@ -7,6 +7,7 @@
 namespace lplb {
 
 enum PlaceReport : int {
+  kPlacePending = -1,   // what the host sets before the launch
   kPlaceOk = 0,
   kPlaceInexact = 1,    // loads of expert groups beyond 2^53: their sums depend on the order of adding; no table was written
   kPlaceUncovered = 2,  // some expert does not sit in exactly one of the ranks' own slots; the tables are not usable
@@ -20,7 +21,9 @@ struct PlaceArgs {
   int n_logical, ep_size, n_group, g, dup, combined, n_nodes;
   // results, and the engine's own copies of them (which keep their addresses)
   int *phy2log, *log2phy, *logcnt, *log2edge;
-  int* report;  // host memory: kPlaceOk before the launch, written only where there is something to report
+  int* report;  // host memory: the outcome, written when everything else is
+  int* anchor_valid;  // [n_anchor] cleared: a new placement is a new LP; may be null
+  int n_anchor;
   int *table_phy2log, *table_log2phy, *table_log2edge, *table_log2slot;
 };
 
