@@ -32,7 +32,7 @@ __host__ __device__ constexpr int cluster_threads(int gp) { return gp == -1 ? 51
 // Indices of one worker at most (8 bytes of shared memory each).  Step and a lookup of its result behind it, grid / cluster, us: 8
 // ranks 1,024 indices 20.2 / 18.0, 16,384 18.5 / 15.8, 32,768 19.2 / 16.2, 65,536 18.5 / 16.5, 131,072 19.2 / 19.2 and with 512
 // experts 26.9 / 24.7; the step alone, 32 ranks, 32,768 indices, 16.3 / 17.7.
-__host__ __device__ constexpr int cluster_max_slice(int gp) { return gp == -1 ? 10240 : 1024; }
+__host__ __device__ constexpr int cluster_max_slice(int gp) { return gp == -1 ? 10240 : gp == -2 ? 2560 : 1024; }
 
 __host__ __device__ inline int cluster_row(int e) { return (e + 3) & ~3; }  // a row of counts, in words: whole messages
 __host__ __device__ inline int cluster_slice(long long n, int n_workers, int threads) {  // indices of a worker, in whole rounds of its threads
@@ -154,7 +154,7 @@ __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& e
   const int solving = Step::solving(tp), first_sender = solving <= kWarps / 2 ? solving : 0;
   const bool rehearsal = ex.n_ranks <= 1 && Step::rehearses(tp), rehearses = rehearsal && warp == Step::kRehearsing;
   const int n_threads = rehearsal ? kBlock - 32 : kBlock;  // those that do not rehearse
-  const TileLane mine = load_step_lane<GP, D>(tp, prm, rehearses, status);
+  const TileLane mine = load_step_lane<GP, D, true>(tp, prm, rehearses, status);
   const uint32_t my_bar = sm100::smem_u32(bar);
   if (threadIdx.x == 0) {
     sm100::mbar_init(my_bar, 1);
@@ -218,7 +218,7 @@ __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& e
     if (tracing) trace[3] = global_timer_ns();
   }
   if (rehearses || warp < solving)
-    solve_step_tiles<GP, D>(bundle, made_up, rehearses, tp, prm, mine, probs, share, avail, status, [&] {
+    solve_step_tiles<GP, D, true>(bundle, made_up, rehearses, tp, prm, mine, probs, share, avail, status, [&] {
       if (!rehearses && first_sender > 0) asm volatile("bar.arrive 3, %0;" ::"r"(n_threads) : "memory");
     });
   const int n_senders = n_threads - first_sender * 32, sender = (int)threadIdx.x - first_sender * 32;

@@ -254,7 +254,7 @@ long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_ct
   if (!shape_ok(topo, true, solver) || tp.e > kClusterMaxExperts) return 0;
   SolveParams prm{1, 1.0};
   prm.solver = solver;
-  const long long n = (long long)(n_cta - 1) * cluster_max_slice(tile_rows(tp.g) == 1 ? -1 : -2);
+  const long long n = (long long)(n_cta - 1) * cluster_max_slice(-tile_rows(tp.g));
   int fits = 0;
   const cudaError_t err = (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(
       nullptr, n, tp, Exchange{}, prm, nullptr, nullptr, Counter{}, nullptr, nullptr, n_cta, 0, nullptr, nullptr, &fits);
