@@ -90,6 +90,8 @@ class PlannerEngine {
     o2r_ = to_dev_i32(o2r);
     const auto to = r2o.to(torch::kCPU, torch::kInt64).contiguous(), from = o2r.to(torch::kCPU, torch::kInt64).contiguous();
     const int64_t *t = to.data_ptr<int64_t>(), *f = from.data_ptr<int64_t>();
+    const auto to32 = to.to(torch::kInt32), from32 = from.to(torch::kInt32);
+    lplb::plan_topology(g_, d_, to32.data_ptr<int>(), from32.data_ptr<int>(), &tile_rounds_, &tile_near_);
     inverse_topology_ = true;
     for (int rank = 0; rank < g_; ++rank)
       for (int d = 0; d < d_; ++d) {
@@ -571,7 +573,7 @@ class PlannerEngine {
   lplb::TopoDesc topo() const {
     return lplb::TopoDesc{r2o_.data_ptr<int>(),     o2r_.data_ptr<int>(),      phy2log_.data_ptr<int>(),
                           log2phy_.data_ptr<int>(), log2edge_.data_ptr<int>(), log2slot_.data_ptr<int>(),
-                          n_group_, g_, d_, ll_, c_};
+                          n_group_, g_, d_, ll_, c_, tile_rounds_, tile_near_};
   }
 
   int n_group_, g_, d_, ll_, c_, e_, device_;
@@ -580,6 +582,7 @@ class PlannerEngine {
   torch::Tensor r2o_, o2r_, phy2log_, log2phy_, log2edge_, log2slot_;
   bool warm_ = false;
   torch::Tensor workspace_, status_, probs_, trace_, anchor_, anchor_valid_;
+  unsigned long long tile_rounds_ = 0, tile_near_ = 0;
   bool inverse_topology_ = false;  // r2o_ and o2r_ are each other's inverse
   std::mutex place_mutex_;
   torch::Tensor place_report_;  // pinned [1], written by place_kernel

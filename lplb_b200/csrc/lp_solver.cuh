@@ -35,6 +35,11 @@
 
 namespace lplb {
 
+// Tile solver, groups of several warps: see plan_tiles.
+struct TilePlan {
+  unsigned long long rounds = 0, near = 0;
+};
+
 struct IpmParams {
   int max_iters;   // hard cap on iterations
   double tol;      // relative duality gap and feasibility target
@@ -56,6 +61,7 @@ struct IpmParams {
   // Tile solver, groups of fewer than 8 ranks: the rows up to 8 take part as ranks without load,
   // as they do in the warp solver.
   bool pad_rows = false;
+  TilePlan plan;
 };
 
 struct IpmOutcome {

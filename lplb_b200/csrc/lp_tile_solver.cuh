@@ -28,8 +28,8 @@
 //
 // Solve kernel, two replicas per rank, unrelated instances, us a call back to back (the warp solver
 // for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 11.2, 64 groups of 8 ranks
-// 26.2 -> 12.4, 16 ranks 40.6 -> 18.0, 32 ranks 64.4 -> 26.1, 64 ranks 147 -> 52.  An iteration: 8 ranks 3.5 -> 1.4,
-// 64 ranks 22.5 -> 7.4 us.
+// 26.2 -> 12.0, 16 ranks 40.6 -> 18.0, 32 ranks 64.4 -> 25.9, 64 ranks 147 -> 46.  An iteration: 8 ranks 3.5 -> 1.4,
+// 64 ranks 22.5 -> 6.6 us.
 #pragma once
 
 #include "lp_solver.cuh"
@@ -96,6 +96,12 @@ __device__ __forceinline__ double rcp2(double x) {
   const double r = rcp_seed(x);
   return fma(r, fma(-x, r, 1.0), r);
 }
+
+#ifdef LPLB_HOST_SIM
+inline int lowest_bit(unsigned x) { return __builtin_ctz(x); }
+#else
+__device__ __forceinline__ int lowest_bit(unsigned x) { return __ffs((int)x) - 1; }
+#endif
 
 #ifdef LPLB_HOST_SIM
 using lplb_sim::from_words;
@@ -198,6 +204,8 @@ enum TileSum : int { kSumStart, kSumCold, kSumMu, kSumDual, kSumX, kSumX1, kSumA
 enum TileMax : int { kMaxLoad, kMaxDown, kMaxCount };
 constexpr int kTileKeys = 4;
 
+constexpr int kRoundsFrom = 8;  // tile rows from which on pivots go in rounds, see sweep_matrix
+
 struct TileLayout {
   int sweep, rows_mat, u, pi, vec, edge, sums, maxes, keys, total;  // in doubles; every part starts on 16 bytes
 };
@@ -206,9 +214,9 @@ __host__ __device__ constexpr TileLayout tile_layout(int nb, int d) {
   const int n = 8 * nb, many = nb > 1;
   int o = 0;
   l.sweep = o, o += nb * kSweepScratch;
-  l.rows_mat = o, o += many * nb * nb * 64;  // normal matrix, tile by tile
-  l.u = o, o += many * 2 * nb * 64;          // pivot columns, two alternating copies
-  l.pi = o, o += many * 2 * 64;              // minus the inverse of the pivot tile, likewise
+  l.rows_mat = o, o += many * nb * nb * 64;  // normal matrix, tile by tile; during the inversion what is left of the pivots' columns
+  l.u = o, o += (many && nb < kRoundsFrom) * 2 * nb * 64;  // pivot columns, two alternating copies
+  l.pi = o, o += many * nb * 64;             // minus the inverses of the pivot tiles
   l.vec = o, o += many * kVecCount * n;
   l.edge = o, o += many * kEdgeCount * d * n;
   l.sums = o, o += many * kSumCount * nb * 2;
@@ -236,9 +244,10 @@ struct TileTeam {
   __device__ __forceinline__ double2* sums(int v) const { return reinterpret_cast<double2*>(sm + kLay.sums) + v * NB; }
   __device__ __forceinline__ double* maxes(int v) const { return sm + kLay.maxes + v * NB; }
   __device__ __forceinline__ unsigned* keys(int v) const { return reinterpret_cast<unsigned*>(sm + kLay.keys) + v * NB; }
-  __device__ __forceinline__ double2* mat() const { return reinterpret_cast<double2*>(sm + kLay.rows_mat) + warp * NB * 32; }
+  __device__ __forceinline__ double2* mat() const { return mat(warp); }  // the warp's tile row
+  __device__ __forceinline__ double2* mat(int row) const { return reinterpret_cast<double2*>(sm + kLay.rows_mat) + row * NB * 32; }
   __device__ __forceinline__ double2* pivot_col(int parity) const { return reinterpret_cast<double2*>(sm + kLay.u) + parity * NB * 32; }
-  __device__ __forceinline__ double2* pivot_inv(int parity) const { return reinterpret_cast<double2*>(sm + kLay.pi) + parity * 32; }
+  __device__ __forceinline__ double2* pivot_inv(int p) const { return reinterpret_cast<double2*>(sm + kLay.pi) + p * 32; }
 
   __device__ __forceinline__ void sync() const {
     if constexpr (NB > 1) {
@@ -360,16 +369,57 @@ struct TileTeam {
   }
 };
 
+// The order in which the tiles of the diagonal become pivots, from the topology.  Pivots that are not coupled at their turn
+// do not touch each other's rows, so they go in one round: of a torus's ring of eight tile rows 0, 2, 4, 6, then 1, 5, then
+// 3, then 7.  Byte r of `rounds` is the set of round r, byte p of `near` the rows that are coupled to pivot p at its turn, those
+// of earlier pivots included.
+// Edges (i, to[i * d + k]) of both tables; entries outside of the group are skipped.
+inline TilePlan plan_tiles(int g, int d, const int* const (&tables)[2]) {
+  const int nb = tile_rows(g);
+  unsigned coupled[8] = {};
+  for (const int* to : tables)
+    for (int i = 0; i < g; ++i)
+      for (int k = 0; k < d; ++k) {
+        const int j = to[i * d + k];
+        if (j < 0 || j >= g || j / 8 == i / 8) continue;
+        coupled[i / 8] |= 1u << (j / 8);
+        coupled[j / 8] |= 1u << (i / 8);
+      }
+  TilePlan plan;
+  unsigned left = (1u << nb) - 1u;
+  for (int r = 0; left != 0; ++r) {
+    unsigned set = 0, blocked = 0;
+    for (int p = 0; p < nb; ++p)
+      if (((left & ~blocked) >> p) & 1u) {
+        set |= 1u << p;
+        blocked |= coupled[p];
+      }
+    for (int p = 0; p < nb; ++p) {
+      if (!((set >> p) & 1u)) continue;
+      plan.near |= (unsigned long long)coupled[p] << (8 * p);
+      for (int i = 0; i < nb; ++i)  // a sweep couples all that its pivot is coupled to
+        if ((coupled[p] >> i) & 1u) coupled[i] |= coupled[p] & ~(1u << i);
+    }
+    plan.rounds |= (unsigned long long)set << (8 * r);
+    left &= ~set;
+  }
+  return plan;
+}
+
 // The inverse of the normal matrix, one tile row per warp: on entry n[j] is tile (I, j) of the
 // matrix, on return minus the inverse's tile.  Block sweeps over the tiles of the diagonal: with P the
 // pivot tile's inverse and U_I the tiles of its column, tile (I, J) becomes N_IJ - U_I P U_J^T, the
-// pivot's column U_I P, its row P U_J^T and the pivot itself -P.  The tiles of a row are kept rotated, so
-// that the pivot's column is always the first and the loop over pivots stays rolled.
+// pivot's column U_I P, its row P U_J^T and the pivot itself -P.  What bounds it is the chain of tile inversions, a round of
+// pivots each, so as many pivots go at once as the topology leaves uncoupled, and tiles that are zero are left out.  (64 ranks
+// of a torus in four rounds instead of eight pivots one after the other: a call 52.0 -> 49.3 us; 40 ranks of a ring with the line
+// before scratch_after 42.9 -> 35.3.)  A column is published in the matrix's place in shared memory, every tile by the warp that
+// owns its row.  Up to four tile rows leave little to do at once, and the plain loop is faster (32 ranks 10.6 us for
+// three iterations in rounds, 10.1 one after the other).
 template <int NB, int D>
-__device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (&n0)[NB], double (&n1)[NB]) {
+__device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, const TilePlan& plan, double (&n0)[NB], double (&n1)[NB]) {
   if constexpr (NB == 1) {
     sweep_tile(n0[0], n1[0], tm.lane, tm.sweep());
-  } else {
+  } else if constexpr (NB < kRoundsFrom) {
     if (tm.warp == 0) {
       double p0 = n0[0], p1 = n1[0];
       sweep_tile(p0, p1, tm.lane, tm.sweep());
@@ -398,7 +448,7 @@ __device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (
       update(1);
       if (tm.warp == p + 1) {
         // The next pivot tile is ready: invert it while the others update theirs.  (The other tiles of
-        // this row are due to be replaced by P U_J^T, so they need no update: 62 -> 52 us at 64 ranks.)
+        // this row are due to be replaced by P U_J^T, so they need no update.)
         double p0 = n0[0], p1 = n1[0];
         sweep_tile(p0, p1, tm.lane, tm.sweep());
         tm.pivot_inv((p + 1) & 1)[tm.lane] = double2{p0, p1};
@@ -409,6 +459,70 @@ __device__ __forceinline__ void sweep_matrix(const TileTeam<NB, D>& tm, double (
       n0[NB - 1] = f0;
       n1[NB - 1] = f1;
     }
+  } else {
+    double2* row = tm.mat();
+    const double2 diag = row[tm.warp * 32 + tm.lane];
+    double g0 = diag.x, g1 = diag.y;  // the row's own pivot tile
+    constexpr int kAtOnce = NB < 4 ? NB : 4;
+#pragma unroll 1
+    for (unsigned long long rounds = plan.rounds; rounds != 0; rounds >>= 8) {
+      const unsigned set = (unsigned)rounds & 0xFFu, next = (unsigned)(rounds >> 8) & 0xFFu;
+      const bool turn = (set >> tm.warp) & 1u;
+      if (turn) {
+        sweep_tile(g0, g1, tm.lane, tm.sweep());
+        tm.pivot_inv(tm.warp)[tm.lane] = double2{g0, g1};
+      }
+      // What the updates below add to is zero in the pivots' columns and in their rows, and in its own column a pivot
+      // stands for minus the identity: so N_IJ + (-U_I P) U_J^T, U_I P and P U_J^T are all one product, without a choice.
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        if ((set >> j) & 1u) {
+          if (j == tm.warp) row[j * 32 + tm.lane] = double2{tm.r == 2 * tm.c ? -1.0 : 0.0, tm.r == 2 * tm.c + 1 ? -1.0 : 0.0};
+          else row[j * 32 + tm.lane] = double2{n0[j], n1[j]};
+          n0[j] = n1[j] = 0.0;
+        } else if (turn) {
+          n0[j] = n1[j] = 0.0;
+        }
+      }
+      tm.sync();
+#pragma unroll 1
+      for (unsigned pivots = set; pivots != 0; pivots &= pivots - 1) {
+        const int p = lowest_bit(pivots);
+        const unsigned near = (unsigned)(plan.near >> (8 * p)) & 0xFFu;
+        const bool pivot = p == tm.warp;
+        if (!pivot && !((near >> tm.warp) & 1u)) continue;
+        const double2 m = tm.pivot_inv(p)[tm.lane];  // -P
+        double a0 = -m.x, a1 = -m.y;
+        if (!pivot) {
+          const double2 u = row[p * 32 + tm.lane];
+          a0 = a1 = 0.0;  // -U_I P
+          mma8(a0, a1, u.x, m.x, a0, a1);
+          mma8(a0, a1, u.y, m.y, a0, a1);
+          mma8(g0, g1, a0, u.x, g0, g1);
+          mma8(g0, g1, a1, u.y, g0, g1);
+          // The other tiles of a row that holds a pivot of the next round are due to be replaced by P U_J^T, so they need no
+          // update, and its pivot can be inverted at once.
+          if ((next >> tm.warp) & 1u) continue;
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < NB; j0 += kAtOnce) {
+          if ((((near | 1u << p) >> j0) & ((1u << kAtOnce) - 1u)) == 0) continue;
+          double2 b[kAtOnce];
+#pragma unroll
+          for (int j = 0; j < kAtOnce; ++j) b[j] = tm.mat(j0 + j)[p * 32 + tm.lane];
+#pragma unroll
+          for (int j = 0; j < kAtOnce; ++j) mma8(n0[j0 + j], n1[j0 + j], a0, b[j].x, n0[j0 + j], n1[j0 + j]);
+#pragma unroll
+          for (int j = 0; j < kAtOnce; ++j) mma8(n0[j0 + j], n1[j0 + j], a1, b[j].y, n0[j0 + j], n1[j0 + j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j == tm.warp) {
+        n0[j] = g0;
+        n1[j] = g1;
+      }
   }
 }
 
@@ -490,7 +604,8 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
         }
     } else {
       double2* mat = tm.mat();
-      for (int j = 0; j < NB; ++j) mat[j * 32 + lane] = double2{0.0, 0.0};
+      if constexpr (NB < kRoundsFrom)
+        for (int j = 0; j < NB; ++j) mat[j * 32 + lane] = double2{0.0, 0.0};
       auto at = [&](int col) { return reinterpret_cast<double*>(mat) + ((col >> 3) * 32 + 4 * tm.r + ((col & 7) >> 1)) * 2 + (col & 1); };
 #pragma unroll
       for (int d = 0; d < D; ++d) {
@@ -622,6 +737,12 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
           at_dst -= (same_dst >> k) & 1u ? val[k] : 0.0;
           at_src -= (same_src >> k) & 1u ? val[k] : 0.0;
         }
+        if constexpr (NB >= kRoundsFrom) {  // the last inversion has left its columns here; several barriers are behind it
+          double2* mat = tm.mat();
+#pragma unroll
+          for (int j = 0; j < NB; ++j) mat[j * 32 + lane] = double2{0.0, 0.0};
+          __syncwarp();
+        }
         if (place_dst != nullptr) *place_dst = at_dst;
         if (place_src != nullptr) *place_src = at_src;
         if (place_diag != nullptr) *place_diag = diag;
@@ -675,7 +796,7 @@ __device__ __forceinline__ IpmOutcome ipm_solve_tiles(const int warp, const int 
     }
     tm.put(kVecG, g);
     tm.put(kVecG1, g_one);
-    sweep_matrix<NB, D>(tm, n0, n1);  // with several warps its barriers also publish the right-hand sides
+    sweep_matrix<NB, D>(tm, prm.plan, n0, n1);  // with several warps its barriers also publish the right-hand sides
     double x, x1, border, same;
     {
       double rs = 0.0;

@@ -22,7 +22,10 @@ struct TopoDesc {
   const int* log2edge;
   const int* log2slot;  // [E] rank * (d + 1) + bundle of the expert (d = the rank's non-replicated ones)
   int n_group, g, d, ll, c;
+  unsigned long long tile_rounds, tile_near;  // from plan_topology
 };
+// The order of pivots that the tile solver takes for a topology (its tables in host memory); shapes that it does not cover: zeros.
+void plan_topology(int g, int d, const int* r2o, const int* o2r, unsigned long long* rounds, unsigned long long* near);
 
 struct ExchangeDesc {
   unsigned long long* const* recv;  // device array of n_ranks pointers (nullptr when n_ranks == 1);

@@ -81,9 +81,10 @@ cudaError_t dispatch_shape(int g, int d, int solver, bool packed, Fn&& fn) {
 // solves with the same code as the stand-alone kernel, bit for bit; beyond, shares agree to rounding (1e-6 of their norm).
 bool pack_groups(const Topo& tp) { return tp.n_group > 2 * kWarps; }
 
-IpmParams make_params(const SolveParams& prm, int g, int d) {
+IpmParams make_params(const SolveParams& prm, const TopoDesc& t) {
   IpmParams p{prm.max_iters, prm.tol, prm.anchor, prm.anchor_valid, prm.guard, prm.snap_mu};
-  p.pad_rows = resolve_solver(g, d, prm.solver) == kSolverWarp;
+  p.pad_rows = resolve_solver(t.g, t.d, prm.solver) == kSolverWarp;
+  p.plan = TilePlan{t.tile_rounds, t.tile_near};
   return p;
 }
 
@@ -115,6 +116,13 @@ const char* solver_code(const TopoDesc& topo, int requested, bool fused) {
   return name;
 }
 
+void plan_topology(int g, int d, const int* r2o, const int* o2r, unsigned long long* rounds, unsigned long long* near) {
+  TilePlan plan;
+  if (g <= kTileMaxGroup && d <= kTileMaxDup) plan = plan_tiles(g, d, {r2o, o2r});
+  *rounds = plan.rounds;
+  *near = plan.near;
+}
+
 int anchor_dup(int g, int d, int requested) { return resolve_solver(g, d, requested) == kSolverBlock ? padded_dup(d) : d; }
 
 size_t planner_workspace_bytes(int n_logical) { return workspace_bytes(n_logical); }
@@ -136,7 +144,7 @@ cudaError_t launch_count(const void* idx, int idx_is64, long long n, int n_logic
 cudaError_t launch_solve(const int* workload, const TopoDesc& topo, SolveParams prm, float* probs, float* normalised,
                          void* avail, int avail_is64, int* status, cudaStream_t stream) {
   if (!shape_ok(topo, true, prm.solver)) return cudaErrorInvalidValue;
-  SolveLaunch l{workload, make_topo(topo), make_params(prm, topo.g, topo.d), probs, normalised, Counter{avail, avail_is64}, status,
+  SolveLaunch l{workload, make_topo(topo), make_params(prm, topo), probs, normalised, Counter{avail, avail_is64}, status,
                 stream};
   return dispatch_shape(topo.g, topo.d, prm.solver, false, l);
 }
@@ -209,12 +217,12 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
   if (!shape_ok(topo, true, prm.solver) || n_cta < 2 || exd.n_ranks > kMaxRanks) return cudaErrorInvalidValue;
   Exchange ex{exd.recv, exd.n_ranks, exd.my_rank, exd.node_size, exd.timeout_ns};
   if (idx_is64) {
-    FusedLaunch<int64_t> l{static_cast<const int64_t*>(idx), n, make_topo(topo), ex, make_params(prm, topo.g, topo.d),
+    FusedLaunch<int64_t> l{static_cast<const int64_t*>(idx), n, make_topo(topo), ex, make_params(prm, topo),
                            static_cast<Workspace*>(workspace), probs, Counter{avail, avail_is64}, status,
                            static_cast<int64_t*>(out), n_cta, grid_timeout_ns, trace, cooperative, stream};
     return dispatch_shape(topo.g, topo.d, prm.solver, pack_groups(l.tp), l);
   }
-  FusedLaunch<int32_t> l{static_cast<const int32_t*>(idx), n, make_topo(topo), ex, make_params(prm, topo.g, topo.d),
+  FusedLaunch<int32_t> l{static_cast<const int32_t*>(idx), n, make_topo(topo), ex, make_params(prm, topo),
                          static_cast<Workspace*>(workspace), probs, Counter{avail, avail_is64}, status,
                          static_cast<int32_t*>(out), n_cta, grid_timeout_ns, trace, cooperative, stream};
   return dispatch_shape(topo.g, topo.d, prm.solver, pack_groups(l.tp), l);
@@ -222,13 +230,13 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
 
 namespace {
 template <typename IdxT>
-cudaError_t cluster_step(const void* idx, long long n, const Topo& tp, const Exchange& ex, const SolveParams& prm, void* workspace,
+cudaError_t cluster_step(const void* idx, long long n, const Topo& tp, const Exchange& ex, const IpmParams& prm, int solver, void* workspace,
                          float* probs, Counter avail, int* status, void* out, int n_cta, unsigned long long timeout_ns,
                          unsigned long long* trace, cudaStream_t stream, int* fits) {
-  const ClusterLaunch<IdxT> l{static_cast<const IdxT*>(idx), n, tp, ex, make_params(prm, tp.g, tp.d),
+  const ClusterLaunch<IdxT> l{static_cast<const IdxT*>(idx), n, tp, ex, prm,
                               static_cast<Workspace*>(workspace), probs, avail, status, static_cast<IdxT*>(out), n_cta,
                               timeout_ns, trace, stream, fits};
-  return dispatch_shape(tp.g, tp.d, prm.solver, pack_groups(tp), l);
+  return dispatch_shape(tp.g, tp.d, solver, pack_groups(tp), l);
 }
 }  // namespace
 
@@ -239,7 +247,7 @@ cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const Top
   const Topo tp = make_topo(topo);
   if (tp.e > kClusterMaxExperts) return cudaErrorInvalidValue;
   const Exchange ex{exd.recv, exd.n_ranks, exd.my_rank, exd.node_size, exd.timeout_ns};
-  return (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(idx, n, tp, ex, prm, workspace, probs, Counter{avail, avail_is64},
+  return (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(idx, n, tp, ex, make_params(prm, topo), prm.solver, workspace, probs, Counter{avail, avail_is64},
                                                                      status, out, n_cta, timeout_ns, trace, stream, nullptr);
 }
 
@@ -252,12 +260,10 @@ int cluster_ctas(long long n) {
 long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_cta) {
   const Topo tp = make_topo(topo);
   if (!shape_ok(topo, true, solver) || tp.e > kClusterMaxExperts) return 0;
-  SolveParams prm{1, 1.0};
-  prm.solver = solver;
   const long long n = (long long)(n_cta - 1) * cluster_max_slice(-tile_rows(tp.g));
   int fits = 0;
   const cudaError_t err = (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(
-      nullptr, n, tp, Exchange{}, prm, nullptr, nullptr, Counter{}, nullptr, nullptr, n_cta, 0, nullptr, nullptr, &fits);
+      nullptr, n, tp, Exchange{}, IpmParams{1, 1.0}, solver, nullptr, nullptr, Counter{}, nullptr, nullptr, n_cta, 0, nullptr, nullptr, &fits);
   if (err != cudaSuccess) cudaGetLastError();  // this shape does not run in a cluster
   return err == cudaSuccess && fits > 0 ? n : 0;
 }

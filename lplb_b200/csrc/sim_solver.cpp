@@ -91,6 +91,7 @@ template <int NB, int D>
 void solve_batch_tiles(int g, int rows, const int* r2o, const int* o2r, int nb, const double* w, const double* fixed,
                        int max_iters, double tol, double* f_out, int* iters, int* converged, double* anchor,
                        int* anchor_valid, double guard, double snap_mu) {
+  const lplb::TilePlan plan = lplb::plan_tiles(g, D, {r2o, o2r});
   std::vector<double> scratch(lplb::tile_layout(NB, D).total);  // exactly, so that a sanitizer sees an overrun
   for (int b = 0; b < nb; ++b) {
     lplb_sim::run_block(32 * NB, [&](int tid) {
@@ -102,6 +103,7 @@ void solve_batch_tiles(int g, int rows, const int* r2o, const int* o2r, int nb, 
       if (live) own = fixed[(size_t)b * g + rank];
       for (int k = 0; live && k < D; ++k) own += mine[k];
       lplb::IpmParams prm{max_iters, tol, anchor, anchor_valid, guard, snap_mu};
+      prm.plan = plan;
       double* group = anchor ? anchor + (size_t)b * g * (4 * D + 3) : nullptr;
       double* slot = live && anchor ? group + (size_t)rank * (4 * D + 3) : nullptr;
       int* flag = anchor ? anchor_valid + b : nullptr;
