@@ -110,7 +110,7 @@ def run_ours(args) -> dict:
     n_routed = N_LOGICAL + RED_PER_RANK * EP_SIZE
     extra = {"warm_start": False} if args.cold else {}  # otherwise the library default
     planner = Planner(cube(), n_routed, N_LOGICAL, EP_SIZE, group, device=dev, comm=args.comm, **extra)
-    n_sms = args.n_sms or None  # None: the library picks (one CTA per SM, fewer for small batches)
+    n_sms = args.n_sms or None  # None: the library picks (one cluster of 16 CTAs for this batch)
     pl = planner.n_local_routed_experts
 
     total_steps = args.warmup + args.steps
@@ -330,7 +330,7 @@ def run_ours(args) -> dict:
             "comm": planner.comm,
             "lp_warm_start": planner.warm_start,
             "planner_configuration": "library defaults" if not args.cold and args.comm == "auto" else "non-default flags",
-            "n_sms": n_sms or planner._default_ctas(TOKENS_PER_RANK * TOP_K),
+            "n_sms": n_sms or "library default",
             "l2": "256 MiB buffer written between timed iterations",
             "first_step": step0,
             "bias_redraws_inside_timed_steps": redraws_timed,

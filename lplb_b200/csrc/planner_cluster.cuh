@@ -421,6 +421,9 @@ __device__ __forceinline__ void cluster_worker(const ClusterHead<IdxT>& head, Wo
   if (late) wait_messages(bar_result, timeout_ns);  // nothing may be on its way here when this CTA leaves
 }
 
+// It starts early, but does not let its successor do so: a MoE pass behind it, whose kernels then all started and waited while it
+// ran, took 4.6 us longer (64 tokens x 2048: behind the grid-wide step 148, here 147, with early successors 153).
+//
 // Grid = one cluster: a solver CTA and gridDim.x - 1 worker CTAs.  Shapes of the tile solver for up to 32 ranks (GP = -1, -2, -4;
 // with 64 a step is the solve, 52.7 us against 53.3 here).
 template <int GP, int D, typename IdxT>
@@ -431,7 +434,6 @@ __global__ void __launch_bounds__(cluster_threads(GP), 1) cluster_run_kernel(con
   extern __shared__ __align__(16) int smem[];
   __shared__ __align__(8) uint64_t bar;       // the solver's: counts; a worker's: results
   __shared__ int counts[kNumberWords];
-  allow_successor();
   wait_predecessors();
   constexpr int T = cluster_threads(GP);
   const int n_workers = (int)gridDim.x - 1;

@@ -460,9 +460,11 @@ class Planner:
         """Logical expert ids ``[-1, E)`` in, physical expert ids ``[-1, P)`` out, same shape
         (reference ``lplb/planner.py:245-266``).
 
-        ``n_sms`` CTAs are launched (default: one per SM, fewer for batches of less than 384
-        indices per SM, never fewer than two): one of them exchanges the statistics and solves
-        the LPs, the others count and rewrite the indices.
+        ``n_sms`` CTAs are launched, never fewer than two: one of them exchanges the statistics and solves
+        the LPs, the others count and rewrite the indices.  By default the library picks: one
+        thread-block cluster of up to 16 CTAs for batches that so many can count (up to 1024 experts;
+        153,600 indices with groups of up to 8 ranks, 38,400 with 16, 15,360 with 32), beyond
+        one CTA per SM, fewer for less than 384 indices per SM.
 
         ``idx`` normally lives on the planner's GPU.  It may instead be a *pinned host* tensor:
         the kernel then reads it over PCIe itself (no separate host-to-device copy), and the
