@@ -30,8 +30,9 @@ constexpr int kClusterAhead = 2;          // indices of one thread on their way 
 // of several warps are slower that way (16 ranks 8.0 -> 8.9 us, 32 ranks 11.0 -> 12.3, from the same source without spills).
 __host__ __device__ constexpr int cluster_threads(int gp) { return gp == -1 ? 512 : 256; }
 // Indices of one worker at most (8 bytes of shared memory each).  Step and a lookup of its result behind it, grid / cluster, us: 8
-// ranks 1,024 indices 20.2 / 18.0, 16,384 18.5 / 15.8, 32,768 19.2 / 16.2, 65,536 18.5 / 16.5, 131,072 19.2 / 19.2 and with 512
-// experts 26.9 / 24.7; the step alone, 32 ranks, 32,768 indices, 16.3 / 17.7.
+// ranks 1,024 indices 20.2 / 17.1, 16,384 18.5 / 15.0, 32,768 19.4 / 15.8, 65,536 18.5 / 16.0, 131,072 19.2 / 18.4 and with 512
+// experts 27.0 / 23.7; 16 ranks 32,768 indices 21.9 / 19.9, the step alone at 65,536 13.9 / 17.2; 32 ranks 15,200 indices 34.7 /
+// 32.4, the step alone at 32,768 15.8 / 17.4 (in a captured graph 28.2 / 28.6 with a copy and a lookup).
 __host__ __device__ constexpr int cluster_max_slice(int gp) { return gp == -1 ? 10240 : gp == -2 ? 2560 : 1024; }
 
 __host__ __device__ inline int cluster_row(int e) { return (e + 3) & ~3; }  // a row of counts, in words: whole messages
