@@ -76,14 +76,20 @@ __device__ __forceinline__ bool even_pick(unsigned k, unsigned quota, unsigned t
 
 // Waits for the first phase of `bar`; false when `budget_ns` ran out.
 __device__ __forceinline__ bool wait_messages(uint32_t bar, uint64_t budget_ns) {
-  if (sm100::mbar_try_wait_cluster(bar, 0)) return true;
+  const uint32_t nap_ns = (uint32_t)(budget_ns < sm100::kSuspendNs ? budget_ns : sm100::kSuspendNs);
+  if (sm100::mbar_try_wait_cluster(bar, 0, nap_ns)) return true;
   const uint64_t t0 = global_timer_ns();
   do {
-    for (int i = 0; i < 16; ++i)
-      if (sm100::mbar_try_wait_cluster(bar, 0)) return true;
+    if (sm100::mbar_try_wait_cluster(bar, 0, nap_ns)) return true;
   } while (global_timer_ns() - t0 <= budget_ns);
   return false;
 }
+
+// A CTA whose wait has run out may not leave before the messages that it stopped waiting for are there: they are stores to its
+// shared memory.  All have been issued when it gets here (the cluster barrier), so this has nothing to do with the caller's
+// budget, which may be as short as the caller likes.
+constexpr uint64_t kLandingNs = 1000000000;
+__device__ __forceinline__ void await_landing(uint32_t bar) { wait_messages(bar, kLandingNs); }
 
 // Numbers the experts with a replica in ascending order: has(j, i) and put(j, i, number) of the calling thread's j-th
 // expert i = j T + thread.  Called by the first T threads of a CTA, all that have not exited; `counts` is
@@ -273,7 +279,7 @@ __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& e
   __syncwarp();
   cluster_arrive();
   cluster_wait();  // the workers have what was sent; nobody's shared memory goes before that
-  if (late) wait_messages(my_bar, timeout_ns);
+  if (late) await_landing(my_bar);
 }
 
 // What the workers need, in one place: the first of their instructions wait for it.
@@ -419,7 +425,7 @@ __device__ __forceinline__ void cluster_worker(const ClusterHead<IdxT>& head, Wo
   }
   __syncwarp();
   cluster_wait();
-  if (late) wait_messages(bar_result, timeout_ns);  // nothing may be on its way here when this CTA leaves
+  if (late) await_landing(bar_result);
 }
 
 // It starts early, but does not let its successor do so: a MoE pass behind it, whose kernels then all started and waited while it

@@ -22,6 +22,16 @@ def test_the_cluster_kernel_waits_for_its_predecessor_first():
     assert text.count("wait_predecessors") == 1  # both roles run behind it
 
 
+def test_a_cta_that_gave_up_waits_for_its_messages_beyond_the_callers_budget():
+    text = re.sub(r"//[^\n]*", "", (CSRC / "planner_cluster.cuh").read_text())
+    for role in ("cluster_solver", "cluster_worker"):
+        body = text[text.index(f"void {role}(") :]
+        body = body[: body.index("\n}")]
+        after = body[body.rindex("cluster_wait();") + len("cluster_wait();") :]
+        assert "if (late) await_landing(" in after and "timeout_ns" not in after
+    assert "timeout_ns" not in text[text.index("void await_landing(") :].split("}")[0]
+
+
 def _planner(r2o, groups, ll, combined=1, **kw):
     g, d = r2o.shape
     ep = g * groups
@@ -166,3 +176,54 @@ def test_the_exchange_runs_in_a_cluster_too():
     st = planner.check_status(clear=True)
     assert st["error"] == "peer_timeout" and st["detail"] == 0b10 and st["timeouts"] == 1
     assert int(eng.warm_start_valid().sum()) == 0
+
+
+def _clean_step(planner, idx, use_exchange=False, cluster=8):
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = eng.run_fused(idx, avail, 16, use_exchange, None, cluster)
+    want = eng.map_idx(idx, eng.last_probs(), planner.count_workload(idx, 8)[1], 8)
+    assert torch.equal(_counts(planner, out), _counts(planner, want)) and planner.check_status().ok
+
+
+@gpu
+@pytest.mark.parametrize("cluster", [2, 4, 16])
+def test_workers_whose_wait_runs_out_leave_half_of_the_tokens(cluster):
+    """The solver still waits for a peer that never publishes when the workers give up."""
+    planner = _planner(topology.cube(), 1, 8, peer_timeout_us=3000.0, grid_timeout_us=300.0)
+    eng = planner._engine
+    eng.open_exchange_loopback(2, 0)
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    idx = _indices(planner, 6000, torch.int64, seed=11)
+    out = eng.run_fused(idx, avail, 16, True, None, cluster)
+    st = planner.check_status(clear=True)
+    assert st["error"] == "lp_timeout" and st["timeouts"] == cluster  # every worker, and the missing peer
+    live = idx >= 0
+    assert torch.equal(planner.phy2log[out[live].long()].long(), idx[live]) and bool((out[~live] == -1).all())
+    replicated = planner.mapping.log2phy[:, 1] >= 0
+    moved = torch.bincount(idx[live & (out == planner.mapping.log2phy[idx.clamp_min(0), 1])], minlength=64)
+    counts = torch.bincount(idx[live], minlength=64)
+    assert bool((moved[~replicated] == 0).all())
+    # every other one of a worker's tokens, the first of them
+    assert bool((moved[replicated] >= counts[replicated] // 2).all())
+    assert bool((moved[replicated] <= (counts[replicated] + cluster - 1) // 2).all())
+    eng.debug_fill_slot(1, torch.zeros(64, dtype=torch.int32), eng.completed_launches() + 1)
+    _clean_step(planner, idx, use_exchange=True)
+
+
+@gpu
+@pytest.mark.parametrize("cluster", [2, 16])
+def test_a_solver_whose_wait_runs_out_reports_it(cluster):
+    planner = _planner(topology.cube(), 1, 32)
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    idx = _indices(planner, 10240 * (cluster - 1), torch.int64, seed=cluster)
+    eng.set_params(24, 1e-4, 1e6, 1e-3)  # the ids come over PCIe, so no count is there within a nanosecond
+    for _ in range(3):
+        out = eng.run_fused(idx.cpu().pin_memory(), avail, 16, False, torch.empty_like(idx), cluster)
+        st = planner.check_status(clear=True)
+        assert st["error"] in ("grid_timeout", "lp_timeout") and st["timeouts"] >= 1
+        live = idx >= 0
+        assert torch.equal(planner.phy2log[out[live].long()].long(), idx[live]) and bool((out[~live] == -1).all())
+    eng.set_params(24, 1e-4, 1e6, 1e6)
+    _clean_step(planner, idx, cluster=16)
