@@ -162,6 +162,9 @@ __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& e
   const bool rehearsal = ex.n_ranks <= 1 && Step::rehearses(tp), rehearses = rehearsal && warp == Step::kRehearsing;
   const int n_threads = rehearsal ? kBlock - 32 : kBlock;  // those that do not rehearse
   const TileLane mine = load_step_lane<GP, D, true>(tp, prm, rehearses, status);
+  // The rows start at zero: what is summed when the wait for them runs out is a part of the counts and nothing else.  (The tables
+  // are on their way meanwhile.)
+  for (int i = threadIdx.x; i < n_workers * row / 4; i += kBlock) reinterpret_cast<int4*>(rows)[i] = int4{0, 0, 0, 0};
   const uint32_t my_bar = sm100::smem_u32(bar);
   if (threadIdx.x == 0) {
     sm100::mbar_init(my_bar, 1);

@@ -227,3 +227,30 @@ def test_a_solver_whose_wait_runs_out_reports_it(cluster):
         assert torch.equal(planner.phy2log[out[live].long()].long(), idx[live]) and bool((out[~live] == -1).all())
     eng.set_params(24, 1e-4, 1e6, 1e6)
     _clean_step(planner, idx, cluster=16)
+
+
+def test_the_rows_of_counts_are_cleared_before_a_worker_may_write_them():
+    text = re.sub(r"//[^\n]*", "", (CSRC / "planner_cluster.cuh").read_text())
+    body = text[text.index("void cluster_solver(") :]
+    assert "reinterpret_cast<int4*>(rows)[i] = int4{0, 0, 0, 0}" in body[: body.index("cluster_arrive();")]
+
+
+@gpu
+def test_counts_that_came_late_are_a_part_of_the_batch():
+    """Every batch is drawn from experts of its own, so whatever else lies in shared memory shows up as a token too many."""
+    planner = _planner(topology.cube(), 1, 32)
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gen = torch.Generator("cuda").manual_seed(2)
+    for step in range(24):
+        own = torch.arange(256, device="cuda")[step % 8 :: 8]
+        idx = own[torch.randint(32, (150000,), device="cuda", generator=gen)]
+        eng.set_params(24, 1e-4, 1e6, 1e6 if step % 2 == 0 else 1e-3)
+        src = idx if step % 2 == 0 else idx.cpu().pin_memory()
+        eng.run_fused(src, avail, 16, False, torch.empty_like(idx), 16)
+        counts = torch.bincount(idx, minlength=256)
+        glob = eng.workspace()[8 + 2 * 256 : 8 + 3 * 256]
+        assert bool((glob >= 0).all()) and bool((glob <= counts).all())
+        st = planner.check_status(clear=True)
+        assert st.ok == (step % 2 == 0)
+        assert not st.ok or torch.equal(glob.long(), counts)
