@@ -91,6 +91,15 @@ __device__ __forceinline__ bool wait_messages(uint32_t bar, uint64_t budget_ns) 
 constexpr uint64_t kLandingNs = 1000000000;
 __device__ __forceinline__ void await_landing(uint32_t bar) { wait_messages(bar, kLandingNs); }
 
+// Threads wait each for themselves, so one may give up on what another still sees arrive: whichever does so first reports it,
+// once per CTA.
+__device__ __forceinline__ void report_late(bool late, int* reported, int* status, int code, int phase, int detail) {
+  if (late && atomicExch(reported, 1) == 0) {
+    atomicAdd(&status[kStTimeouts], 1);
+    raise_status(status, code, phase, detail);
+  }
+}
+
 // Numbers the experts with a replica in ascending order: has(j, i) and put(j, i, number) of the calling thread's j-th
 // expert i = j T + thread.  Called by the first T threads of a CTA, all that have not exited; `counts` is
 // kNumberWords of shared memory.
@@ -130,7 +139,7 @@ template <int GP, int D>
 __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& ex, IpmParams prm, Workspace* ws,
                                                float* __restrict__ probs, Counter avail, int* status, int n_workers,
                                                unsigned long long timeout_ns, unsigned long long* __restrict__ trace, int* smem,
-                                               uint64_t* bar, int* counts) {
+                                               uint64_t* bar, int* counts, int* reported) {
   const int e = tp.e, row = cluster_row(e), n_rep = cluster_replicated(tp), warp = threadIdx.x >> 5;
   const bool tracing = trace != nullptr && threadIdx.x == 0;
   int* rows = smem;                                    // [n_workers][row]
@@ -167,6 +176,7 @@ __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& e
   for (int i = threadIdx.x; i < n_workers * row / 4; i += kBlock) reinterpret_cast<int4*>(rows)[i] = int4{0, 0, 0, 0};
   const uint32_t my_bar = sm100::smem_u32(bar);
   if (threadIdx.x == 0) {
+    *reported = 0;
     sm100::mbar_init(my_bar, 1);
     sm100::mbar_expect_tx(my_bar, (uint32_t)(n_workers * row) * sizeof(int));
     sm100::fence_barrier_init();
@@ -198,10 +208,7 @@ __device__ __forceinline__ void cluster_solver(const Topo& tp, const Exchange& e
   if (!rehearses) {
     late = !wait_messages(my_bar, timeout_ns);
     if (tracing) trace[2] = global_timer_ns();
-    if (late && threadIdx.x == 0) {
-      atomicAdd(&status[kStTimeouts], 1);
-      raise_status(status, kErrGridTimeout, kPhCount, 0);
-    }
+    report_late(late, reported, status, kErrGridTimeout, kPhCount, 0);
 #pragma unroll 1
     for (int i = threadIdx.x; i < e; i += n_threads) {
       const int slot = slots[i];
@@ -300,7 +307,7 @@ struct ClusterHead {
 template <int T, typename IdxT>
 __device__ __forceinline__ void cluster_worker(const ClusterHead<IdxT>& head, Workspace* ws, int* status, int q, int n_workers,
                                                unsigned long long timeout_ns, unsigned long long* __restrict__ trace, int* smem,
-                                               uint64_t* bar, int* counts) {
+                                               uint64_t* bar, int* counts, int* reported) {
   const long long begin = min((long long)q * head.slice, head.n);
   const int m = (int)min((long long)head.slice, head.n - begin), e = head.e, row = cluster_row(e), n_rep = head.n_rep;
   const IdxT* __restrict__ idx = head.idx + begin;
@@ -325,6 +332,7 @@ __device__ __forceinline__ void cluster_worker(const ClusterHead<IdxT>& head, Wo
     if (j * T + (int)threadIdx.x < e) table[j] = head.log2phy[j * T + threadIdx.x];
   const uint32_t bar_result = sm100::smem_u32(bar);
   if (threadIdx.x == 0) {
+    *reported = 0;
     sm100::mbar_init(bar_result, 1);
     sm100::mbar_expect_tx(bar_result, (uint32_t)n_rep * 16);
     sm100::fence_barrier_init();
@@ -411,10 +419,7 @@ __device__ __forceinline__ void cluster_worker(const ClusterHead<IdxT>& head, Wo
       if (round == 1) out[it.x] = (IdxT)(int)(stay ? ph & 0xFFFFu : ph >> 16);
     }
   }
-  if (late && threadIdx.x == 0) {
-    atomicAdd(&status[kStTimeouts], 1);
-    raise_status(status, kErrLpTimeout, kPhRedirect, q);
-  }
+  report_late(late, reported, status, kErrLpTimeout, kPhRedirect, q);
   if (trace != nullptr) {  // tracing only: find the worker that leaves last
     __syncthreads();
     if (tracing) trace[5] = global_timer_ns();
@@ -444,6 +449,7 @@ __global__ void __launch_bounds__(cluster_threads(GP), 1) cluster_run_kernel(con
   extern __shared__ __align__(16) int smem[];
   __shared__ __align__(8) uint64_t bar;       // the solver's: counts; a worker's: results
   __shared__ int counts[kNumberWords];
+  __shared__ int reported;  // that a wait of this CTA ran out
   wait_predecessors();
   constexpr int T = cluster_threads(GP);
   const int n_workers = (int)gridDim.x - 1;
@@ -457,9 +463,9 @@ __global__ void __launch_bounds__(cluster_threads(GP), 1) cluster_run_kernel(con
       }
       asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     }
-    cluster_solver<GP, D>(tp, ex, prm, ws, probs, avail, status, n_workers, timeout_ns, trace, smem, &bar, counts);
+    cluster_solver<GP, D>(tp, ex, prm, ws, probs, avail, status, n_workers, timeout_ns, trace, smem, &bar, counts, &reported);
   } else {
-    cluster_worker<T, IdxT>(head, ws, status, (int)blockIdx.x - 1, n_workers, timeout_ns, trace, smem, &bar, counts);
+    cluster_worker<T, IdxT>(head, ws, status, (int)blockIdx.x - 1, n_workers, timeout_ns, trace, smem, &bar, counts, &reported);
   }
 }
 

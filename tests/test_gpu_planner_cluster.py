@@ -254,3 +254,37 @@ def test_counts_that_came_late_are_a_part_of_the_batch():
         st = planner.check_status(clear=True)
         assert st.ok == (step % 2 == 0)
         assert not st.ok or torch.equal(glob.long(), counts)
+
+
+def test_whichever_thread_gives_up_reports_it():
+    text = re.sub(r"//[^\n]*", "", (CSRC / "planner_cluster.cuh").read_text())
+    assert not re.search(r"late && threadIdx|threadIdx\.x == 0 && late", text)
+    for role, code in (("cluster_solver", "kErrGridTimeout"), ("cluster_worker", "kErrLpTimeout")):
+        body = text[text.index(f"void {role}(") :]
+        assert re.search(rf"\n *report_late\(late, reported, status, {code}", body[: body.index("\n}")])
+
+
+@gpu
+@pytest.mark.parametrize("cluster", [2, 16])
+def test_a_step_without_a_report_had_all_counts(cluster):
+    """Budgets around the time at which the counts arrive (the ids come over PCIe): some warps give up on them, others
+    still see them."""
+    planner = _planner(topology.cube(), 1, 32)
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    idx = _indices(planner, 10240 * (cluster - 1), torch.int64, seed=21)
+    host, out = idx.cpu().pin_memory(), torch.empty_like(idx)
+    counts = torch.bincount(idx + 1, minlength=257)[1:]
+    by_cta = planner.count_workload(idx, 8)[1]
+    reported = 0
+    for step in range(250):
+        eng.set_params(24, 1e-4, 1e6, 0.001 + 0.2 * step)
+        eng.run_fused(host, avail, 16, False, out, cluster)
+        glob = eng.workspace()[8 + 2 * 256 : 8 + 3 * 256].clone()
+        st = planner.check_status(clear=True)
+        reported += not st.ok
+        if st.ok:
+            assert torch.equal(glob.long(), counts)
+            want = eng.map_idx(idx, eng.last_probs(), by_cta, 8)
+            assert torch.equal(_counts(planner, out), _counts(planner, want))
+    assert 0 < reported < 250
