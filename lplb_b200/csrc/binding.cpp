@@ -333,6 +333,15 @@ class PlannerEngine {
     return out;
   }
 
+  // CTAs of the cluster that run_fused takes for n indices when it may choose; 0: the grid-wide kernel.
+  int cluster_choice(int64_t n, bool is64, bool host_result) {
+    const int cluster = lplb::cluster_ctas(n, host_result);
+    if (cluster == 0) return 0;
+    long long& most = cluster_limit_[{is64, cluster}];  // asked once
+    if (most < 0) most = lplb::cluster_limit(topo(), prm_.solver, is64, cluster);
+    return n > most ? 0 : cluster;
+  }
+
   // ---- single launch ------------------------------------------------------------------
   // `idx` may also be a pinned host tensor: the kernel then reads it over PCIe itself and,
   // if `out` is a pinned host tensor too, writes the result straight back, which replaces two
@@ -357,12 +366,7 @@ class PlannerEngine {
                                         << " ranks with at most " << lplb::kMaxDup << " replicas each");
     LPLB_CHECK(!use_exchange || n_ranks_ <= 32, "the in-kernel exchange covers at most 32 ranks");
     const auto topology = topo();
-    if (cluster < 0) {
-      cluster = lplb::cluster_ctas(idx.numel());
-      long long& most = cluster_limit_[{is64, cluster}];  // asked once
-      if (most < 0) most = lplb::cluster_limit(topology, prm_.solver, is64, cluster);
-      if (idx.numel() > most) cluster = 0;
-    }
+    if (cluster < 0) cluster = cluster_choice(idx.numel(), is64, out_opt.has_value() && !out_opt->is_cuda());
     int& limit = is64 ? max_cta64_ : max_cta32_;
     if (limit < 0) limit = lplb::max_fused_ctas(topo(), prm_.solver, is64);
     LPLB_CHECK(limit >= 2, "fused kernel cannot be resident on this device");
@@ -634,6 +638,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("map_idx", &PlannerEngine::map_idx)
       .def("run_fused", &PlannerEngine::run_fused, py::arg("idx"), py::arg("avail"), py::arg("n_cta"),
            py::arg("use_exchange"), py::arg("out") = py::none(), py::arg("cluster") = 0)
+      .def("cluster_choice", &PlannerEngine::cluster_choice, py::arg("n"), py::arg("is64") = true, py::arg("host_result") = false)
       .def("all_reduce_counts", &PlannerEngine::all_reduce_counts)
       .def("alloc_exchange", &PlannerEngine::alloc_exchange)
       .def("open_exchange", &PlannerEngine::open_exchange)

@@ -99,8 +99,8 @@ cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const Top
                            SolveParams prm, void* workspace, float* probs, void* avail, int avail_is64, int* status,
                            void* out, int n_cta, unsigned long long timeout_ns, unsigned long long* trace, cudaStream_t stream);
 // The cluster that suits a batch of n indices, and how many a cluster takes: up to there it is faster than the grid-wide
-// kernel.  0 where shape or device cannot run one.
-int cluster_ctas(long long n);
+// kernel.  0 where shape or device cannot run one, or where the result goes to host memory and is too large for it.
+int cluster_ctas(long long n, bool host_result);
 long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_cta);
 
 // Co-resident CTA limit of the fused kernel for this topology on the current device (0 when the

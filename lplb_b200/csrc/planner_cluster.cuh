@@ -24,6 +24,12 @@ constexpr int kClusterMaxCtas = 16;       // the largest cluster that sm_100a sc
 constexpr uint32_t kNoReplica = 0xFFFF;   // physical ids in 16 bits: there are at most two per expert
 constexpr int kClusterMaxExperts = 1024;  // a row of counts per worker in the solver's shared memory
 constexpr long long kClusterShare = 256;  // indices per worker before a step takes a larger cluster
+// Indices of a result in host memory: a worker writes its slice in two passes, each with holes where the other writes, so every
+// line crosses PCIe in pieces, from 15 SMs.  Ids and result in pinned memory, one call and the wait for it, grid / cluster, us:
+// 8 ranks 256 experts 8,192 indices 29.5 / 26.6, 14,336 27.9 / 27.0, 16,384 30.0 / 31.3, 32,768 35.2 / 44.4, 131,072 64.9 / 114;
+// 512 experts 16,384 32.0 / 31.5; 16 ranks 12,288 31.6 / 31.2, 16,384 34.9 / 36.1; 32 ranks 15,200 44.3 / 43.4.  Ids alone may be there
+// whatever their number (32,768 27.3 / 26.2, 131,072 41.8 / 41.2).
+constexpr long long kClusterHostResult = 15360;
 constexpr int kClusterAhead = 2;          // indices of one thread on their way at once
 
 // Threads of a CTA.  With 512 the solver CTA keeps the first kBlock, and the registers of the others, which exit; the solvers

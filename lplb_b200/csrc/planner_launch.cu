@@ -251,7 +251,8 @@ cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const Top
                                                                      status, out, n_cta, timeout_ns, trace, stream, nullptr);
 }
 
-int cluster_ctas(long long n) {
+int cluster_ctas(long long n, bool host_result) {
+  if (host_result && n > kClusterHostResult) return 0;
   int n_cta = 2;
   while (n_cta < kClusterMaxCtas && n > (long long)(n_cta - 1) * kClusterShare) n_cta *= 2;
   return n_cta;

@@ -288,3 +288,24 @@ def test_a_step_without_a_report_had_all_counts(cluster):
             want = eng.map_idx(idx, eng.last_probs(), by_cta, 8)
             assert torch.equal(_counts(planner, out), _counts(planner, want))
     assert 0 < reported < 250
+
+
+@gpu
+@pytest.mark.parametrize("r2o,ll", [(topology.cube(), 32), (topology.hypercube(), 16), (topology.torus(8, 4), 8)])
+@pytest.mark.parametrize("n", [8, 4096, 15360, 15368, 32768])
+def test_a_result_in_host_memory_takes_the_cluster_for_small_batches_only(r2o, ll, n):
+    planner = _planner(r2o, 1, ll)
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    idx = _indices(planner, n, torch.int64, seed=n).reshape(-1, 8)
+    by_cta = planner.count_workload(idx, 8)[1]
+    host = idx.cpu().pin_memory()
+    assert (eng.cluster_choice(n, host_result=True) > 0) == (n <= 15360)
+    for src, out in ((host, None), (host, torch.empty_like(idx)), (idx, torch.empty_like(host).pin_memory())):
+        got = planner.run(src, avail, out=out)
+        torch.cuda.synchronize()
+        assert got.is_cuda == (out is not None and out.is_cuda)
+        want = eng.map_idx(idx, eng.last_probs(), by_cta, 8)
+        assert torch.equal(_counts(planner, got.cuda()), _counts(planner, want))
+        assert torch.equal(planner.phy2log[got.cuda()[idx >= 0]].long(), idx[idx >= 0])
+    assert planner.check_status().ok
