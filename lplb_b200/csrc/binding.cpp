@@ -339,7 +339,7 @@ class PlannerEngine {
     if (cluster == 0) return 0;
     long long& most = cluster_limit_[{is64, cluster}];  // asked once
     if (most < 0) most = lplb::cluster_limit(topo(), prm_.solver, is64, cluster);
-    return n > most ? 0 : cluster;
+    return most == 0 || n > most ? 0 : cluster;
   }
 
   // ---- single launch ------------------------------------------------------------------

@@ -309,3 +309,14 @@ def test_a_result_in_host_memory_takes_the_cluster_for_small_batches_only(r2o, l
         assert torch.equal(_counts(planner, got.cuda()), _counts(planner, want))
         assert torch.equal(planner.phy2log[got.cuda()[idx >= 0]].long(), idx[idx >= 0])
     assert planner.check_status().ok
+
+
+@gpu
+@pytest.mark.parametrize("r2o,groups,ll", [(topology.torus(8, 8), 1, 2), (topology.cube(), 17, 2), (topology.cube(), 1, 150), (topology.ring(80), 1, 2),
+                                            (topology.cube(), 1, 2), (topology.hypercube(), 1, 2), (topology.torus(8, 4), 1, 2)])
+def test_an_empty_batch_runs_on_every_shape(r2o, groups, ll):
+    planner = _planner(r2o, groups, ll)
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = planner.run(torch.zeros(0, 8, dtype=torch.int64, device="cuda"), avail)
+    assert out.shape == (0, 8) and int(avail) == groups and planner.check_status().ok
+    assert bool((planner.last_probs == 1).all())
