@@ -23,7 +23,10 @@ namespace lplb {
 constexpr int kClusterMaxCtas = 16;       // the largest cluster that sm_100a schedules
 constexpr uint32_t kNoReplica = 0xFFFF;   // physical ids in 16 bits: there are at most two per expert
 constexpr int kClusterMaxExperts = 1024;  // a row of counts per worker in the solver's shared memory
-constexpr long long kClusterShare = 256;  // indices per worker before a step takes a larger cluster
+// Indices per worker before a step takes a larger cluster.  2 / 4 / 8 / 16 CTAs, one after the other and from a graph, us: 256
+// indices 15.1 each, 18.5 / 17.7 / 17.6 / 18.9; 1,024 15.8 each, 20.8 / 18.7 / 18.7 / 18.5; 2,048 16.7 / 16.2 / 16.2 / 15.9, 20.9 each; 4,096 15.8 /
+// 14.9 / 14.5 / 14.2, 19.6 / 19.1 / 18.4 / 17.8.
+constexpr long long kClusterShare = 256;
 // Indices of a result in host memory: a worker writes its slice in two passes, each with holes where the other writes, so every
 // line crosses PCIe in pieces, from 15 SMs.  Ids and result in pinned memory, one call and the wait for it, grid / cluster, us:
 // 8 ranks 256 experts 8,192 indices 29.5 / 26.6, 14,336 27.9 / 27.0, 16,384 30.0 / 31.3, 32,768 35.2 / 44.4, 131,072 64.9 / 114;
@@ -35,11 +38,27 @@ constexpr int kClusterAhead = 2;          // indices of one thread on their way 
 // Threads of a CTA.  With 512 the solver CTA keeps the first kBlock, and the registers of the others, which exit; the solvers
 // of several warps are slower that way (16 ranks 8.0 -> 8.9 us, 32 ranks 11.0 -> 12.3, from the same source without spills).
 __host__ __device__ constexpr int cluster_threads(int gp) { return gp == -1 ? 512 : 256; }
-// Indices of one worker at most (8 bytes of shared memory each).  Step and a lookup of its result behind it, grid / cluster, us: 8
-// ranks 1,024 indices 20.2 / 17.1, 16,384 18.5 / 15.0, 32,768 19.4 / 15.8, 65,536 18.5 / 16.0, 131,072 19.2 / 18.4 and with 512
-// experts 27.0 / 23.7; 16 ranks 32,768 indices 21.9 / 19.9, the step alone at 65,536 13.9 / 17.2; 32 ranks 15,200 indices 34.7 /
-// 32.4, the step alone at 32,768 15.8 / 17.4 (in a captured graph 28.2 / 28.6 with a copy and a lookup).
+// Indices of one worker at most (8 bytes of shared memory each).
 __host__ __device__ constexpr int cluster_max_slice(int gp) { return gp == -1 ? 10240 : gp == -2 ? 2560 : 1024; }
+// Indices of one worker up to which the cluster is the faster one: where a step and a lookup of its result, one after the other, replayed
+// from a graph behind a copy of the ids, and as single calls that are waited for, together stop gaining.  With groups of 8 ranks this
+// depends on how many experts have a replica, whose tokens a worker handles twice.  Grid / cluster of 16, us, the three in
+// this order, at the last size that gains and the first that loses:
+//   1 of 32 (512 experts)   131,072: 20.5/18.5 22.6/22.6 29.9/29.3   -
+//   1 of 16 (256 experts)   114,688: 19.5/18.5 22.6/23.5 28.9/28.6   131,072: 18.5/18.5 20.5/22.6 27.9/29.1
+//   1 of 8 (256 experts)     81,920: 19.8/17.8 22.0/22.6 28.9/28.4    98,304: 19.2/18.5 20.8/22.6 28.6/28.7
+//   1 of 4 (256 experts)     65,536: 20.6/19.2 22.6/23.3 29.9/29.7    81,920: 19.4/19.2 21.5/23.9 29.9/31.5
+//   1 of 2 (256 experts)     16,384: 20.1/17.8 20.8/21.4 31.9/30.6    32,768: 18.5/18.4 19.5/21.5 28.6/29.7
+//   all (48 experts)         32,768: 17.8/15.8 19.2/19.9 27.6/27.1    65,536: 17.1/16.5 19.4/21.2 26.7/27.4
+//   16 ranks                 38,400: 22.6/20.6 23.7/23.7 32.0/31.4   32 ranks 15,360: 28.0/24.0 29.1/28.0 34.4/33.7
+// Above those two the kernel alone loses (16 ranks 65,536 indices 13.9 / 17.2, 32 ranks 32,768 15.8 / 17.4), though a step and a lookup
+// of 32 ranks gains one after the other (32,768: 24.6 / 22.6, from a graph 28.2 / 28.6).
+__host__ __device__ constexpr int cluster_paying_slice(int gp, int e, int n_rep) {
+  int slice = cluster_max_slice(gp);
+  if (gp == -1)
+    for (int share = 32 * n_rep; share > e && slice > 2048; share /= 2) slice -= 2048;
+  return slice;
+}
 
 __host__ __device__ inline int cluster_row(int e) { return (e + 3) & ~3; }  // a row of counts, in words: whole messages
 __host__ __device__ inline int cluster_slice(long long n, int n_workers, int threads) {  // indices of a worker, in whole rounds of its threads

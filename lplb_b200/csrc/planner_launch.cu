@@ -261,7 +261,7 @@ int cluster_ctas(long long n, bool host_result) {
 long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_cta) {
   const Topo tp = make_topo(topo);
   if (!shape_ok(topo, true, solver) || tp.e > kClusterMaxExperts) return 0;
-  const long long n = (long long)(n_cta - 1) * cluster_max_slice(-tile_rows(tp.g));
+  const long long n = (long long)(n_cta - 1) * cluster_paying_slice(-tile_rows(tp.g), tp.e, cluster_replicated(tp));
   int fits = 0;
   const cudaError_t err = (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(
       nullptr, n, tp, Exchange{}, IpmParams{1, 1.0}, solver, nullptr, nullptr, Counter{}, nullptr, nullptr, n_cta, 0, nullptr, nullptr, &fits);

@@ -462,9 +462,10 @@ class Planner:
 
         ``n_sms`` CTAs are launched, never fewer than two: one of them exchanges the statistics and solves
         the LPs, the others count and rewrite the indices.  By default the library picks: one
-        thread-block cluster of up to 16 CTAs for batches that so many can count (up to 1024 experts;
-        153,600 indices with groups of up to 8 ranks, 38,400 with 16, 15,360 with 32), beyond
-        one CTA per SM, fewer for less than 384 indices per SM.
+        thread-block cluster of up to 16 CTAs for batches that so many can count (up to 1024 experts; with
+        groups of up to 8 ranks 153,600 indices where one expert in 32 has a replica, 30,720 fewer
+        each time that share doubles, down to 30,720; 38,400 with 16 ranks, 15,360 with 32 and for a
+        result in host memory), beyond one CTA per SM, fewer for less than 384 indices per SM.
 
         ``idx`` normally lives on the planner's GPU.  It may instead be a *pinned host* tensor:
         the kernel then reads it over PCIe itself (no separate host-to-device copy), and the

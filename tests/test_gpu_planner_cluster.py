@@ -320,3 +320,18 @@ def test_an_empty_batch_runs_on_every_shape(r2o, groups, ll):
     out = planner.run(torch.zeros(0, 8, dtype=torch.int64, device="cuda"), avail)
     assert out.shape == (0, 8) and int(avail) == groups and planner.check_status().ok
     assert bool((planner.last_probs == 1).all())
+
+
+@gpu
+@pytest.mark.parametrize("r2o,groups,ll,combined,most", [
+    (topology.cube(), 1, 64, 1, 153600), (topology.cube(), 1, 32, 1, 122880), (topology.cube(), 1, 32, 2, 92160), (topology.cube(), 2, 16, 1, 92160),
+    (topology.cube(), 4, 8, 1, 61440), (topology.ring(3), 1, 9, 1, 92160), (topology.cube(), 4, 8, 2, 30720), (topology.circulant(8, (1, 2, 5)), 1, 6, 2, 30720),
+    (topology.hypercube(), 1, 4, 2, 38400), (topology.torus(8, 4), 1, 8, 1, 15360), (topology.torus(8, 8), 1, 8, 1, 0), (topology.cube(), 17, 8, 1, 0),
+])
+@pytest.mark.parametrize("is64", [True, False])
+def test_the_largest_batch_of_a_cluster_follows_the_share_of_replicated_experts(r2o, groups, ll, combined, most, is64):
+    eng = _planner(r2o, groups, ll, combined)._engine
+    assert eng.cluster_choice(0, is64) == (2 if most else 0)
+    assert eng.cluster_choice(most + 1, is64) == 0
+    if most:
+        assert eng.cluster_choice(most, is64) == 16 and eng.cluster_choice(256, is64) == 2 and eng.cluster_choice(257, is64) == 4
