@@ -76,6 +76,38 @@ def _check(planner, idx, cluster, in_place=False):
     assert planner.check_status().ok
 
 
+@gpu
+@pytest.mark.parametrize("r2o,groups,ll", [(topology.cube(), 1, 32), (topology.cube(), 4, 8), (topology.cube(), 5, 4), (topology.ring(5), 2, 7),
+                                            (topology.hypercube(), 1, 16), (topology.torus(8, 4), 1, 8)])
+def test_each_kernel_continues_from_the_iterates_it_saved_itself(r2o, groups, ll):
+    """The same batches on two planners, one always grid-wide, the other always in a cluster."""
+    grid, cluster = (_planner(r2o, groups, ll, warm_start=True) for _ in range(2))
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gen = torch.Generator("cuda").manual_seed(ll)
+    e = grid.n_logical_routed_experts
+    popularity = torch.rand(e, device="cuda", generator=gen) ** 3 + 1e-3
+    for p in (grid, cluster):
+        p.update_redundancy_mapping((popularity * 1e6).long())
+    warm = 0
+    for step in range(14):
+        if step == 7:  # another distribution: the saved iterates do not fit
+            popularity = torch.rand(e, device="cuda", generator=gen) ** 3 + 1e-3
+        if step == 11:
+            for p in (grid, cluster):
+                p.invalidate_warm_start()
+        idx = torch.multinomial(popularity, 15000, replacement=True, generator=gen)
+        grid._engine.run_fused(idx, avail, 16, False, None, 0)
+        out = cluster._engine.run_fused(idx, avail, 16, False, None, 16)
+        assert torch.equal(cluster._engine.last_probs(), grid._engine.last_probs())
+        assert torch.equal(cluster._engine.warm_start_valid(), grid._engine.warm_start_valid())
+        want = grid._engine.map_idx(idx, grid._engine.last_probs(), grid.count_workload(idx, 8)[1], 8)
+        assert torch.equal(_counts(cluster, out), _counts(grid, want))
+        iters = [p.check_status(clear=True)["lp_iters"] for p in (grid, cluster)]
+        assert iters[0] == iters[1]
+        warm += step > 0 and iters[1] <= 3
+    assert warm  # warm starts were among them
+
+
 # 512 threads and slices in rounds of them with groups of 8 ranks, 256 with larger ones
 @gpu
 @pytest.mark.parametrize("n", [0, 1, 3, 31, 511, 512, 513, 1024, 1537, 4095, 7681, 30721, 153600])
