@@ -367,3 +367,23 @@ def test_the_largest_batch_of_a_cluster_follows_the_share_of_replicated_experts(
     assert eng.cluster_choice(most + 1, is64) == 0
     if most:
         assert eng.cluster_choice(most, is64) == 16 and eng.cluster_choice(256, is64) == 2 and eng.cluster_choice(257, is64) == 4
+
+
+# 224 threads take the totals two at a time while one warp rehearses, 256 one at a time where none does (five groups)
+@gpu
+@pytest.mark.parametrize("groups,ll", [(1, 27), (1, 28), (1, 29), (1, 32), (1, 56), (1, 57), (4, 14), (1, 112), (1, 113), (1, 200), (5, 8), (5, 13)])
+@pytest.mark.parametrize("r2o", [topology.ring(8), topology.circulant(8, (1, 2, 5))])
+def test_the_grid_wide_step_at_the_edges_of_its_rounds_of_experts(r2o, groups, ll):
+    planner = _planner(r2o, groups, ll, warm_start=False)
+    eng = planner._engine
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for n in (500, 20000):
+        idx = _indices(planner, n, torch.int64, seed=n + ll)
+        out = eng.run_fused(idx, avail, 16, False, None, 0)
+        counts, by_cta = planner.count_workload(idx, 8)
+        shares = eng.last_probs().clone()
+        glob = eng.workspace()[8 + 2 * counts.numel() : 8 + 3 * counts.numel()]
+        assert torch.equal(glob, counts)
+        assert torch.equal(shares, planner.solve_probs(counts, avail)[0])
+        assert torch.equal(_counts(planner, out), _counts(planner, eng.map_idx(idx, shares, by_cta, 8)))
+    assert planner.check_status().ok
