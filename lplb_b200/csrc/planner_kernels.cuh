@@ -528,13 +528,21 @@ __global__ void __launch_bounds__(kBlock) solve_kernel(const int* __restrict__ w
 __host__ __device__ inline size_t bundle_bytes_aligned(int n_ranks, int d) {
   return ((sizeof(int) * (size_t)n_ranks * (d + 1)) + 15 + 16) & ~(size_t)15;
 }
-// (Reached by adding to `bundle`, not through an integer: the compiler then still knows that it is shared memory, and
-// does not access the solvers' matrices and vectors as if they could be anywhere: a call with 64 ranks 49.3 -> 44.4 us, 64 groups
-// of 8 ranks 12.4 -> 12.0, three iterations with 32 ranks 10.6 -> 10.1.)
+// With KNOWN it is reached by adding to `bundle`, not through an integer: the compiler then still knows that it is shared memory,
+// and does not access the solvers' matrices and vectors as if they could be anywhere: a call with 64 ranks 49.3 -> 44.4 us, 64
+// groups of 8 ranks 12.4 -> 12.0, three iterations with 32 ranks 10.6 -> 10.1.  Not so for some shapes of two warps, whose code it
+// makes slower to fetch (in the caches they are equal, 7.65 / 7.68): generic / known, us, the grid-wide step's solve with three
+// replicas 8.8 / 9.1, with four 8.75 / 9.0, a call with four 11.0 / 11.3; but (with what else came at the time) the step's solve
+// with one or two 8.2 / 8.0 and 9.0 / 8.7, a call with three 11.4 / 10.7.
+template <bool KNOWN = true>
 __device__ __forceinline__ double* scratch_after(int* bundle, int n_ranks, int d) {
   int* end = bundle + (size_t)n_ranks * (d + 1);
-  const unsigned past = (unsigned)__cvta_generic_to_shared(end) & 15u;
-  return reinterpret_cast<double*>(end + ((16u - past) & 15u) / sizeof(int));
+  if constexpr (KNOWN) {
+    const unsigned past = (unsigned)__cvta_generic_to_shared(end) & 15u;
+    return reinterpret_cast<double*>(end + ((16u - past) & 15u) / sizeof(int));
+  } else {
+    return reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(end) + 15) & ~(uintptr_t)15);
+  }
 }
 
 // Stand-alone solve kernel, tile solver: `teams` groups per CTA (several warps per group: one), and a last
@@ -557,7 +565,7 @@ __global__ void __launch_bounds__(kBlock) tile_solve_kernel(const int* __restric
   if (warp < teams * NB) {
     const TileLane mine = load_tile_lane<NB, D>(tp, team_warp, status);
     solve_groups_tiles<NB, D, false>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, team_warp, prm, mine, probs, nullptr, avail, status,
-                              scratch_after(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total, [] {});
+                              scratch_after<!(NB == 2 && D == 4)>(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total, [] {});
   }
 }
 
@@ -875,7 +883,7 @@ __device__ __forceinline__ void solve_step_tiles(int* bundle, const int* made_up
                                                  const TileLane& mine, float* __restrict__ probs, float* share, Counter avail,
                                                  int* status, Shared shared) {
   const int warp = threadIdx.x >> 5;
-  double* scratch = scratch_after(bundle, tp.n_group * tp.g, tp.d);
+  double* scratch = scratch_after<EARLY || !(GP == -2 && D >= 3)>(bundle, tp.n_group * tp.g, tp.d);
   if constexpr (GP == -1) {
     Topo t = tp;
     if (rehearses) {
