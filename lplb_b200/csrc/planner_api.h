@@ -94,7 +94,7 @@ cudaError_t launch_fused(const void* idx, int idx_is64, long long n, const TopoD
                          int cooperative, cudaStream_t stream);
 
 // The same step in one thread-block cluster of n_cta CTAs (2 to 16; CTA 0 exchanges and solves): up to 1024 experts, groups of
-// up to 32 ranks, and at most cluster_max_slice() indices per worker (cudaErrorInvalidValue otherwise).
+// up to 32 ranks, at least one replica, and at most cluster_max_slice() indices per worker (cudaErrorInvalidValue otherwise).
 cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const TopoDesc& topo, const ExchangeDesc& ex,
                            SolveParams prm, void* workspace, float* probs, void* avail, int avail_is64, int* status,
                            void* out, int n_cta, unsigned long long timeout_ns, unsigned long long* trace, cudaStream_t stream);

@@ -245,7 +245,7 @@ cudaError_t launch_cluster(const void* idx, int idx_is64, long long n, const Top
                            void* out, int n_cta, unsigned long long timeout_ns, unsigned long long* trace, cudaStream_t stream) {
   if (!shape_ok(topo, true, prm.solver) || n_cta < 2 || n_cta > kClusterMaxCtas || exd.n_ranks > kMaxRanks) return cudaErrorInvalidValue;
   const Topo tp = make_topo(topo);
-  if (tp.e > kClusterMaxExperts) return cudaErrorInvalidValue;
+  if (tp.e > kClusterMaxExperts || cluster_replicated(tp) < 1) return cudaErrorInvalidValue;
   const Exchange ex{exd.recv, exd.n_ranks, exd.my_rank, exd.node_size, exd.timeout_ns};
   return (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(idx, n, tp, ex, make_params(prm, topo), prm.solver, workspace, probs, Counter{avail, avail_is64},
                                                                      status, out, n_cta, timeout_ns, trace, stream, nullptr);
@@ -260,7 +260,7 @@ int cluster_ctas(long long n, bool host_result) {
 
 long long cluster_limit(const TopoDesc& topo, int solver, int idx_is64, int n_cta) {
   const Topo tp = make_topo(topo);
-  if (!shape_ok(topo, true, solver) || tp.e > kClusterMaxExperts) return 0;
+  if (!shape_ok(topo, true, solver) || tp.e > kClusterMaxExperts || cluster_replicated(tp) < 1) return 0;
   const long long n = (long long)(n_cta - 1) * cluster_paying_slice(-tile_rows(tp.g), tp.e, cluster_replicated(tp));
   int fits = 0;
   const cudaError_t err = (idx_is64 ? cluster_step<int64_t> : cluster_step<int32_t>)(

@@ -387,3 +387,20 @@ def test_the_grid_wide_step_at_the_edges_of_its_rounds_of_experts(r2o, groups, l
         assert torch.equal(shares, planner.solve_probs(counts, avail)[0])
         assert torch.equal(_counts(planner, out), _counts(planner, eng.map_idx(idx, shares, by_cta, 8)))
     assert planner.check_status().ok
+
+
+@gpu
+def test_an_engine_without_replicas_takes_the_grid_wide_kernel():
+    """The planner refuses such a placement, the engine does not; a cluster's messages are one per replicated expert."""
+    from lplb_b200 import _native
+
+    eng = _native.load().PlannerEngine(1, 8, 2, 4, 0, 0)
+    eng.set_topology(topology.cube(), topology.invert_r2o(topology.cube()))
+    ids = torch.arange(32, device="cuda")
+    eng.set_mapping(ids, torch.stack([ids, torch.full_like(ids, -1)], 1).contiguous(), torch.full_like(ids, -1))
+    avail = torch.zeros(1, dtype=torch.int32, device="cuda")
+    idx = torch.arange(-1, 1000, device="cuda") % 33 - 1
+    with pytest.raises(RuntimeError):
+        eng.run_fused(idx, avail, 16, False, None, 2)
+    assert eng.cluster_choice(idx.numel()) == 0
+    assert torch.equal(eng.run_fused(idx, avail, 16, False, None, -1), idx)
