@@ -531,9 +531,10 @@ __host__ __device__ inline size_t bundle_bytes_aligned(int n_ranks, int d) {
 // With KNOWN it is reached by adding to `bundle`, not through an integer: the compiler then still knows that it is shared memory,
 // and does not access the solvers' matrices and vectors as if they could be anywhere: a call with 64 ranks 49.3 -> 44.4 us, 64
 // groups of 8 ranks 12.4 -> 12.0, three iterations with 32 ranks 10.6 -> 10.1.  Not so for some shapes of two warps, whose code it
-// makes slower to fetch (in the caches they are equal, 7.65 / 7.68): generic / known, us, the grid-wide step's solve with three
-// replicas 8.8 / 9.1, with four 8.75 / 9.0, a call with four 11.0 / 11.3; but (with what else came at the time) the step's solve
-// with one or two 8.2 / 8.0 and 9.0 / 8.7, a call with three 11.4 / 10.7.
+// makes slower: generic / known, us, the grid-wide step's solve with three replicas 8.8 / 9.1, with four 8.75 / 9.0 (its code comes
+// cold; in the caches they are equal, 7.65 / 7.68), a call of the solve kernel, 16 ranks, with two 16.30 / 16.45, with four 11.0 /
+// 11.3; but one replica 14.05 / 13.15, three 18.42 / 17.28, and (with what else came at the time) the step's solve with one or two
+// 8.2 / 8.0 and 9.0 / 8.7.
 template <bool KNOWN = true>
 __device__ __forceinline__ double* scratch_after(int* bundle, int n_ranks, int d) {
   int* end = bundle + (size_t)n_ranks * (d + 1);
@@ -565,7 +566,7 @@ __global__ void __launch_bounds__(kBlock) tile_solve_kernel(const int* __restric
   if (warp < teams * NB) {
     const TileLane mine = load_tile_lane<NB, D>(tp, team_warp, status);
     solve_groups_tiles<NB, D, false>(bundle, tp, first + (NB == 1 ? warp : 0), tp.n_group, team_warp, prm, mine, probs, nullptr, avail, status,
-                              scratch_after<!(NB == 2 && D == 4)>(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total, [] {});
+                              scratch_after<!(NB == 2 && D % 2 == 0)>(bundle, tp.n_group * tp.g, tp.d) + (NB == 1 ? warp : 0) * tile_layout(NB, D).total, [] {});
   }
 }
 
