@@ -27,8 +27,8 @@
 //   * A product with an inverse is not as good as a substitution, so the step is refined once (kDamping).
 //
 // Solve kernel, two replicas per rank, unrelated instances, us a call back to back (the warp solver
-// for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 11.2, 64 groups of 8 ranks
-// 26.2 -> 12.0, 16 ranks 40.6 -> 18.0, 32 ranks 64.4 -> 25.9, 64 ranks 147 -> 46.  An iteration: 8 ranks 3.5 -> 1.4,
+// for 8 ranks, the thread-block solver above -> this one): 8 ranks 22.6 -> 10.4, 64 groups of 8 ranks
+// 26.2 -> 12.3, 16 ranks 40.6 -> 17.9, 32 ranks 64.4 -> 24.8, 64 ranks 147 -> 46.  An iteration: 8 ranks 3.5 -> 1.4,
 // 64 ranks 22.5 -> 6.6 us.
 #pragma once
 

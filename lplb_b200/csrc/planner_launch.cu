@@ -36,7 +36,7 @@ bool shape_ok(const TopoDesc& t, bool need_solver = true, int solver = kSolverAu
 // Calls fn.template operator()<GP, D>() for the instantiation that covers the topology: GP = -1, -2, -4,
 // -8 for the tile solver with that many warps per group, 8, 16, 32 for the warp solver, 0 for the
 // thread-block solver (D is then the padded count).  The tile solver takes every group that it
-// covers (8 ranks 22.6 -> 11.2 us a call, 16 ranks 40.6 -> 18.0, 32 ranks 64 -> 26, 64 ranks 147 -> 52 against the
+// covers (8 ranks 22.6 -> 10.4 us a call, 16 ranks 40.6 -> 17.9, 32 ranks 64 -> 25, 64 ranks 147 -> 46 against the
 // other two), except that the warp solver packs four groups of 8 ranks into a warp: `packed` asks for
 // that where one CTA has many of them.  The warp solver's larger groups run on request only.
 template <typename Fn>
